@@ -113,21 +113,34 @@ SwWorkspace* workspace(char* errmsg, int32_t errmsg_len, int* rc) {
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// per-column scratch bytes of the three kernels
+
+// per-column scratch bytes of the kernels
 size_t scratch_per_col(int nlay) {
   const int nw = (nlay + 31) / 32;
-  return (size_t)(2 * nlay * sw::kSwNg + sw::kSwNg + 3 * nlay * 14 + 2 * nlay + 2 + (nlay + 1) * 10 * 32) * 8 + 4 +
-         (size_t)sw::kSwNg * nw * 4 + 64;
+  return (sw::tg_doubles(nlay) + sw::rt_col_store(nlay) + (size_t)9 * nlay + sw::kSwNg + 3 * nlay * 14 + 2 * nlay + 2) * 8 +
+         4 + (size_t)sw::kSwNg * nw * 4 + 64;
 }
 
-// carve one chunk's scratch out of the workspace
-sw::SwScratch carve(char* base, int nc, int nlay) {
+// Columns of a chunk of a call of n: equal chunks that fit the scratch budget,
+// in whole waves of the upward kernel.
+int chunk_columns(int n, int nlay) {
+  const int most = (int)std::max<size_t>(1, kScratchBudget / scratch_per_col(nlay));
+  if (n <= most) return std::max(n, 1);
+  const int wave = sw::kRtPerSm * g.num_sms, chunks = (n + most - 1) / most, even = (n + chunks - 1) / chunks;
+  const int whole = (even + wave - 1) / wave * wave;
+  return whole <= most ? whole : std::max(most / wave * wave, std::min(most, wave));
+}
+
+// carve one chunk's scratch out of the workspace (base null: only its size;
+// transfer false: the gas optics alone)
+size_t carve(char* base, int nc, int nlay, bool transfer, sw::SwScratch* out) {
   sw::SwScratch s{};
   const int nw = (nlay + 31) / 32;
   size_t off = 0;
-  auto take = [&](size_t bytes) { char* p = base + off; off += align256(bytes); return p; };
-  s.taug = (double*)take((size_t)nc * nlay * sw::kSwNg * 8);
-  s.taur = (double*)take((size_t)nc * nlay * sw::kSwNg * 8);
+  auto take = [&](size_t bytes) { char* p = base ? base + off : nullptr; off += align256(bytes); return p; };
+  s.taug = (double*)take((size_t)nc * sw::tg_doubles(nlay) * 8);
+  s.colmol = (double*)take((size_t)nc * nlay * 8);
+  s.ray24 = (double*)take((size_t)nc * nlay * 8 * 8);
   s.sflux = (double*)take((size_t)nc * sw::kSwNg * 8);
   s.taucw = (double*)take((size_t)nc * nlay * 14 * 8);
   s.ssacw = (double*)take((size_t)nc * nlay * 14 * 8);
@@ -138,20 +151,17 @@ sw::SwScratch carve(char* base, int nc, int nlay) {
   s.zcf0 = (double*)take((size_t)nc * 8);
   s.seed = (int32_t*)take((size_t)nc * 4);
   s.bits = (uint32_t*)take((size_t)nc * sw::kSwNg * nw * 4);
-  s.lane_store = (double*)take((size_t)nc * (nlay + 1) * 10 * 32 * 8);
+  s.rt_store = transfer ? (double*)take((size_t)nc * sw::rt_col_store(nlay) * 8) : nullptr;
+  s.num_sms = g.num_sms;
   s.nw = nw;
-  return s;
+  if (out) *out = s;
+  return off;
 }
-size_t carve_bytes(int nc, int nlay) {
-  const int nw = (nlay + 31) / 32;
-  const size_t parts[13] = {(size_t)nc * 8, (size_t)nc * nlay * 8, (size_t)nc * (nlay + 1) * 10 * 32 * 8, (size_t)nc * nlay * sw::kSwNg * 8, (size_t)nc * nlay * sw::kSwNg * 8,
-                            (size_t)nc * sw::kSwNg * 8,        (size_t)nc * nlay * 14 * 8,
-                            (size_t)nc * nlay * 14 * 8,        (size_t)nc * nlay * 14 * 8,
-                            (size_t)nc * nlay * 8,             (size_t)nc * 8,
-                            (size_t)nc * 4,                    (size_t)nc * sw::kSwNg * nw * 4};
-  size_t t = 0;
-  for (size_t p : parts) t += align256(p);
-  return t;
+size_t carve_bytes(int nc, int nlay, bool transfer = true) { return carve(nullptr, nc, nlay, transfer, nullptr); }
+sw::SwScratch carve(char* base, int nc, int nlay, bool transfer = true) {
+  sw::SwScratch s;
+  carve(base, nc, nlay, transfer, &s);
+  return s;
 }
 
 // Sizes (in elements) of the caller's arrays.
@@ -262,8 +272,7 @@ cudaError_t zero_outputs(const sw::SwArgs& d, const Sizes& z, int nlay, cudaStre
 int run_device(SwWorkspace* w, const sw::SwArgs& d, int nday, cudaStream_t st, float* kernel_ms, char* errmsg,
                int32_t errmsg_len, const Sizes& z) {
   CK(zero_outputs(d, z, d.nlay, st), "zeroing the outputs");
-  const size_t per = scratch_per_col(d.nlay);
-  int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)nday, kScratchBudget / per));
+  const int chunk = chunk_columns(nday, d.nlay);
   CK(grow(&w->scratch, &w->scratch_bytes, carve_bytes(chunk, d.nlay)), "scratch allocation");
   cudaEvent_t ev[4] = {};
   if (kernel_ms) {
@@ -290,7 +299,7 @@ int run_device(SwWorkspace* w, const sw::SwArgs& d, int nday, cudaStream_t st, f
       CK(lw::mcica_sw_two_set_launch(nc, d.nlay, d.iovr, ms, s.bits, g.num_sms, st), "McICA kernel launch");
     }
     if (first) CK(cudaEventRecord(ev[2], st), "cudaEventRecord");
-    CK(sw::rt_launch(d, s, p0, nc, g.etab, st), "transfer kernel launch");
+    CK(sw::rt_launch(d, s, p0, nc, g.tab, g.etab, st), "transfer kernel launch");
     if (first) CK(cudaEventRecord(ev[3], st), "cudaEventRecord");
   }
   if (kernel_ms) {
@@ -383,8 +392,7 @@ int run_host_pipelined(SwWorkspace* w, const rrtmg_sw_run_args* a, cudaStream_t 
   }
   CK(grow(&w->pbuf, &w->pbuf_bytes, 2 * per), "staging allocation");
   // the kernels' scratch for a whole chunk, allocated before any launch
-  const size_t chunk_cols = std::min<size_t>(kSwHostChunk, kScratchBudget / scratch_per_col(nlay));
-  CK(grow(&w->scratch, &w->scratch_bytes, carve_bytes((int)chunk_cols, nlay)), "scratch allocation");
+  CK(grow(&w->scratch, &w->scratch_bytes, carve_bytes(chunk_columns(kSwHostChunk, nlay), nlay)), "scratch allocation");
   CK(cudaMemsetAsync(w->bad, 0, sizeof(int), st), "cudaMemsetAsync");
   for (int j = 0; j < nch; ++j) {
     const int b = j & 1, c0 = j * kSwHostChunk, n = std::min(kSwHostChunk, npts - c0);
@@ -606,15 +614,13 @@ extern "C" int rrtmg_sw_gpu_gas_optics(const rrtmg_sw_run_args* a, double* taug,
   sw::SwArgs d = device_args(a);
   d.cldtau = nullptr;
   const int nday = a->nday, nlay = a->nlay;
-  CK(grow(&w->scratch, &w->scratch_bytes, carve_bytes(nday, nlay)), "scratch allocation");
-  sw::SwScratch s = carve(w->scratch, nday, nlay);
+  CK(grow(&w->scratch, &w->scratch_bytes, carve_bytes(nday, nlay, false)), "scratch allocation");
+  sw::SwScratch s = carve(w->scratch, nday, nlay, false);
   s.bad = w->bad;
   d.gas_only = 1;
   CK(cudaMemsetAsync(w->bad, 0, sizeof(int), st), "cudaMemsetAsync");
   CK(sw::optics_launch(d, s, 0, nday, g.tab, st), "optics kernel launch");
-  const size_t n = (size_t)nday * nlay * sw::kSwNg;
-  CK(cudaMemcpyAsync(taug, s.taug, n * 8, cudaMemcpyDeviceToDevice, st), "cudaMemcpyAsync");
-  CK(cudaMemcpyAsync(taur, s.taur, n * 8, cudaMemcpyDeviceToDevice, st), "cudaMemcpyAsync");
+  CK(sw::gas_unpack_launch(s, nday, nlay, g.tab, taug, taur, st), "unpacking kernel launch");
   CK(cudaMemcpyAsync(sfluxzen, s.sflux, (size_t)nday * sw::kSwNg * 8, cudaMemcpyDeviceToDevice, st), "cudaMemcpyAsync");
   return check_bad(w, st, errmsg, errmsg_len);
 }
@@ -681,8 +687,7 @@ extern "C" int rrtmg_sw_gpu_run_blocks(const rrtmg_sw_run_args* blocks, int32_t 
   CK(sw::blocks_prepare(d_tab, d_pre, d_pre + nb, nb, total_cols, d_pts, w->bad, st), "block table kernels");
   // the kernels over all daytime points, in scratch-sized chunks
   const sw::SwArgs& f = w->h_tab[0];
-  const size_t per = scratch_per_col(nlay);
-  const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)std::max(ndays, 1), kScratchBudget / per));
+  const int chunk = chunk_columns(ndays, nlay);
   CK(grow(&w->scratch, &w->scratch_bytes, carve_bytes(chunk, nlay)), "scratch allocation");
   cudaEvent_t ev[4] = {};
   float* kms = x->kernel_ms;
@@ -706,7 +711,7 @@ extern "C" int rrtmg_sw_gpu_run_blocks(const rrtmg_sw_run_args* blocks, int32_t 
     else if (f.isubcsw > 0)
       CK(lw::mcica_sw_two_set_launch(nc, nlay, f.iovr, ms, sc.bits, g.num_sms, st), "McICA kernel launch");
     if (first_chunk) CK(cudaEventRecord(ev[2], st), "cudaEventRecord");
-    CK(sw::rt_blocks_launch(d_tab, d_pts, f.isubcsw <= 0, f.hswb != nullptr, sc, p0, nc, nlay, g.etab, st),
+    CK(sw::rt_blocks_launch(d_tab, d_pts, f.isubcsw <= 0, f.hswb != nullptr, sc, p0, nc, nlay, g.tab, g.etab, st),
        "transfer kernel launch");
     if (first_chunk) CK(cudaEventRecord(ev[3], st), "cudaEventRecord");
   }

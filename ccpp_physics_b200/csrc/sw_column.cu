@@ -10,19 +10,14 @@
 //                     the solar source sfluxzen, the clear/cloudy column test
 //                     (RSM:1101-1125) and cldprop (RSM:1566-1938);
 //   lw_mcica_kernel<112>  the sub-column generator (lw_mcica.cu);
-//   sw_rt_kernel      one warp per column, lanes over g-points: spcvrtm
+//   sw_rt_kernel      two columns per CTA, one g-point per thread: spcvrtm
 //                     (RSM:3228-3942) with vrtqdr (RSM:3959-4051) and the
 //                     flux / heating-rate outputs (RSM:1225-1373).
-// Per lane (g-point) the clear-sky and all-sky sweeps run side by side: the
-// upward sweep evaluates each layer's clear two-stream optics once (the
-// all-sky sweep re-evaluates only the layers whose McICA flag is set) and
-// keeps them, with both adding recurrences (zrupb, zrupd), in global
-// scratch; the downward sweep reads them back and produces both sweeps'
-// fluxes level by level.  Fluxes are summed over g-points with warp
-// butterflies in a fixed order.
 //
-// Built with -fmad=false: every statement keeps the reference's evaluation
-// order and rounding.
+// Built with -fmad=false: every statement that feeds a table index or a
+// difference of nearly equal numbers keeps the reference's evaluation order
+// and rounding; the recurrences behind them use fma() where that is exact
+// enough (see sw_rt_kernel).
 #include <cstdint>
 #include <cstdio>
 #include <cuda_runtime.h>
@@ -166,27 +161,10 @@ __device__ __forceinline__ double forc(const Tab& f, const Lay& L, int j) {
 }
 
 __device__ void taumol_layer(const Lay& L, bool lower, const int id0[14], const int id1[14],
-                             const double* __restrict__ T, double* __restrict__ tg, double* __restrict__ tr) {
+                             const double* __restrict__ T, double* __restrict__ tg, double* __restrict__ t24) {
   int js;
   double fs, f[8];
   const double* strr = T + swtab::strrat;
-  // Rayleigh: one coefficient for bands 16-22, 28, 29
-  const double rs[14] = {T[swtab::b16_rayl], T[swtab::b17_rayl], T[swtab::b18_rayl], T[swtab::b19_rayl],
-                         T[swtab::b20_rayl], T[swtab::b21_rayl], T[swtab::b22_rayl], 0.0, 0.0, 0.0, 0.0, 0.0,
-                         T[swtab::b28_rayl], T[swtab::b29_rayl]};
-#pragma unroll 1
-  for (int b = 0; b < 14; ++b) {
-    if (b == 7 || b == 8 || b == 9 || b == 10 || b == 11) continue;
-    const double tauray = L.colmol * rs[b];
-    for (int j = 0; j < c_ng[b]; ++j) tr[c_ns[b] + j] = tauray;
-  }
-  {  // per-g Rayleigh of bands 23, 25, 26, 27
-    const int bands[4] = {7, 9, 10, 11};
-    const int offs[4] = {swtab::b23_rayl, swtab::b25_rayl, swtab::b26_rayl, swtab::b27_rayl};
-#pragma unroll 1
-    for (int q = 0; q < 4; ++q)
-      for (int j = 0; j < c_ng[bands[q]]; ++j) tr[c_ns[bands[q]] + j] = L.colmol * __ldg(T + offs[q] + j);
-  }
   const double o2tem = 4.35e-4 / (350.0 * 2.0), o2adj = 1.6;
   // bands 16, 17, 18, 19, 21, 22: binary species in the lower atmosphere
   {
@@ -213,22 +191,22 @@ __device__ void taumol_layer(const Lay& L, bool lower, const int id0[14], const 
         for (int j = 1; j <= ng; ++j) {
           double t = speccomb * k8(absa, f, i01, 9, i11, j) + L.colamt[0] * (selfc(selfref, L, j) + forc(forref, L, j));
           if (b == 6) t = t + o2cont;
-          tg[ns + j - 1] = t;
+          tg[kTgStride * (ns + j - 1)] = t;
         }
       } else if (b == 1 || b == 5) {   // 17, 21: binary species above too
         const double speccomb = spec8(L, 0, 1, strr[b], 4.0, js, fs, f);
         const int i01 = id0[b] + js, i11 = id1[b] + js;
         for (int j = 1; j <= ng; ++j) {
           const int a0 = L.indfor, a1 = a0 + 1;
-          tg[ns + j - 1] = speccomb * k8(absb, f, i01, 5, i11, j) +
+          tg[kTgStride * (ns + j - 1)] = speccomb * k8(absb, f, i01, 5, i11, j) +
                            L.colamt[0] * L.forfac * (forref(a0, j) + L.forfrac * (forref(a1, j) - forref(a0, j)));
         }
       } else {
         const int i01 = id0[b] + 1, i11 = id1[b] + 1;
         const double o2cont = o2tem * L.colamt[5];
         for (int j = 1; j <= ng; ++j) {
-          if (b == 6) tg[ns + j - 1] = L.colamt[5] * o2adj * k4(absb, L, i01, i11, j) + o2cont;
-          else tg[ns + j - 1] = L.colamt[b == 3 ? 1 : 4] * k4(absb, L, i01, i11, j);
+          if (b == 6) tg[kTgStride * (ns + j - 1)] = L.colamt[5] * o2adj * k4(absb, L, i01, i11, j) + o2cont;
+          else tg[kTgStride * (ns + j - 1)] = L.colamt[b == 3 ? 1 : 4] * k4(absb, L, i01, i11, j);
         }
       }
     }
@@ -241,10 +219,10 @@ __device__ void taumol_layer(const Lay& L, bool lower, const int id0[14], const 
     const int i01 = id0[b] + 1, i11 = id1[b] + 1;
     for (int j = 1; j <= 10; ++j) {
       if (lower)
-        tg[ns + j - 1] = L.colamt[0] * (k4(absa, L, i01, i11, j) + selfc(selfref, L, j) + forc(forref, L, j)) +
+        tg[kTgStride * (ns + j - 1)] = L.colamt[0] * (k4(absa, L, i01, i11, j) + selfc(selfref, L, j) + forc(forref, L, j)) +
                          L.colamt[4] * __ldg(absch4 + j - 1);
       else
-        tg[ns + j - 1] = L.colamt[0] * (k4(absb, L, i01, i11, j) + forc(forref, L, j)) + L.colamt[4] * __ldg(absch4 + j - 1);
+        tg[kTgStride * (ns + j - 1)] = L.colamt[0] * (k4(absb, L, i01, i11, j) + forc(forref, L, j)) + L.colamt[4] * __ldg(absch4 + j - 1);
     }
   }
   {  // band 23: H2O below, nothing above
@@ -253,7 +231,7 @@ __device__ void taumol_layer(const Lay& L, bool lower, const int id0[14], const 
     const double givfac = T[swtab::b23_givfac];
     const int i01 = id0[b] + 1, i11 = id1[b] + 1;
     for (int j = 1; j <= 10; ++j)
-      tg[ns + j - 1] = lower ? L.colamt[0] * (givfac * k4(absa, L, i01, i11, j) + selfc(selfref, L, j) + forc(forref, L, j))
+      tg[kTgStride * (ns + j - 1)] = lower ? L.colamt[0] * (givfac * k4(absa, L, i01, i11, j) + selfc(selfref, L, j) + forc(forref, L, j))
                              : 0.0;
   }
   {  // band 24: H2O/O2 below, O2 above; O3 both; Rayleigh from the species bin
@@ -266,16 +244,16 @@ __device__ void taumol_layer(const Lay& L, bool lower, const int id0[14], const 
       const double speccomb = spec8(L, 0, 5, strr[b], 8.0, js, fs, f);
       const int i01 = id0[b] + js, i11 = id1[b] + js;
       for (int j = 1; j <= 8; ++j) {
-        tg[ns + j - 1] = speccomb * k8(absa, f, i01, 9, i11, j) + L.colamt[2] * __ldg(abso3a + j - 1) +
+        tg[kTgStride * (ns + j - 1)] = speccomb * k8(absa, f, i01, 9, i11, j) + L.colamt[2] * __ldg(abso3a + j - 1) +
                          L.colamt[0] * (selfc(selfref, L, j) + forc(forref, L, j));
         const double ra = __ldg(rayla + (j - 1) + 8 * (js - 1)), rb = __ldg(rayla + (j - 1) + 8 * js);
-        tr[ns + j - 1] = L.colmol * (ra + fs * (rb - ra));
+        t24[j - 1] = L.colmol * (ra + fs * (rb - ra));
       }
     } else {
       const int i01 = id0[b] + 1, i11 = id1[b] + 1;
       for (int j = 1; j <= 8; ++j) {
-        tg[ns + j - 1] = L.colamt[5] * k4(absb, L, i01, i11, j) + L.colamt[2] * __ldg(abso3b + j - 1);
-        tr[ns + j - 1] = L.colmol * __ldg(raylb + j - 1);
+        tg[kTgStride * (ns + j - 1)] = L.colamt[5] * k4(absb, L, i01, i11, j) + L.colamt[2] * __ldg(abso3b + j - 1);
+        t24[j - 1] = L.colmol * __ldg(raylb + j - 1);
       }
     }
   }
@@ -285,16 +263,16 @@ __device__ void taumol_layer(const Lay& L, bool lower, const int id0[14], const 
     const double *abso3a = T + swtab::b25_abso3a, *abso3b = T + swtab::b25_abso3b;
     const int i01 = id0[b] + 1, i11 = id1[b] + 1;
     for (int j = 1; j <= 6; ++j)
-      tg[ns + j - 1] = lower ? L.colamt[0] * k4(absa, L, i01, i11, j) + L.colamt[2] * __ldg(abso3a + j - 1)
+      tg[kTgStride * (ns + j - 1)] = lower ? L.colamt[0] * k4(absa, L, i01, i11, j) + L.colamt[2] * __ldg(abso3a + j - 1)
                              : L.colamt[2] * __ldg(abso3b + j - 1);
   }
-  for (int j = 0; j < 6; ++j) tg[c_ns[10] + j] = 0.0;   // band 26: Rayleigh only
+  for (int j = 0; j < 6; ++j) tg[kTgStride * (c_ns[10] + j)] = 0.0;   // band 26: Rayleigh only
   {  // band 27: O3
     const int b = 11, ns = c_ns[b];
     const Tab absa{T + swtab::b27_absa, 65}, absb{T + swtab::b27_absb, 235};
     const int i01 = id0[b] + 1, i11 = id1[b] + 1;
     for (int j = 1; j <= 8; ++j)
-      tg[ns + j - 1] = L.colamt[2] * (lower ? k4(absa, L, i01, i11, j) : k4(absb, L, i01, i11, j));
+      tg[kTgStride * (ns + j - 1)] = L.colamt[2] * (lower ? k4(absa, L, i01, i11, j) : k4(absb, L, i01, i11, j));
   }
   {  // band 28: O3/O2 both
     const int b = 12, ns = c_ns[b];
@@ -302,7 +280,7 @@ __device__ void taumol_layer(const Lay& L, bool lower, const int id0[14], const 
     const double speccomb = spec8(L, 2, 5, strr[b], lower ? 8.0 : 4.0, js, fs, f);
     const int i01 = id0[b] + js, i11 = id1[b] + js;
     for (int j = 1; j <= 6; ++j)
-      tg[ns + j - 1] = speccomb * (lower ? k8(absa, f, i01, 9, i11, j) : k8(absb, f, i01, 5, i11, j));
+      tg[kTgStride * (ns + j - 1)] = speccomb * (lower ? k8(absa, f, i01, 9, i11, j) : k8(absb, f, i01, 5, i11, j));
   }
   {  // band 29: H2O + CO2 below, CO2 + H2O above
     const int b = 13, ns = c_ns[b];
@@ -312,10 +290,10 @@ __device__ void taumol_layer(const Lay& L, bool lower, const int id0[14], const 
     const int i01 = id0[b] + 1, i11 = id1[b] + 1;
     for (int j = 1; j <= 12; ++j) {
       if (lower)
-        tg[ns + j - 1] = L.colamt[0] * (k4(absa, L, i01, i11, j) + selfc(selfref, L, j) + forc(forref, L, j)) +
+        tg[kTgStride * (ns + j - 1)] = L.colamt[0] * (k4(absa, L, i01, i11, j) + selfc(selfref, L, j) + forc(forref, L, j)) +
                          L.colamt[1] * __ldg(absco2 + j - 1);
       else
-        tg[ns + j - 1] = L.colamt[1] * k4(absb, L, i01, i11, j) + L.colamt[0] * __ldg(absh2o + j - 1);
+        tg[kTgStride * (ns + j - 1)] = L.colamt[1] * k4(absb, L, i01, i11, j) + L.colamt[0] * __ldg(absh2o + j - 1);
     }
   }
 }
@@ -416,6 +394,51 @@ __device__ void cloud_layer(const SwArgs& a, size_t x, const double* __restrict_
   }
 }
 
+// ---- Rayleigh optical depth of g-point g (RSM:4094-5573) --------------------
+// colmol * coefficient, except band 24, whose coefficient depends on the
+// layer's species bin: the optics kernel writes those eight values per layer.
+// p[stride * k] * coef is taur of layer k in either case.
+struct RaySrc {
+  const double* p;
+  int stride;
+  double coef;
+};
+__device__ __forceinline__ RaySrc ray_src(const SwScratch& s, size_t pl, int nlay, int g, int b,
+                                          const double* __restrict__ T) {
+  if (b == 8) return {s.ray24 + pl * nlay * 8 + (g - c_ns[8]), 8, 1.0};
+  const int j = g - c_ns[b];
+  int off = 0;
+  switch (b) {
+    case 0: off = swtab::b16_rayl; break;
+    case 1: off = swtab::b17_rayl; break;
+    case 2: off = swtab::b18_rayl; break;
+    case 3: off = swtab::b19_rayl; break;
+    case 4: off = swtab::b20_rayl; break;
+    case 5: off = swtab::b21_rayl; break;
+    case 6: off = swtab::b22_rayl; break;
+    case 7: off = swtab::b23_rayl + j; break;
+    case 9: off = swtab::b25_rayl + j; break;
+    case 10: off = swtab::b26_rayl + j; break;
+    case 11: off = swtab::b27_rayl + j; break;
+    case 12: off = swtab::b28_rayl; break;
+    default: off = swtab::b29_rayl; break;
+  }
+  return {s.colmol + pl * nlay, 1, __ldg(T + off)};
+}
+
+// the stage entry point's outputs: taug and taur as [column][layer][112]
+__global__ void sw_gas_unpack_kernel(SwScratch s, int nc, int nlay, const double* __restrict__ T,
+                                     double* __restrict__ taug, double* __restrict__ taur) {
+  const long long n = (long long)nc * nlay * kSwNg;
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+    const int g = (int)(q % kSwNg), k = (int)(q / kSwNg % nlay);
+    const size_t pl = (size_t)(q / kSwNg / nlay);
+    const RaySrc r = ray_src(s, pl, nlay, g, band_of(g), T);
+    taug[q] = s.taug[tg_offset(nlay, pl, k, g)];
+    taur[q] = r.p[(size_t)r.stride * k] * r.coef;
+  }
+}
+
 // ---- kernel 1: optics ------------------------------------------------------
 constexpr int kOptWarps = 4;
 
@@ -457,9 +480,8 @@ __device__ __forceinline__ void optics_body(const SwArgs& a, const SwScratch& s,
         id1[b] = ((L.jp - 12) * 5 + (L.jt1 - 1)) * c_nspb[b];
       }
     }
-    double* tg = s.taug + ((size_t)pl * nlay + k) * kSwNg;
-    double* tr = s.taur + ((size_t)pl * nlay + k) * kSwNg;
-    taumol_layer(L, lower, id0, id1, T, tg, tr);
+    s.colmol[(size_t)pl * nlay + k] = L.colmol;
+    taumol_layer(L, lower, id0, id1, T, s.taug + tg_offset(nlay, pl, k, 0), s.ray24 + ((size_t)pl * nlay + k) * 8);
   }
 
   // solar source per band (RSM:4225-4310), one band per lane
@@ -585,25 +607,88 @@ struct LayOpt {
   double rb, rd, tb, td, e3, e4;
 };
 
-__device__ __forceinline__ double exp_tab(const double* __restrict__ ET, double z) {
-  // itind = ftind*NTBMX + 0.5 with truncation; ftind in [0, 1) so the
-  // clamped form of RSM:3601-3602 selects the same entry
-  const double ftind = z / (kBpade + z);
-  return __ldg(ET + (int)(ftind * kNtbmx + 0.5));
+// Quotients and roots from the hardware estimate (2^-20) and Newton's
+// iteration, for operands that are normal numbers far from the ends of the
+// range: no range check and no slow path, about two thirds of the instructions
+// of the compiled IEEE operations.  recip_newton is 1/x to about 2^-52;
+// div_markstein and sqrt_markstein add Markstein's residual step (IBM J. Res.
+// Dev. 34, 1990), which rounds correctly but for a reciprocal whose own last
+// bit was misrounded.
+__device__ __forceinline__ double recip_newton(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+__device__ __forceinline__ double div_markstein(double a, double b) {
+  const double y = recip_newton(b), q = a * y;
+  return fma(fma(-b, q, a), y, q);
+}
+__device__ __forceinline__ double sqrt_markstein(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(0.5 * y, fma(-x * y, y, 1.0), y);
+  y = fma(0.5 * y, fma(-x * y, y, 1.0), y);
+  const double r = x * y;
+  return fma(fma(-r, r, x), 0.5 * y, r);
+}
+// fmax / fmin with a constant: NaN gives the constant, as fmax and fmin do
+__device__ __forceinline__ double at_least(double c, double x) { return x > c ? x : c; }
+__device__ __forceinline__ double at_most(double c, double x) { return x < c ? x : c; }
+__device__ __forceinline__ double clamp01(double x) { return at_least(0.0, at_most(1.0, x)); }
+
+// exp_tbl in global or in shared memory
+struct TblGlobal {
+  const double* p;
+  __device__ __forceinline__ double operator()(int i) const { return __ldg(p + i); }
+};
+struct TblShared {
+  unsigned base;
+  __device__ __forceinline__ double operator()(int i) const {
+    double v;
+    asm("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(base + 8u * (unsigned)i));
+    return v;
+  }
+};
+
+// exp_tbl at index int(z / (bpade + z) * NTBMX + 0.5) (RSM:3601-3602; ftind in
+// [0, 1), so the clamped and the truncated form select the same entry).  The
+// quotient comes from one Newton step (error below 1e-8 in index units) and is
+// rounded by adding 1.5 2^52; only a value within 1e-6 of a tie takes the IEEE
+// division, so the entry is the reference's in every case.
+template <typename Tbl>
+__device__ __forceinline__ double exp_tab(const Tbl& ET, double z) {
+  constexpr double kRound = 6755399441055744.0;
+  const double d = kBpade + z;
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  y = fma(y, fma(-d, y, 1.0), y);
+  const double q = z * y, t = fma(q, (double)kNtbmx, kRound);
+  int i = __double2loint(t);
+  const double f = fma(q, (double)kNtbmx, kRound - t);
+  if (!(fabs(f) < 0.5 - 1.0e-6)) i = (int)(z / d * kNtbmx + 0.5);
+  return ET(i);
 }
 __device__ __forceinline__ double exp_small(double z) { return 1.0 - z + 0.5 * z * z; }
+template <typename Tbl>
+__device__ __forceinline__ double exp_of(const Tbl& ET, double z) {   // od_lo = 0.06
+  return (z <= 0.06) ? exp_small(z) : exp_tab(ET, z);
+}
 
-// the two-stream layer reflectance / transmittance of spcvrtm (RSM:3447-3600)
+// The two-stream layer reflectance / transmittance of spcvrtm (RSM:3447-3600).
+// Thin layers difference nearly equal numbers here, so everything up to the
+// two final quotients keeps the reference's operations and their order.
+template <typename Tbl>
 __device__ __forceinline__ void two_stream(double ztau0, double zssa0, double zasy0, double cosz, double sntz,
-                                           int iswmode, const double* __restrict__ ET, LayOpt& o) {
-  const double zcrit = 0.9999995, od_lo = 0.06, eps1 = 1.0e-8;
-  const double zssaw = fmin(kOneMinus, zssa0 / ztau0);
-  const double zasyw = zasy0 / fmax(kFtiny, zssa0);
+                                           int iswmode, const Tbl& ET, LayOpt& o) {
+  const double zcrit = 0.9999995, eps1 = 1.0e-8;
+  const double zssaw = at_most(kOneMinus, div_markstein(zssa0, ztau0));
+  const double zasyw = div_markstein(zasy0, at_least(kFtiny, zssa0));
   double za1 = zasyw * zasyw;
   double za2 = zssaw * za1;
   const double ztau1 = (1.0 - za2) * ztau0;
-  const double zssa1 = (zssaw - za2) / (1.0 - za2);
-  const double zasy1 = zasyw / (1.0 + zasyw);
+  const double zssa1 = div_markstein(zssaw - za2, 1.0 - za2);
+  const double zasy1 = div_markstein(zasyw, 1.0 + zasyw);
   const double zasy3 = 0.75 * zasy1;
   double zgam1, zgam2, zgam3;
   if (iswmode == 1) {
@@ -621,25 +706,29 @@ __device__ __forceinline__ void two_stream(double ztau0, double zssa0, double za
     zgam3 = (1.0 - zsr3 * zasy1 * cosz) * 0.5;
   }
   const double zgam4 = 1.0 - zgam3;
+  // direct-beam transmittance of the scaled optical depth; the layer optics
+  // use it capped at 500, the beam (e3) does not
+  const double zbeam = ztau1 * sntz;
+  const double zexm2 = exp_of(ET, at_most(500.0, zbeam));
+  o.e3 = (zbeam <= 500.0) ? zexm2 : exp_of(ET, zbeam);
+  o.e4 = exp_of(ET, ztau0 * sntz);
   if (zssaw >= zcrit) {
     za1 = zgam1 * cosz - zgam3;
     za2 = zgam1 * ztau1;
-    const double zb1 = fmin(ztau1 * sntz, 500.0);
-    const double zb2 = (zb1 <= od_lo) ? exp_small(zb1) : exp_tab(ET, zb1);
-    o.rb = fmax(0.0, fmin(1.0, (za2 - za1 * (1.0 - zb2)) / (1.0 + za2)));
-    o.tb = fmax(0.0, fmin(1.0, 1.0 - o.rb));
-    o.rd = fmax(0.0, fmin(1.0, za2 / (1.0 + za2)));
-    o.td = fmax(0.0, fmin(1.0, 1.0 - o.rd));
+    o.rb = clamp01((za2 - za1 * (1.0 - zexm2)) / (1.0 + za2));
+    o.tb = clamp01(1.0 - o.rb);
+    o.rd = clamp01(za2 / (1.0 + za2));
+    o.td = clamp01(1.0 - o.rd);
   } else {
     za1 = zgam1 * zgam4 + zgam2 * zgam3;
     za2 = zgam1 * zgam3 + zgam2 * zgam4;
     double zrk = (zgam1 - zgam2) * (zgam1 + zgam2);
-    zrk = (zrk > eps1) ? sqrt(zrk) : 0.0;
+    zrk = (zrk > eps1) ? sqrt_markstein(zrk) : 0.0;
     const double zrk2 = zrk + zrk;
     const double zrp = zrk * cosz;
     const double zrp1 = 1.0 + zrp, zrm1 = 1.0 - zrp;
     const double zrpp1 = 1.0 - zrp * zrp;
-    const double zrpp = copysign(fmax(kFlimit, fabs(zrpp1)), zrpp1);
+    const double zrpp = copysign(at_least(kFlimit, fabs(zrpp1)), zrpp1);
     const double zrkg1 = zrk + zgam1, zrkg3 = zrk * zgam3, zrkg4 = zrk * zgam4;
     const double zr1 = zrm1 * (za2 + zrkg3);
     const double zr2 = zrp1 * (za2 - zrkg3);
@@ -649,56 +738,45 @@ __device__ __forceinline__ void two_stream(double ztau0, double zssa0, double za
     const double zt1 = zrp1 * (za1 + zrkg4);
     const double zt2 = zrm1 * (za1 - zrkg4);
     const double zt3 = zrk2 * (zgam4 + za1 * cosz);
-    const double zb1 = fmin(zrk * ztau1, 500.0);
-    const double zexm1 = (zb1 <= od_lo) ? exp_small(zb1) : exp_tab(ET, zb1);
-    const double zexp1 = 1.0 / zexm1;
-    const double zb2 = fmin(sntz * ztau1, 500.0);
-    const double zexm2 = (zb2 <= od_lo) ? exp_small(zb2) : exp_tab(ET, zb2);
-    const double zexp2 = 1.0 / zexm2;
+    const double zexm1 = exp_of(ET, at_most(500.0, zrk * ztau1));
+    const double zexp1 = div_markstein(1.0, zexm1);
+    const double zexp2 = div_markstein(1.0, zexm2);
     const double ze1r45 = zr4 * zexp1 + zr5 * zexm1;
+    // zden1 of the beam (zssa1 / ze1r45) and of the diffuse light
+    // (zr4 / (ze1r45 zrkg1), its denominator kept eps1 from 0)
+    const double zb = ze1r45 * zrkg1;
+    double dbeam, ddiff;
+    if (fabs(zb) > eps1 && fabs(ze1r45) > eps1) {
+      const double q = recip_newton(zb);
+      dbeam = zssa1 * (zrkg1 * q);
+      ddiff = zr4 * q;
+    } else {
+      dbeam = zssa1 / ze1r45;
+      ddiff = (ze1r45 >= 0.0) ? zr4 / fmax(eps1, zb) : zr4 / fmin(-eps1, zb);
+    }
     if (fabs(ze1r45) <= eps1) {
       o.rb = eps1;
       o.tb = zexm2;
     } else {
-      const double zden1 = zssa1 / ze1r45;
-      o.rb = fmax(0.0, fmin(1.0, (zr1 * zexp1 - zr2 * zexm1 - zr3 * zexm2) * zden1));
-      o.tb = fmax(0.0, fmin(1.0, zexm2 * (1.0 - (zt1 * zexp1 - zt2 * zexm1 - zt3 * zexp2) * zden1)));
+      o.rb = clamp01((zr1 * zexp1 - zr2 * zexm1 - zr3 * zexm2) * dbeam);
+      o.tb = clamp01(zexm2 * (1.0 - (zt1 * zexp1 - zt2 * zexm1 - zt3 * zexp2) * dbeam));
     }
-    const double zden1 = (ze1r45 >= 0.0) ? zr4 / fmax(eps1, ze1r45 * zrkg1) : zr4 / fmin(-eps1, ze1r45 * zrkg1);
-    o.rd = fmax(0.0, fmin(1.0, zgam2 * (zexp1 - zexm1) * zden1));
-    o.td = fmax(0.0, fmin(1.0, zrk2 * zden1));
+    o.rd = clamp01(zgam2 * (zexp1 - zexm1) * ddiff);
+    o.td = clamp01(zrk2 * ddiff);
   }
-  const double od_lo2 = 0.06;
-  double zr = ztau1 * sntz;
-  o.e3 = (zr <= od_lo2) ? exp_small(zr) : exp_tab(ET, zr);
-  zr = ztau0 * sntz;
-  o.e4 = (zr <= od_lo2) ? exp_small(zr) : exp_tab(ET, zr);
 }
 
-struct ColIn {
-  const double* taug;   // row k at taug + k*112
-  const double* taur;
-  const double *aod, *ssa, *asy;   // caller arrays, (i, r, b)
-  const double *tcw, *scw, *gcw;   // [k][14]
-  const uint32_t* bits;            // this g-point's nw words (McICA)
-  const double* cfr;               // normalised cloud fraction, layer k at cfr[k * cfs] (grid-mean)
-  size_t cfs;
-  size_t i;
-  int ld, nlay, top_at_1, nw;
-  double cosz, sntz;
-  int iswmode;
-};
-
-__device__ __forceinline__ bool cloud_bit(const ColIn& c, int k) { return (c.bits[k >> 5] >> (k & 31)) & 1u; }
-// the all-sky sweep treats layer k as cloudy: its McICA flag, or cldfrc > ftiny (RSM:2885)
-template <bool GRID>
-__device__ __forceinline__ bool cloudy_layer(const ColIn& c, int k) {
-  return GRID ? (c.cfr[(size_t)k * c.cfs] > kFtiny) : cloud_bit(c, k);
+// read-once inputs: no L1 line, which stays with exp_tbl
+__device__ __forceinline__ double2 ld_once2(const double* p) {
+  double2 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
 }
+
 // spcvrtc's mixing of a cloudy layer's optics with its clear optics o
 // (RSM:3039-3042, 3057, 3072): zc0 * clear + zc1 * cloudy
-__device__ __forceinline__ void mix_grid(const ColIn& c, int k, const LayOpt& o, LayOpt& w) {
-  const double zc1 = c.cfr[(size_t)k * c.cfs], zc0 = 1.0 - zc1;
+__device__ __forceinline__ void mix_grid(double zc1, const LayOpt& o, LayOpt& w) {
+  const double zc0 = 1.0 - zc1;
   w.rb = zc0 * o.rb + zc1 * w.rb;
   w.rd = zc0 * o.rd + zc1 * w.rd;
   w.tb = zc0 * o.tb + zc1 * w.tb;
@@ -707,280 +785,457 @@ __device__ __forceinline__ void mix_grid(const ColIn& c, int k, const LayOpt& o,
   w.e4 = zc0 * o.e4 + zc1 * w.e4;
 }
 
-// the inputs of layer k of g-point g (band b): gas, Rayleigh and aerosol
-// optics, plus the cloud optics when the cloudy pass flags the layer
-struct LayIn {
-  double tr, tg, tae, sae, gae, tcw, scw, gcw;
-  bool cld;
-};
-template <bool GRID>
-__device__ __forceinline__ void layer_in(const ColIn& c, int g, int b, int k, bool cloudy_pass, LayIn& v) {
-  const int r = c.top_at_1 ? c.nlay - 1 - k : k;
-  const size_t xa = c.i + (size_t)c.ld * ((size_t)r + (size_t)c.nlay * b);
-  v.tr = c.taur[(size_t)k * kSwNg + g];
-  v.tg = c.taug[(size_t)k * kSwNg + g];
-  v.tae = __ldg(c.aod + xa);
-  v.sae = __ldg(c.ssa + xa);
-  v.gae = __ldg(c.asy + xa);
-  v.cld = cloudy_pass && cloudy_layer<GRID>(c, k);
-  if (v.cld) {
-    v.tcw = c.tcw[(size_t)k * 14 + b];
-    v.scw = c.scw[(size_t)k * 14 + b];
-    v.gcw = c.gcw[(size_t)k * 14 + b];
-  }
-}
-// the layer's two-stream optics (RSM:3447-3449 clear, 3678-3680 cloudy)
-__device__ __forceinline__ void layer_opt(const ColIn& c, const LayIn& v, const double* __restrict__ ET, LayOpt& o) {
-  double ztau0 = fmax(kFtiny, v.tr + v.tg + v.tae);
-  double zssa0 = v.tr + v.tae * v.sae;
-  double zasy0 = v.gae * v.sae * v.tae;
-  if (v.cld) {
-    ztau0 = ztau0 + v.tcw;
-    zssa0 = zssa0 + v.scw;
-    zasy0 = zasy0 + v.gcw;
-  }
-  two_stream(ztau0, zssa0, zasy0, c.cosz, c.sntz, c.iswmode, ET, o);
-}
-
-__device__ __forceinline__ double warp_sum(double v) {
+// Sums of N values (a power of two) over the 16 lanes of a half-warp: each
+// step exchanges half of the values with the partner lane, so N values take
+// N - 1 + log2(16 / N) exchanges instead of 4 N.  Lane j ends with the sum of
+// value bits(j) (see sum_index).
+template <int N>
+__device__ __forceinline__ double half_sums(double (&v)[N], int lane, unsigned mask) {
+  int o = 8;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+  for (int n = N / 2; n >= 1; n >>= 1, o >>= 1) {
+    const bool hi = (lane & o) != 0;
+#pragma unroll
+    for (int q = 0; q < n; ++q) {
+      const double keep = hi ? v[q + n] : v[q], send = hi ? v[q] : v[q + n];
+      v[q] = keep + __shfl_xor_sync(mask, send, o);
+    }
+  }
+  double r = v[0];
+  for (; o >= 1; o >>= 1) r += __shfl_xor_sync(mask, r, o);
+  return r;
+}
+// the value whose sum lane j of the half-warp holds, -1 where another lane has it too
+template <int N>
+__device__ __forceinline__ int sum_index(int lane) {
+  int idx = 0, o = 8;
+#pragma unroll
+  for (int n = N / 2; n >= 1; n >>= 1, o >>= 1)
+    if (lane & o) idx += n;
+  return (lane & (2 * o - 1)) ? -1 : idx;
 }
 
-constexpr int kRtWarps = 4;   // GRID: isubcsw <= 0, spcvrtc's cloud-fraction mixing; else McICA flags
-constexpr int kLaneVals = 10;   // per-lane stored values per level
+// Transfer, thread = g-point (112 per column; columns share warps, so no lane
+// idles), in two kernels.
+//
+// sw_up_kernel, bottom to top: each layer's two-stream optics are evaluated
+// once for the clear sky (and before that once more where the layer is cloudy),
+// and vrtqdr's upward recurrence (RSM:4011-4020) gives the reflectances
+// (zrupb, zrupd) of everything below a level.  With those known, the way down
+// needs no second adding recurrence: for the beam D and the diffuse flux F
+// entering a layer,
+//   D' = e3 D,  F' = (td F + ((tb - e3) + e3 zrupb rd) D) / (1 - rd zrupd),
+// and the level's fluxes are D + F down and zrupb D + zrupd F up, which is
+// what vrtqdr's zrdnd / ztdn form (RSM:4026-4046) gives, with one quotient per
+// layer and sweep in place of four.  sw_down_kernel does that and the outputs.
+//
+// Two kernels, because they want different things: the way up is a chain of
+// FP64 operations per layer (128 registers, sixteen warps per SM, 58 % of the
+// issue slots), the way down streams the stored layers (80 registers, 4.9 TB/s).
+// As phases of one kernel, with a slot of the store per resident column, the
+// same loops took 13.0 ms at 16,384 x 127; as two they take 9.1 ms (a column
+// per warp, both adding recurrences and four 10-shuffle sums per level took
+// 21.3 ms).  Down at 4, 5, 6 and 7 CTAs per SM: 9.4, 9.1, 9.1 and 9.8 ms.
+constexpr int kRtAhead = 2;   // layers whose stored records are in flight on the way down (even)
+constexpr int kRtLay = kRtVals * kSwNg;   // store doubles of a layer
 
-// One column's transfer and outputs: a = the argument record of the call
-// (or of the physics block) the column belongs to, j1 its 1-based column
-// there, acc0 this warp's shared-memory slice.
+// a thread's view of its column
+struct RtCol {
+  const double *aod, *ssa, *asy;    // layer 0 of the g-point's band, xstep per layer
+  const double *tg;                 // taug of layers 0..3
+  RaySrc ray;
+  ptrdiff_t xstep;
+  const double *tcw, *scw, *gcw;    // cloud optics of the band, 14 per layer
+  const uint32_t* bits;             // McICA flags
+  const double* cfr;                // normalised cloud fraction, cfs per layer (grid-mean)
+  size_t cfs;
+  double* st;                       // the g-point's layer store
+  double cosz, sntz;
+  int nlay, nw, iswmode;
+  bool cloudy;
+};
+
+// layer k is cloudy for this g-point: its McICA flag, or cldfrc > ftiny
+// (RSM:2885); word = the flags of layers 32 (k / 32) ..
 template <bool GRID>
-__device__ __forceinline__ void rt_body(const SwArgs& a, const SwScratch& s, int pl, int nc, int j1, int lane,
-                                        double* acc0, const double* __restrict__ ET) {
-  const int nlay = a.nlay, nlp1 = nlay + 1;
-  const bool want_b = a.hswb != nullptr;
-  double* acc = acc0;
-  double *up0 = acc, *dn0 = acc + nlp1, *upc = acc + 2 * nlp1, *dnc = acc + 3 * nlp1;
-  double* accb = acc + 4 * nlp1;   // [14][2][nlp1] total-sky band fluxes (hswb)
-  for (int q = lane; q < (want_b ? 32 : 4) * nlp1; q += 32) acc[q] = 0.0;
-  __syncwarp();
+__device__ __forceinline__ uint32_t flags_of(const RtCol& c, int w) {
+  return (!GRID && c.cloudy && w >= 0 && w < c.nw) ? __ldg(c.bits + w) : 0u;
+}
+template <bool GRID>
+__device__ __forceinline__ bool cloud_at(const RtCol& c, int k, uint32_t word) {
+  return GRID ? (c.cloudy && c.cfr[(size_t)k * c.cfs] > kFtiny) : ((word >> (k & 31)) & 1u);
+}
 
-  const size_t i = (size_t)(j1 - 1);
-  ColIn c;
-  c.taug = s.taug + (size_t)pl * nlay * kSwNg;
-  c.taur = s.taur + (size_t)pl * nlay * kSwNg;
-  c.aod = a.aod; c.ssa = a.ssa; c.asy = a.asy;
-  c.tcw = s.taucw + (size_t)pl * nlay * 14;
-  c.scw = s.ssacw + (size_t)pl * nlay * 14;
-  c.gcw = s.asycw + (size_t)pl * nlay * 14;
-  c.i = i; c.ld = a.ld; c.nlay = nlay; c.top_at_1 = a.top_at_1; c.nw = s.nw;
-  c.cosz = a.cosz[i];
-  c.sntz = 1.0 / a.cosz[i];
-  c.iswmode = a.iswmode;
-  const double ssolar = a.s0fac * a.cosz[i];
-  const double albbm[2] = {a.alb_nir_dir[i], a.alb_uvis_dir[i]};
-  const double albdf[2] = {a.alb_nir_dif[i], a.alb_uvis_dif[i]};
-  const double cf1 = s.zcf1[pl], cf0 = s.zcf0[pl];
-  const bool cloudy = cf1 > kEps;
+// all-sky optics of the cloudy layers, into store values 8..13
+template <bool GRID, typename Tbl>
+__device__ __forceinline__ void rt_cloudy(const RtCol& c, const Tbl& ET) {
+#pragma unroll 1
+  for (int w = 0; w < c.nw; ++w) {
+    uint32_t m = flags_of<GRID>(c, w);
+    if (GRID)
+      for (int k = 32 * w; k < min(32 * w + 32, c.nlay); ++k) m |= (cloud_at<true>(c, k, 0) ? 1u : 0u) << (k & 31);
+    while (m) {   // each lane its own layers: a warp's rounds are the most cloudy layers of one lane
+      const int k = 32 * w + __ffs(m) - 1;
+      m &= m - 1;
+      const ptrdiff_t xo = c.xstep * k;
+      const double tae = __ldg(c.aod + xo), sae = __ldg(c.ssa + xo), gae = __ldg(c.asy + xo);
+      const double tr = c.ray.p[c.ray.stride * k] * c.ray.coef, tg = c.tg[(size_t)(k >> 2) * kSwNg * kTgStride + (k & 3)];
+      const double ztau0 = fmax(kFtiny, tr + tg + tae);
+      const double zssa0 = tr + tae * sae;
+      const double zasy0 = gae * sae * tae;
+      const size_t x = (size_t)k * 14;
+      LayOpt v;
+      two_stream(ztau0 + c.tcw[x], zssa0 + c.scw[x], zasy0 + c.gcw[x], c.cosz, c.sntz, c.iswmode, ET, v);
+      if (GRID) {
+        LayOpt o;
+        two_stream(ztau0, zssa0, zasy0, c.cosz, c.sntz, c.iswmode, ET, o);
+        mix_grid(c.cfr[(size_t)k * c.cfs], o, v);
+      }
+      double* q = c.st + (size_t)k * kRtLay;
+      __stcg(q + 8 * kSwNg, v.td);
+      __stcg(q + 9 * kSwNg, v.tb - v.e3);
+      __stcg(q + 10 * kSwNg, v.e3);
+      __stcg(q + 11 * kSwNg, v.rd);
+      __stcg(q + 12 * kSwNg, v.rb);
+      __stcg(q + 13 * kSwNg, v.e4);
+    }
+  }
+}
+
+// bottom to top from the surface's (ub, ud): store values td, tb - e3, e3, rd
+// of each layer and zrupb, zrupd (clear, all-sky) below it; above the top
+// layer the unscaled beam transmittances of the column and zrupb, zrupd
+template <bool GRID, typename Tbl>
+__device__ __forceinline__ void rt_up(const RtCol& c, const Tbl& ET, double ub, double ud) {
+  double ubw = ub, udw = ud, beam0 = 1.0, beam0w = 1.0;
+  const double *aod = c.aod, *ssa = c.ssa, *asy = c.asy, *ray = c.ray.p, *tgp = c.tg;
+  double* st = c.st;
+  struct In { double tr, tae, sae, gae; } nx;
+  auto fetch = [&](In& v) {
+    v.tr = *ray;
+    v.tae = __ldg(aod);
+    v.sae = __ldg(ssa);
+    v.gae = __ldg(asy);
+    ray += c.ray.stride;
+    aod += c.xstep;
+    ssa += c.xstep;
+    asy += c.xstep;
+  };
+  fetch(nx);
+  double2 n01 = ld_once2(tgp), n23 = ld_once2(tgp + 2);
+  uint32_t word = 0, nword = flags_of<GRID>(c, 0);
+#pragma unroll 1
+  for (int k0 = 0; k0 < c.nlay; k0 += 4) {
+    if ((k0 & 31) == 0) {
+      word = nword;
+      nword = flags_of<GRID>(c, (k0 >> 5) + 1);
+    }
+    const double2 c01 = n01, c23 = n23;
+    if (k0 + 4 < c.nlay) {
+      tgp += kSwNg * kTgStride;
+      n01 = ld_once2(tgp);
+      n23 = ld_once2(tgp + 2);
+    }
+#pragma unroll 1
+    for (int kk = 0; kk < 4; ++kk) {
+      const int k = k0 + kk;
+      if (k >= c.nlay) break;
+      const In cur = nx;
+      if (k + 1 < c.nlay) fetch(nx);   // issued ahead of this layer's arithmetic
+      const double tg = (kk & 2) ? ((kk & 1) ? c23.y : c23.x) : ((kk & 1) ? c01.y : c01.x);
+      const double tr = cur.tr * c.ray.coef;
+      LayOpt o;
+      two_stream(fmax(kFtiny, tr + tg + cur.tae), tr + cur.tae * cur.sae, cur.gae * cur.sae * cur.tae, c.cosz, c.sntz,
+                 c.iswmode, ET, o);
+      double tbd = o.tb - o.e3;
+      __stcg(st, o.td);
+      __stcg(st + kSwNg, tbd);
+      __stcg(st + 2 * kSwNg, o.e3);
+      __stcg(st + 3 * kSwNg, o.rd);
+      __stcg(st + 4 * kSwNg, ub);
+      __stcg(st + 5 * kSwNg, ud);
+      beam0 *= o.e4;
+      const double q = recip_newton(fma(-ud, o.rd, 1.0));
+      ub = fma(o.td * fma(tbd, ud, o.e3 * ub), q, o.rb);
+      ud = fma(o.td * o.td * ud, q, o.rd);
+      if (c.cloudy) {
+        __stcg(st + 6 * kSwNg, ubw);
+        __stcg(st + 7 * kSwNg, udw);
+        if (cloud_at<GRID>(c, k, word)) {
+          o.td = __ldcg(st + 8 * kSwNg);
+          tbd = __ldcg(st + 9 * kSwNg);
+          o.e3 = __ldcg(st + 10 * kSwNg);
+          o.rd = __ldcg(st + 11 * kSwNg);
+          o.rb = __ldcg(st + 12 * kSwNg);
+          o.e4 = __ldcg(st + 13 * kSwNg);
+        }
+        beam0w *= o.e4;
+        const double qw = recip_newton(fma(-udw, o.rd, 1.0));
+        ubw = fma(o.td * fma(tbd, udw, o.e3 * ubw), qw, o.rb);
+        udw = fma(o.td * o.td * udw, qw, o.rd);
+      }
+      st += kRtLay;
+    }
+  }
+  __stcg(st, beam0);
+  __stcg(st + kSwNg, beam0w);
+  __stcg(st + 4 * kSwNg, ub);
+  __stcg(st + 5 * kSwNg, ud);
+  __stcg(st + 6 * kSwNg, ubw);
+  __stcg(st + 7 * kSwNg, udw);
+}
+
+// where the way down puts its sums: a group's [4][nlp1] up, down clear, up,
+// down all-sky; with hswb also [kRtBandSlots][2][nlp1] total-sky band fluxes
+struct RtSums {
+  double *part, *accb;
+  double cf1, cf0;
+  int nlp1, grp, b, blo, nbg;   // the g-point's band, the group's first band and their number - 1 (at most 2)
+};
+
+// top to bottom from (ub, ud) at the top level: fluxes of every level, summed
+// over the group's g-points two levels at a time
+template <bool GRID, bool BANDS>
+__device__ __forceinline__ void rt_down(const RtCol& c, double zsolar, const RtSums& S, double (&end)[4]) {
+  const int half = threadIdx.x & 15;
+  const unsigned hmask = 0xffffu << (threadIdx.x & 16);
+  const int idx8 = sum_index<8>(half), idx4 = sum_index<4>(half);
+  const double* st = c.st + (size_t)c.nlay * kRtLay;   // the layer at hand
+  double ub = __ldcg(st + 4 * kSwNg), ud = __ldcg(st + 5 * kSwNg), ubw = __ldcg(st + 6 * kSwNg),
+         udw = __ldcg(st + 7 * kSwNg), D = zsolar, F = 0.0, Dw = zsolar, Fw = 0.0;
+  st -= kRtLay;
+  double v[8];
+  auto level = [&](int slot) {   // fluxes of the level reached into v[4 * slot ..]
+    v[4 * slot + 0] = fma(F, ud, D * ub);
+    v[4 * slot + 1] = D + F;
+    v[4 * slot + 2] = c.cloudy ? fma(Fw, udw, Dw * ubw) : 0.0;
+    v[4 * slot + 3] = c.cloudy ? Dw + Fw : 0.0;
+  };
+  auto flush = [&](int m, int nlev) {   // sums of levels m (slot 0) and m - 1 (slot 1)
+    if (BANDS) {   // total-sky band fluxes (spcvrtc: cf1 all-sky + cf0 clear, RSM:3160-3161)
+#pragma unroll 1
+      for (int q = 0; q < 3; ++q) {
+        double u[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const double c0 = v[4 * (e >> 1) + (e & 1)], c1 = v[4 * (e >> 1) + 2 + (e & 1)];
+          const double t = c.cloudy ? (GRID ? S.cf1 * c1 + S.cf0 * c0 : c1) : c0;
+          u[e] = (S.b == S.blo + q) ? t : 0.0;
+        }
+        const double r = half_sums<4>(u, half, hmask);
+        const int lev = idx4 >> 1;
+        if (q <= S.nbg && idx4 >= 0 && lev < nlev)
+          S.accb[((size_t)2 * (S.blo + q + S.grp) + (idx4 & 1)) * S.nlp1 + (m - lev)] = r;
+      }
+    }
+    const double r = half_sums<8>(v, half, hmask);
+    const int lev = idx8 >> 2;
+    if (idx8 >= 0 && lev < nlev) S.part[(size_t)(idx8 & 3) * S.nlp1 + (m - lev)] = r;
+  };
+  struct Rec { double td, tbd, e3, rd, ub, ud, ubw, udw; };
+  auto load = [&](int below, Rec& r) {   // the record `below` layers under it
+    const double* p = st - below * kRtLay;
+    r.td = __ldcg(p);
+    r.tbd = __ldcg(p + kSwNg);
+    r.e3 = __ldcg(p + 2 * kSwNg);
+    r.rd = __ldcg(p + 3 * kSwNg);
+    r.ub = __ldcg(p + 4 * kSwNg);
+    r.ud = __ldcg(p + 5 * kSwNg);
+    if (c.cloudy) {
+      r.ubw = __ldcg(p + 6 * kSwNg);
+      r.udw = __ldcg(p + 7 * kSwNg);
+    }
+  };
+  uint32_t word = flags_of<GRID>(c, (c.nlay - 1) >> 5), nword = flags_of<GRID>(c, ((c.nlay - 1) >> 5) - 1);
+  auto step = [&](int m, const Rec& r) {   // through layer m
+    if ((m & 31) == 31 && m < c.nlay - 1) {
+      word = nword;
+      nword = flags_of<GRID>(c, (m >> 5) - 1);
+    }
+    ub = r.ub;
+    ud = r.ud;
+    const double q = recip_newton(fma(-r.rd, ud, 1.0));
+    F = fma(r.td, F, fma(r.e3 * ub, r.rd, r.tbd) * D) * q;
+    D *= r.e3;
+    if (c.cloudy) {
+      ubw = r.ubw;
+      udw = r.udw;
+      double td = r.td, tbd = r.tbd, e3 = r.e3, rd = r.rd;
+      if (cloud_at<GRID>(c, m, word)) {
+        td = __ldcg(st + 8 * kSwNg);
+        tbd = __ldcg(st + 9 * kSwNg);
+        e3 = __ldcg(st + 10 * kSwNg);
+        rd = __ldcg(st + 11 * kSwNg);
+      }
+      const double qw = recip_newton(fma(-rd, udw, 1.0));
+      Fw = fma(td, Fw, fma(e3 * ubw, rd, tbd) * Dw) * qw;
+      Dw *= e3;
+    }
+  };
+  level(0);
+  Rec r[kRtAhead];   // the next layers' records
+#pragma unroll
+  for (int q = 0; q < kRtAhead; ++q)
+    if (c.nlay > q) load(q, r[q]);
+#pragma unroll 1
+  for (int m0 = c.nlay - 1; m0 >= 0; m0 -= kRtAhead) {
+#pragma unroll
+    for (int q = 0; q < kRtAhead; ++q) {
+      const int m = m0 - q;
+      if (m >= 0) {
+        step(m, r[q]);
+        if (m >= kRtAhead) load(kRtAhead, r[q]);
+        st -= kRtLay;
+        level((q & 1) ? 0 : 1);
+        if ((q & 1) == 0) flush(m + 1, 2);
+      }
+    }
+  }
+  if ((c.nlay & 1) == 0) {   // an odd number of levels: the last one is alone in slot 0
+    v[4] = v[5] = v[6] = v[7] = 0.0;
+    flush(0, 1);
+  }
+  end[0] = D;
+  end[1] = F;
+  end[2] = Dw;
+  end[3] = Fw;
+}
+
+// thread g's view of column j1 of record a, column pl of the chunk
+__device__ __forceinline__ RtCol rt_col(const SwArgs& a, const SwScratch& s, int pl, int nc, int j1, int g, int b,
+                                        const double* __restrict__ T) {
+  const int nlay = a.nlay, top = a.top_at_1;
+  const size_t i = (size_t)(j1 - 1), ld = (size_t)a.ld;
+  RtCol c;
+  const size_t xb = i + ld * ((size_t)nlay * b + (top ? nlay - 1 : 0));
+  c.aod = a.aod + xb;
+  c.ssa = a.ssa + xb;
+  c.asy = a.asy + xb;
+  c.tg = s.taug + tg_offset(nlay, pl, 0, g);
+  c.ray = ray_src(s, pl, nlay, g, b, T);
+  c.xstep = top ? -(ptrdiff_t)ld : (ptrdiff_t)ld;
+  const size_t cx = (size_t)pl * nlay * 14 + b;
+  c.tcw = s.taucw + cx;
+  c.scw = s.ssacw + cx;
+  c.gcw = s.asycw + cx;
+  c.bits = s.bits + ((size_t)pl * kSwNg + g) * s.nw;
   c.cfr = s.aux + pl;
   c.cfs = (size_t)nc;
-  // surface partition and UV-B sums of lane 0: [pass][bm1, bm2, df1, df2, uvb]
-  double sfc[2][5] = {{0, 0, 0, 0, 0}, {0, 0, 0, 0, 0}};
+  c.st = s.rt_store + (size_t)pl * rt_col_store(nlay) + g;
+  c.cosz = a.cosz[i];
+  c.sntz = 1.0 / c.cosz;
+  c.nlay = nlay;
+  c.nw = s.nw;
+  c.iswmode = a.iswmode;
+  c.cloudy = s.zcf1[pl] > kEps;
+  return c;
+}
 
-  // per-lane storage in global scratch, [level][value][lane] per column
-  // (values: 6 clear-sky layer optics, clear zrupb/zrupd, cloudy
-  // zrupb/zrupd): a warp touches 256 contiguous bytes per value, and the
-  // L2-only (.cg) accesses keep L1 for exp_tbl and the streamed optical depths
-  double* lst = s.lane_store + (size_t)pl * (size_t)(nlay + 1) * kLaneVals * 32 + lane;
-  auto st8 = [&](int k, int q, double v) { __stcg(lst + ((size_t)k * kLaneVals + q) * 32, v); };
-  auto ld8 = [&](int k, int q) { return __ldcg(lst + ((size_t)k * kLaneVals + q) * 32); };
+template <bool GRID, typename Tbl>
+__device__ __forceinline__ void up_body(const SwArgs& a, const SwScratch& s, int pl, int nc, int j1, int g,
+                                        const double* __restrict__ T, const Tbl& ET) {
+  const int b = band_of(g), ibd = c_idxsfc[b];
+  const size_t i = (size_t)(j1 - 1);
+  const RtCol c = rt_col(a, s, pl, nc, j1, g, b, T);
+  if (c.cloudy) rt_cloudy<GRID>(c, ET);
+  rt_up<GRID>(c, ET, ibd ? (ibd == 1 ? a.alb_nir_dir[i] : a.alb_uvis_dir[i]) : 0.5 * (a.alb_nir_dir[i] + a.alb_uvis_dir[i]),
+              ibd ? (ibd == 1 ? a.alb_nir_dif[i] : a.alb_uvis_dif[i]) : 0.5 * (a.alb_nir_dif[i] + a.alb_uvis_dif[i]));
+}
 
-  for (int r0 = 0; r0 < kSwNg; r0 += 32) {
-    const int g = r0 + lane;
-    const bool valid = g < kSwNg;
-    const int gg = valid ? g : kSwNg - 1;
-    const int b = band_of(gg), ibd = c_idxsfc[b];
-    const double zsolar = ssolar * s.sflux[(size_t)pl * kSwNg + gg];
-    const double wgt = valid ? zsolar : 0.0;
-    const int blo = band_of(r0), bhi = band_of(min(r0 + 31, kSwNg - 1));
-    c.bits = s.bits + ((size_t)pl * kSwNg + gg) * s.nw;
-    const double refb1 = ibd ? albbm[ibd - 1] : 0.5 * (albbm[0] + albbm[1]);
-    const double refd1 = ibd ? albdf[ibd - 1] : 0.5 * (albdf[0] + albdf[1]);
-    // The clear-sky sweep and, in a cloudy column, the all-sky sweep of
-    // spcvrtm (RSM:3444-3667, 3668-3893) run side by side: a layer's clear
-    // optics are evaluated once and serve both, and the all-sky sweep
-    // re-evaluates only the layers its sub-column flags cloudy, as spcvrtm
-    // keeps the clear-pass arrays for clear layers (RSM:3849-3850).
-    // upward adding (vrtqdr, RSM:4011-4020)
-    double ub = refb1, ud = refd1, ubw = refb1, udw = refd1;
-    st8(0, 6, ub);
-    st8(0, 7, ud);
-    if (cloudy) {
-      st8(0, 8, ubw);
-      st8(0, 9, udw);
-    }
-    LayIn vin;
-    layer_in<GRID>(c, gg, b, 0, cloudy, vin);
-    for (int k = 0; k < nlay; ++k) {
-      const LayIn cur = vin;
-      if (k + 1 < nlay) layer_in<GRID>(c, gg, b, k + 1, cloudy, vin);   // issued ahead of this layer's arithmetic
-      LayIn clr = cur;
-      clr.cld = false;
-      LayOpt o;
-      layer_opt(c, clr, ET, o);
-      st8(k, 0, o.rb); st8(k, 1, o.rd); st8(k, 2, o.tb); st8(k, 3, o.td); st8(k, 4, o.e3); st8(k, 5, o.e4);
-      {
-        const double zden1 = 1.0 / (1.0 - ud * o.rd);
-        const double nb = o.rb + (o.td * ((o.tb - o.e3) * ud + o.e3 * ub)) * zden1;
-        const double nd = o.rd + o.td * o.td * ud * zden1;
-        ub = nb;
-        ud = nd;
-        st8(k + 1, 6, ub);
-        st8(k + 1, 7, ud);
-      }
-      if (cloudy) {
-        LayOpt w = o;
-        if (cur.cld) {
-          layer_opt(c, cur, ET, w);
-          if (GRID) mix_grid(c, k, o, w);
-        }
-        const double zden1 = 1.0 / (1.0 - udw * w.rd);
-        const double nb = w.rb + (w.td * ((w.tb - w.e3) * udw + w.e3 * ubw)) * zden1;
-        const double nd = w.rd + w.td * w.td * udw * zden1;
-        ubw = nb;
-        udw = nd;
-        st8(k + 1, 8, ubw);
-        st8(k + 1, 9, udw);
-      }
-    }
-    // downward sweep (RSM:4026-4040) with the fluxes of each level (RSM:4041-4046)
-    auto fetch = [&](int m, LayOpt& o, LayOpt& w) {
-      o.rb = ld8(m, 0); o.rd = ld8(m, 1); o.tb = ld8(m, 2); o.td = ld8(m, 3); o.e3 = ld8(m, 4); o.e4 = ld8(m, 5);
-      w = o;
-      if (cloudy && cloudy_layer<GRID>(c, m)) {
-        LayIn v;
-        layer_in<GRID>(c, gg, b, m, true, v);
-        layer_opt(c, v, ET, w);
-        if (GRID) mix_grid(c, m, o, w);
-      }
-    };
-    // one downward step of a sweep: layer optics o, state (tdbt, tdn, rdnd, tdbt0)
-    auto down = [&](int m, const LayOpt& o, double& tdbt, double& tdn, double& rdnd, double& tdbt0) {
-      double tdn_m, rdnd_m;
-      if (m == nlay - 1) {
-        tdn_m = o.tb;
-        rdnd_m = o.rd;
-      } else {
-        const double zden1 = 1.0 / (1.0 - o.rd * rdnd);
-        tdn_m = tdbt * o.tb + (o.td * ((tdn - tdbt) + tdbt * o.rb * rdnd)) * zden1;
-        rdnd_m = o.rd + o.td * o.td * rdnd * zden1;
-      }
-      tdbt = o.e3 * tdbt;
-      tdbt0 = o.e4 * tdbt0;
-      tdn = tdn_m;
-      rdnd = rdnd_m;
-    };
-    auto flux = [&](double tdbt, double tdn, double rdnd, double rub, double rud, double& fu, double& fd) {
-      const double zden1 = 1.0 / (1.0 - rdnd * rud);
-      fu = (tdbt * rub + (tdn - tdbt) * rud) * zden1;
-      fd = tdbt + (tdn - tdbt + tdbt * rub * rdnd) * zden1;
-    };
-    double tdbt = 1.0, tdn = 1.0, rdnd = 0.0, tdbt0 = 1.0, fd0 = 0.0;
-    double tdbtw = 1.0, tdnw = 1.0, rdndw = 0.0, tdbt0w = 1.0, fd0w = 0.0;
-    LayOpt nx, nxw;
-    fetch(nlay - 1, nx, nxw);
-    for (int m = nlay; m >= 0; --m) {
-      if (m < nlay) {
-        const LayOpt o = nx, w = nxw;
-        if (m > 0) fetch(m - 1, nx, nxw);   // the next layer's loads overlap this layer's recurrences
-        down(m, o, tdbt, tdn, rdnd, tdbt0);
-        if (cloudy) down(m, w, tdbtw, tdnw, rdndw, tdbt0w);
-      }
-      double fu, fd, fuw = 0.0, fdw = 0.0;
-      flux(tdbt, tdn, rdnd, ld8(m, 6), ld8(m, 7), fu, fd);
-      if (cloudy) flux(tdbtw, tdnw, rdndw, ld8(m, 8), ld8(m, 9), fuw, fdw);
-      if (m == 0) {
-        fd0 = fd;
-        fd0w = fdw;
-      }
-      const double su = warp_sum(wgt * fu), sd = warp_sum(wgt * fd);
-      if (lane == 0) {
-        up0[m] += su;
-        dn0[m] += sd;
-      }
-      if (cloudy) {
-        const double suw = warp_sum(wgt * fuw), sdw = warp_sum(wgt * fdw);
-        if (lane == 0) {
-          upc[m] += suw;
-          dnc[m] += sdw;
-        }
-      }
-      if (want_b) {   // total-sky band fluxes (spcvrtc: cf1 * all-sky + cf0 * clear, RSM:3160-3161)
-        const double tu = cloudy ? (GRID ? cf1 * fuw + cf0 * fu : fuw) : fu;
-        const double td = cloudy ? (GRID ? cf1 * fdw + cf0 * fd : fdw) : fd;
-        for (int bb = blo; bb <= bhi; ++bb) {
-          const double mu = warp_sum(b == bb ? wgt * tu : 0.0), md = warp_sum(b == bb ? wgt * td : 0.0);
-          if (lane == 0) {
-            accb[(size_t)(2 * bb) * nlp1 + m] += mu;
-            accb[(size_t)(2 * bb + 1) * nlp1 + m] += md;
-          }
-        }
-      }
-    }
-    // surface direct / diffuse partition (RSM:3641-3655) and UV-B (RSM:3907)
-    for (int pass = 0; pass < (cloudy ? 2 : 1); ++pass) {
-      const double t0 = pass ? tdbt0w : tdbt0, f0 = pass ? fd0w : fd0;
-      const double zb1 = wgt * t0, zb2 = wgt * (f0 - t0);
-      const double bm1 = (ibd == 1) ? zb1 : (ibd == 0 ? 0.5 * zb1 : 0.0);
-      const double bm2 = (ibd == 2) ? zb1 : (ibd == 0 ? 0.5 * zb1 : 0.0);
-      const double df1 = (ibd == 1) ? zb2 : (ibd == 0 ? 0.5 * zb2 : 0.0);
-      const double df2 = (ibd == 2) ? zb2 : (ibd == 0 ? 0.5 * zb2 : 0.0);
-      const double uv = (b == 27 - 16) ? wgt * f0 : 0.0;
-      const double v[5] = {warp_sum(bm1), warp_sum(bm2), warp_sum(df1), warp_sum(df2), warp_sum(uv)};
-      if (lane == 0)
-        for (int q = 0; q < 5; ++q) sfc[pass][q] += v[q];
+template <bool GRID, bool BANDS>
+__device__ __forceinline__ void down_body(const SwArgs& a, const SwScratch& s, int pl, int nc, int j1, int g,
+                                          double* __restrict__ acc, const double* __restrict__ T) {
+  const int nlay = a.nlay, nlp1 = nlay + 1, grp = g >> 4, top = a.top_at_1;
+  double* accb = acc + (size_t)4 * kRtGroups * nlp1;
+  double* sfc = accb + (BANDS ? (size_t)2 * kRtBandSlots * nlp1 : 0);   // [kRtGroups][2][5]
+  const size_t i = (size_t)(j1 - 1), ld = (size_t)a.ld;
+  const int b = band_of(g), ibd = c_idxsfc[b];
+  const double cf1 = s.zcf1[pl], cf0 = s.zcf0[pl];
+  const bool cloudy = cf1 > kEps;
+  const double zsolar = a.s0fac * a.cosz[i] * s.sflux[(size_t)pl * kSwNg + g];
+  double end[4];   // beam and diffuse flux at the surface, clear and all-sky
+  {
+    const RtCol c = rt_col(a, s, pl, nc, j1, g, b, T);
+    RtSums S;
+    S.part = acc + (size_t)grp * 4 * nlp1;
+    S.accb = accb;
+    S.cf1 = cf1;
+    S.cf0 = cf0;
+    S.nlp1 = nlp1;
+    S.grp = grp;
+    S.b = b;
+    S.blo = band_of(g & ~15);
+    S.nbg = band_of(g | 15) - S.blo;
+    rt_down<GRID, BANDS>(c, zsolar, S, end);
+  }
+  const double* tops = s.rt_store + (size_t)pl * rt_col_store(nlay) + (size_t)nlay * kRtLay + g;
+  const double beam[2] = {__ldcg(tops), __ldcg(tops + kSwNg)};
+
+  // surface direct / diffuse partition (RSM:3641-3655) and UV-B (RSM:3907)
+  {
+    const int half = threadIdx.x & 15, idx8 = sum_index<8>(half);
+    const unsigned hmask = 0xffffu << (threadIdx.x & 16);
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+      const double zb1 = zsolar * beam[pass], f0 = end[2 * pass] + end[2 * pass + 1], zb2 = f0 - zb1;
+      double w[8] = {(ibd == 1) ? zb1 : (ibd == 0 ? 0.5 * zb1 : 0.0), (ibd == 2) ? zb1 : (ibd == 0 ? 0.5 * zb1 : 0.0),
+                     (ibd == 1) ? zb2 : (ibd == 0 ? 0.5 * zb2 : 0.0), (ibd == 2) ? zb2 : (ibd == 0 ? 0.5 * zb2 : 0.0),
+                     (b == 27 - 16) ? f0 : 0.0, 0.0, 0.0, 0.0};
+      const double r = half_sums<8>(w, half, hmask);
+      if (idx8 >= 0 && idx8 < 5) sfc[(grp * 2 + pass) * 5 + idx8] = r;
     }
   }
-  __syncwarp();
+  __syncthreads();
+
+  // ---- sums over the column's groups, in a fixed order ----
+  for (int q = g; q < 4 * nlp1; q += kSwNg) {
+    double t = 0.0;
+#pragma unroll
+    for (int p = 0; p < kRtGroups; ++p) t += acc[(size_t)p * 4 * nlp1 + q];
+    acc[q] = t;
+  }
+  __syncthreads();
+  double *up0 = acc, *dn0 = acc + nlp1, *upc = acc + 2 * nlp1, *dnc = acc + 3 * nlp1;
   if (cloudy && GRID) {   // spcvrtc's total-sky fluxes (RSM:3158-3178)
-    for (int m = lane; m < nlp1; m += 32) {
+    for (int m = g; m < nlp1; m += kSwNg) {
       upc[m] = cf1 * upc[m] + cf0 * up0[m];
       dnc[m] = cf1 * dnc[m] + cf0 * dn0[m];
     }
-    if (lane == 0)
-      for (int q = 0; q < 5; ++q) sfc[1][q] = cf1 * sfc[1][q] + cf0 * sfc[0][q];
-    __syncwarp();
   }
+  if (GRID) __syncthreads();
 
   // outputs (RSM:1225-1373)
-  const int ld = a.ld;
   const double* fu_t = cloudy ? upc : up0;
   const double* fd_t = cloudy ? dnc : dn0;
-  auto row = [&](int m) { return a.top_at_1 ? nlay - 1 - m : m; };     // internal layer -> caller row
-  auto lev = [&](int k) { return a.top_at_1 ? nlay - k : k; };         // internal level -> caller level
-  for (int m = lane; m < nlay; m += 32) {
+  auto row = [&](int m) { return top ? nlay - 1 - m : m; };     // internal layer -> caller row
+  auto lev = [&](int k) { return top ? nlay - k : k; };         // internal level -> caller level
+  for (int m = g; m < nlay; m += kSwNg) {
     const int r = row(m);
-    const size_t x = i + (size_t)ld * r;
+    const size_t x = i + ld * r;
     const double rfdelp = a.heatfac / a.delp[x];
     a.hswc[x] = ((fd_t[m + 1] - fu_t[m + 1]) - (fd_t[m] - fu_t[m])) * rfdelp;
     if (a.hsw0) a.hsw0[x] = ((dn0[m + 1] - up0[m + 1]) - (dn0[m] - up0[m])) * rfdelp;
-    if (want_b)
-      for (int bb = 0; bb < 14; ++bb) {
-        const double* bu = accb + (size_t)(2 * bb) * nlp1;
-        const double* bd = accb + (size_t)(2 * bb + 1) * nlp1;
-        a.hswb[i + (size_t)ld * ((size_t)r + (size_t)nlay * bb)] = ((bd[m + 1] - bu[m + 1]) - (bd[m] - bu[m])) * rfdelp;
+    if (BANDS)
+      for (int bb = 0; bb < 14; ++bb) {   // a band's g-points lie in one or two groups
+        const int p0 = c_ns[bb] >> 4, p1 = (c_ns[bb] + c_ng[bb] - 1) >> 4;
+        double u0 = 0.0, u1 = 0.0, d0 = 0.0, d1 = 0.0;
+        for (int p = p0; p <= p1; ++p) {
+          const double* bu = accb + (size_t)(2 * (bb + p)) * nlp1;
+          const double* bd = bu + nlp1;
+          u0 += bu[m]; u1 += bu[m + 1]; d0 += bd[m]; d1 += bd[m + 1];
+        }
+        a.hswb[i + ld * ((size_t)r + (size_t)nlay * bb)] = ((d1 - u1) - (d0 - u0)) * rfdelp;
       }
   }
   if (a.flxprf)
-    for (int k = lane; k < nlp1; k += 32) {
-      double* rec = a.flxprf + 4 * (i + (size_t)ld * lev(k));
+    for (int k = g; k < nlp1; k += kSwNg) {
+      double* rec = a.flxprf + 4 * (i + ld * lev(k));
       rec[0] = fu_t[k];
       rec[1] = fd_t[k];
       rec[2] = up0[k];
       rec[3] = dn0[k];
     }
-  if (lane == 0) {
-    const int t = cloudy ? 1 : 0;
+  if (g == 0) {
     double* tf = a.topflx + 3 * i;
     tf[0] = fu_t[nlay];
     tf[1] = dn0[nlay];
@@ -990,40 +1245,87 @@ __device__ __forceinline__ void rt_body(const SwArgs& a, const SwScratch& s, int
     sf[1] = fd_t[0];
     sf[2] = up0[0];
     sf[3] = dn0[0];
-    if (a.fdncmp) {
-      double* r = a.fdncmp + 6 * i;
-      r[0] = sfc[t][4];
-      r[1] = sfc[0][4];
-      r[2] = sfc[t][0];
-      r[3] = sfc[t][2];
-      r[4] = sfc[t][1];
-      r[5] = sfc[t][3];
+  }
+  if (a.fdncmp && g < 6) {
+    // records uvbfc, uvbf0, nirbm, nirdf, visbm, visdf from the sums bm1, bm2, df1, df2, uvb
+    const int from[6] = {4, 4, 0, 2, 1, 3};
+    int q = from[0];
+#pragma unroll
+    for (int e = 1; e < 6; ++e) q = (g == e) ? from[e] : q;
+    double clr = 0.0, all = 0.0;
+    for (int p = 0; p < kRtGroups; ++p) {
+      clr += sfc[(p * 2 + 0) * 5 + q];
+      all += sfc[(p * 2 + 1) * 5 + q];
     }
+    if (GRID) all = cf1 * all + cf0 * clr;
+    a.fdncmp[6 * i + g] = (cloudy && g != 1) ? all : clr;
   }
 }
 
-template <bool GRID>
-__global__ void __launch_bounds__(32 * kRtWarps, 4)   // 128 registers: sixteen warps per SM
-sw_rt_kernel(SwArgs a, SwScratch s, int p0, int nc, const double* __restrict__ ET) {
+// exp_tbl of the upward kernel: SHT in shared memory, else gathered through L1
+template <bool SHT>
+struct RtTable;
+template <>
+struct RtTable<false> {
+  typedef TblGlobal type;
+  static __device__ __forceinline__ type get(const double* ET, double*) { return {ET}; }
+};
+template <>
+struct RtTable<true> {
+  typedef TblShared type;
+  static __device__ __forceinline__ type get(const double* ET, double* sm) {
+    for (int q = threadIdx.x; q <= kNtbmx; q += blockDim.x) sm[q] = ET[q];
+    __syncthreads();
+    return {(unsigned)__cvta_generic_to_shared(sm)};
+  }
+};
+template <bool SHT>
+__host__ __device__ constexpr size_t rt_table_doubles() { return SHT ? kNtbmx + 1 : 0; }
+
+// COLS columns at a time per CTA, which walks the chunk
+template <bool GRID, int COLS, bool SHT>
+__global__ void __launch_bounds__(COLS* kSwNg, kRtPerSm / COLS)
+sw_up_kernel(SwArgs a, SwScratch s, int p0, int nc, const double* __restrict__ T, const double* __restrict__ ET) {
   extern __shared__ double sm[];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int pl = blockIdx.x * kRtWarps + w;
-  if (pl >= nc) return;
-  const int j1 = a.idxday[p0 + pl];
-  if (j1 < 1 || j1 > a.npts) return;   // reported by the optics kernel
-  rt_body<GRID>(a, s, pl, nc, j1, lane, sm + (size_t)w * rt_warp_doubles(a.nlay, a.hswb != nullptr), ET);
+  const auto tbl = RtTable<SHT>::get(ET, sm);
+  const int h = threadIdx.x / kSwNg, g = threadIdx.x - h * kSwNg;
+  for (int pl = blockIdx.x * COLS + h; pl < nc; pl += gridDim.x * COLS) {
+    const int j1 = a.idxday[p0 + pl];
+    if (j1 < 1 || j1 > a.npts) continue;   // reported by the optics kernel
+    up_body<GRID>(a, s, pl, nc, j1, g, T, tbl);
+  }
 }
 
-template <bool GRID>
-__global__ void __launch_bounds__(32 * kRtWarps, 4)
-sw_rt_blocks_kernel(const SwArgs* __restrict__ tab, const int2* __restrict__ pts, bool want_b, SwScratch s, int p0,
-                    int nc, int nlay, const double* __restrict__ ET) {
+template <bool GRID, int COLS, bool SHT>
+__global__ void __launch_bounds__(COLS* kSwNg, kRtPerSm / COLS)
+sw_up_blocks_kernel(const SwArgs* __restrict__ tab, const int2* __restrict__ pts, SwScratch s, int p0, int nc,
+                    const double* __restrict__ T, const double* __restrict__ ET) {
   extern __shared__ double sm[];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int pl = blockIdx.x * kRtWarps + w;
-  if (pl >= nc) return;
-  const int2 q = pts[p0 + pl];
-  rt_body<GRID>(tab[q.x], s, pl, nc, q.y, lane, sm + (size_t)w * rt_warp_doubles(nlay, want_b), ET);
+  const auto tbl = RtTable<SHT>::get(ET, sm);
+  const int h = threadIdx.x / kSwNg, g = threadIdx.x - h * kSwNg;
+  for (int pl = blockIdx.x * COLS + h; pl < nc; pl += gridDim.x * COLS) {
+    const int2 q = pts[p0 + pl];
+    up_body<GRID>(tab[q.x], s, pl, nc, q.y, g, T, tbl);
+  }
+}
+
+// a column per CTA
+template <bool GRID, bool BANDS>
+__global__ void __launch_bounds__(kSwNg, BANDS ? 2 : kDownPerSm)
+sw_down_kernel(SwArgs a, SwScratch s, int p0, int nc, const double* __restrict__ T) {
+  extern __shared__ double sm[];
+  const int j1 = a.idxday[p0 + blockIdx.x];
+  if (j1 < 1 || j1 > a.npts) return;
+  down_body<GRID, BANDS>(a, s, blockIdx.x, nc, j1, threadIdx.x, sm, T);
+}
+
+template <bool GRID, bool BANDS>
+__global__ void __launch_bounds__(kSwNg, BANDS ? 2 : kDownPerSm)
+sw_down_blocks_kernel(const SwArgs* __restrict__ tab, const int2* __restrict__ pts, SwScratch s, int p0, int nc,
+                      const double* __restrict__ T) {
+  extern __shared__ double sm[];
+  const int2 q = pts[p0 + blockIdx.x];
+  down_body<GRID, BANDS>(tab[q.x], s, blockIdx.x, nc, q.y, threadIdx.x, sm, T);
 }
 
 // Zeroes every output of every column of the physics blocks (RSM:824-845):
@@ -1098,6 +1400,12 @@ cudaError_t overlap_aux_launch(int ncols, int nlay, int ld, int iovr, const doub
   return cudaGetLastError();
 }
 
+cudaError_t gas_unpack_launch(const SwScratch& s, int nc, int nlay, const double* T, double* taug, double* taur,
+                              cudaStream_t st) {
+  sw_gas_unpack_kernel<<<1024, 256, 0, st>>>(s, nc, nlay, T, taug, taur);
+  return cudaGetLastError();
+}
+
 cudaError_t optics_launch(const SwArgs& a, const SwScratch& s, int p0, int nc, const double* T, cudaStream_t st) {
   if (nc <= 0) return cudaSuccess;
   const int grid = (nc + kOptWarps - 1) / kOptWarps;
@@ -1105,15 +1413,22 @@ cudaError_t optics_launch(const SwArgs& a, const SwScratch& s, int p0, int nc, c
   return cudaGetLastError();
 }
 
-size_t rt_smem_bytes(int nlay, bool hswb) { return (size_t)kRtWarps * rt_warp_doubles(nlay, hswb) * sizeof(double); }
+size_t down_smem(int nlay, bool hswb) { return rt_col_doubles(nlay, hswb) * sizeof(double); }
+constexpr size_t kUpSmem = rt_table_doubles<true>() * sizeof(double);
 
 cudaError_t rt_prepare(int max_smem) {
-  cudaError_t e = cudaFuncSetAttribute(sw_rt_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(sw_rt_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(sw_rt_blocks_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(sw_rt_blocks_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+  const void* up[] = {(const void*)sw_up_kernel<false, kRtPerSm, true>, (const void*)sw_up_kernel<true, kRtPerSm, true>,
+                      (const void*)sw_up_blocks_kernel<false, kRtPerSm, true>,
+                      (const void*)sw_up_blocks_kernel<true, kRtPerSm, true>};
+  const void* down[] = {(const void*)sw_down_kernel<false, false>,        (const void*)sw_down_kernel<true, false>,
+                        (const void*)sw_down_kernel<false, true>,         (const void*)sw_down_kernel<true, true>,
+                        (const void*)sw_down_blocks_kernel<false, false>, (const void*)sw_down_blocks_kernel<true, false>,
+                        (const void*)sw_down_blocks_kernel<false, true>,  (const void*)sw_down_blocks_kernel<true, true>};
+  cudaError_t e = cudaSuccess;
+  for (const void* f : up)
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUpSmem);
+  for (const void* f : down)
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
   return e;
 }
 
@@ -1134,21 +1449,37 @@ cudaError_t optics_blocks_launch(const SwArgs* tab, const int2* pts, const SwScr
 }
 
 cudaError_t rt_blocks_launch(const SwArgs* tab, const int2* pts, bool grid, bool want_b, const SwScratch& s, int p0,
-                             int nc, int nlay, const double* ET, cudaStream_t st) {
+                             int nc, int nlay, const double* T, const double* ET, cudaStream_t st) {
   if (nc <= 0) return cudaSuccess;
-  const int g = (nc + kRtWarps - 1) / kRtWarps;
-  const size_t smem = rt_smem_bytes(nlay, want_b);
-  if (grid) sw_rt_blocks_kernel<true><<<g, 32 * kRtWarps, smem, st>>>(tab, pts, want_b, s, p0, nc, nlay, ET);
-  else sw_rt_blocks_kernel<false><<<g, 32 * kRtWarps, smem, st>>>(tab, pts, want_b, s, p0, nc, nlay, ET);
+  // as many columns per CTA as an SM holds, exp_tbl in shared memory, once every SM gets such a CTA; below that a
+  // column per CTA, which spreads a small call over the SMs
+  if (nc >= s.num_sms * kRtPerSm) {
+    const auto up = grid ? sw_up_blocks_kernel<true, kRtPerSm, true> : sw_up_blocks_kernel<false, kRtPerSm, true>;
+    up<<<s.num_sms, kRtPerSm * kSwNg, kUpSmem, st>>>(tab, pts, s, p0, nc, T, ET);
+  } else {
+    const auto up = grid ? sw_up_blocks_kernel<true, 1, false> : sw_up_blocks_kernel<false, 1, false>;
+    up<<<nc, kSwNg, 0, st>>>(tab, pts, s, p0, nc, T, ET);
+  }
+  const auto down = want_b ? (grid ? sw_down_blocks_kernel<true, true> : sw_down_blocks_kernel<false, true>)
+                           : (grid ? sw_down_blocks_kernel<true, false> : sw_down_blocks_kernel<false, false>);
+  down<<<nc, kSwNg, down_smem(nlay, want_b), st>>>(tab, pts, s, p0, nc, T);
   return cudaGetLastError();
 }
 
-cudaError_t rt_launch(const SwArgs& a, const SwScratch& s, int p0, int nc, const double* ET, cudaStream_t st) {
+cudaError_t rt_launch(const SwArgs& a, const SwScratch& s, int p0, int nc, const double* T, const double* ET,
+                      cudaStream_t st) {
   if (nc <= 0) return cudaSuccess;
-  const int grid = (nc + kRtWarps - 1) / kRtWarps;
-  const size_t smem = rt_smem_bytes(a.nlay, a.hswb != nullptr);
-  if (a.isubcsw <= 0) sw_rt_kernel<true><<<grid, 32 * kRtWarps, smem, st>>>(a, s, p0, nc, ET);
-  else sw_rt_kernel<false><<<grid, 32 * kRtWarps, smem, st>>>(a, s, p0, nc, ET);
+  const bool want_b = a.hswb != nullptr, grid = a.isubcsw <= 0;
+  if (nc >= s.num_sms * kRtPerSm) {   // as in rt_blocks_launch
+    const auto up = grid ? sw_up_kernel<true, kRtPerSm, true> : sw_up_kernel<false, kRtPerSm, true>;
+    up<<<s.num_sms, kRtPerSm * kSwNg, kUpSmem, st>>>(a, s, p0, nc, T, ET);
+  } else {
+    const auto up = grid ? sw_up_kernel<true, 1, false> : sw_up_kernel<false, 1, false>;
+    up<<<nc, kSwNg, 0, st>>>(a, s, p0, nc, T, ET);
+  }
+  const auto down = want_b ? (grid ? sw_down_kernel<true, true> : sw_down_kernel<false, true>)
+                           : (grid ? sw_down_kernel<true, false> : sw_down_kernel<false, false>);
+  down<<<nc, kSwNg, down_smem(a.nlay, want_b), st>>>(a, s, p0, nc, T);
   return cudaGetLastError();
 }
 

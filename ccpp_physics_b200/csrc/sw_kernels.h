@@ -27,7 +27,9 @@ struct SwArgs {
 
 // per-chunk scratch (pl = column within the chunk, k = internal layer)
 struct SwScratch {
-  double *taug, *taur;               // [pl][k][112]
+  double* taug;                      // gas optical depths, tg_offset(nlay, pl, k, g)
+  double* colmol;                    // [pl][k] total molecules (Rayleigh)
+  double* ray24;                     // [pl][k][8] band 24's Rayleigh optical depths
   double* sflux;                     // [pl][112]
   double *taucw, *ssacw, *asycw;     // [pl][k][14]
   double* cldf;                      // [pl + nc*k], floored cloud fraction (McICA input)
@@ -35,19 +37,42 @@ struct SwScratch {
   int32_t* seed;                     // [pl]
   double *zcf1, *zcf0;               // [pl] cloudy / clear column fractions (RSM:1101-1125)
   uint32_t* bits;                    // [pl][112][nw] McICA cloudy flags
-  double* lane_store;                // [pl][k][10][32] the transfer's per-lane layer optics and recurrences
+  double* rt_store;                  // [pl][k][kRtVals][112] the transfer's layer optics and recurrences
+  int num_sms;
   int nw;
   int* bad;                          // set when idxday names a column outside 1..npts
 };
 
-__host__ __device__ inline size_t rt_warp_doubles(int nlay, bool hswb) { return (size_t)(hswb ? 32 : 4) * (nlay + 1); }
+// taug: four layers of a g-point are one 32-byte sector, so the optics
+// kernel (thread = layer) writes and the transfer kernel (thread = g-point)
+// reads whole sectors
+constexpr int kTgStride = 4;   // between g-points of a layer
+__host__ __device__ inline size_t tg_doubles(int nlay) { return (size_t)((nlay + 3) / 4) * kSwNg * kTgStride; }
+__host__ __device__ inline size_t tg_offset(int nlay, size_t pl, int k, int g) {
+  return pl * tg_doubles(nlay) + ((size_t)(k >> 2) * kSwNg + g) * kTgStride + (k & 3);
+}
+
+// transfer kernels: 112 threads per column; kRtPerSm columns per SM on the way
+// up, kDownPerSm on the way down
+constexpr int kRtPerSm = 4, kDownPerSm = 6;
+constexpr int kRtGroups = kSwNg / 16;       // 16-lane groups of a column
+constexpr int kRtVals = 14;                 // stored values per layer and g-point
+constexpr int kRtBandSlots = 14 + kRtGroups - 1;   // (band, group) pairs: slot band + group
+__host__ __device__ inline size_t rt_col_store(int nlay) { return (size_t)(nlay + 1) * kRtVals * kSwNg; }
+// shared memory of one column: the groups' partial flux sums
+__host__ __device__ inline size_t rt_col_doubles(int nlay, bool hswb) {
+  return (size_t)(4 * kRtGroups + (hswb ? 2 * kRtBandSlots : 0)) * (nlay + 1) + 10 * kRtGroups;
+}
 
 cudaError_t overlap_aux_launch(int ncols, int nlay, int ld, int iovr, const double* dz, const double* delg,
                                const double* alpha, double* aux, int ldo, cudaStream_t st);
 cudaError_t optics_launch(const SwArgs& a, const SwScratch& s, int p0, int nc, const double* T, cudaStream_t st);
 cudaError_t rt_prepare(int max_smem);
-size_t rt_smem_bytes(int nlay, bool hswb);
-cudaError_t rt_launch(const SwArgs& a, const SwScratch& s, int p0, int nc, const double* ET, cudaStream_t st);
+cudaError_t rt_launch(const SwArgs& a, const SwScratch& s, int p0, int nc, const double* T, const double* ET,
+                      cudaStream_t st);
+// taug / taur of the chunk's columns as [column][layer][112] (stage entry point)
+cudaError_t gas_unpack_launch(const SwScratch& s, int nc, int nlay, const double* T, double* taug, double* taur,
+                              cudaStream_t st);
 // physics blocks in one call: tab[b] = block b's record (device), colpre[b] / dayp[b]
 // = columns / daytime points before block b (dayp has nb + 1 entries)
 cudaError_t blocks_prepare(const SwArgs* tab, const int* colpre, const int* dayp, int nb, int total_cols,
@@ -55,6 +80,6 @@ cudaError_t blocks_prepare(const SwArgs* tab, const int* colpre, const int* dayp
 cudaError_t optics_blocks_launch(const SwArgs* tab, const int2* pts, const SwScratch& s, int p0, int nc,
                                  const double* T, cudaStream_t st);
 cudaError_t rt_blocks_launch(const SwArgs* tab, const int2* pts, bool grid, bool want_b, const SwScratch& s, int p0,
-                             int nc, int nlay, const double* ET, cudaStream_t st);
+                             int nc, int nlay, const double* T, const double* ET, cudaStream_t st);
 
 }  // namespace sw
