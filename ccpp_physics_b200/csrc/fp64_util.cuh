@@ -1,0 +1,90 @@
+// fp64_util.cuh -- FP64 helpers of the transfer kernels (lw_rt64.cuh,
+// sw_column.cu): quotients without the IEEE slow path, table indices that
+// equal the reference's, sums over lanes.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace fp64 {
+
+// Quotients and roots from the hardware estimate (2^-20) and Newton's
+// iteration, for operands that are normal numbers far from the ends of the
+// range: no range check and no slow path, about two thirds of the instructions
+// of the compiled IEEE operations.  recip_newton is 1/x to about 2^-52;
+// div_markstein and sqrt_markstein add Markstein's residual step (IBM J. Res.
+// Dev. 34, 1990), which rounds correctly but for a reciprocal whose own last
+// bit was misrounded.
+__device__ __forceinline__ double recip_newton(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+__device__ __forceinline__ double div_markstein(double a, double b) {
+  const double y = recip_newton(b), q = a * y;
+  return fma(fma(-b, q, a), y, q);
+}
+__device__ __forceinline__ double sqrt_markstein(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(0.5 * y, fma(-x * y, y, 1.0), y);
+  y = fma(0.5 * y, fma(-x * y, y, 1.0), y);
+  const double r = x * y;
+  return fma(fma(-r, r, x), 0.5 * y, r);
+}
+// int(z / (bpade + z) * 10000 + 0.5) for z > 0 (RSM:3601-3602, RLM:3602-3614),
+// the index of the 10,001-entry transmittance tables.  The quotient comes from
+// one Newton step (error below 1e-8 in index units) and is rounded by adding
+// 1.5 2^52; only a value within 1e-6 of a tie takes the IEEE division, so the
+// entry is the reference's in every case.
+__device__ __forceinline__ int pade_index(double z) {
+  constexpr double kBpade = 1.0 / 0.278, kRound = 6755399441055744.0;
+  const double d = kBpade + z;
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  y = fma(y, fma(-d, y, 1.0), y);
+  const double q = z * y, t = fma(q, 10000.0, kRound);
+  int i = __double2loint(t);
+  const double f = fma(q, 10000.0, kRound - t);
+  if (!(fabs(f) < 0.5 - 1.0e-6)) i = (int)(z / d * 10000 + 0.5);
+  return i;
+}
+
+// read-once inputs: no L1 line, which stays with exp_tbl
+__device__ __forceinline__ double2 ld_once2(const double* p) {
+  double2 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+
+// Sums of N values (a power of two) over the L lanes (16 or 32) of a group:
+// each step exchanges half of the values with the partner lane, so N values
+// take N - 1 + log2(L / N) exchanges instead of N log2(L).  Lane j of the group
+// ends with the sum of value sum_index<N, L>(j).
+template <int N, int L>
+__device__ __forceinline__ double lane_sums(double (&v)[N], int lane, unsigned mask) {
+  int o = L / 2;
+#pragma unroll
+  for (int n = N / 2; n >= 1; n >>= 1, o >>= 1) {
+    const bool hi = (lane & o) != 0;
+#pragma unroll
+    for (int q = 0; q < n; ++q) {
+      const double keep = hi ? v[q + n] : v[q], send = hi ? v[q] : v[q + n];
+      v[q] = keep + __shfl_xor_sync(mask, send, o);
+    }
+  }
+  double r = v[0];
+#pragma unroll
+  for (; o >= 1; o >>= 1) r += __shfl_xor_sync(mask, r, o);
+  return r;
+}
+// the value whose sum lane j of the group holds, -1 where another lane has it too
+template <int N, int L>
+__device__ __forceinline__ int sum_index(int lane) {
+  int idx = 0, o = L / 2;
+#pragma unroll
+  for (int n = N / 2; n >= 1; n >>= 1, o >>= 1)
+    if (lane & o) idx += n;
+  return (lane & (2 * o - 1)) ? -1 : idx;
+}
+
+}  // namespace fp64

@@ -38,7 +38,7 @@ struct DeviceState {
   int num_sms = 0;
   double* kt64 = nullptr;
   float* kt32 = nullptr;
-  double* tbl64 = nullptr;   // records {exp, tfn, tau, 0} (4 x (NTBL+1))
+  double* tbl64 = nullptr;   // rlwinit tables (lw_common.cuh, Tables)
   float* tbl32 = nullptr;
   Consts cs{};
   bool sgpath = false;       // the learned-gas-optics column path (lw_sg_path.cu) is usable on this device
@@ -205,14 +205,17 @@ extern "C" int rrtmg_lw_gpu_init(const rrtmg_lw_init_args* a, char* errmsg, int3
     ex[i] = (ta[i] >= explimit) ? expeps : std::exp(-ta[i]);
     tf[i] = (ta[i] < 0.06) ? ta[i] / 6.0 : 1.0 - 2.0 * ((1.0 / ta[i]) - (ex[i] / (1.0 - ex[i])));
   }
-  // interleave: record i = {exp_tbl(i), tfn_tbl(i), tau_tbl(i), 0}
-  std::vector<double> rec(4 * (NTBL + 1), 0.0);
+  // interleaved for the kernels (lw_common.cuh, Tables)
+  std::vector<double> rec(3 * (NTBL + 1));
+  std::vector<float> rec32(4 * (NTBL + 1), 0.0f);
   for (int i = 0; i <= NTBL; ++i) {
-    rec[4 * i + 0] = ex[i];
-    rec[4 * i + 1] = tf[i];
-    rec[4 * i + 2] = ta[i];
+    rec[2 * i + 0] = ex[i];
+    rec[2 * i + 1] = tf[i];
+    rec[2 * (NTBL + 1) + i] = ta[i];
+    rec32[4 * i + 0] = (float)ex[i];
+    rec32[4 * i + 1] = (float)tf[i];
+    rec32[4 * i + 2] = (float)ta[i];
   }
-  std::vector<float> rec32(rec.begin(), rec.end());
 
   size_t nblob = (size_t)(rrtmg_lw_tables_blob_end - rrtmg_lw_tables_blob);
   if (nblob != sizeof(double) * RRTMG_LW_TABLES_NDOUBLE) {

@@ -11,25 +11,14 @@
 
 #include "lw_common.cuh"
 
-// Unrolling of the per-band g-point loops.  Full unrolling makes every table
-// gather a constant offset from a per-layer row pointer, but the sixteen
-// unrolled bands overflow the instruction cache: measured on B200 (16,384
-// columns x 127 layers) the rolled loops run the FP32 gas-optics kernel 25%
-// faster (6.4 -> 4.8 ms) and the FP64 one 3% faster, with identical results.
-#ifndef LW_GLOOP_FULL
-#define LW_GLOOP_FULL 0
-#endif
-#ifndef LW_GLOOP_N
-#define LW_GLOOP_N 1
-#endif
-#define LW_PRAGMA_(x) _Pragma(#x)
-#define LW_PRAGMA(x) LW_PRAGMA_(x)
-#if LW_GLOOP_FULL
-#define LW_GLOOP _Pragma("unroll")
-#else
-#define LW_GLOOP LW_PRAGMA(unroll LW_GLOOP_N)
-#endif
-
+// The g loop takes two g-points at a time: every band has an even number of
+// them and every table starts at a multiple of eight values, so a pair is one
+// 16-byte (FP64) or 8-byte (FP32) gather.  A lane's gathers touch a row of
+// their own, so a warp's load costs a wavefront per row whatever its width:
+// pairs halve them: 16,384 x
+// 127, FP64 7.87 -> 5.05 ms (with the sector hand-off of lw_rt64.cuh; one
+// value at a time in rows of layers it took 5.47), FP32 3.93 -> 3.65 ms.
+// Unrolled further, the sixteen bands overflow the instruction cache.
 namespace lw {
 
 // Per-layer state produced by setcoef (RLM:2151-2406) and the driver
@@ -88,27 +77,53 @@ struct LayRef {
   }
 };
 
+// The values of two consecutive g-points, with element-wise arithmetic.
+template <typename R>
+struct G2 {
+  R x, y;
+};
+template <typename R> __device__ __forceinline__ G2<R> operator+(G2<R> a, G2<R> b) { return {a.x + b.x, a.y + b.y}; }
+template <typename R> __device__ __forceinline__ G2<R> operator-(G2<R> a, G2<R> b) { return {a.x - b.x, a.y - b.y}; }
+template <typename R> __device__ __forceinline__ G2<R> operator*(R a, G2<R> b) { return {a * b.x, a * b.y}; }
+template <typename R> __device__ __forceinline__ G2<R> operator*(G2<R> a, R b) { return {a.x * b, a.y * b}; }
+// products that no addition is contracted into
+__device__ __forceinline__ G2<double> mul_rn(G2<double> a, double b, double c) { return {__dmul_rn(a.x, b), __dmul_rn(a.y, c)}; }
+__device__ __forceinline__ G2<float> mul_rn(G2<float> a, float b, float c) { return {__fmul_rn(a.x, b), __fmul_rn(a.y, c)}; }
+__device__ __forceinline__ G2<double> ldg2(const double* p) {
+  const double2 v = __ldg(reinterpret_cast<const double2*>(p));
+  return {v.x, v.y};
+}
+__device__ __forceinline__ G2<float> ldg2(const float* p) {
+  const float2 v = __ldg(reinterpret_cast<const float2*>(p));
+  return {v.x, v.y};
+}
+
 template <typename R>
 struct KT {
   const R* __restrict__ p;
-  // Fortran-order accessors, 1-based indices
-  __device__ __forceinline__ R at(long long o) const {
+  // Fortran-order accessors, 1-based indices: elements i and i + 1 (i odd) of
+  // the leading dimension n1 (even)
+  __device__ __forceinline__ G2<R> at(long long o) const {
+    if (!LW_OK(o >= 0 && o + 1 < RRTMG_LW_TABLES_NDOUBLE && (o & 1) == 0, 1, o)) return {R(0), R(0)};
+    return ldg2(p + o);
+  }
+  __device__ __forceinline__ G2<R> a1(int off, int i) const { return at(off + (i - 1)); }
+  __device__ __forceinline__ G2<R> a2(int off, int n1, int i, int j) const {
+    return at(off + (i - 1) + n1 * (j - 1));
+  }
+  __device__ __forceinline__ G2<R> a3(int off, int n1, int n2, int i, int j, int k) const {
+    return at(off + (i - 1) + n1 * ((j - 1) + n2 * (k - 1)));
+  }
+  __device__ __forceinline__ R chi(int m, int j) const {
+    const long long o = lwtab::chi_mls + (m - 1) + 7 * (j - 1);
     if (!LW_OK(o >= 0 && o < RRTMG_LW_TABLES_NDOUBLE, 1, o)) return R(0);
     return ldg(p + o);
   }
-  __device__ __forceinline__ R a1(int off, int i) const { return at(off + (i - 1)); }
-  __device__ __forceinline__ R a2(int off, int n1, int i, int j) const {
-    return at(off + (i - 1) + n1 * (j - 1));
-  }
-  __device__ __forceinline__ R a3(int off, int n1, int n2, int i, int j, int k) const {
-    return at(off + (i - 1) + n1 * ((j - 1) + n2 * (k - 1)));
-  }
-  __device__ __forceinline__ R chi(int m, int j) const { return a2(lwtab::chi_mls, 7, m, j); }
 };
 
 template <typename R> __device__ __forceinline__ R one() { return R(1); }
 template <typename R> __device__ __forceinline__ R oneminus() { return R(1) - R(1.0e-6); }
-template <typename R> __device__ __forceinline__ R lerp(R a, R f, R b) { return a + f * (b - a); }
+template <typename R> __device__ __forceinline__ G2<R> lerp(G2<R> a, R f, G2<R> b) { return a + f * (b - a); }
 template <typename R> __device__ __forceinline__ R fracpart(R x) { return x - trunc(x); }  // mod(x,1), x>=0
 
 // binary-species parameter of a pair of key gases
@@ -154,7 +169,7 @@ __device__ __forceinline__ Maj6<R> major_setup(R specparm, R fs, int ind, R facA
   return m;
 }
 template <typename R>
-__device__ __forceinline__ R major6(const KT<R>& t, int off, int ng, int ig, const Maj6<R>& m) {
+__device__ __forceinline__ G2<R> major6(const KT<R>& t, int off, int ng, int ig, const Maj6<R>& m) {
   return m.w0 * t.a2(off, ng, ig, m.i0) + m.w1 * t.a2(off, ng, ig, m.i1) +
          m.w2 * t.a2(off, ng, ig, m.i2) + m.w3 * t.a2(off, ng, ig, m.i3) +
          m.w4 * t.a2(off, ng, ig, m.i4) + m.w5 * t.a2(off, ng, ig, m.i5);
@@ -175,7 +190,7 @@ __device__ __forceinline__ Low<R> low_setup(const Lay<R>& L, R a, R r0, R r1, R 
   return o;
 }
 template <typename R>
-__device__ __forceinline__ R low_major(const KT<R>& t, int off, int ng, int ig, const Low<R>& o) {
+__device__ __forceinline__ G2<R> low_major(const KT<R>& t, int off, int ng, int ig, const Low<R>& o) {
   return o.s0.comb * major6(t, off, ng, ig, o.m0) + o.s1.comb * major6(t, off, ng, ig, o.m1);
 }
 
@@ -197,17 +212,17 @@ __device__ __forceinline__ Up<R> up_setup(const Lay<R>& L, R a, R r0, R r1, R b)
   return u;
 }
 template <typename R>
-__device__ __forceinline__ R up_major(const KT<R>& t, int off, int ng, int ig, const Up<R>& u) {
-  R a = u.f000 * t.a2(off, ng, ig, u.ind0) + u.f010 * t.a2(off, ng, ig, u.ind0 + 5) +
+__device__ __forceinline__ G2<R> up_major(const KT<R>& t, int off, int ng, int ig, const Up<R>& u) {
+  const G2<R> a = u.f000 * t.a2(off, ng, ig, u.ind0) + u.f010 * t.a2(off, ng, ig, u.ind0 + 5) +
         u.f100 * t.a2(off, ng, ig, u.ind0 + 1) + u.f110 * t.a2(off, ng, ig, u.ind0 + 6);
-  R b = u.f001 * t.a2(off, ng, ig, u.ind1) + u.f011 * t.a2(off, ng, ig, u.ind1 + 5) +
+  const G2<R> b = u.f001 * t.a2(off, ng, ig, u.ind1) + u.f011 * t.a2(off, ng, ig, u.ind1 + 5) +
         u.f101 * t.a2(off, ng, ig, u.ind1 + 1) + u.f111 * t.a2(off, ng, ig, u.ind1 + 6);
   return u.comb0 * a + u.comb1 * b;
 }
 
 // single-key-species 4-point interpolation
 template <typename R>
-__device__ __forceinline__ R absk(const KT<R>& t, int off, int ng, int ig, const Lay<R>& L, int ind0, int ind1) {
+__device__ __forceinline__ G2<R> absk(const KT<R>& t, int off, int ng, int ig, const Lay<R>& L, int ind0, int ind1) {
   return L.fac00 * t.a2(off, ng, ig, ind0) + L.fac10 * t.a2(off, ng, ig, ind0 + 1) +
          L.fac01 * t.a2(off, ng, ig, ind1) + L.fac11 * t.a2(off, ng, ig, ind1 + 1);
 }
@@ -217,26 +232,26 @@ template <typename R, int B> __device__ __forceinline__ int up0(const Lay<R>& L)
 template <typename R, int B> __device__ __forceinline__ int up1(const Lay<R>& L) { return ((L.jp - 12) * 5 + (L.jt1 - 1)) * nspb_of(B) + 1; }
 
 template <typename R>
-__device__ __forceinline__ R selfc(const KT<R>& t, int off, int ng, int ig, const Lay<R>& L) {
+__device__ __forceinline__ G2<R> selfc(const KT<R>& t, int off, int ng, int ig, const Lay<R>& L) {
   return L.selffac * lerp(t.a2(off, ng, ig, L.indself), L.selffrac, t.a2(off, ng, ig, L.indself + 1));
 }
 template <typename R>
-__device__ __forceinline__ R forc(const KT<R>& t, int off, int ng, int ig, const Lay<R>& L) {
+__device__ __forceinline__ G2<R> forc(const KT<R>& t, int off, int ng, int ig, const Lay<R>& L) {
   return L.forfac * lerp(t.a2(off, ng, ig, L.indfor), L.forfrac, t.a2(off, ng, ig, L.indfor + 1));
 }
 template <typename R>
-__device__ __forceinline__ R minor2(const KT<R>& t, int off, int ng, int ig, const Lay<R>& L) {
+__device__ __forceinline__ G2<R> minor2(const KT<R>& t, int off, int ng, int ig, const Lay<R>& L) {
   return lerp(t.a2(off, ng, ig, L.indminor), L.minorfrac, t.a2(off, ng, ig, L.indminor + 1));
 }
 template <typename R>
-__device__ __forceinline__ R minor3(const KT<R>& t, int off, int ng, int nj, int ig, int j, R f, const Lay<R>& L) {
+__device__ __forceinline__ G2<R> minor3(const KT<R>& t, int off, int ng, int nj, int ig, int j, R f, const Lay<R>& L) {
   int m = L.indminor;
-  R m1 = t.a3(off, ng, nj, ig, j, m) + f * (t.a3(off, ng, nj, ig, j + 1, m) - t.a3(off, ng, nj, ig, j, m));
-  R m2 = t.a3(off, ng, nj, ig, j, m + 1) + f * (t.a3(off, ng, nj, ig, j + 1, m + 1) - t.a3(off, ng, nj, ig, j, m + 1));
+  const G2<R> m1 = t.a3(off, ng, nj, ig, j, m) + f * (t.a3(off, ng, nj, ig, j + 1, m) - t.a3(off, ng, nj, ig, j, m));
+  const G2<R> m2 = t.a3(off, ng, nj, ig, j, m + 1) + f * (t.a3(off, ng, nj, ig, j + 1, m + 1) - t.a3(off, ng, nj, ig, j, m + 1));
   return m1 + L.minorfrac * (m2 - m1);
 }
 template <typename R>
-__device__ __forceinline__ R planck(const KT<R>& t, int off, int ng, int ig, int jpl, R fpl) {
+__device__ __forceinline__ G2<R> planck(const KT<R>& t, int off, int ng, int ig, int jpl, R fpl) {
   return lerp(t.a2(off, ng, ig, jpl), fpl, t.a2(off, ng, ig, jpl + 1));
 }
 // minor-gas column adjusted above `thresh` times its reference amount
@@ -248,7 +263,8 @@ __device__ __forceinline__ R adjcol(R col, R ref, R thresh, R base, R expo) {
 }
 
 // ---------------------------------------------------------------------------
-// Each band: for g-points ig = 1..ng call emit(ig-1, taug, fracs).
+// Each band: for g-points ig = 1, 3, .. ng - 1 call emit(ig - 1, taug, fracs)
+// with the values of ig and ig + 1.
 // ---------------------------------------------------------------------------
 
 template <typename R, typename E>  // taugb01, RLM:4023-4125
@@ -260,21 +276,21 @@ __device__ void taugb01(const KT<R>& t, const LayRef<R>& LR, E emit) {
     int i0 = lo0<R, 0>(L), i1 = lo1<R, 0>(L);
     R pp = L.pavel;
     R corradj = (pp < R(250)) ? one<R>() - R(0.15) * (R(250) - pp) / R(154.4) : one<R>();
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R tauself = selfc(t, lwtab::b01_selfref, ng, ig, L);
-      R taufor = forc(t, lwtab::b01_forref, ng, ig, L);
-      R taun2 = scalen2 * minor2(t, lwtab::b01_ka_mn2, ng, ig, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> tauself = selfc(t, lwtab::b01_selfref, ng, ig, L);
+      const G2<R> taufor = forc(t, lwtab::b01_forref, ng, ig, L);
+      const G2<R> taun2 = scalen2 * minor2(t, lwtab::b01_ka_mn2, ng, ig, L);
       emit(ig - 1, corradj * (L.col[0] * absk(t, lwtab::b01_absa, ng, ig, L, i0, i1) + tauself + taufor + taun2),
            t.a1(lwtab::b01_fracrefa, ig));
     }
   } else {
     int i0 = up0<R, 0>(L), i1 = up1<R, 0>(L);
     R corradj = one<R>() - R(0.15) * (L.pavel / R(95.6));
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R taufor = forc(t, lwtab::b01_forref, ng, ig, L);
-      R taun2 = scalen2 * minor2(t, lwtab::b01_kb_mn2, ng, ig, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> taufor = forc(t, lwtab::b01_forref, ng, ig, L);
+      const G2<R> taun2 = scalen2 * minor2(t, lwtab::b01_kb_mn2, ng, ig, L);
       emit(ig - 1, corradj * (L.col[0] * absk(t, lwtab::b01_absb, ng, ig, L, i0, i1) + taufor + taun2),
            t.a1(lwtab::b01_fracrefb, ig));
     }
@@ -288,18 +304,18 @@ __device__ void taugb02(const KT<R>& t, const LayRef<R>& LR, E emit) {
   if (L.lower) {
     int i0 = lo0<R, 1>(L), i1 = lo1<R, 1>(L);
     R corradj = one<R>() - R(0.05) * (L.pavel - R(100)) / R(900);
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R tauself = selfc(t, lwtab::b02_selfref, ng, ig, L);
-      R taufor = forc(t, lwtab::b02_forref, ng, ig, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> tauself = selfc(t, lwtab::b02_selfref, ng, ig, L);
+      const G2<R> taufor = forc(t, lwtab::b02_forref, ng, ig, L);
       emit(ig - 1, corradj * (L.col[0] * absk(t, lwtab::b02_absa, ng, ig, L, i0, i1) + tauself + taufor),
            t.a1(lwtab::b02_fracrefa, ig));
     }
   } else {
     int i0 = up0<R, 1>(L), i1 = up1<R, 1>(L);
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R taufor = forc(t, lwtab::b02_forref, ng, ig, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> taufor = forc(t, lwtab::b02_forref, ng, ig, L);
       emit(ig - 1, L.col[0] * absk(t, lwtab::b02_absb, ng, ig, L, i0, i1) + taufor, t.a1(lwtab::b02_fracrefb, ig));
     }
   }
@@ -315,13 +331,13 @@ __device__ void taugb03(const KT<R>& t, const LayRef<R>& LR, E emit) {
     Low<R> o = low_setup<R, 2>(L, L.col[0], t.chi(1, L.jp) / t.chi(2, L.jp), t.chi(1, L.jp + 1) / t.chi(2, L.jp + 1), L.col[1]);
     Spec<R> sm = spec<R>(L.col[0], rma, L.col[1], R(8));
     Spec<R> sp = spec<R>(L.col[0], rpa, L.col[1], R(8));
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R tauself = selfc(t, lwtab::b03_selfref, ng, ig, L);
-      R taufor = forc(t, lwtab::b03_forref, ng, ig, L);
-      R absn2o = minor3(t, lwtab::b03_ka_mn2o, ng, 9, ig, sm.js, sm.fs, L);
-      R tau_major = o.s0.comb * major6(t, lwtab::b03_absa, ng, ig, o.m0);
-      R tau_major1 = o.s1.comb * major6(t, lwtab::b03_absa, ng, ig, o.m1);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> tauself = selfc(t, lwtab::b03_selfref, ng, ig, L);
+      const G2<R> taufor = forc(t, lwtab::b03_forref, ng, ig, L);
+      const G2<R> absn2o = minor3(t, lwtab::b03_ka_mn2o, ng, 9, ig, sm.js, sm.fs, L);
+      const G2<R> tau_major = o.s0.comb * major6(t, lwtab::b03_absa, ng, ig, o.m0);
+      const G2<R> tau_major1 = o.s1.comb * major6(t, lwtab::b03_absa, ng, ig, o.m1);
       emit(ig - 1, tau_major + tau_major1 + tauself + taufor + adjcoln2o * absn2o,
            planck(t, lwtab::b03_fracrefa, ng, ig, sp.js, sp.fs));
     }
@@ -330,10 +346,10 @@ LW_GLOOP
     Up<R> u = up_setup<R, 2>(L, L.col[0], t.chi(1, L.jp) / t.chi(2, L.jp), t.chi(1, L.jp + 1) / t.chi(2, L.jp + 1), L.col[1]);
     Spec<R> sm = spec<R>(L.col[0], rmb, L.col[1], R(4));
     Spec<R> sp = spec<R>(L.col[0], rpb, L.col[1], R(4));
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R taufor = forc(t, lwtab::b03_forref, ng, ig, L);
-      R absn2o = minor3(t, lwtab::b03_kb_mn2o, ng, 5, ig, sm.js, sm.fs, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> taufor = forc(t, lwtab::b03_forref, ng, ig, L);
+      const G2<R> absn2o = minor3(t, lwtab::b03_kb_mn2o, ng, 5, ig, sm.js, sm.fs, L);
       emit(ig - 1, up_major(t, lwtab::b03_absb, ng, ig, u) + taufor + adjcoln2o * absn2o,
            planck(t, lwtab::b03_fracrefb, ng, ig, sp.js, sp.fs));
     }
@@ -348,12 +364,12 @@ __device__ void taugb04(const KT<R>& t, const LayRef<R>& LR, E emit) {
     R rpa = t.chi(1, 11) / t.chi(2, 11);
     Low<R> o = low_setup<R, 3>(L, L.col[0], t.chi(1, L.jp) / t.chi(2, L.jp), t.chi(1, L.jp + 1) / t.chi(2, L.jp + 1), L.col[1]);
     Spec<R> sp = spec<R>(L.col[0], rpa, L.col[1], R(8));
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R tauself = selfc(t, lwtab::b04_selfref, ng, ig, L);
-      R taufor = forc(t, lwtab::b04_forref, ng, ig, L);
-      R tau_major = o.s0.comb * major6(t, lwtab::b04_absa, ng, ig, o.m0);
-      R tau_major1 = o.s1.comb * major6(t, lwtab::b04_absa, ng, ig, o.m1);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> tauself = selfc(t, lwtab::b04_selfref, ng, ig, L);
+      const G2<R> taufor = forc(t, lwtab::b04_forref, ng, ig, L);
+      const G2<R> tau_major = o.s0.comb * major6(t, lwtab::b04_absa, ng, ig, o.m0);
+      const G2<R> tau_major1 = o.s1.comb * major6(t, lwtab::b04_absa, ng, ig, o.m1);
       emit(ig - 1, tau_major + tau_major1 + tauself + taufor, planck(t, lwtab::b04_fracrefa, ng, ig, sp.js, sp.fs));
     }
   } else {
@@ -362,10 +378,10 @@ LW_GLOOP
     Spec<R> sp = spec<R>(L.col[2], rpb, L.col[1], R(4));
     // empirical scalings of g-points 8..14 (RLM:4746-4752)
     const R sc[14] = {R(1), R(1), R(1), R(1), R(1), R(1), R(1), R(0.92), R(0.88), R(1.07), R(1.1), R(0.99), R(0.88), R(0.943)};
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R tau = up_major(t, lwtab::b04_absb, ng, ig, u);
-      if (ig >= 8) tau = tau * sc[ig - 1];
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      G2<R> tau = up_major(t, lwtab::b04_absb, ng, ig, u);
+      if (ig >= 7) tau = mul_rn(tau, sc[ig - 1], sc[ig]);
       emit(ig - 1, tau, planck(t, lwtab::b04_fracrefb, ng, ig, sp.js, sp.fs));
     }
   }
@@ -380,11 +396,11 @@ __device__ void taugb05(const KT<R>& t, const LayRef<R>& LR, E emit) {
     Low<R> o = low_setup<R, 4>(L, L.col[0], t.chi(1, L.jp) / t.chi(2, L.jp), t.chi(1, L.jp + 1) / t.chi(2, L.jp + 1), L.col[1]);
     Spec<R> sm = spec<R>(L.col[0], rma, L.col[1], R(8));
     Spec<R> sp = spec<R>(L.col[0], rpa, L.col[1], R(8));
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R tauself = selfc(t, lwtab::b05_selfref, ng, ig, L);
-      R taufor = forc(t, lwtab::b05_forref, ng, ig, L);
-      R abso3 = minor3(t, lwtab::b05_ka_mo3, ng, 9, ig, sm.js, sm.fs, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> tauself = selfc(t, lwtab::b05_selfref, ng, ig, L);
+      const G2<R> taufor = forc(t, lwtab::b05_forref, ng, ig, L);
+      const G2<R> abso3 = minor3(t, lwtab::b05_ka_mo3, ng, 9, ig, sm.js, sm.fs, L);
       emit(ig - 1, low_major(t, lwtab::b05_absa, ng, ig, o) + tauself + taufor + abso3 * L.col[2] +
                        L.wx[0] * t.a1(lwtab::b05_ccl4, ig),
            planck(t, lwtab::b05_fracrefa, ng, ig, sp.js, sp.fs));
@@ -393,8 +409,8 @@ LW_GLOOP
     R rpb = t.chi(3, 43) / t.chi(2, 43);
     Up<R> u = up_setup<R, 4>(L, L.col[2], t.chi(3, L.jp) / t.chi(2, L.jp), t.chi(3, L.jp + 1) / t.chi(2, L.jp + 1), L.col[1]);
     Spec<R> sp = spec<R>(L.col[2], rpb, L.col[1], R(4));
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig)
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2)
       emit(ig - 1, up_major(t, lwtab::b05_absb, ng, ig, u) + L.wx[0] * t.a1(lwtab::b05_ccl4, ig),
            planck(t, lwtab::b05_fracrefb, ng, ig, sp.js, sp.fs));
   }
@@ -407,18 +423,18 @@ __device__ void taugb06(const KT<R>& t, const LayRef<R>& LR, E emit) {
   if (L.lower) {
     int i0 = lo0<R, 5>(L), i1 = lo1<R, 5>(L);
     R adjcolco2 = adjcol<R>(L.col[1], L.coldry * t.chi(2, L.jp + 1), R(3), R(2), R(0.77));
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R tauself = selfc(t, lwtab::b06_selfref, ng, ig, L);
-      R taufor = forc(t, lwtab::b06_forref, ng, ig, L);
-      R absco2 = minor2(t, lwtab::b06_ka_mco2, ng, ig, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> tauself = selfc(t, lwtab::b06_selfref, ng, ig, L);
+      const G2<R> taufor = forc(t, lwtab::b06_forref, ng, ig, L);
+      const G2<R> absco2 = minor2(t, lwtab::b06_ka_mco2, ng, ig, L);
       emit(ig - 1, L.col[0] * absk(t, lwtab::b06_absa, ng, ig, L, i0, i1) + tauself + taufor + adjcolco2 * absco2 +
                        L.wx[1] * t.a1(lwtab::b06_cfc11adj, ig) + L.wx[2] * t.a1(lwtab::b06_cfc12, ig),
            t.a1(lwtab::b06_fracrefa, ig));
     }
   } else {
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig)
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2)
       emit(ig - 1, L.wx[1] * t.a1(lwtab::b06_cfc11adj, ig) + L.wx[2] * t.a1(lwtab::b06_cfc12, ig),
            t.a1(lwtab::b06_fracrefa, ig));
   }
@@ -434,11 +450,11 @@ __device__ void taugb07(const KT<R>& t, const LayRef<R>& LR, E emit) {
     Spec<R> sm = spec<R>(L.col[0], rma, L.col[2], R(8));
     Spec<R> sp = spec<R>(L.col[0], rpa, L.col[2], R(8));
     R adjcolco2 = adjcol<R>(L.col[1], L.coldry * t.chi(2, L.jp + 1), R(3), R(3), R(0.79));
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R tauself = selfc(t, lwtab::b07_selfref, ng, ig, L);
-      R taufor = forc(t, lwtab::b07_forref, ng, ig, L);
-      R absco2 = minor3(t, lwtab::b07_ka_mco2, ng, 9, ig, sm.js, sm.fs, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> tauself = selfc(t, lwtab::b07_selfref, ng, ig, L);
+      const G2<R> taufor = forc(t, lwtab::b07_forref, ng, ig, L);
+      const G2<R> absco2 = minor3(t, lwtab::b07_ka_mco2, ng, 9, ig, sm.js, sm.fs, L);
       emit(ig - 1, low_major(t, lwtab::b07_absa, ng, ig, o) + tauself + taufor + adjcolco2 * absco2,
            planck(t, lwtab::b07_fracrefa, ng, ig, sp.js, sp.fs));
     }
@@ -447,11 +463,11 @@ LW_GLOOP
     int i0 = up0<R, 6>(L), i1 = up1<R, 6>(L);
     // RLM:5366-5371
     const R sc[12] = {R(1), R(1), R(1), R(1), R(1), R(0.92), R(0.88), R(1.07), R(1.1), R(0.99), R(0.855), R(1)};
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R absco2 = minor2(t, lwtab::b07_kb_mco2, ng, ig, L);
-      R tau = L.col[2] * absk(t, lwtab::b07_absb, ng, ig, L, i0, i1) + adjcolco2 * absco2;
-      if (ig >= 6 && ig <= 11) tau = tau * sc[ig - 1];
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> absco2 = minor2(t, lwtab::b07_kb_mco2, ng, ig, L);
+      G2<R> tau = L.col[2] * absk(t, lwtab::b07_absb, ng, ig, L, i0, i1) + adjcolco2 * absco2;
+      if (ig >= 5) tau = mul_rn(tau, sc[ig - 1], sc[ig]);
       emit(ig - 1, tau, t.a1(lwtab::b07_fracrefb, ig));
     }
   }
@@ -464,13 +480,13 @@ __device__ void taugb08(const KT<R>& t, const LayRef<R>& LR, E emit) {
   R adjcolco2 = adjcol<R>(L.col[1], L.coldry * t.chi(2, L.jp + 1), R(3), R(2), R(0.65));
   if (L.lower) {
     int i0 = lo0<R, 7>(L), i1 = lo1<R, 7>(L);
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R tauself = selfc(t, lwtab::b08_selfref, ng, ig, L);
-      R taufor = forc(t, lwtab::b08_forref, ng, ig, L);
-      R absco2 = minor2(t, lwtab::b08_ka_mco2, ng, ig, L);
-      R abso3 = minor2(t, lwtab::b08_ka_mo3, ng, ig, L);
-      R absn2o = minor2(t, lwtab::b08_ka_mn2o, ng, ig, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> tauself = selfc(t, lwtab::b08_selfref, ng, ig, L);
+      const G2<R> taufor = forc(t, lwtab::b08_forref, ng, ig, L);
+      const G2<R> absco2 = minor2(t, lwtab::b08_ka_mco2, ng, ig, L);
+      const G2<R> abso3 = minor2(t, lwtab::b08_ka_mo3, ng, ig, L);
+      const G2<R> absn2o = minor2(t, lwtab::b08_ka_mn2o, ng, ig, L);
       emit(ig - 1, L.col[0] * absk(t, lwtab::b08_absa, ng, ig, L, i0, i1) + tauself + taufor + adjcolco2 * absco2 +
                        L.col[2] * abso3 + L.col[3] * absn2o + L.wx[2] * t.a1(lwtab::b08_cfc12, ig) +
                        L.wx[3] * t.a1(lwtab::b08_cfc22adj, ig),
@@ -478,10 +494,10 @@ LW_GLOOP
     }
   } else {
     int i0 = up0<R, 7>(L), i1 = up1<R, 7>(L);
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R absco2 = minor2(t, lwtab::b08_kb_mco2, ng, ig, L);
-      R absn2o = minor2(t, lwtab::b08_kb_mn2o, ng, ig, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> absco2 = minor2(t, lwtab::b08_kb_mco2, ng, ig, L);
+      const G2<R> absn2o = minor2(t, lwtab::b08_kb_mn2o, ng, ig, L);
       emit(ig - 1, L.col[2] * absk(t, lwtab::b08_absb, ng, ig, L, i0, i1) + adjcolco2 * absco2 + L.col[3] * absn2o +
                        L.wx[2] * t.a1(lwtab::b08_cfc12, ig) + L.wx[3] * t.a1(lwtab::b08_cfc22adj, ig),
            t.a1(lwtab::b08_fracrefb, ig));
@@ -499,19 +515,19 @@ __device__ void taugb09(const KT<R>& t, const LayRef<R>& LR, E emit) {
     Low<R> o = low_setup<R, 8>(L, L.col[0], t.chi(1, L.jp) / t.chi(6, L.jp), t.chi(1, L.jp + 1) / t.chi(6, L.jp + 1), L.col[4]);
     Spec<R> sm = spec<R>(L.col[0], rma, L.col[4], R(8));
     Spec<R> sp = spec<R>(L.col[0], rpa, L.col[4], R(8));
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R tauself = selfc(t, lwtab::b09_selfref, ng, ig, L);
-      R taufor = forc(t, lwtab::b09_forref, ng, ig, L);
-      R absn2o = minor3(t, lwtab::b09_ka_mn2o, ng, 9, ig, sm.js, sm.fs, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> tauself = selfc(t, lwtab::b09_selfref, ng, ig, L);
+      const G2<R> taufor = forc(t, lwtab::b09_forref, ng, ig, L);
+      const G2<R> absn2o = minor3(t, lwtab::b09_ka_mn2o, ng, 9, ig, sm.js, sm.fs, L);
       emit(ig - 1, low_major(t, lwtab::b09_absa, ng, ig, o) + tauself + taufor + adjcoln2o * absn2o,
            planck(t, lwtab::b09_fracrefa, ng, ig, sp.js, sp.fs));
     }
   } else {
     int i0 = up0<R, 8>(L), i1 = up1<R, 8>(L);
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R absn2o = minor2(t, lwtab::b09_kb_mn2o, ng, ig, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> absn2o = minor2(t, lwtab::b09_kb_mn2o, ng, ig, L);
       emit(ig - 1, L.col[4] * absk(t, lwtab::b09_absb, ng, ig, L, i0, i1) + adjcoln2o * absn2o,
            t.a1(lwtab::b09_fracrefb, ig));
     }
@@ -524,17 +540,17 @@ __device__ void taugb10(const KT<R>& t, const LayRef<R>& LR, E emit) {
   constexpr int ng = 6;
   if (L.lower) {
     int i0 = lo0<R, 9>(L), i1 = lo1<R, 9>(L);
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R tauself = selfc(t, lwtab::b10_selfref, ng, ig, L);
-      R taufor = forc(t, lwtab::b10_forref, ng, ig, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> tauself = selfc(t, lwtab::b10_selfref, ng, ig, L);
+      const G2<R> taufor = forc(t, lwtab::b10_forref, ng, ig, L);
       emit(ig - 1, L.col[0] * absk(t, lwtab::b10_absa, ng, ig, L, i0, i1) + tauself + taufor, t.a1(lwtab::b10_fracrefa, ig));
     }
   } else {
     int i0 = up0<R, 9>(L), i1 = up1<R, 9>(L);
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R taufor = forc(t, lwtab::b10_forref, ng, ig, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> taufor = forc(t, lwtab::b10_forref, ng, ig, L);
       emit(ig - 1, L.col[0] * absk(t, lwtab::b10_absb, ng, ig, L, i0, i1) + taufor, t.a1(lwtab::b10_fracrefb, ig));
     }
   }
@@ -547,20 +563,20 @@ __device__ void taugb11(const KT<R>& t, const LayRef<R>& LR, E emit) {
   R scaleo2 = L.col[5] * L.scaleminor;
   if (L.lower) {
     int i0 = lo0<R, 10>(L), i1 = lo1<R, 10>(L);
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R tauself = selfc(t, lwtab::b11_selfref, ng, ig, L);
-      R taufor = forc(t, lwtab::b11_forref, ng, ig, L);
-      R tauo2 = scaleo2 * minor2(t, lwtab::b11_ka_mo2, ng, ig, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> tauself = selfc(t, lwtab::b11_selfref, ng, ig, L);
+      const G2<R> taufor = forc(t, lwtab::b11_forref, ng, ig, L);
+      const G2<R> tauo2 = scaleo2 * minor2(t, lwtab::b11_ka_mo2, ng, ig, L);
       emit(ig - 1, L.col[0] * absk(t, lwtab::b11_absa, ng, ig, L, i0, i1) + tauself + taufor + tauo2,
            t.a1(lwtab::b11_fracrefa, ig));
     }
   } else {
     int i0 = up0<R, 10>(L), i1 = up1<R, 10>(L);
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R taufor = forc(t, lwtab::b11_forref, ng, ig, L);
-      R tauo2 = scaleo2 * minor2(t, lwtab::b11_kb_mo2, ng, ig, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> taufor = forc(t, lwtab::b11_forref, ng, ig, L);
+      const G2<R> tauo2 = scaleo2 * minor2(t, lwtab::b11_kb_mo2, ng, ig, L);
       emit(ig - 1, L.col[0] * absk(t, lwtab::b11_absb, ng, ig, L, i0, i1) + taufor + tauo2, t.a1(lwtab::b11_fracrefb, ig));
     }
   }
@@ -580,14 +596,14 @@ __device__ void taugb12(const KT<R>& t, const LayRef<R>& LR, E emit) {
     R mult = R(8) * parm;
     int jpl = min(8, max(1, 1 + (int)mult));
     R fpl = fracpart(mult);
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R tauself = selfc(t, lwtab::b12_selfref, ng, ig, L);
-      R taufor = forc(t, lwtab::b12_forref, ng, ig, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> tauself = selfc(t, lwtab::b12_selfref, ng, ig, L);
+      const G2<R> taufor = forc(t, lwtab::b12_forref, ng, ig, L);
       emit(ig - 1, low_major(t, lwtab::b12_absa, ng, ig, o) + tauself + taufor, planck(t, lwtab::b12_fracrefa, ng, ig, jpl, fpl));
     }
   } else {
-    for (int ig = 1; ig <= ng; ++ig) emit(ig - 1, R(0), R(0));
+    for (int ig = 1; ig <= ng; ig += 2) emit(ig - 1, G2<R>{R(0), R(0)}, G2<R>{R(0), R(0)});
   }
 }
 
@@ -602,18 +618,18 @@ __device__ void taugb13(const KT<R>& t, const LayRef<R>& LR, E emit) {
     Spec<R> smco = spec<R>(L.col[0], rma3, L.col[3], R(8));
     Spec<R> sp = spec<R>(L.col[0], rpa, L.col[3], R(8));
     R adjcolco2 = adjcol<R>(L.col[1], L.coldry * R(3.55e-4), R(3), R(2), R(0.68));
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig) {
-      R tauself = selfc(t, lwtab::b13_selfref, ng, ig, L);
-      R taufor = forc(t, lwtab::b13_forref, ng, ig, L);
-      R absco2 = minor3(t, lwtab::b13_ka_mco2, ng, 9, ig, smco2.js, smco2.fs, L);
-      R absco = minor3(t, lwtab::b13_ka_mco, ng, 9, ig, smco.js, smco.fs, L);
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> tauself = selfc(t, lwtab::b13_selfref, ng, ig, L);
+      const G2<R> taufor = forc(t, lwtab::b13_forref, ng, ig, L);
+      const G2<R> absco2 = minor3(t, lwtab::b13_ka_mco2, ng, 9, ig, smco2.js, smco2.fs, L);
+      const G2<R> absco = minor3(t, lwtab::b13_ka_mco, ng, 9, ig, smco.js, smco.fs, L);
       emit(ig - 1, low_major(t, lwtab::b13_absa, ng, ig, o) + tauself + taufor + adjcolco2 * absco2 + L.col[6] * absco,
            planck(t, lwtab::b13_fracrefa, ng, ig, sp.js, sp.fs));
     }
   } else {
-LW_GLOOP
-    for (int ig = 1; ig <= ng; ++ig)
+#pragma unroll 1
+    for (int ig = 1; ig <= ng; ig += 2)
       emit(ig - 1, L.col[2] * minor2(t, lwtab::b13_kb_mo3, ng, ig, L), t.a1(lwtab::b13_fracrefb, ig));
   }
 }
@@ -624,14 +640,14 @@ __device__ void taugb14(const KT<R>& t, const LayRef<R>& LR, E emit) {
   constexpr int ng = 2;
   if (L.lower) {
     int i0 = lo0<R, 13>(L), i1 = lo1<R, 13>(L);
-    for (int ig = 1; ig <= ng; ++ig) {
-      R tauself = selfc(t, lwtab::b14_selfref, ng, ig, L);
-      R taufor = forc(t, lwtab::b14_forref, ng, ig, L);
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> tauself = selfc(t, lwtab::b14_selfref, ng, ig, L);
+      const G2<R> taufor = forc(t, lwtab::b14_forref, ng, ig, L);
       emit(ig - 1, L.col[1] * absk(t, lwtab::b14_absa, ng, ig, L, i0, i1) + tauself + taufor, t.a1(lwtab::b14_fracrefa, ig));
     }
   } else {
     int i0 = up0<R, 13>(L), i1 = up1<R, 13>(L);
-    for (int ig = 1; ig <= ng; ++ig)
+    for (int ig = 1; ig <= ng; ig += 2)
       emit(ig - 1, L.col[1] * absk(t, lwtab::b14_absb, ng, ig, L, i0, i1), t.a1(lwtab::b14_fracrefb, ig));
   }
 }
@@ -646,15 +662,15 @@ __device__ void taugb15(const KT<R>& t, const LayRef<R>& LR, E emit) {
     Spec<R> sm = spec<R>(L.col[3], rma, L.col[1], R(8));
     Spec<R> sp = spec<R>(L.col[3], rpa, L.col[1], R(8));
     R scalen2 = L.colbrd * L.scaleminor;
-    for (int ig = 1; ig <= ng; ++ig) {
-      R tauself = selfc(t, lwtab::b15_selfref, ng, ig, L);
-      R taufor = forc(t, lwtab::b15_forref, ng, ig, L);
-      R taun2 = scalen2 * minor3(t, lwtab::b15_ka_mn2, ng, 9, ig, sm.js, sm.fs, L);
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> tauself = selfc(t, lwtab::b15_selfref, ng, ig, L);
+      const G2<R> taufor = forc(t, lwtab::b15_forref, ng, ig, L);
+      const G2<R> taun2 = scalen2 * minor3(t, lwtab::b15_ka_mn2, ng, 9, ig, sm.js, sm.fs, L);
       emit(ig - 1, low_major(t, lwtab::b15_absa, ng, ig, o) + tauself + taufor + taun2,
            planck(t, lwtab::b15_fracrefa, ng, ig, sp.js, sp.fs));
     }
   } else {
-    for (int ig = 1; ig <= ng; ++ig) emit(ig - 1, R(0), R(0));
+    for (int ig = 1; ig <= ng; ig += 2) emit(ig - 1, G2<R>{R(0), R(0)}, G2<R>{R(0), R(0)});
   }
 }
 
@@ -666,15 +682,15 @@ __device__ void taugb16(const KT<R>& t, const LayRef<R>& LR, E emit) {
     R rpa = t.chi(1, 6) / t.chi(6, 6);
     Low<R> o = low_setup<R, 15>(L, L.col[0], t.chi(1, L.jp) / t.chi(6, L.jp), t.chi(1, L.jp + 1) / t.chi(6, L.jp + 1), L.col[4]);
     Spec<R> sp = spec<R>(L.col[0], rpa, L.col[4], R(8));
-    for (int ig = 1; ig <= ng; ++ig) {
-      R tauself = selfc(t, lwtab::b16_selfref, ng, ig, L);
-      R taufor = forc(t, lwtab::b16_forref, ng, ig, L);
+    for (int ig = 1; ig <= ng; ig += 2) {
+      const G2<R> tauself = selfc(t, lwtab::b16_selfref, ng, ig, L);
+      const G2<R> taufor = forc(t, lwtab::b16_forref, ng, ig, L);
       emit(ig - 1, low_major(t, lwtab::b16_absa, ng, ig, o) + tauself + taufor, planck(t, lwtab::b16_fracrefa, ng, ig, sp.js, sp.fs));
     }
   } else {
     // nspb(16) = 0 (RLM:327): both indices are 1 for every upper layer
     int i0 = up0<R, 15>(L), i1 = up1<R, 15>(L);
-    for (int ig = 1; ig <= ng; ++ig)
+    for (int ig = 1; ig <= ng; ig += 2)
       emit(ig - 1, L.col[4] * absk(t, lwtab::b16_absb, ng, ig, L, i0, i1), t.a1(lwtab::b16_fracrefb, ig));
   }
 }

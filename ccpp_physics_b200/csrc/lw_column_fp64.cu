@@ -5,12 +5,10 @@
 
 #include <type_traits>
 
-// FP64 gas optics runs fastest with its g-point loops unrolled by two (B200,
-// 16,384 columns x 127 layers: 5.5 ms against 6.1 rolled and 6.3 fully unrolled).
-#define LW_GLOOP_N 2
 
 #include "lw_launch.h"
 #include "lw_rt.cuh"
+#include "lw_rt64.cuh"
 #include "lw_rt_grid.cuh"
 
 #define REAL double

@@ -348,8 +348,11 @@ __device__ __forceinline__ void gas_column(int cc, int t, const Sync& S, const G
     // ------------------------------ bands --------------------------------
     // taumol splits at the count laytrop (RLM:2344-2346)
     const LayRef<R> LR{s_lay, s_li, t, NLP, t < laytrop};
-    R* tcol = write_scratch ? sc.tau + (size_t)cc * NGPT * NLP + t : nullptr;
-    R* fcol = write_scratch ? sc.frac + (size_t)cc * NGPT * NLP + t : nullptr;
+    // tau, frac: [g][NLP], or four layers per g-point (lw_rt64.cuh)
+    const size_t hoff = (size_t)cc * NGPT * NLP + (sc.block4 ? (size_t)(t >> 2) * NGPT * 4 + (t & 3) : (size_t)t);
+    const int hstep = sc.block4 ? 4 : NLP;
+    R* tcol = write_scratch ? sc.tau + hoff : nullptr;
+    R* fcol = write_scratch ? sc.frac + hoff : nullptr;
     R* bcol = write_scratch ? sc.band + (size_t)cc * 3 * NBANDS * NLP : nullptr;
 #pragma unroll 1
     for (int b = 0; b < NBANDS; ++b) {
@@ -371,14 +374,18 @@ __device__ __forceinline__ void gas_column(int cc, int t, const Sync& S, const G
         if (!sg_skip && LW_OK(r < nlay && i < B.npts, 15, r)) tauaer = R(B.in[F_AERAOD][ab] * (1.0 - B.in[F_AERSSA][ab]));
         const int ns = ns_of(b);
         const size_t go = ((size_t)c * nlay + t) * NGPT + ns;
-        if (!sg_skip) band_gas_optics<R>(b, kt, LR, [&](int g0, R tau, R frac) {
-          if (tcol && LW_OK(cc < sc.cap && ns + g0 < NGPT, 16, ns + g0)) {
-            __stcs(tcol + (size_t)(ns + g0) * NLP, tau + tauaer);
-            __stcs(fcol + (size_t)(ns + g0) * NLP, frac);
+        if (!sg_skip) band_gas_optics<R>(b, kt, LR, [&](int g0, G2<R> tau, G2<R> frac) {
+          if (tcol && LW_OK(cc < sc.cap && ns + g0 + 1 < NGPT, 16, ns + g0)) {
+            __stcs(tcol + (size_t)(ns + g0) * hstep, tau.x + tauaer);
+            __stcs(tcol + (size_t)(ns + g0 + 1) * hstep, tau.y + tauaer);
+            __stcs(fcol + (size_t)(ns + g0) * hstep, frac.x);
+            __stcs(fcol + (size_t)(ns + g0 + 1) * hstep, frac.y);
           }
           if (f.gas_only && LW_OK(c < sc.ntot, 17, c)) {
-            gas_taug[go + g0] = (double)tau;
-            gas_fracs[go + g0] = (double)frac;
+            gas_taug[go + g0] = (double)tau.x;
+            gas_taug[go + g0 + 1] = (double)tau.y;
+            gas_fracs[go + g0] = (double)frac.x;
+            gas_fracs[go + g0 + 1] = (double)frac.y;
           }
         });
       }

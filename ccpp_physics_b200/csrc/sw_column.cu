@@ -22,10 +22,13 @@
 #include <cstdio>
 #include <cuda_runtime.h>
 
+#include "fp64_util.cuh"
 #include "sw_kernels.h"
 #include "../data/rrtmg_sw_table_layout.h"
 
 namespace sw {
+
+using namespace fp64;
 
 __constant__ int c_ng[14] = {6, 12, 8, 8, 10, 10, 2, 10, 8, 6, 6, 8, 6, 12};   // radsw_param.f NG16..29
 __constant__ int c_ns[14] = {0, 6, 18, 26, 34, 44, 54, 56, 66, 74, 80, 86, 94, 100};
@@ -34,7 +37,7 @@ __constant__ int c_nspb[14] = {1, 5, 1, 1, 1, 5, 1, 0, 1, 0, 0, 1, 5, 1};      /
 __constant__ int c_idxsfc[14] = {1, 1, 1, 1, 1, 1, 1, 1, 0, 2, 2, 2, 2, 1};    // RSM:362
 __constant__ int c_idxebc[14] = {5, 5, 4, 4, 3, 3, 2, 2, 1, 1, 1, 1, 1, 5};    // RSM:363
 
-constexpr double kEps = 1.0e-6, kOneMinus = 1.0 - kEps, kBpade = 1.0 / 0.278, kStpfac = 296.0 / 1013.0;
+constexpr double kEps = 1.0e-6, kOneMinus = 1.0 - kEps, kStpfac = 296.0 / 1013.0;
 constexpr double kFtiny = 1.0e-12, kFlimit = 1.0e-20;
 constexpr double kConG = 9.80665, kConAvgd = 6.0221415e23, kConAmd = 28.9644, kConAmw = 18.0154,
                  kConAmo3 = 47.9982;
@@ -607,31 +610,6 @@ struct LayOpt {
   double rb, rd, tb, td, e3, e4;
 };
 
-// Quotients and roots from the hardware estimate (2^-20) and Newton's
-// iteration, for operands that are normal numbers far from the ends of the
-// range: no range check and no slow path, about two thirds of the instructions
-// of the compiled IEEE operations.  recip_newton is 1/x to about 2^-52;
-// div_markstein and sqrt_markstein add Markstein's residual step (IBM J. Res.
-// Dev. 34, 1990), which rounds correctly but for a reciprocal whose own last
-// bit was misrounded.
-__device__ __forceinline__ double recip_newton(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = fma(y, fma(-x, y, 1.0), y);
-  return fma(y, fma(-x, y, 1.0), y);
-}
-__device__ __forceinline__ double div_markstein(double a, double b) {
-  const double y = recip_newton(b), q = a * y;
-  return fma(fma(-b, q, a), y, q);
-}
-__device__ __forceinline__ double sqrt_markstein(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = fma(0.5 * y, fma(-x * y, y, 1.0), y);
-  y = fma(0.5 * y, fma(-x * y, y, 1.0), y);
-  const double r = x * y;
-  return fma(fma(-r, r, x), 0.5 * y, r);
-}
 // fmax / fmin with a constant: NaN gives the constant, as fmax and fmin do
 __device__ __forceinline__ double at_least(double c, double x) { return x > c ? x : c; }
 __device__ __forceinline__ double at_most(double c, double x) { return x < c ? x : c; }
@@ -651,28 +629,10 @@ struct TblShared {
   }
 };
 
-// exp_tbl at index int(z / (bpade + z) * NTBMX + 0.5) (RSM:3601-3602; ftind in
-// [0, 1), so the clamped and the truncated form select the same entry).  The
-// quotient comes from one Newton step (error below 1e-8 in index units) and is
-// rounded by adding 1.5 2^52; only a value within 1e-6 of a tie takes the IEEE
-// division, so the entry is the reference's in every case.
-template <typename Tbl>
-__device__ __forceinline__ double exp_tab(const Tbl& ET, double z) {
-  constexpr double kRound = 6755399441055744.0;
-  const double d = kBpade + z;
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  y = fma(y, fma(-d, y, 1.0), y);
-  const double q = z * y, t = fma(q, (double)kNtbmx, kRound);
-  int i = __double2loint(t);
-  const double f = fma(q, (double)kNtbmx, kRound - t);
-  if (!(fabs(f) < 0.5 - 1.0e-6)) i = (int)(z / d * kNtbmx + 0.5);
-  return ET(i);
-}
 __device__ __forceinline__ double exp_small(double z) { return 1.0 - z + 0.5 * z * z; }
 template <typename Tbl>
 __device__ __forceinline__ double exp_of(const Tbl& ET, double z) {   // od_lo = 0.06
-  return (z <= 0.06) ? exp_small(z) : exp_tab(ET, z);
+  return (z <= 0.06) ? exp_small(z) : ET(pade_index(z));
 }
 
 // The two-stream layer reflectance / transmittance of spcvrtm (RSM:3447-3600).
@@ -766,13 +726,6 @@ __device__ __forceinline__ void two_stream(double ztau0, double zssa0, double za
   }
 }
 
-// read-once inputs: no L1 line, which stays with exp_tbl
-__device__ __forceinline__ double2 ld_once2(const double* p) {
-  double2 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
-  return v;
-}
-
 // spcvrtc's mixing of a cloudy layer's optics with its clear optics o
 // (RSM:3039-3042, 3057, 3072): zc0 * clear + zc1 * cloudy
 __device__ __forceinline__ void mix_grid(double zc1, const LayOpt& o, LayOpt& w) {
@@ -783,36 +736,6 @@ __device__ __forceinline__ void mix_grid(double zc1, const LayOpt& o, LayOpt& w)
   w.td = zc0 * o.td + zc1 * w.td;
   w.e3 = zc0 * o.e3 + zc1 * w.e3;
   w.e4 = zc0 * o.e4 + zc1 * w.e4;
-}
-
-// Sums of N values (a power of two) over the 16 lanes of a half-warp: each
-// step exchanges half of the values with the partner lane, so N values take
-// N - 1 + log2(16 / N) exchanges instead of 4 N.  Lane j ends with the sum of
-// value bits(j) (see sum_index).
-template <int N>
-__device__ __forceinline__ double half_sums(double (&v)[N], int lane, unsigned mask) {
-  int o = 8;
-#pragma unroll
-  for (int n = N / 2; n >= 1; n >>= 1, o >>= 1) {
-    const bool hi = (lane & o) != 0;
-#pragma unroll
-    for (int q = 0; q < n; ++q) {
-      const double keep = hi ? v[q + n] : v[q], send = hi ? v[q] : v[q + n];
-      v[q] = keep + __shfl_xor_sync(mask, send, o);
-    }
-  }
-  double r = v[0];
-  for (; o >= 1; o >>= 1) r += __shfl_xor_sync(mask, r, o);
-  return r;
-}
-// the value whose sum lane j of the half-warp holds, -1 where another lane has it too
-template <int N>
-__device__ __forceinline__ int sum_index(int lane) {
-  int idx = 0, o = 8;
-#pragma unroll
-  for (int n = N / 2; n >= 1; n >>= 1, o >>= 1)
-    if (lane & o) idx += n;
-  return (lane & (2 * o - 1)) ? -1 : idx;
 }
 
 // Transfer, thread = g-point (112 per column; columns share warps, so no lane
@@ -999,7 +922,7 @@ template <bool GRID, bool BANDS>
 __device__ __forceinline__ void rt_down(const RtCol& c, double zsolar, const RtSums& S, double (&end)[4]) {
   const int half = threadIdx.x & 15;
   const unsigned hmask = 0xffffu << (threadIdx.x & 16);
-  const int idx8 = sum_index<8>(half), idx4 = sum_index<4>(half);
+  const int idx8 = sum_index<8, 16>(half), idx4 = sum_index<4, 16>(half);
   const double* st = c.st + (size_t)c.nlay * kRtLay;   // the layer at hand
   double ub = __ldcg(st + 4 * kSwNg), ud = __ldcg(st + 5 * kSwNg), ubw = __ldcg(st + 6 * kSwNg),
          udw = __ldcg(st + 7 * kSwNg), D = zsolar, F = 0.0, Dw = zsolar, Fw = 0.0;
@@ -1022,13 +945,13 @@ __device__ __forceinline__ void rt_down(const RtCol& c, double zsolar, const RtS
           const double t = c.cloudy ? (GRID ? S.cf1 * c1 + S.cf0 * c0 : c1) : c0;
           u[e] = (S.b == S.blo + q) ? t : 0.0;
         }
-        const double r = half_sums<4>(u, half, hmask);
+        const double r = lane_sums<4, 16>(u, half, hmask);
         const int lev = idx4 >> 1;
         if (q <= S.nbg && idx4 >= 0 && lev < nlev)
           S.accb[((size_t)2 * (S.blo + q + S.grp) + (idx4 & 1)) * S.nlp1 + (m - lev)] = r;
       }
     }
-    const double r = half_sums<8>(v, half, hmask);
+    const double r = lane_sums<8, 16>(v, half, hmask);
     const int lev = idx8 >> 2;
     if (idx8 >= 0 && lev < nlev) S.part[(size_t)(idx8 & 3) * S.nlp1 + (m - lev)] = r;
   };
@@ -1173,7 +1096,7 @@ __device__ __forceinline__ void down_body(const SwArgs& a, const SwScratch& s, i
 
   // surface direct / diffuse partition (RSM:3641-3655) and UV-B (RSM:3907)
   {
-    const int half = threadIdx.x & 15, idx8 = sum_index<8>(half);
+    const int half = threadIdx.x & 15, idx8 = sum_index<8, 16>(half);
     const unsigned hmask = 0xffffu << (threadIdx.x & 16);
 #pragma unroll
     for (int pass = 0; pass < 2; ++pass) {
@@ -1181,7 +1104,7 @@ __device__ __forceinline__ void down_body(const SwArgs& a, const SwScratch& s, i
       double w[8] = {(ibd == 1) ? zb1 : (ibd == 0 ? 0.5 * zb1 : 0.0), (ibd == 2) ? zb1 : (ibd == 0 ? 0.5 * zb1 : 0.0),
                      (ibd == 1) ? zb2 : (ibd == 0 ? 0.5 * zb2 : 0.0), (ibd == 2) ? zb2 : (ibd == 0 ? 0.5 * zb2 : 0.0),
                      (b == 27 - 16) ? f0 : 0.0, 0.0, 0.0, 0.0};
-      const double r = half_sums<8>(w, half, hmask);
+      const double r = lane_sums<8, 16>(w, half, hmask);
       if (idx8 >= 0 && idx8 < 5) sfc[(grp * 2 + pass) * 5 + idx8] = r;
     }
   }
