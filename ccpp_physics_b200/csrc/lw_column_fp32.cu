@@ -7,6 +7,10 @@
 
 #include <type_traits>
 
+// FP32 gas optics at 4 CTAs per SM (128 registers, no spills), 16,384 x 127: 2.74 ms, against 3.91, 3.12,
+// 2.74 and 4.59 ms at 2, 3, 5 and 6; FP64 runs best at 3 (4.40 ms, against 5.41 at 2 and 4.65 at 4).
+#define LW_GAS_MINB 4
+
 #include "lw_launch.h"
 #include "lw_rt.cuh"
 #include "lw_rt_grid.cuh"

@@ -4,10 +4,10 @@
 // Replaces, per column, the driver prologue of rrtmg_lw_run
 // (physics/Radiation/RRTMG/radlw_main.F90, RLM:785-1050), the band cloud
 // optics of cldprop (RLM:1589-1799), setcoef (RLM:2151-2406) and taumol
-// (RLM:3836-6840).  One CTA owns one column at a time, one thread one layer;
-// the setcoef state of the layer stays in that thread's registers and the 16
-// bands are walked in order, so every table gather of a band happens while
-// the band's coefficients are hot in L1/L2.
+// (RLM:3836-6840).  One warp owns 32 layers of a column at a time, one lane one
+// layer; the layer's setcoef record waits in shared memory and the bands are
+// walked in order, so every table gather of a band happens while the band's
+// coefficients are hot in L1/L2.
 //
 // Output (device scratch, read by kernel B in lw_rt.cuh), per column c of the
 // chunk and layer k (0-based, surface first), NLP = 32*V >= nlay+1:
@@ -36,22 +36,18 @@ constexpr double kAbsrain = 0.33e-3, kAbssnow0 = 1.5;   // radlw_datatb.f:941,94
 constexpr int kColRec = 48;                     // doubles per column record
 
 // Minimum resident CTAs per SM requested from the register allocator
-// (measured on B200, 16,384 columns x 127 layers: gas optics 3 in both
-// precisions, transfer 4, gas optics behind the network 5).  The V = 8
-// kernels (128..255 layers) are left uncapped: with the caps their
+// (measured on B200, 16,384 columns x 127 layers: gas optics 3 in FP64 and 4
+// in FP32, transfer 4, gas optics behind the network 5).  The V = 8
+// transfer kernels (128..255 layers) are left uncapped: with the caps their
 // transfer kernel spilled ~1 KB per thread and an illegal address was
 // observed that reading the code did not explain.
 #ifndef LW_GAS_MINB
-#ifdef LW_GAS_MINB_SMALL   // build-time override for V <= 4 (tuning builds)
-#define LW_GAS_MINB (V > 4 ? 1 : LW_GAS_MINB_SMALL)
-#else
-#define LW_GAS_MINB (V > 4 ? 1 : 3)
-#endif
+#define LW_GAS_MINB 3
 #endif
 // gas optics behind the learned gas optics (setcoef/taumol only for
 // out-of-envelope layers): light enough for more resident CTAs
 #ifndef LW_GAS_MINB_SG
-#define LW_GAS_MINB_SG (V > 4 ? 1 : 5)
+#define LW_GAS_MINB_SG 5
 #endif
 #ifndef LW_RT_MINB
 #ifdef LW_RT_MINB_SMALL
@@ -127,56 +123,66 @@ __device__ __forceinline__ double planck_int(const double* kt, int b, int ind, d
   return c_delwave[b] * (p0 + frac * (p1 - p0));
 }
 
+// Per-warp working arrays of gas_unit.
 template <typename R>
-__host__ __device__ constexpr size_t gas_smem_bytes(int V) {
-  const size_t NLP = 32 * (size_t)V;
-  return sizeof(double) * (2 * NLP + 24 + 8 * NLP) + sizeof(R) * N_LF * NLP + sizeof(int) * (NLP + 4);
-}
-
-// Per-column working arrays of gas_column (shared memory in lw_gas_kernel,
-// any memory the caller's threads can reach elsewhere); gas_smem_bytes<R>(V).
-template <typename R, int V>
 struct GasWork {
-  double* red;   // [2 NLP]
-  double* col;   // [24]
-  double* cld;   // [8 NLP] cloud inputs of the layer
-  R* lay;        // [N_LF NLP] setcoef record (LayRef)
-  int* li;       // [NLP]
-  int* ci;       // [4]
-  __device__ __forceinline__ static GasWork at(void* base) {
-    constexpr int NLP = 32 * V;
+  double* red;   // [2 NLP] coldry and h2o column amounts of the whole column
+  double* cld;   // [8][32] cloud inputs of the layer
+  R* lay;        // [N_LF][32] setcoef record (LayRef)
+  int* li;       // [32]
+  __host__ __device__ static constexpr size_t bytes(int NLP) {
+    return sizeof(double) * (2 * (size_t)NLP + 8 * 32) + sizeof(R) * N_LF * 32 + sizeof(int) * 32;
+  }
+  __device__ __forceinline__ static GasWork at(void* base, int NLP) {
     GasWork w;
     w.red = reinterpret_cast<double*>(base);
-    w.col = w.red + 2 * NLP;
-    w.cld = w.col + 24;
-    w.lay = reinterpret_cast<R*>(w.cld + 8 * NLP);
-    w.li = reinterpret_cast<int*>(w.lay + N_LF * NLP);
-    w.ci = w.li + NLP;
+    w.cld = w.red + 2 * NLP;
+    w.lay = reinterpret_cast<R*>(w.cld + 8 * 32);
+    w.li = reinterpret_cast<int*>(w.lay + N_LF * 32);
     return w;
   }
 };
 
-// Kernel A's work for one column cc of the chunk (global column sc.c0 + cc),
-// run by the 32 V threads t = 0 .. 32 V - 1 that S synchronizes.
-template <typename R, int V, bool SG, typename Sync>
-__device__ __forceinline__ void gas_column(int cc, int t, const Sync& S, const GasWork<R, V>& W,
-                                           const Block* __restrict__ blocks, int nblocks, const Block& b0,
-                                           const Flags& f, const Tables<R>& tab, const Tables<double>& tab64,
-                                           const Scratch<R>& sc, double* __restrict__ gas_taug,
-                                           double* __restrict__ gas_fracs) {
-  constexpr int NLP = 32 * V;
-  double* s_red = W.red;
-  double* s_col = W.col;
-  double* s_cld = W.cld;
+// ln p > 4.56 (the lower atmosphere, RLM:2344): p against e^4.56 =
+// 95.58347984, by the logarithm itself where rounding could decide.
+__device__ __forceinline__ bool lower_atm(double p) {
+  return (p > 95.5834 && p < 95.5836) ? log(p) > 4.56 : p > 95.5835;
+}
+
+// dry-air and water-vapour column amounts of a layer (RLM:823-836)
+struct ColAmt {
+  double coldry, h2ovmr;
+};
+__device__ __forceinline__ ColAmt col_amounts(double q, double delp) {
+  const double amdw = kConAmd / kConAmw;
+  const double tem1c = 100.0 * kConG, tem2c = 1.0e-20 * 1.0e3 * kConAvgd;
+  ColAmt o;
+  o.h2ovmr = fmax(0.0, q * amdw / (1.0 - q));
+  const double tem0 = (1.0 - o.h2ovmr) * kConAmd + o.h2ovmr * kConAmw;
+  o.coldry = tem2c * delp / (tem1c * tem0 * (1.0 + o.h2ovmr));
+  return o;
+}
+
+// Kernel A's work for 32 layers (segment seg) and bands b_lo .. b_hi - 1 of
+// column cc of the chunk (global column sc.c0 + cc), by one warp, a lane per
+// layer.  What the layers share (the split of the atmosphere, the cloudy-column
+// test, the precipitable water) each warp finds for itself, so no warp waits
+// for another: with a CTA per column, the warps of the upper atmosphere waited
+// at every column's barrier for the one whose layers lie on both sides.
+// 16,384 x 127: FP64 5.03 -> 4.40 ms; 32 x 64, in eight band groups, 100 -> 31 us.
+template <typename R, bool SG>
+__device__ __forceinline__ void gas_unit(int cc, int seg, int b_lo, int b_hi, int lane, int NLP, const GasWork<R>& W,
+                                         const Block* __restrict__ blocks, int nblocks, const Block& b0,
+                                         const Flags& f, const Tables<R>& tab, const Tables<double>& tab64,
+                                         const Scratch<R>& sc, double* __restrict__ gas_taug,
+                                         double* __restrict__ gas_fracs) {
   R* s_lay = W.lay;
-  int* s_li = W.li;
-  int* s_ci = W.ci;
+  const int t = 32 * seg + lane;   // layer
+  const bool first = b_lo == 0;    // of the segment's band groups
   const int nlay = f.nlay, nlp1 = nlay + 1;
-  const KT<R> kt{tab.kt};
   const double* kt64 = tab64.kt;
   {
     const int c = sc.c0 + cc;                        // global column
-    S.sync();
     const Block& B = (nblocks == 1) ? b0 : blocks[find_block(blocks, nblocks, c)];
     const int i = c - B.col0;
     const size_t ld = (size_t)B.ld;
@@ -186,23 +192,43 @@ __device__ __forceinline__ void gas_column(int cc, int t, const Sync& S, const G
       return B.in[fld][i + ld * row];
     };
 
+    // what the column's layers share: laytrop (a count, RLM:2344-2346), any cloud
+    // (RLM:1101), and for the column record the amounts of every layer
+    const bool write_scratch = sc.tau != nullptr;
+    const bool rec = first && seg == 0 && write_scratch;
+    int laytrop = 0;
+    bool lcf1 = false;
+    for (int k0 = 0; k0 < nlay; k0 += 32) {
+      const int k = k0 + lane;
+      bool lo = false, cl = false;
+      if (k < nlay) {
+        const int rk = top ? nlay - 1 - k : k;
+        lo = lower_atm(IN(F_PLYR, rk));
+        cl = IN(F_CLDCF, rk) > kEps;
+        if (rec) {
+          const ColAmt ca = col_amounts(IN(F_QLYR, rk), IN(F_DELPIN, rk));
+          W.red[k] = ca.coldry;
+          W.red[NLP + k] = fmax(0.0, ca.coldry * ca.h2ovmr);
+        }
+      }
+      laytrop += __popc(__ballot_sync(0xffffffffu, lo));
+      lcf1 |= __any_sync(0xffffffffu, cl) != 0;
+    }
+    __syncwarp();
+
     // ------------------------------ prologue + setcoef, FP64 -------------
     double tlyrfr = 0.0, tlvlfr = 0.0;
     int indlay = 1, indlev = 1, r = 0;
-    bool lowerk = false, cldk = false;
     bool sg_skip = false;   // learned gas optics already wrote this layer's tau/frac
     if (t < nlay) {
       const int kref = t + 1;
       r = top ? nlp1 - kref - 1 : t;                  // 0-based input row of the layer
       const int rl = top ? nlp1 - kref - 1 : t + 1;   // 0-based input row of its top level
       double pavel = IN(F_PLYR, r), delp = IN(F_DELPIN, r), tavel = IN(F_TLYR, r), tz = IN(F_TLVL, rl);
-      double q = IN(F_QLYR, r);
-      const double amdw = kConAmd / kConAmw, amdo3 = kConAmd / kConAmo3;
-      double h2ovmr = fmax(0.0, q * amdw / (1.0 - q));
+      const double amdo3 = kConAmd / kConAmo3;
+      const ColAmt ca = col_amounts(IN(F_QLYR, r), delp);
+      const double h2ovmr = ca.h2ovmr, coldry = ca.coldry;
       double o3vmr = fmax(0.0, IN(F_OLYR, r) * amdo3);
-      double tem0 = (1.0 - h2ovmr) * kConAmd + h2ovmr * kConAmw;
-      const double tem1c = 100.0 * kConG, tem2c = 1.0e-20 * 1.0e3 * kConAvgd;
-      double coldry = tem2c * delp / (tem1c * tem0 * (1.0 + h2ovmr));
       double temcol = 1.0e-12 * coldry;
       const double colh2o = fmax(0.0, coldry * h2ovmr);
       // the learned gas optics already wrote tau/frac of layers inside its training
@@ -211,15 +237,14 @@ __device__ __forceinline__ void gas_column(int cc, int t, const Sync& S, const G
         float xf[SG_NFEAT];
         layer_features(pavel, tavel, h2ovmr, o3vmr, IN(F_CO2, r), IN(F_CH4, r), IN(F_N2O, r), xf);
         sg_skip = in_envelope(xf, f.sg_norm);
-        if (!sg_skip && f.sg_fallback) atomicAdd(f.sg_fallback, 1u);
+        if (!sg_skip && first && f.sg_fallback) atomicAdd(f.sg_fallback, 1u);
       }
       indlay = min(180, max(1, (int)(tavel - 159.0)));
       tlyrfr = tavel - (int)tavel;
       indlev = min(180, max(1, (int)(tz - 159.0)));
       tlvlfr = tz - (int)tz;
-      double plog = log(pavel);
-      lowerk = plog > 4.56;
       if (!sg_skip) {
+        const double plog = log(pavel);
         double colv[7], wxv[4];
         colv[0] = colh2o;
         colv[1] = fmax(temcol, coldry * IN(F_CO2, r));
@@ -261,7 +286,7 @@ __device__ __forceinline__ void gas_column(int cc, int t, const Sync& S, const G
         double minorfrac = tem1 - (double)indminor;
         int indfor, indself;
         double forfrac, selffrac;
-        if (lowerk) {
+        if (plog > 4.56) {
           tem1 = (332.0 - tavel) / 36.0;
           indfor = min(2, max(1, (int)tem1));
           forfrac = tem1 - (double)indfor;
@@ -278,76 +303,62 @@ __device__ __forceinline__ void gas_column(int cc, int t, const Sync& S, const G
         selffac = colv[0] * selffac;
         forfac = colv[0] * forfac;
 
-        R* ls = s_lay + t;
-        ls[LF_FAC00 * NLP] = R(fac00); ls[LF_FAC01 * NLP] = R(fac01);
-        ls[LF_FAC10 * NLP] = R(fac10); ls[LF_FAC11 * NLP] = R(fac11);
-        ls[LF_SELFFAC * NLP] = R(selffac); ls[LF_SELFFRAC * NLP] = R(selffrac);
-        ls[LF_FORFAC * NLP] = R(forfac); ls[LF_FORFRAC * NLP] = R(forfrac);
-        ls[LF_MINORFRAC * NLP] = R(minorfrac);
-        ls[LF_SCALEMINOR * NLP] = R(scaleminor); ls[LF_SCALEMINORN2 * NLP] = R(scaleminorn2);
-        for (int m = 0; m < 7; ++m) ls[(LF_COL1 + m) * NLP] = R(colv[m]);
-        ls[LF_COLDRY * NLP] = R(coldry); ls[LF_COLBRD * NLP] = R(colbrd);
-        for (int m = 0; m < 4; ++m) ls[(LF_WX1 + m) * NLP] = R(wxv[m]);
-        ls[LF_PAVEL * NLP] = R(pavel);
-        s_li[t] = jp | (jt << 8) | (jt1 << 12) | (indself << 16) | (indfor << 20) | (indminor << 24);
+        R* ls = s_lay + lane;
+        ls[LF_FAC00 * 32] = R(fac00); ls[LF_FAC01 * 32] = R(fac01);
+        ls[LF_FAC10 * 32] = R(fac10); ls[LF_FAC11 * 32] = R(fac11);
+        ls[LF_SELFFAC * 32] = R(selffac); ls[LF_SELFFRAC * 32] = R(selffrac);
+        ls[LF_FORFAC * 32] = R(forfac); ls[LF_FORFRAC * 32] = R(forfrac);
+        ls[LF_MINORFRAC * 32] = R(minorfrac);
+        ls[LF_SCALEMINOR * 32] = R(scaleminor); ls[LF_SCALEMINORN2 * 32] = R(scaleminorn2);
+        for (int m = 0; m < 7; ++m) ls[(LF_COL1 + m) * 32] = R(colv[m]);
+        ls[LF_COLDRY * 32] = R(coldry); ls[LF_COLBRD * 32] = R(colbrd);
+        for (int m = 0; m < 4; ++m) ls[(LF_WX1 + m) * 32] = R(wxv[m]);
+        ls[LF_PAVEL * 32] = R(pavel);
+        W.li[lane] = jp | (jt << 8) | (jt1 << 12) | (indself << 16) | (indfor << 20) | (indminor << 24);
       }
-      double cf = IN(F_CLDCF, r);
-      cldk = cf > kEps;
-      double* cl = s_cld + t;
-      cl[0 * NLP] = cf;
+      double* cl = W.cld + lane;
+      cl[0 * 32] = IN(F_CLDCF, r);
       if (f.ilwcliq > 0) {
-        cl[1 * NLP] = IN(F_LWP, r); cl[2 * NLP] = IN(F_RELIQ, r); cl[3 * NLP] = IN(F_IWP, r);
-        cl[4 * NLP] = IN(F_REICE, r); cl[5 * NLP] = IN(F_RWP, r); cl[6 * NLP] = IN(F_SWP, r);
-        cl[7 * NLP] = IN(F_RESNOW, r);
+        cl[1 * 32] = IN(F_LWP, r); cl[2 * 32] = IN(F_RELIQ, r); cl[3 * 32] = IN(F_IWP, r);
+        cl[4 * 32] = IN(F_REICE, r); cl[5 * 32] = IN(F_RWP, r); cl[6 * 32] = IN(F_SWP, r);
+        cl[7 * 32] = IN(F_RESNOW, r);
       } else {
-        cl[5 * NLP] = IN(F_CLDOD, r);
+        cl[5 * 32] = IN(F_CLDOD, r);
       }
-      s_red[t] = coldry;
-      s_red[NLP + t] = colh2o;
     }
-    const int laytrop = S.count(lowerk);
-    const int lcf1 = S.any(cldk);
-    if (t == 0) {
+    if (rec && LW_OK(cc < sc.cap, 18, cc)) {
       // precipitable water (RLM:910-919 / 1012-1019): sequential, reference order
-      double tem1 = 0.0, tem2 = 0.0;
-      for (int k = 0; k < nlay; ++k) {
-        tem1 = tem1 + s_red[k] + s_red[NLP + k];
-        tem2 = tem2 + s_red[NLP + k];
+      double pw = 0.0;
+      if (lane == 0) {
+        double tem1 = 0.0, tem2 = 0.0;
+        for (int k = 0; k < nlay; ++k) {
+          tem1 = tem1 + W.red[k] + W.red[NLP + k];
+          tem2 = tem2 + W.red[NLP + k];
+        }
+        const double amdw = kConAmd / kConAmw;
+        double tem0 = 10.0 * tem2 / (amdw * tem1 * kConG);
+        pw = tem0 * (top ? IN(F_PLVL, nlay) : IN(F_PLVL, 0));
       }
-      const double amdw = kConAmd / kConAmw;
-      double tem0 = 10.0 * tem2 / (amdw * tem1 * kConG);
-      s_col[17] = tem0 * (top ? IN(F_PLVL, nlay) : IN(F_PLVL, 0));
-      double sfe = B.in[F_SFEMIS][i];
-      s_col[16] = (sfe > kEps && sfe <= 1.0) ? sfe : 1.0;
-      double stemp = B.in[F_SFGTMP][i];
-      double tz0 = top ? IN(F_TLVL, nlay) : IN(F_TLVL, 0);
-      s_col[18] = stemp - (int)stemp;
-      s_col[19] = tz0 - (int)tz0;
-      s_ci[0] = min(180, max(1, (int)(stemp - 159.0)));
-      s_ci[1] = min(180, max(1, (int)(tz0 - 159.0)));
-    }
-    S.sync();
-    const bool write_scratch = sc.tau != nullptr;
-    double* crec = write_scratch ? sc.col + (size_t)cc * kColRec : nullptr;
-    if (crec && !LW_OK(cc < sc.cap, 18, cc)) crec = nullptr;
-    if (t < NBANDS) {
-      // diffusivity angle (RLM:1041-1050) and surface Planck terms (RLM:2251-2262)
-      double secd = (t == 0 || t == 3 || t == 9)
-                        ? 1.66
-                        : fmin(1.80, fmax(1.50, c_a0[t] + c_a1[t] * exp(c_a2[t] * s_col[17])));
-      if (crec) {
-        crec[t] = secd;
-        crec[16 + t] = planck_int(kt64, t, s_ci[0], s_col[18]);   // pklay(b, 0): stemp
+      pw = __shfl_sync(0xffffffffu, pw, 0);
+      double* crec = sc.col + (size_t)cc * kColRec;
+      if (lane < NBANDS) {
+        // diffusivity angle (RLM:1041-1050) and surface Planck terms (RLM:2251-2262)
+        const double stemp = B.in[F_SFGTMP][i];
+        crec[lane] = (lane == 0 || lane == 3 || lane == 9)
+                         ? 1.66
+                         : fmin(1.80, fmax(1.50, c_a0[lane] + c_a1[lane] * exp(c_a2[lane] * pw)));
+        crec[16 + lane] = planck_int(kt64, lane, min(180, max(1, (int)(stemp - 159.0))), stemp - (int)stemp);   // pklay(b, 0): stemp
       }
-    }
-    if (t == 0 && crec) {
-      crec[32] = s_col[16];
-      crec[33] = lcf1 ? 1.0 : 0.0;
+      if (lane == 0) {
+        const double sfe = B.in[F_SFEMIS][i];
+        crec[32] = (sfe > kEps && sfe <= 1.0) ? sfe : 1.0;
+        crec[33] = lcf1 ? 1.0 : 0.0;
+      }
     }
 
     // ------------------------------ bands --------------------------------
     // taumol splits at the count laytrop (RLM:2344-2346)
-    const LayRef<R> LR{s_lay, s_li, t, NLP, t < laytrop};
+    const LayRef<R> LR{s_lay, W.li, lane, 32, t < laytrop};
     // tau, frac: [g][NLP], or four layers per g-point (lw_rt64.cuh)
     const size_t hoff = (size_t)cc * NGPT * NLP + (sc.block4 ? (size_t)(t >> 2) * NGPT * 4 + (t & 3) : (size_t)t);
     const int hstep = sc.block4 ? 4 : NLP;
@@ -355,13 +366,13 @@ __device__ __forceinline__ void gas_column(int cc, int t, const Sync& S, const G
     R* fcol = write_scratch ? sc.frac + hoff : nullptr;
     R* bcol = write_scratch ? sc.band + (size_t)cc * 3 * NBANDS * NLP : nullptr;
 #pragma unroll 1
-    for (int b = 0; b < NBANDS; ++b) {
+    for (int b = b_lo; b < b_hi; ++b) {
       if (t < nlay) {
         double tcld = 0.0;
         if (lcf1) {
-          const double* cl = s_cld + t;
-          tcld = band_taucld(b, f, kt64, cl[0], cl[NLP], cl[2 * NLP], cl[3 * NLP], cl[4 * NLP], cl[5 * NLP],
-                             cl[6 * NLP], cl[7 * NLP]);
+          const double* cl = W.cld + lane;
+          tcld = band_taucld(b, f, kt64, cl[0], cl[32], cl[2 * 32], cl[3 * 32], cl[4 * 32], cl[5 * 32], cl[6 * 32],
+                             cl[7 * 32]);
         }
         if (b == 6 && !f.gas_only && LW_OK(r < nlay && i < B.npts, 13, r)) B.out[O_CLDTAU][i + ld * r] = lcf1 ? tcld : 0.0;   // band 7 (RLM:1087-1097)
         if (bcol && LW_OK(cc < sc.cap && t + 1 < NLP, 14, cc)) {   // evict-first stores: the hand-off must not push the tables out of L2
@@ -374,35 +385,52 @@ __device__ __forceinline__ void gas_column(int cc, int t, const Sync& S, const G
         if (!sg_skip && LW_OK(r < nlay && i < B.npts, 15, r)) tauaer = R(B.in[F_AERAOD][ab] * (1.0 - B.in[F_AERSSA][ab]));
         const int ns = ns_of(b);
         const size_t go = ((size_t)c * nlay + t) * NGPT + ns;
-        if (!sg_skip) band_gas_optics<R>(b, kt, LR, [&](int g0, G2<R> tau, G2<R> frac) {
+        if (!sg_skip) band_gas_optics<R>(b, tab.kt, LR, [&](int g0, auto tau, auto frac) {
           if (tcol && LW_OK(cc < sc.cap && ns + g0 + 1 < NGPT, 16, ns + g0)) {
-            __stcs(tcol + (size_t)(ns + g0) * hstep, tau.x + tauaer);
-            __stcs(tcol + (size_t)(ns + g0 + 1) * hstep, tau.y + tauaer);
-            __stcs(fcol + (size_t)(ns + g0) * hstep, frac.x);
-            __stcs(fcol + (size_t)(ns + g0 + 1) * hstep, frac.y);
+            each(tau, [&](int q, R v) { __stcs(tcol + (size_t)(ns + g0 + q) * hstep, v + tauaer); });
+            each(frac, [&](int q, R v) { __stcs(fcol + (size_t)(ns + g0 + q) * hstep, v); });
           }
           if (f.gas_only && LW_OK(c < sc.ntot, 17, c)) {
-            gas_taug[go + g0] = (double)tau.x;
-            gas_taug[go + g0 + 1] = (double)tau.y;
-            gas_fracs[go + g0] = (double)frac.x;
-            gas_fracs[go + g0 + 1] = (double)frac.y;
+            each(tau, [&](int q, R v) { gas_taug[go + g0 + q] = (double)v; });
+            each(frac, [&](int q, R v) { gas_fracs[go + g0 + q] = (double)v; });
           }
         });
       }
-      if (t == 0 && bcol) __stcs(bcol + (1 * NBANDS + b) * NLP, R(planck_int(kt64, b, s_ci[1], s_col[19])));
+      if (t == 0 && bcol) {   // pklev(b, 0): the level below the first layer
+        const double tz0 = top ? IN(F_TLVL, nlay) : IN(F_TLVL, 0);
+        __stcs(bcol + (1 * NBANDS + b) * NLP, R(planck_int(kt64, b, min(180, max(1, (int)(tz0 - 159.0))), tz0 - (int)tz0)));
+      }
     }
+    __syncwarp();   // the warp's next unit writes the working arrays
   }
 }
 
-template <typename R, int V, bool SG>
-__global__ void __launch_bounds__(32 * V, SG ? LW_GAS_MINB_SG : LW_GAS_MINB)
-lw_gas_kernel(const Block* __restrict__ blocks, int nblocks, const Block b0, int ncols, Flags f,
+constexpr int kGasWarps = 4;   // per CTA
+// first bands of the nsplit band groups of a segment (about equal numbers of
+// g-points), by nsplit = 1, 2, 4, 8
+static __device__ __constant__ int c_gas_split[4][9] = {
+    {0, 16}, {0, 5, 16}, {0, 3, 5, 9, 16}, {0, 2, 3, 4, 5, 7, 9, 12, 16}};
+
+// Units of 32 layers x a band group, strided over the grid's warps; lsplit =
+// log2 of the band groups per segment.  A column's segments are dealt out from
+// another one in each round of the grid, so that a warp's share of the costlier
+// lower atmosphere evens out.
+template <typename R, bool SG>
+__global__ void __launch_bounds__(32 * kGasWarps, SG ? LW_GAS_MINB_SG : LW_GAS_MINB)
+lw_gas_kernel(const Block* __restrict__ blocks, int nblocks, const Block b0, int ncols, int NLP, int lsplit, Flags f,
               Tables<R> tab, Tables<double> tab64, Scratch<R> sc, double* __restrict__ gas_taug,
               double* __restrict__ gas_fracs) {
-  extern __shared__ __align__(16) char smem_raw[];   // gas_smem_bytes<R>(V)
-  const GasWork<R, V> W = GasWork<R, V>::at(smem_raw);
-  for (int cc = blockIdx.x; cc < ncols; cc += gridDim.x)
-    gas_column<R, V, SG>(cc, threadIdx.x, CtaSync{}, W, blocks, nblocks, b0, f, tab, tab64, sc, gas_taug, gas_fracs);
+  extern __shared__ __align__(16) char smem_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const GasWork<R> W = GasWork<R>::at(smem_raw + warp * GasWork<R>::bytes(NLP), NLP);
+  const int nseg = (f.nlay + 31) >> 5, per = nseg << lsplit;
+  const long long units = (long long)ncols * per, stride = (long long)gridDim.x * kGasWarps;
+  for (long long u = (long long)blockIdx.x * kGasWarps + warp; u < units; u += stride) {
+    const int cc = (int)(u / per), r = (int)(u % per), part = r / nseg;
+    const int seg = (int)((r + u / per * per / stride) % nseg);   // the round of the column's first unit: the same for all of them
+    gas_unit<R, SG>(cc, seg, c_gas_split[lsplit][part], c_gas_split[lsplit][part + 1], lane, NLP, W, blocks, nblocks,
+                    b0, f, tab, tab64, sc, gas_taug, gas_fracs);
+  }
 }
 
 }  // namespace lw

@@ -12,8 +12,8 @@
 // layers across the lanes (both sweeps as affine scans: a composition, five
 // shuffle steps and a replay per g-point, lw_rt.cuh), a layer's terms cost two
 // evaluations but no scan, a column spreads over five warps, and a layer count
-// of 64 leaves no lane idle.  16,384 x 127: 5.02 ms as scans, 4.66 here
-// (3.3 down, 1.3 up); 1,024 x 64: 493 -> 170 us; 32 x 64: 569 -> 51 us.
+// of 64 leaves no lane idle.  16,384 x 127: 5.02 ms as scans, 4.22 here
+// (3.3 down, 1.3 up); 1,024 x 64: 493 -> 150 us; 32 x 64: 569 -> 46 us.
 // The way down leaves {transmittance, upward source} in place of {tau, frac}
 // (recomputing both on the way up: 6.06 ms); with exp_tbl and tfn_tbl in shared
 // memory, three columns per CTA: 5.83 ms; four CTAs per SM at 96 registers:
@@ -30,7 +30,7 @@ constexpr int kRt64Threads = 160, kRt64Warps = kRt64Threads / 32;
 // tau and frac of this path, [c][kb][140][4]: four layers of a g-point are one
 // 32-byte sector, written by the layers' threads (lw_gas.cuh) and read by the
 // g-point's
-__host__ __device__ constexpr int kRt64Block = NGPT * 4;
+constexpr int kRt64Block = NGPT * 4;
 
 __host__ __device__ inline size_t rt64_smem_bytes(int nlay) {   // the warps' partial sums
   return (size_t)kRt64Warps * 4 * (nlay + 1) * sizeof(double);

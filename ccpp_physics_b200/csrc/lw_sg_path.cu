@@ -605,7 +605,7 @@ __global__ void __launch_bounds__(SR_THREADS, 1) lw_sg_rt_kernel(SrArgs a) {
 // Out-of-envelope layers: plain FP32 taumol (the FP32 path's gas optics) for
 // the listed columns, written over the network's values in the hand-off.
 constexpr int FB_V = 4;                        // 128 layer threads
-constexpr size_t FB_NLP = 32 * FB_V;
+constexpr int FB_NLP = 32 * FB_V;
 constexpr size_t FB_SLOT_BYTES = (((2 * NGPT + 3 * NBANDS) * FB_NLP * sizeof(float) + kColRec * sizeof(double)) + 255) &
                                  ~(size_t)255;
 constexpr int FB_GRID = 64;
@@ -626,8 +626,8 @@ struct FbArgs {
 };
 
 __global__ void __launch_bounds__(32 * FB_V) lw_sg_fallback_kernel(FbArgs a) {
-  extern __shared__ __align__(16) char fsm[];   // gas_smem_bytes<float>(FB_V)
-  const GasWork<float, FB_V> W = GasWork<float, FB_V>::at(fsm);
+  extern __shared__ __align__(16) char fsm[];   // a GasWork per warp
+  const GasWork<float> W = GasWork<float>::at(fsm + (threadIdx.x >> 5) * GasWork<float>::bytes(FB_NLP), FB_NLP);
   const int n = *a.count;
   const int t = threadIdx.x, nlay = a.f.nlay;
   float* slot = reinterpret_cast<float*>(a.slots + (size_t)blockIdx.x * FB_SLOT_BYTES);
@@ -641,8 +641,9 @@ __global__ void __launch_bounds__(32 * FB_V) lw_sg_fallback_kernel(FbArgs a) {
     sc.c0 = c;
     sc.cap = 1;
     sc.ntot = c + 1;
-    gas_column<float, FB_V, true>(0, t, CtaSync{}, W, a.blocks, a.nblocks, a.b0, a.f, a.tab, a.tab64, sc, nullptr,
-                                  nullptr);
+    if ((t & ~31) < nlay)
+      gas_unit<float, true>(0, t >> 5, 0, NBANDS, t & 31, FB_NLP, W, a.blocks, a.nblocks, a.b0, a.f, a.tab, a.tab64, sc,
+                            nullptr, nullptr);
     __syncthreads();
     if (t < nlay) {
       // the network kernel's envelope test on the same features
@@ -728,7 +729,7 @@ cudaError_t sg_path_prepare() {
   cudaError_t e = cudaFuncSetAttribute(lw_sg_rt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SR_SMEM);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(lw_sg_fallback_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)gas_smem_bytes<float>(FB_V));
+                           (int)(FB_V * GasWork<float>::bytes(FB_NLP)));
   if (e != cudaSuccess) return e;
   int occ = 0;
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, lw_sg_rt_kernel, SR_THREADS, SR_SMEM)) != cudaSuccess)
@@ -783,7 +784,7 @@ cudaError_t sg_path_launch(const Block* blocks, int nblocks, const Block& b0, in
     fa.slots = fbs;
     {
       NvtxRange r("taumol fallback (out of envelope)");
-      lw_sg_fallback_kernel<<<FB_GRID, 32 * FB_V, gas_smem_bytes<float>(FB_V), st>>>(fa);
+      lw_sg_fallback_kernel<<<FB_GRID, 32 * FB_V, FB_V * GasWork<float>::bytes(FB_NLP), st>>>(fa);
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     SrArgs ra;
