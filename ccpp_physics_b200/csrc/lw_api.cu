@@ -23,6 +23,7 @@
 
 #include "../../include/rrtmg_lw_gpu.h"
 #include "lw_common.cuh"
+#include "host_stage.h"
 #include "lw_launch.h"
 
 extern "C" const unsigned char rrtmg_lw_tables_blob[];
@@ -55,6 +56,7 @@ struct Workspace {
   cudaStream_t stream = nullptr;
   char* dbuf = nullptr;       // device staging for host-memory calls
   size_t dbuf_bytes = 0;
+  HostStage stage;            // pinned staging of small host-memory calls
   uint32_t* bits = nullptr;   // McICA sub-column flags
   size_t bits_bytes = 0;
   char* scratch = nullptr;    // gas optics -> transfer hand-off (kernel A -> B)
@@ -784,26 +786,34 @@ extern "C" int rrtmg_lw_gpu_run_ex(const rrtmg_lw_run_args* a, const rrtmg_lw_ex
   if (d.icseed) total += al(fs.n1 * sizeof(int32_t));
   CK(cudaStreamSynchronize(st), "cudaStreamSynchronize");
   CK(grow(&w->dbuf, &w->dbuf_bytes, total), "cudaMalloc(workspace)");
-  char* p = w->dbuf;
+  const bool staged = w->stage.ensure(total);
+  HostGather up{w->stage.p, w->dbuf, st};
+  size_t off = 0;
+  auto put = [&](const void* src, size_t bytes) -> cudaError_t {   // the next field of the device buffer
+    const size_t at = off;
+    off += al(bytes);
+    if (staged) return up.put(at, src, bytes, off);
+    return cudaMemcpyAsync(w->dbuf + at, src, bytes, cudaMemcpyHostToDevice, st);
+  };
   for (int k = 0; k < nin; ++k) {
     if (!*ins[k]) continue;
-    size_t bytes = in_n[k] * sizeof(double);
-    CK(cudaMemcpyAsync(p, *ins[k], bytes, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync(H2D)");
-    *ins[k] = reinterpret_cast<const double*>(p);
-    p += al(bytes);
+    const double* dp = reinterpret_cast<const double*>(w->dbuf + off);
+    CK(put(*ins[k], in_n[k] * sizeof(double)), "cudaMemcpyAsync(H2D)");
+    *ins[k] = dp;
   }
   if (d.icseed) {
-    size_t bytes = fs.n1 * sizeof(int32_t);
-    CK(cudaMemcpyAsync(p, d.icseed, bytes, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync(H2D)");
-    d.icseed = reinterpret_cast<const int32_t*>(p);
-    p += al(bytes);
+    const int32_t* dp = reinterpret_cast<const int32_t*>(w->dbuf + off);
+    CK(put(d.icseed, fs.n1 * sizeof(int32_t)), "cudaMemcpyAsync(H2D)");
+    d.icseed = dp;
   }
+  if (staged) CK(up.send(off), "cudaMemcpyAsync(H2D)");
+  const size_t out0 = off;
   double* host_out[N_OUT];
   for (int k = 0; k < nout; ++k) {
     host_out[k] = *outs[k];
     if (!*outs[k]) continue;
-    *outs[k] = reinterpret_cast<double*>(p);
-    p += al(out_n[k] * sizeof(double));
+    *outs[k] = reinterpret_cast<double*>(w->dbuf + off);
+    off += al(out_n[k] * sizeof(double));
   }
   Block B;
   block_from_args(&d, &B);
@@ -811,6 +821,20 @@ extern "C" int rrtmg_lw_gpu_run_ex(const rrtmg_lw_run_args* a, const rrtmg_lw_ex
   int r = launch(w, st, &B, 1, a->npts, f, kp, default_shape(kp, pick_v(f.nlay)), x->kernel_ms, errmsg,
                  errmsg_len);
   if (r) return r;
+  if (staged) {
+    CK(cudaMemcpyAsync(w->stage.p + out0, w->dbuf + out0, off - out0, cudaMemcpyDeviceToHost, st),
+       "cudaMemcpyAsync(D2H)");
+    CK(cudaStreamSynchronize(st), "kernel execution");
+    const size_t ld = a->ldim > 0 ? (size_t)a->ldim : (size_t)a->npts, np = (size_t)a->npts, L = (size_t)a->nlay;
+    const size_t width[] = {1, 2, 4, 1, 1, 1, 4}, rows[] = {L, 0, 0, L, L, L * NBANDS, L + 1};   // 0: per-column records
+    for (int k = 0; k < nout; ++k) {
+      if (!host_out[k]) continue;
+      const char* src = w->stage.p + (reinterpret_cast<char*>(*outs[k]) - w->dbuf);
+      if (rows[k]) copy_rows(host_out[k], src, rows[k], ld, np, width[k] * sizeof(double));
+      else std::memcpy(host_out[k], src, np * width[k] * sizeof(double));
+    }
+    return 0;
+  }
   for (int k = 0; k < nout; ++k) {
     if (!host_out[k]) continue;
     CK(cudaMemcpyAsync(host_out[k], *outs[k], out_n[k] * sizeof(double), cudaMemcpyDeviceToHost, st),
@@ -1110,6 +1134,7 @@ extern "C" void rrtmg_lw_gpu_finalize(void) {
     for (GraphEntry* e : w->graphs) drop_graph(e);
     w->graphs.clear();
     if (w->dbuf) cudaFree(w->dbuf);
+    w->stage.release();
     if (w->pbuf) cudaFree(w->pbuf);
     if (w->h2d) cudaStreamDestroy(w->h2d);
     if (w->d2h) cudaStreamDestroy(w->d2h);

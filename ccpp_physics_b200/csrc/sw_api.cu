@@ -19,6 +19,7 @@
 
 #include "../../include/rrtmg_sw_gpu.h"
 #include "../data/rrtmg_sw_table_layout.h"
+#include "host_stage.h"
 #include "lw_common.cuh"
 #include "lw_launch.h"
 #include "sw_kernels.h"
@@ -57,6 +58,7 @@ struct SwWorkspace {
   size_t pbuf_bytes = 0;
   // physics blocks: the block table, its prefixes and the point table on the
   // device, and the host copies they are uploaded from
+  HostStage pin;   // pinned staging of small host-array calls
   char* btab = nullptr;
   size_t btab_bytes = 0;
   std::vector<sw::SwArgs> h_tab;
@@ -313,15 +315,16 @@ int run_device(SwWorkspace* w, const sw::SwArgs& d, int nday, cudaStream_t st, f
   return 0;
 }
 
+int bad_day(int bad, char* errmsg, int32_t errmsg_len) {
+  if (!bad) return 0;
+  set_msg(errmsg, errmsg_len, "rrtmg_sw_gpu: idxday names a column outside 1..npts (those points were skipped)");
+  return 1;
+}
 int check_bad(SwWorkspace* w, cudaStream_t st, char* errmsg, int32_t errmsg_len) {
   int bad = 0;
   CK(cudaMemcpyAsync(&bad, w->bad, sizeof(int), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
   CK(cudaStreamSynchronize(st), "kernel execution");
-  if (bad) {
-    set_msg(errmsg, errmsg_len, "rrtmg_sw_gpu: idxday names a column outside 1..npts (those points were skipped)");
-    return 1;
-  }
-  return 0;
+  return bad_day(bad, errmsg, errmsg_len);
 }
 
 // Host arrays of many columns: chunks of kSwHostChunk columns, double-
@@ -552,25 +555,32 @@ extern "C" int rrtmg_sw_gpu_run_ex(const rrtmg_sw_run_args* a, const rrtmg_sw_ex
   size_t total = align256(z.np * 4) + align256(z.nd * 4);
   for (auto& p : ins) if (*p.first) total += align256(p.second * 8);
   for (auto& p : outs) if (*p.p) total += align256(p.n * 8);
+  CK(cudaStreamSynchronize(st), "cudaStreamSynchronize");   // an earlier call that failed may still read the staging
   CK(grow(&w->stage, &w->stage_bytes, total), "staging allocation");
+  const bool staged = w->pin.ensure(total + 256);   // and the flag of a bad idxday
+  HostGather up{w->pin.p, w->stage, st};
   size_t off = 0;
   auto place = [&](size_t bytes) { char* p = w->stage + off; off += align256(bytes); return p; };
+  auto put = [&](const void* src, size_t bytes, cudaError_t* e) {   // the next field of the device buffer
+    const size_t at = off;
+    char* p = place(bytes);
+    *e = staged ? up.put(at, src, bytes, off) : cudaMemcpyAsync(p, src, bytes, cudaMemcpyHostToDevice, st);
+    return p;
+  };
+  cudaError_t ce = cudaSuccess;
   if (a->icseed) {
-    int32_t* p = (int32_t*)place(z.np * 4);
-    CK(cudaMemcpyAsync(p, a->icseed, z.np * 4, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync");
-    da.icseed = p;
+    da.icseed = (int32_t*)put(a->icseed, z.np * 4, &ce);
+    CK(ce, "cudaMemcpyAsync");
   }
-  {
-    int32_t* p = (int32_t*)place(z.nd * 4);
-    CK(cudaMemcpyAsync(p, a->idxday, z.nd * 4, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync");
-    da.idxday = p;
-  }
+  da.idxday = (int32_t*)put(a->idxday, z.nd * 4, &ce);
+  CK(ce, "cudaMemcpyAsync");
   for (auto& p : ins) {
     if (!*p.first) continue;
-    double* d = (double*)place(p.second * 8);
-    CK(cudaMemcpyAsync(d, *p.first, p.second * 8, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync");
-    *p.first = d;
+    *p.first = (double*)put(*p.first, p.second * 8, &ce);
+    CK(ce, "cudaMemcpyAsync");
   }
+  if (staged) CK(up.send(off), "cudaMemcpyAsync");
+  const size_t out0 = off;
   struct Back { double* host; double* dev; Out o; };
   std::vector<Back> back;
   for (auto& p : outs) {
@@ -582,6 +592,18 @@ extern "C" int rrtmg_sw_gpu_run_ex(const rrtmg_sw_run_args* a, const rrtmg_sw_ex
   sw::SwArgs d = device_args(&da);
   int r = run_device(w, d, a->nday, st, x->kernel_ms, errmsg, errmsg_len, z);
   if (r) return r;
+  if (staged) {
+    int* bad = (int*)(w->pin.p + total);
+    CK(cudaMemcpyAsync(w->pin.p + out0, w->stage + out0, off - out0, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
+    CK(cudaMemcpyAsync(bad, w->bad, sizeof(int), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
+    CK(cudaStreamSynchronize(st), "kernel execution");
+    for (const Back& b : back) {
+      const char* src = w->pin.p + ((char*)b.dev - w->stage);
+      if (b.o.w == 0) std::memcpy(b.host, src, b.o.n * 8);
+      else copy_rows(b.host, src, b.o.rows, ldz, (size_t)a->npts, b.o.w * 8);
+    }
+    return bad_day(*bad, errmsg, errmsg_len);
+  }
   for (const Back& b : back) {
     if (b.o.w == 0) {   // per-column records: exactly npts of them
       CK(cudaMemcpyAsync(b.host, b.dev, b.o.n * 8, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
@@ -772,6 +794,7 @@ extern "C" void rrtmg_sw_gpu_finalize(void) {
     if (w->stream) cudaStreamSynchronize(w->stream);
     cudaFree(w->scratch);
     cudaFree(w->stage);
+    w->pin.release();
     cudaFree(w->bad);
     cudaFree(w->pbuf);
     cudaFree(w->btab);
