@@ -37,6 +37,7 @@ struct SwState {
   bool ready = false;
   int device = 0, num_sms = 0;
   double* tab = nullptr;     // coefficient blob
+  double* ktab = nullptr;    // the same, g-point fastest in the k-tables
   double* etab = nullptr;    // exp_tbl(0:NTBMX)
   double heatfac = 0.0;
 };
@@ -286,7 +287,7 @@ int run_device(SwWorkspace* w, const sw::SwArgs& d, int nday, cudaStream_t st, f
     s.bad = w->bad;
     const bool first = kernel_ms && p0 == 0;
     if (first) CK(cudaEventRecord(ev[0], st), "cudaEventRecord");
-    CK(sw::optics_launch(d, s, p0, nc, g.tab, st), "optics kernel launch");
+    CK(sw::optics_launch(d, s, p0, nc, g.tab, g.ktab, st), "optics kernel launch");
     if (first) CK(cudaEventRecord(ev[1], st), "cudaEventRecord");
     lw::McicaStage ms;
     ms.cldf = s.cldf;
@@ -494,6 +495,11 @@ extern "C" int rrtmg_sw_gpu_init(const rrtmg_sw_init_args* a, char* errmsg, int3
     }
     CK(cudaMalloc((void**)&g.tab, nb), "cudaMalloc tables");
     CK(cudaMemcpy(g.tab, rrtmg_sw_tables_blob, nb, cudaMemcpyHostToDevice), "table upload");
+    std::vector<double> k(RRTMG_SW_TABLES_NDOUBLE);
+    std::memcpy(k.data(), rrtmg_sw_tables_blob, nb);
+    sw::gpoint_fastest(k.data());
+    CK(cudaMalloc((void**)&g.ktab, nb), "cudaMalloc tables");
+    CK(cudaMemcpy(g.ktab, k.data(), nb, cudaMemcpyHostToDevice), "table upload");
     CK(cudaMalloc((void**)&g.etab, (kNtbmx + 1) * 8), "cudaMalloc exp_tbl");
     int max_smem = 0;
     CK(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, g.device), "cudaDeviceGetAttribute");
@@ -641,7 +647,7 @@ extern "C" int rrtmg_sw_gpu_gas_optics(const rrtmg_sw_run_args* a, double* taug,
   s.bad = w->bad;
   d.gas_only = 1;
   CK(cudaMemsetAsync(w->bad, 0, sizeof(int), st), "cudaMemsetAsync");
-  CK(sw::optics_launch(d, s, 0, nday, g.tab, st), "optics kernel launch");
+  CK(sw::optics_launch(d, s, 0, nday, g.tab, g.ktab, st), "optics kernel launch");
   CK(sw::gas_unpack_launch(s, nday, nlay, g.tab, taug, taur, st), "unpacking kernel launch");
   CK(cudaMemcpyAsync(sfluxzen, s.sflux, (size_t)nday * sw::kSwNg * 8, cudaMemcpyDeviceToDevice, st), "cudaMemcpyAsync");
   return check_bad(w, st, errmsg, errmsg_len);
@@ -721,7 +727,7 @@ extern "C" int rrtmg_sw_gpu_run_blocks(const rrtmg_sw_run_args* blocks, int32_t 
     sc.bad = w->bad;
     const bool first_chunk = kms && p0 == 0;
     if (first_chunk) CK(cudaEventRecord(ev[0], st), "cudaEventRecord");
-    CK(sw::optics_blocks_launch(d_tab, d_pts, sc, p0, nc, g.tab, st), "optics kernel launch");
+    CK(sw::optics_blocks_launch(d_tab, d_pts, sc, p0, nc, nlay, g.tab, g.ktab, st), "optics kernel launch");
     if (first_chunk) CK(cudaEventRecord(ev[1], st), "cudaEventRecord");
     lw::McicaStage ms;
     ms.cldf = sc.cldf;
@@ -811,6 +817,7 @@ extern "C" void rrtmg_sw_gpu_finalize(void) {
   g_ws.clear();
   tl_ws = nullptr;
   if (g.tab) cudaFree(g.tab);
+  if (g.ktab) cudaFree(g.ktab);
   if (g.etab) cudaFree(g.etab);
   g = SwState{};
 }

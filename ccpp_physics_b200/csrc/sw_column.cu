@@ -3,7 +3,7 @@
 // rrtmg_sw_run (physics/Radiation/RRTMG/radsw_main.F90:493-1379, RSM below)
 // for the McICA configurations runs as three launches over a chunk of
 // daytime columns:
-//   sw_optics_kernel  one warp per column, lanes over layers: the driver's
+//   sw_optics_kernel  one warp per 32 layers of a column, a lane per layer: the driver's
 //                     layer prologue (RSM:910-1094), setcoef (RSM:2242-2389),
 //                     taumol16..29 (RSM:4094-5573; every lane runs the same
 //                     band's code, so the band branches never diverge),
@@ -20,6 +20,8 @@
 // enough (see sw_rt_kernel).
 #include <cstdint>
 #include <cstdio>
+#include <vector>
+
 #include <cuda_runtime.h>
 
 #include "fp64_util.cuh"
@@ -32,8 +34,6 @@ using namespace fp64;
 
 __constant__ int c_ng[14] = {6, 12, 8, 8, 10, 10, 2, 10, 8, 6, 6, 8, 6, 12};   // radsw_param.f NG16..29
 __constant__ int c_ns[14] = {0, 6, 18, 26, 34, 44, 54, 56, 66, 74, 80, 86, 94, 100};
-__constant__ int c_nspa[14] = {9, 9, 9, 9, 1, 9, 9, 1, 9, 1, 0, 1, 9, 1};      // RSM:359
-__constant__ int c_nspb[14] = {1, 5, 1, 1, 1, 5, 1, 0, 1, 0, 0, 1, 5, 1};      // RSM:360
 __constant__ int c_idxsfc[14] = {1, 1, 1, 1, 1, 1, 1, 1, 0, 2, 2, 2, 2, 1};    // RSM:362
 __constant__ int c_idxebc[14] = {5, 5, 4, 4, 3, 3, 2, 2, 1, 1, 1, 1, 1, 5};    // RSM:363
 
@@ -58,6 +58,12 @@ struct Lay {
   int jp, jt, jt1, indfor, indself;
   bool lower_plog;   // plog > 4.56
 };
+
+// ln p > 4.56 (RSM:2305): p against e^4.56 = 95.58347983, by the logarithm
+// itself where rounding could decide.
+__device__ __forceinline__ bool lower_atm(double p) {
+  return (p > 95.5834 && p < 95.5836) ? log(p) > 4.56 : p > 95.5835;
+}
 
 // rrtmg_sw_run's layer prologue (RSM:910-946 / 1001-1040) for internal
 // layer k (0-based, surface first) of caller column i, then setcoef.
@@ -120,20 +126,59 @@ __device__ void layer_record(const SwArgs& a, int i, int k, const double* __rest
 }
 
 // ---- taumol for one layer, every g-point (RSM:4094-5573) ------------------
-// Table views with Fortran subscripts: ka(ind, j) of a (rows, ng) array.
-struct Tab {
-  const double* p;
-  int rows;
-  __device__ __forceinline__ double operator()(int ind, int j) const { return __ldg(p + (ind - 1) + rows * (j - 1)); }
+// Two g-points at a time: every band has an even number of them, and in the
+// device copy of the k-tables (rswinit's, g-point fastest; sw_api.cu) a pair is
+// one 16-byte gather from the layer's row.  With the tables as the reference
+// holds them (row fastest) each g-point of a row is a sector of its own.  With
+// a warp per 32 layers instead of per column: 16,384 x 127, 3.85 -> 2.6 ms; 57 x
+// 127, 187 -> 74 us.
+struct D2 {
+  double x, y;
 };
+__device__ __forceinline__ D2 operator+(D2 a, D2 b) { return {a.x + b.x, a.y + b.y}; }
+__device__ __forceinline__ D2 operator-(D2 a, D2 b) { return {a.x - b.x, a.y - b.y}; }
+__device__ __forceinline__ D2 operator*(double a, D2 b) { return {a * b.x, a * b.y}; }
+__device__ __forceinline__ D2 operator+(D2 a, double b) { return {a.x + b, a.y + b}; }
+
+// bands 16..29 as 0..13 (radsw_param.f NG16..29, RSM:359-360)
+__host__ __device__ constexpr int ng_of(int b) {
+  return b == 0 ? 6 : b == 1 ? 12 : b == 2 || b == 3 ? 8 : b == 4 || b == 5 ? 10 : b == 6 ? 2 : b == 7 ? 10
+       : b == 8 ? 8 : b == 9 || b == 10 ? 6 : b == 11 ? 8 : b == 12 ? 6 : 12;
+}
+__host__ __device__ constexpr int ns_of(int b) { return b == 0 ? 0 : ns_of(b - 1) + ng_of(b - 1); }
+__host__ __device__ constexpr int nspa_of(int b) { return b == 4 || b == 7 || b == 9 || b == 11 || b == 13 ? 1 : b == 10 ? 0 : 9; }
+__host__ __device__ constexpr int nspb_of(int b) {
+  return b == 1 || b == 5 || b == 12 ? 5 : b == 7 || b == 9 || b == 10 ? 0 : 1;
+}
+
+// k-table view with Fortran row subscripts: the pair (j, j + 1) of row ind.
+// ODD: a layer whose jp lies on the other side of the split than the layer
+// itself (an inverted pressure profile, or a column without a lower layer, where
+// laytrop is nlay) has rows beyond its tables; it reads what the reference's
+// subscripts reach in the blob as it stands.
+template <int NG, int ROWS, bool ODD>
+struct Tab {
+  const double* p;   // in the blob if ODD, else in its copy with the g-point fastest
+  __device__ __forceinline__ D2 operator()(int ind, int j) const {
+    if (ODD) return {__ldg(p + (ind - 1) + ROWS * (j - 1)), __ldg(p + (ind - 1) + ROWS * j)};
+    const double2 v = __ldg(reinterpret_cast<const double2*>(p + (ind - 1) * NG + (j - 1)));
+    return {v.x, v.y};
+  }
+};
+__device__ __forceinline__ D2 pair_at(const double* p, int j) {
+  const double2 v = __ldg(reinterpret_cast<const double2*>(p + (j - 1)));
+  return {v.x, v.y};
+}
 
 // the eight-point binary-species interpolation (fac000*k(i01) + fac100*k(i01+1)
 // + fac010*k(i01+d) + fac110*k(i01+d+1) + the same at i11), left to right
-__device__ __forceinline__ double k8(const Tab& t, const double (&f)[8], int i01, int d, int i11, int j) {
+template <int NG, int ROWS, bool ODD>
+__device__ __forceinline__ D2 k8(const Tab<NG, ROWS, ODD>& t, const double (&f)[8], int i01, int d, int i11, int j) {
   return f[0] * t(i01, j) + f[2] * t(i01 + 1, j) + f[1] * t(i01 + d, j) + f[3] * t(i01 + d + 1, j) +
          f[4] * t(i11, j) + f[6] * t(i11 + 1, j) + f[5] * t(i11 + d, j) + f[7] * t(i11 + d + 1, j);
 }
-__device__ __forceinline__ double k4(const Tab& t, const Lay& L, int i01, int i11, int j) {
+template <int NG, int ROWS, bool ODD>
+__device__ __forceinline__ D2 k4(const Tab<NG, ROWS, ODD>& t, const Lay& L, int i01, int i11, int j) {
   return L.fac00 * t(i01, j) + L.fac10 * t(i01 + 1, j) + L.fac01 * t(i11, j) + L.fac11 * t(i11 + 1, j);
 }
 // speccomb/specmult/js/fs and the eight weights (RSM:4386-4399)
@@ -154,152 +199,196 @@ __device__ __forceinline__ double spec8(const Lay& L, int g1, int g2, double str
   f[7] = fs * L.fac11;
   return speccomb;
 }
-__device__ __forceinline__ double selfc(const Tab& s, const Lay& L, int j) {
+template <int NG, int ROWS, bool ODD>
+__device__ __forceinline__ D2 selfc(const Tab<NG, ROWS, ODD>& s, const Lay& L, int j) {
   const int a = L.indself, b = a + 1;
   return L.selffac * (s(a, j) + L.selffrac * (s(b, j) - s(a, j)));
 }
-__device__ __forceinline__ double forc(const Tab& f, const Lay& L, int j) {
+template <int NG, int ROWS, bool ODD>
+__device__ __forceinline__ D2 forc(const Tab<NG, ROWS, ODD>& f, const Lay& L, int j) {
   const int a = L.indfor, b = a + 1;
   return L.forfac * (f(a, j) + L.forfrac * (f(b, j) - f(a, j)));
 }
+// first table rows of a band (RSM:4187-4202)
+template <int B>
+__device__ __forceinline__ int row0(const Lay& L, bool lower) {
+  return lower ? ((L.jp - 1) * 5 + (L.jt - 1)) * nspa_of(B) : ((L.jp - 13) * 5 + (L.jt - 1)) * nspb_of(B);
+}
+template <int B>
+__device__ __forceinline__ int row1(const Lay& L, bool lower) {
+  return lower ? (L.jp * 5 + (L.jt1 - 1)) * nspa_of(B) : ((L.jp - 12) * 5 + (L.jt1 - 1)) * nspb_of(B);
+}
+// band B's values of g-points j, j + 1
+template <int B>
+__device__ __forceinline__ void put(double* tg, int j, D2 v) {
+  tg[kTgStride * (ns_of(B) + j - 1)] = v.x;
+  tg[kTgStride * (ns_of(B) + j)] = v.y;
+}
 
-__device__ void taumol_layer(const Lay& L, bool lower, const int id0[14], const int id1[14],
-                             const double* __restrict__ T, double* __restrict__ tg, double* __restrict__ t24) {
+// bands 16, 17, 18, 19, 21, 22: binary species in the lower atmosphere (and
+// above in 17 and 21); absa at table offset A, absb AB, selfref S, forref F
+template <bool ODD, int B, int G2, int A, int AB, int S, int F>
+__device__ __forceinline__ void binary_band(const Lay& L, bool lower, const double* __restrict__ T,
+                                            const double* __restrict__ K, double* __restrict__ tg) {
+  constexpr int ng = ng_of(B);
+  constexpr double o2tem = 4.35e-4 / (350.0 * 2.0), o2adj = 1.6;
+  const Tab<ng, 585, ODD> absa{K + A};
+  const Tab<ng, B == 1 || B == 5 ? 1175 : 235, ODD> absb{K + AB};
+  const Tab<ng, 10, ODD> selfref{K + S};
+  const Tab<ng, B == 1 || B == 5 ? 4 : 3, ODD> forref{K + F};
+  const int id0 = row0<B>(L, lower), id1 = row1<B>(L, lower);
   int js;
   double fs, f[8];
-  const double* strr = T + swtab::strrat;
-  const double o2tem = 4.35e-4 / (350.0 * 2.0), o2adj = 1.6;
-  // bands 16, 17, 18, 19, 21, 22: binary species in the lower atmosphere
-  {
-    const int bands[6] = {0, 1, 2, 3, 5, 6};
-    const int g2s[6] = {4, 1, 4, 1, 1, 5};
-    const int oa[6] = {swtab::b16_absa, swtab::b17_absa, swtab::b18_absa, swtab::b19_absa, swtab::b21_absa,
-                       swtab::b22_absa};
-    const int ob[6] = {swtab::b16_absb, swtab::b17_absb, swtab::b18_absb, swtab::b19_absb, swtab::b21_absb,
-                       swtab::b22_absb};
-    const int os[6] = {swtab::b16_selfref, swtab::b17_selfref, swtab::b18_selfref, swtab::b19_selfref,
-                       swtab::b21_selfref, swtab::b22_selfref};
-    const int of[6] = {swtab::b16_forref, swtab::b17_forref, swtab::b18_forref, swtab::b19_forref,
-                       swtab::b21_forref, swtab::b22_forref};
-    const int mfr[6] = {3, 4, 3, 3, 4, 3};
+  if (lower) {
+    const double speccomb = spec8(L, 0, G2, T[swtab::strrat + B], 8.0, js, fs, f);
+    const int i01 = id0 + js, i11 = id1 + js;
+    const double o2cont = o2tem * L.colamt[5];
 #pragma unroll 1
-    for (int q = 0; q < 6; ++q) {
-      const int b = bands[q], ns = c_ns[b], ng = c_ng[b];
-      const Tab absa{T + oa[q], 585}, selfref{T + os[q], 10}, forref{T + of[q], mfr[q]};
-      const Tab absb{T + ob[q], (b == 1 || b == 5) ? 1175 : 235};
-      if (lower) {
-        const double speccomb = spec8(L, 0, g2s[q], strr[b], 8.0, js, fs, f);
-        const int i01 = id0[b] + js, i11 = id1[b] + js;
-        const double o2cont = o2tem * L.colamt[5];
-        for (int j = 1; j <= ng; ++j) {
-          double t = speccomb * k8(absa, f, i01, 9, i11, j) + L.colamt[0] * (selfc(selfref, L, j) + forc(forref, L, j));
-          if (b == 6) t = t + o2cont;
-          tg[kTgStride * (ns + j - 1)] = t;
-        }
-      } else if (b == 1 || b == 5) {   // 17, 21: binary species above too
-        const double speccomb = spec8(L, 0, 1, strr[b], 4.0, js, fs, f);
-        const int i01 = id0[b] + js, i11 = id1[b] + js;
-        for (int j = 1; j <= ng; ++j) {
-          const int a0 = L.indfor, a1 = a0 + 1;
-          tg[kTgStride * (ns + j - 1)] = speccomb * k8(absb, f, i01, 5, i11, j) +
-                           L.colamt[0] * L.forfac * (forref(a0, j) + L.forfrac * (forref(a1, j) - forref(a0, j)));
-        }
-      } else {
-        const int i01 = id0[b] + 1, i11 = id1[b] + 1;
-        const double o2cont = o2tem * L.colamt[5];
-        for (int j = 1; j <= ng; ++j) {
-          if (b == 6) tg[kTgStride * (ns + j - 1)] = L.colamt[5] * o2adj * k4(absb, L, i01, i11, j) + o2cont;
-          else tg[kTgStride * (ns + j - 1)] = L.colamt[b == 3 ? 1 : 4] * k4(absb, L, i01, i11, j);
-        }
-      }
+    for (int j = 1; j <= ng; j += 2) {
+      D2 t = speccomb * k8(absa, f, i01, 9, i11, j) + L.colamt[0] * (selfc(selfref, L, j) + forc(forref, L, j));
+      if (B == 6) t = t + o2cont;
+      put<B>(tg, j, t);
+    }
+  } else if (B == 1 || B == 5) {
+    const double speccomb = spec8(L, 0, 1, T[swtab::strrat + B], 4.0, js, fs, f);
+    const int i01 = id0 + js, i11 = id1 + js;
+#pragma unroll 1
+    for (int j = 1; j <= ng; j += 2) {
+      const int a0 = L.indfor, a1 = a0 + 1;
+      put<B>(tg, j, speccomb * k8(absb, f, i01, 5, i11, j) +
+                        L.colamt[0] * L.forfac * (forref(a0, j) + L.forfrac * (forref(a1, j) - forref(a0, j))));
+    }
+  } else {
+    const int i01 = id0 + 1, i11 = id1 + 1;
+    const double o2cont = o2tem * L.colamt[5];
+#pragma unroll 1
+    for (int j = 1; j <= ng; j += 2) {
+      if (B == 6) put<B>(tg, j, L.colamt[5] * o2adj * k4(absb, L, i01, i11, j) + o2cont);
+      else put<B>(tg, j, L.colamt[B == 3 ? 1 : 4] * k4(absb, L, i01, i11, j));
     }
   }
+}
+
+// T = the coefficient blob, K = its copy with the g-point fastest in the k-tables (ODD: the blob itself)
+template <bool ODD>
+__device__ void taumol_layer(const Lay& L, bool lower, const double* __restrict__ T, const double* __restrict__ K,
+                             double* __restrict__ tg, double* __restrict__ t24) {
+  int js;
+  double fs, f[8];
+  using namespace swtab;
+  binary_band<ODD, 0, 4, b16_absa, b16_absb, b16_selfref, b16_forref>(L, lower, T, K, tg);
+  binary_band<ODD, 1, 1, b17_absa, b17_absb, b17_selfref, b17_forref>(L, lower, T, K, tg);
+  binary_band<ODD, 2, 4, b18_absa, b18_absb, b18_selfref, b18_forref>(L, lower, T, K, tg);
+  binary_band<ODD, 3, 1, b19_absa, b19_absb, b19_selfref, b19_forref>(L, lower, T, K, tg);
+  binary_band<ODD, 5, 1, b21_absa, b21_absb, b21_selfref, b21_forref>(L, lower, T, K, tg);
+  binary_band<ODD, 6, 5, b22_absa, b22_absb, b22_selfref, b22_forref>(L, lower, T, K, tg);
   {  // band 20: H2O, CH4
-    const int b = 4, ns = c_ns[b];
-    const Tab absa{T + swtab::b20_absa, 65}, absb{T + swtab::b20_absb, 235}, selfref{T + swtab::b20_selfref, 10},
-        forref{T + swtab::b20_forref, 4};
-    const double* absch4 = T + swtab::b20_absch4;
-    const int i01 = id0[b] + 1, i11 = id1[b] + 1;
-    for (int j = 1; j <= 10; ++j) {
-      if (lower)
-        tg[kTgStride * (ns + j - 1)] = L.colamt[0] * (k4(absa, L, i01, i11, j) + selfc(selfref, L, j) + forc(forref, L, j)) +
-                         L.colamt[4] * __ldg(absch4 + j - 1);
-      else
-        tg[kTgStride * (ns + j - 1)] = L.colamt[0] * (k4(absb, L, i01, i11, j) + forc(forref, L, j)) + L.colamt[4] * __ldg(absch4 + j - 1);
+    constexpr int b = 4, ng = ng_of(b);
+    const Tab<ng, 65, ODD> absa{K + b20_absa};
+    const Tab<ng, 235, ODD> absb{K + b20_absb};
+    const Tab<ng, 10, ODD> selfref{K + b20_selfref};
+    const Tab<ng, 4, ODD> forref{K + b20_forref};
+    const int i01 = row0<b>(L, lower) + 1, i11 = row1<b>(L, lower) + 1;
+#pragma unroll 1
+    for (int j = 1; j <= ng; j += 2) {
+      const D2 ch4 = L.colamt[4] * pair_at(K + b20_absch4, j);
+      if (lower) put<b>(tg, j, L.colamt[0] * (k4(absa, L, i01, i11, j) + selfc(selfref, L, j) + forc(forref, L, j)) + ch4);
+      else put<b>(tg, j, L.colamt[0] * (k4(absb, L, i01, i11, j) + forc(forref, L, j)) + ch4);
     }
   }
   {  // band 23: H2O below, nothing above
-    const int b = 7, ns = c_ns[b];
-    const Tab absa{T + swtab::b23_absa, 65}, selfref{T + swtab::b23_selfref, 10}, forref{T + swtab::b23_forref, 3};
-    const double givfac = T[swtab::b23_givfac];
-    const int i01 = id0[b] + 1, i11 = id1[b] + 1;
-    for (int j = 1; j <= 10; ++j)
-      tg[kTgStride * (ns + j - 1)] = lower ? L.colamt[0] * (givfac * k4(absa, L, i01, i11, j) + selfc(selfref, L, j) + forc(forref, L, j))
-                             : 0.0;
+    constexpr int b = 7, ng = ng_of(b);
+    const Tab<ng, 65, ODD> absa{K + b23_absa};
+    const Tab<ng, 10, ODD> selfref{K + b23_selfref};
+    const Tab<ng, 3, ODD> forref{K + b23_forref};
+    const double givfac = T[b23_givfac];
+    const int i01 = row0<b>(L, lower) + 1, i11 = row1<b>(L, lower) + 1;
+#pragma unroll 1
+    for (int j = 1; j <= ng; j += 2)
+      put<b>(tg, j, lower ? L.colamt[0] * (givfac * k4(absa, L, i01, i11, j) + selfc(selfref, L, j) + forc(forref, L, j))
+                          : D2{0.0, 0.0});
   }
   {  // band 24: H2O/O2 below, O2 above; O3 both; Rayleigh from the species bin
-    const int b = 8, ns = c_ns[b];
-    const Tab absa{T + swtab::b24_absa, 585}, absb{T + swtab::b24_absb, 235}, selfref{T + swtab::b24_selfref, 10},
-        forref{T + swtab::b24_forref, 3};
-    const double *abso3a = T + swtab::b24_abso3a, *abso3b = T + swtab::b24_abso3b, *rayla = T + swtab::b24_rayla,
-                 *raylb = T + swtab::b24_raylb;
+    constexpr int b = 8, ng = ng_of(b);
+    const Tab<ng, 585, ODD> absa{K + b24_absa};
+    const Tab<ng, 235, ODD> absb{K + b24_absb};
+    const Tab<ng, 10, ODD> selfref{K + b24_selfref};
+    const Tab<ng, 3, ODD> forref{K + b24_forref};
     if (lower) {
-      const double speccomb = spec8(L, 0, 5, strr[b], 8.0, js, fs, f);
-      const int i01 = id0[b] + js, i11 = id1[b] + js;
-      for (int j = 1; j <= 8; ++j) {
-        tg[kTgStride * (ns + j - 1)] = speccomb * k8(absa, f, i01, 9, i11, j) + L.colamt[2] * __ldg(abso3a + j - 1) +
-                         L.colamt[0] * (selfc(selfref, L, j) + forc(forref, L, j));
-        const double ra = __ldg(rayla + (j - 1) + 8 * (js - 1)), rb = __ldg(rayla + (j - 1) + 8 * js);
-        t24[j - 1] = L.colmol * (ra + fs * (rb - ra));
+      const double speccomb = spec8(L, 0, 5, T[strrat + b], 8.0, js, fs, f);
+      const int i01 = row0<b>(L, lower) + js, i11 = row1<b>(L, lower) + js;
+#pragma unroll 1
+      for (int j = 1; j <= ng; j += 2) {
+        put<b>(tg, j, speccomb * k8(absa, f, i01, 9, i11, j) + L.colamt[2] * pair_at(K + b24_abso3a, j) +
+                          L.colamt[0] * (selfc(selfref, L, j) + forc(forref, L, j)));
+        const D2 ra = pair_at(K + b24_rayla + 8 * (js - 1), j), rb = pair_at(K + b24_rayla + 8 * js, j);
+        const D2 r = L.colmol * (ra + fs * (rb - ra));
+        t24[j - 1] = r.x;
+        t24[j] = r.y;
       }
     } else {
-      const int i01 = id0[b] + 1, i11 = id1[b] + 1;
-      for (int j = 1; j <= 8; ++j) {
-        tg[kTgStride * (ns + j - 1)] = L.colamt[5] * k4(absb, L, i01, i11, j) + L.colamt[2] * __ldg(abso3b + j - 1);
-        t24[j - 1] = L.colmol * __ldg(raylb + j - 1);
+      const int i01 = row0<b>(L, lower) + 1, i11 = row1<b>(L, lower) + 1;
+#pragma unroll 1
+      for (int j = 1; j <= ng; j += 2) {
+        put<b>(tg, j, L.colamt[5] * k4(absb, L, i01, i11, j) + L.colamt[2] * pair_at(K + b24_abso3b, j));
+        const D2 r = L.colmol * pair_at(K + b24_raylb, j);
+        t24[j - 1] = r.x;
+        t24[j] = r.y;
       }
     }
   }
   {  // band 25: H2O below; O3 both
-    const int b = 9, ns = c_ns[b];
-    const Tab absa{T + swtab::b25_absa, 65};
-    const double *abso3a = T + swtab::b25_abso3a, *abso3b = T + swtab::b25_abso3b;
-    const int i01 = id0[b] + 1, i11 = id1[b] + 1;
-    for (int j = 1; j <= 6; ++j)
-      tg[kTgStride * (ns + j - 1)] = lower ? L.colamt[0] * k4(absa, L, i01, i11, j) + L.colamt[2] * __ldg(abso3a + j - 1)
-                             : L.colamt[2] * __ldg(abso3b + j - 1);
+    constexpr int b = 9, ng = ng_of(b);
+    const Tab<ng, 65, ODD> absa{K + b25_absa};
+    const int i01 = row0<b>(L, lower) + 1, i11 = row1<b>(L, lower) + 1;
+#pragma unroll 1
+    for (int j = 1; j <= ng; j += 2)
+      put<b>(tg, j, lower ? L.colamt[0] * k4(absa, L, i01, i11, j) + L.colamt[2] * pair_at(K + b25_abso3a, j)
+                          : L.colamt[2] * pair_at(K + b25_abso3b, j));
   }
-  for (int j = 0; j < 6; ++j) tg[kTgStride * (c_ns[10] + j)] = 0.0;   // band 26: Rayleigh only
+#pragma unroll
+  for (int j = 1; j <= ng_of(10); j += 2) put<10>(tg, j, D2{0.0, 0.0});   // band 26: Rayleigh only
   {  // band 27: O3
-    const int b = 11, ns = c_ns[b];
-    const Tab absa{T + swtab::b27_absa, 65}, absb{T + swtab::b27_absb, 235};
-    const int i01 = id0[b] + 1, i11 = id1[b] + 1;
-    for (int j = 1; j <= 8; ++j)
-      tg[kTgStride * (ns + j - 1)] = L.colamt[2] * (lower ? k4(absa, L, i01, i11, j) : k4(absb, L, i01, i11, j));
+    constexpr int b = 11, ng = ng_of(b);
+    const Tab<ng, 65, ODD> absa{K + b27_absa};
+    const Tab<ng, 235, ODD> absb{K + b27_absb};
+    const int i01 = row0<b>(L, lower) + 1, i11 = row1<b>(L, lower) + 1;
+#pragma unroll 1
+    for (int j = 1; j <= ng; j += 2) put<b>(tg, j, L.colamt[2] * (lower ? k4(absa, L, i01, i11, j) : k4(absb, L, i01, i11, j)));
   }
   {  // band 28: O3/O2 both
-    const int b = 12, ns = c_ns[b];
-    const Tab absa{T + swtab::b28_absa, 585}, absb{T + swtab::b28_absb, 1175};
-    const double speccomb = spec8(L, 2, 5, strr[b], lower ? 8.0 : 4.0, js, fs, f);
-    const int i01 = id0[b] + js, i11 = id1[b] + js;
-    for (int j = 1; j <= 6; ++j)
-      tg[kTgStride * (ns + j - 1)] = speccomb * (lower ? k8(absa, f, i01, 9, i11, j) : k8(absb, f, i01, 5, i11, j));
+    constexpr int b = 12, ng = ng_of(b);
+    const Tab<ng, 585, ODD> absa{K + b28_absa};
+    const Tab<ng, 1175, ODD> absb{K + b28_absb};
+    const double speccomb = spec8(L, 2, 5, T[strrat + b], lower ? 8.0 : 4.0, js, fs, f);
+    const int i01 = row0<b>(L, lower) + js, i11 = row1<b>(L, lower) + js;
+#pragma unroll 1
+    for (int j = 1; j <= ng; j += 2) put<b>(tg, j, speccomb * (lower ? k8(absa, f, i01, 9, i11, j) : k8(absb, f, i01, 5, i11, j)));
   }
   {  // band 29: H2O + CO2 below, CO2 + H2O above
-    const int b = 13, ns = c_ns[b];
-    const Tab absa{T + swtab::b29_absa, 65}, absb{T + swtab::b29_absb, 235}, selfref{T + swtab::b29_selfref, 10},
-        forref{T + swtab::b29_forref, 4};
-    const double *absco2 = T + swtab::b29_absco2, *absh2o = T + swtab::b29_absh2o;
-    const int i01 = id0[b] + 1, i11 = id1[b] + 1;
-    for (int j = 1; j <= 12; ++j) {
+    constexpr int b = 13, ng = ng_of(b);
+    const Tab<ng, 65, ODD> absa{K + b29_absa};
+    const Tab<ng, 235, ODD> absb{K + b29_absb};
+    const Tab<ng, 10, ODD> selfref{K + b29_selfref};
+    const Tab<ng, 4, ODD> forref{K + b29_forref};
+    const int i01 = row0<b>(L, lower) + 1, i11 = row1<b>(L, lower) + 1;
+#pragma unroll 1
+    for (int j = 1; j <= ng; j += 2) {
       if (lower)
-        tg[kTgStride * (ns + j - 1)] = L.colamt[0] * (k4(absa, L, i01, i11, j) + selfc(selfref, L, j) + forc(forref, L, j)) +
-                         L.colamt[1] * __ldg(absco2 + j - 1);
+        put<b>(tg, j, L.colamt[0] * (k4(absa, L, i01, i11, j) + selfc(selfref, L, j) + forc(forref, L, j)) +
+                          L.colamt[1] * pair_at(K + b29_absco2, j));
       else
-        tg[kTgStride * (ns + j - 1)] = L.colamt[1] * k4(absb, L, i01, i11, j) + L.colamt[0] * __ldg(absh2o + j - 1);
+        put<b>(tg, j, L.colamt[1] * k4(absb, L, i01, i11, j) + L.colamt[0] * pair_at(K + b29_absh2o, j));
     }
   }
 }
+
+// a (rows, bands) table of the cloud optics with Fortran subscripts
+struct Rows {
+  const double* p;
+  int rows;
+  __device__ __forceinline__ double operator()(int ind, int j) const { return __ldg(p + (ind - 1) + rows * (j - 1)); }
+};
 
 // ---- cldprop for one layer (RSM:1687-1903) --------------------------------
 __device__ void cloud_layer(const SwArgs& a, size_t x, const double* __restrict__ T, double* __restrict__ tw,
@@ -323,9 +412,9 @@ __device__ void cloud_layer(const SwArgs& a, size_t x, const double* __restrict_
       const double factor = refliq - 1.5;
       const int index = max(1, min(57, (int)factor));
       const double fint = factor - (double)index;
-      const Tab ext{T + (a.iswcliq == 1 ? swtab::extliq1 : swtab::extliq2), 58};
-      const Tab ssa{T + (a.iswcliq == 1 ? swtab::ssaliq1 : swtab::ssaliq2), 58};
-      const Tab asy{T + (a.iswcliq == 1 ? swtab::asyliq1 : swtab::asyliq2), 58};
+      const Rows ext{T + (a.iswcliq == 1 ? swtab::extliq1 : swtab::extliq2), 58};
+      const Rows ssa{T + (a.iswcliq == 1 ? swtab::ssaliq1 : swtab::ssaliq2), 58};
+      const Rows asy{T + (a.iswcliq == 1 ? swtab::asyliq1 : swtab::asyliq2), 58};
       for (int b = 0; b < 14; ++b) {
         const int c = b + 1;
         const double e = fmax(0.0, ext(index, c) + fint * (ext(index + 1, c) - ext(index, c)));
@@ -364,9 +453,9 @@ __device__ void cloud_layer(const SwArgs& a, size_t x, const double* __restrict_
           fint = factor - (double)index;
           rows = 46;
         }
-        const Tab ext{T + (a.iswcice == 2 ? swtab::extice2 : swtab::extice3), rows};
-        const Tab ssa{T + (a.iswcice == 2 ? swtab::ssaice2 : swtab::ssaice3), rows};
-        const Tab asy{T + (a.iswcice == 2 ? swtab::asyice2 : swtab::asyice3), rows};
+        const Rows ext{T + (a.iswcice == 2 ? swtab::extice2 : swtab::extice3), rows};
+        const Rows ssa{T + (a.iswcice == 2 ? swtab::ssaice2 : swtab::ssaice3), rows};
+        const Rows asy{T + (a.iswcice == 2 ? swtab::asyice2 : swtab::asyice3), rows};
         for (int b = 0; b < 14; ++b) {
           const int c = b + 1;
           const double e = fmax(0.0, ext(index, c) + fint * (ext(index + 1, c) - ext(index, c)));
@@ -443,96 +532,107 @@ __global__ void sw_gas_unpack_kernel(SwScratch s, int nc, int nlay, const double
 }
 
 // ---- kernel 1: optics ------------------------------------------------------
-constexpr int kOptWarps = 4;
+constexpr int kOptWarps = 4;   // per CTA
+// 128 registers at 4 CTAs per SM, 16,384 x 127: 2.55 ms, against 3.69, 2.83 and
+// 2.52 ms at 2, 3 and 5 (which slows 1,800 x 64 from 209 to 241 us)
+constexpr int kOptPerSm = 4;
 
-// One column's optics: a = the argument record of the call (or of the
-// physics block) the column belongs to, j1 its 1-based column there.
-__device__ __forceinline__ void optics_body(const SwArgs& a, const SwScratch& s, int pl, int nc, int j1, int lane,
-                                            int* s_jp_w, const double* __restrict__ T) {
-  const int i = j1 - 1, nlay = a.nlay;
+// Optics of 32 layers (segment seg) of one column by one warp, a lane per
+// layer: a = the argument record of the call (or of the physics block) the
+// column belongs to, j1 its 1-based column there.  Each warp finds what the
+// layers share (laytrop, the cloudy fraction) for itself; segment 0 also writes
+// the column's values.  s_col: kSwMaxLay doubles of the warp's.
+__device__ __forceinline__ void optics_body(const SwArgs& a, const SwScratch& s, int pl, int nc, int j1, int seg,
+                                            int lane, double* s_col, const double* __restrict__ T,
+                                            const double* __restrict__ K) {
+  const int i = j1 - 1, nlay = a.nlay, k = 32 * seg + lane;
+  const size_t ld = (size_t)a.ld;
+  auto row = [&](int kk) { return a.top_at_1 ? nlay - 1 - kk : kk; };
   // laytrop: the last layer with ln p > 4.56, nlay if none (RSM:2305, 2353)
   int laytrop = 0;
   for (int k0 = 0; k0 < nlay; k0 += 32) {
-    const int k = k0 + lane;
-    bool hi = false;
-    if (k < nlay) {
-      const int r = a.top_at_1 ? nlay - 1 - k : k;
-      const double plog = log(a.plyr[(size_t)i + (size_t)a.ld * r]);
-      s_jp_w[k] = max(1, min(58, (int)(36.0 - 5.0 * (plog + 0.04))));
-      hi = plog > 4.56;
-    }
+    const int kk = k0 + lane;
+    const bool hi = kk < nlay && lower_atm(a.plyr[i + ld * row(kk)]);
     const unsigned m = __ballot_sync(0xffffffffu, hi);
     if (m) laytrop = k0 + 32 - __clz(m);
   }
   if (laytrop == 0) laytrop = nlay;
-  __syncwarp();
 
-  // gas optics, one layer per lane
-  for (int k = lane; k < nlay; k += 32) {
+  // gas optics
+  if (k < nlay) {
     Lay L;
     layer_record(a, i, k, T, L);
-    const bool lower = (k + 1) <= laytrop;
-    int id0[14], id1[14];
-#pragma unroll
-    for (int b = 0; b < 14; ++b) {
-      if (lower) {
-        id0[b] = ((L.jp - 1) * 5 + (L.jt - 1)) * c_nspa[b];
-        id1[b] = (L.jp * 5 + (L.jt1 - 1)) * c_nspa[b];
-      } else {
-        id0[b] = ((L.jp - 13) * 5 + (L.jt - 1)) * c_nspb[b];
-        id1[b] = ((L.jp - 12) * 5 + (L.jt1 - 1)) * c_nspb[b];
-      }
-    }
     s.colmol[(size_t)pl * nlay + k] = L.colmol;
-    taumol_layer(L, lower, id0, id1, T, s.taug + tg_offset(nlay, pl, k, 0), s.ray24 + ((size_t)pl * nlay + k) * 8);
+    const bool lower = (k + 1) <= laytrop;
+    double *tg = s.taug + tg_offset(nlay, pl, k, 0), *t24 = s.ray24 + ((size_t)pl * nlay + k) * 8;
+    if (lower != (L.jp < 13)) taumol_layer<true>(L, lower, T, T, tg, t24);
+    else taumol_layer<false>(L, lower, T, K, tg, t24);
   }
 
   // solar source per band (RSM:4225-4310), one band per lane
-  if (lane < 14) {
-    const int b = lane, jb = 16 + b, ng = c_ng[b], ns = c_ns[b];
-    const int ibd = (int)T[swtab::ibx + b];
-    double* sf = s.sflux + (size_t)pl * kSwNg + ns;
-    if (jb == 16 || jb == 20 || jb == 23 || jb == 25 || jb == 26 || jb == 29) {
-      for (int j = 0; j < ng; ++j) sf[j] = T[swtab::sfluxref01 + j + 16 * (ibd - 1)];
-    } else if (jb == 27) {
-      for (int j = 0; j < ng; ++j) sf[j] = T[swtab::scalekur] * T[swtab::sfluxref01 + j + 16 * (ibd - 1)];
-    } else {
-      const int lref = (int)T[swtab::layreffr + b];
-      int ks;   // 1-based
-      if (jb == 17 || jb == 28) {
-        ks = nlay;
-        for (int k = laytrop; k <= nlay - 1; ++k)
-          if (s_jp_w[k - 1] < lref && s_jp_w[k] >= lref) { ks = k + 1; break; }
+  if (seg == 0) {
+    int* s_jp = reinterpret_cast<int*>(s_col);
+    for (int kk = lane; kk < nlay; kk += 32) {
+      const double plog = log(a.plyr[i + ld * row(kk)]);
+      s_jp[kk] = max(1, min(58, (int)(36.0 - 5.0 * (plog + 0.04))));
+    }
+    __syncwarp();
+    if (lane < 14) {
+      const int b = lane, jb = 16 + b, ng = c_ng[b], ns = c_ns[b];
+      const int ibd = (int)T[swtab::ibx + b];
+      double* sf = s.sflux + (size_t)pl * kSwNg + ns;
+      if (jb == 16 || jb == 20 || jb == 23 || jb == 25 || jb == 26 || jb == 29) {
+        for (int j = 0; j < ng; ++j) sf[j] = T[swtab::sfluxref01 + j + 16 * (ibd - 1)];
+      } else if (jb == 27) {
+        for (int j = 0; j < ng; ++j) sf[j] = T[swtab::scalekur] * T[swtab::sfluxref01 + j + 16 * (ibd - 1)];
       } else {
-        ks = laytrop;
-        for (int k = 1; k <= laytrop - 1; ++k)
-          if (s_jp_w[k - 1] < lref && s_jp_w[k] >= lref) { ks = k + 1; break; }
-      }
-      Lay L;
-      layer_record(a, i, ks - 1, T, L);
-      const double colm1 = L.colamt[(int)T[swtab::ix1 + b] - 1], colm2 = L.colamt[(int)T[swtab::ix2 + b] - 1];
-      const double speccomb = colm1 + T[swtab::strrat + b] * colm2;
-      const double specmult = T[swtab::specwt + b] * fmin(kOneMinus, colm1 / speccomb);
-      const int js = 1 + (int)specmult;
-      const double fs = fmod(specmult, 1.0);
-      const bool two = (jb == 17 || jb == 28);
-      const double* ref = T + (two ? swtab::sfluxref02 : swtab::sfluxref03);
-      const int nbin = two ? 5 : 9;
-      for (int j = 0; j < ng; ++j) {
-        const double r0 = ref[j + 16 * ((js - 1) + nbin * (ibd - 1))], r1 = ref[j + 16 * (js + nbin * (ibd - 1))];
-        sf[j] = r0 + fs * (r1 - r0);
+        const int lref = (int)T[swtab::layreffr + b];
+        int ks;   // 1-based
+        if (jb == 17 || jb == 28) {
+          ks = nlay;
+          for (int kk = laytrop; kk <= nlay - 1; ++kk)
+            if (s_jp[kk - 1] < lref && s_jp[kk] >= lref) { ks = kk + 1; break; }
+        } else {
+          ks = laytrop;
+          for (int kk = 1; kk <= laytrop - 1; ++kk)
+            if (s_jp[kk - 1] < lref && s_jp[kk] >= lref) { ks = kk + 1; break; }
+        }
+        Lay L;
+        layer_record(a, i, ks - 1, T, L);
+        const int m1 = (int)T[swtab::ix1 + b] - 1, m2 = (int)T[swtab::ix2 + b] - 1;
+        double colm1 = 0.0, colm2 = 0.0;
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+          colm1 = (m == m1) ? L.colamt[m] : colm1;
+          colm2 = (m == m2) ? L.colamt[m] : colm2;
+        }
+        const double speccomb = colm1 + T[swtab::strrat + b] * colm2;
+        const double specmult = T[swtab::specwt + b] * fmin(kOneMinus, colm1 / speccomb);
+        const int js = 1 + (int)specmult;
+        const double fs = fmod(specmult, 1.0);
+        const bool two = (jb == 17 || jb == 28);
+        const double* ref = T + (two ? swtab::sfluxref02 : swtab::sfluxref03);
+        const int nbin = two ? 5 : 9;
+        for (int j = 0; j < ng; ++j) {
+          const double r0 = ref[j + 16 * ((js - 1) + nbin * (ibd - 1))], r1 = ref[j + 16 * (js + nbin * (ibd - 1))];
+          sf[j] = r0 + fs * (r1 - r0);
+        }
       }
     }
+    __syncwarp();
   }
 
   if (a.gas_only) return;
-  // clear / cloudy column (RSM:1101-1125), in layer order on lane 0
+  // clear / cloudy column (RSM:1101-1125), in layer order on lane 0 from a
+  // shared copy: read from memory, its 127 dependent loads were a third of the
+  // kernel's time
+  for (int kk = lane; kk < nlay; kk += 32) s_col[kk] = a.cf[i + ld * row(kk)];
+  __syncwarp();
   double zcf1 = 0.0;
   if (lane == 0) {
     double zcf0 = 1.0, z1 = 1.0;
-    for (int k = 0; k < nlay; ++k) {
-      const int r = a.top_at_1 ? nlay - 1 - k : k;
-      const double cf = a.cf[(size_t)i + (size_t)a.ld * r];
+    for (int kk = 0; kk < nlay; ++kk) {
+      const double cf = s_col[kk];
       if (a.iovr == a.iovr_rand) {
         zcf0 = zcf0 * (1.0 - cf);
       } else if (a.iovr == a.iovr_maxrand) {
@@ -546,28 +646,26 @@ __device__ __forceinline__ void optics_body(const SwArgs& a, const SwScratch& s,
     if (zcf0 <= kFtiny) zcf0 = 0.0;
     if (zcf0 > kOneMinus) zcf0 = 1.0;
     zcf1 = 1.0 - zcf0;
-    s.zcf1[pl] = zcf1;
-    s.zcf0[pl] = zcf0;
-    // McICA seed: ipsdsw0 + i or icseed(i) (RSM:875-883); grid-mean clouds draw none
-    s.seed[pl] = (a.isubcsw == 2) ? a.icseed[i] : 1 + a.seed0 + j1;
+    if (seg == 0) {
+      s.zcf1[pl] = zcf1;
+      s.zcf0[pl] = zcf0;
+      // McICA seed: ipsdsw0 + i or icseed(i) (RSM:875-883); grid-mean clouds draw none
+      s.seed[pl] = (a.isubcsw == 2) ? a.icseed[i] : 1 + a.seed0 + j1;
+    }
   }
   zcf1 = __shfl_sync(0xffffffffu, zcf1, 0);
-  for (int k = lane; k < nlay; k += 32) {
-    const int r = a.top_at_1 ? nlay - 1 - k : k;
-    const size_t x = (size_t)i + (size_t)a.ld * r;
-    const double cf = a.cf[x];
+  if (k < nlay) {
+    const size_t x = i + ld * row(k);
+    const double cf = s_col[k];
     s.cldf[(size_t)pl + (size_t)nc * k] = (cf < kFtiny) ? 0.0 : cf;   // mcica_subcol input (RSM:1904-1908)
     if (a.isubcsw <= 0) {   // grid-mean clouds: cldfrc = cfrac / cf1 (RSM:1930-1934)
       s.aux[(size_t)pl + (size_t)nc * k] = (zcf1 > 0.0) ? cf / zcf1 : 0.0;
     } else if (a.iovr == 3) {   // fac_lcf between layers k-1 and k (RSM:2106-2108), dz in internal order
       double f = 0.0;
-      if (k > 0) {
-        const int r1 = a.top_at_1 ? nlay - k : k - 1;
-        f = exp(-0.5 * (a.dz[x] + a.dz[(size_t)i + (size_t)a.ld * r1]) / a.delg[i]);
-      }
+      if (k > 0) f = exp(-0.5 * (a.dz[x] + a.dz[i + ld * row(k - 1)]) / a.delg[i]);
       s.aux[(size_t)pl + (size_t)nc * k] = f;
     } else if (a.iovr == 4 || a.iovr == 5) {   // alpha, in the caller's row order (RSM:921, 1012)
-      s.aux[(size_t)pl + (size_t)nc * k] = a.alpha[(size_t)i + (size_t)a.ld * k];
+      s.aux[(size_t)pl + (size_t)nc * k] = a.alpha[i + ld * k];
     }
     if (zcf1 > 0.0) {
       double* tw = s.taucw + ((size_t)pl * nlay + k) * 14;
@@ -577,32 +675,33 @@ __device__ __forceinline__ void optics_body(const SwArgs& a, const SwScratch& s,
       a.cldtau[x] = tw[9];   // band 25 (RSM:1144-1152)
     }
   }
+  __syncwarp();
 }
 
-__global__ void __launch_bounds__(32 * kOptWarps, 3)   // 168 registers: twelve warps per SM hide the table gathers better than eight
-sw_optics_kernel(SwArgs a, SwScratch s, int p0, int nc, const double* __restrict__ T) {
-  __shared__ int s_jp[kOptWarps][kSwMaxLay];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int pl = blockIdx.x * kOptWarps + w;
+__global__ void __launch_bounds__(32 * kOptWarps, kOptPerSm)
+sw_optics_kernel(SwArgs a, SwScratch s, int p0, int nc, const double* __restrict__ T, const double* __restrict__ K) {
+  __shared__ double s_col[kOptWarps][kSwMaxLay];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nseg = (a.nlay + 31) >> 5;
+  const int u = blockIdx.x * kOptWarps + w, pl = u / nseg, seg = u - pl * nseg;
   if (pl >= nc) return;   // whole warps only: no block barrier below
   const int j1 = a.idxday[p0 + pl];
   if (j1 < 1 || j1 > a.npts) {   // idxday outside 1..npts: skip the column, report
     if (lane == 0) atomicOr(s.bad, 1);
     return;
   }
-  optics_body(a, s, pl, nc, j1, lane, s_jp[w], T);
+  optics_body(a, s, pl, nc, j1, seg, lane, s_col[w], T, K);
 }
 
 // many physics blocks in one launch: daytime point p is column pts[p].y of block pts[p].x
-__global__ void __launch_bounds__(32 * kOptWarps, 3)
+__global__ void __launch_bounds__(32 * kOptWarps, kOptPerSm)
 sw_optics_blocks_kernel(const SwArgs* __restrict__ tab, const int2* __restrict__ pts, SwScratch s, int p0, int nc,
-                        const double* __restrict__ T) {
-  __shared__ int s_jp[kOptWarps][kSwMaxLay];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int pl = blockIdx.x * kOptWarps + w;
+                        const double* __restrict__ T, const double* __restrict__ K) {
+  __shared__ double s_col[kOptWarps][kSwMaxLay];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nseg = (tab[0].nlay + 31) >> 5;
+  const int u = blockIdx.x * kOptWarps + w, pl = u / nseg, seg = u - pl * nseg;
   if (pl >= nc) return;
   const int2 q = pts[p0 + pl];
-  optics_body(tab[q.x], s, pl, nc, q.y, lane, s_jp[w], T);
+  optics_body(tab[q.x], s, pl, nc, q.y, seg, lane, s_col[w], T, K);
 }
 
 // ---- kernel 3: transfer ------------------------------------------------------
@@ -1329,10 +1428,37 @@ cudaError_t gas_unpack_launch(const SwScratch& s, int nc, int nlay, const double
   return cudaGetLastError();
 }
 
-cudaError_t optics_launch(const SwArgs& a, const SwScratch& s, int p0, int nc, const double* T, cudaStream_t st) {
+static int optics_grid(int nc, int nlay) { return (int)(((long)nc * ((nlay + 31) / 32) + kOptWarps - 1) / kOptWarps); }
+
+// Reorders every (rows, ng) k-table of the coefficient blob from row fastest to
+// g-point fastest, in place.
+void gpoint_fastest(double* blob) {
+  using namespace swtab;
+  const struct { int off, rows, ng; } t[] = {
+      {b16_absa, 585, 6},  {b16_absb, 235, 6},  {b16_selfref, 10, 6},  {b16_forref, 3, 6},
+      {b17_absa, 585, 12}, {b17_absb, 1175, 12}, {b17_selfref, 10, 12}, {b17_forref, 4, 12},
+      {b18_absa, 585, 8},  {b18_absb, 235, 8},  {b18_selfref, 10, 8},  {b18_forref, 3, 8},
+      {b19_absa, 585, 8},  {b19_absb, 235, 8},  {b19_selfref, 10, 8},  {b19_forref, 3, 8},
+      {b20_absa, 65, 10},  {b20_absb, 235, 10}, {b20_selfref, 10, 10}, {b20_forref, 4, 10},
+      {b21_absa, 585, 10}, {b21_absb, 1175, 10}, {b21_selfref, 10, 10}, {b21_forref, 4, 10},
+      {b22_absa, 585, 2},  {b22_absb, 235, 2},  {b22_selfref, 10, 2},  {b22_forref, 3, 2},
+      {b23_absa, 65, 10},  {b23_selfref, 10, 10}, {b23_forref, 3, 10},
+      {b24_absa, 585, 8},  {b24_absb, 235, 8},  {b24_selfref, 10, 8},  {b24_forref, 3, 8},
+      {b25_absa, 65, 6},   {b27_absa, 65, 8},   {b27_absb, 235, 8},
+      {b28_absa, 585, 6},  {b28_absb, 1175, 6},
+      {b29_absa, 65, 12},  {b29_absb, 235, 12}, {b29_selfref, 10, 12}, {b29_forref, 4, 12}};
+  std::vector<double> row;
+  for (const auto& q : t) {
+    row.assign(blob + q.off, blob + q.off + (size_t)q.rows * q.ng);
+    for (int i = 0; i < q.rows; ++i)
+      for (int j = 0; j < q.ng; ++j) blob[q.off + (size_t)i * q.ng + j] = row[(size_t)j * q.rows + i];
+  }
+}
+
+cudaError_t optics_launch(const SwArgs& a, const SwScratch& s, int p0, int nc, const double* T, const double* K,
+                          cudaStream_t st) {
   if (nc <= 0) return cudaSuccess;
-  const int grid = (nc + kOptWarps - 1) / kOptWarps;
-  sw_optics_kernel<<<grid, 32 * kOptWarps, 0, st>>>(a, s, p0, nc, T);
+  sw_optics_kernel<<<optics_grid(nc, a.nlay), 32 * kOptWarps, 0, st>>>(a, s, p0, nc, T, K);
   return cudaGetLastError();
 }
 
@@ -1364,10 +1490,10 @@ cudaError_t blocks_prepare(const SwArgs* tab, const int* colpre, const int* dayp
   return cudaGetLastError();
 }
 
-cudaError_t optics_blocks_launch(const SwArgs* tab, const int2* pts, const SwScratch& s, int p0, int nc,
-                                 const double* T, cudaStream_t st) {
+cudaError_t optics_blocks_launch(const SwArgs* tab, const int2* pts, const SwScratch& s, int p0, int nc, int nlay,
+                                 const double* T, const double* K, cudaStream_t st) {
   if (nc <= 0) return cudaSuccess;
-  sw_optics_blocks_kernel<<<(nc + kOptWarps - 1) / kOptWarps, 32 * kOptWarps, 0, st>>>(tab, pts, s, p0, nc, T);
+  sw_optics_blocks_kernel<<<optics_grid(nc, nlay), 32 * kOptWarps, 0, st>>>(tab, pts, s, p0, nc, T, K);
   return cudaGetLastError();
 }
 

@@ -66,7 +66,10 @@ __host__ __device__ inline size_t rt_col_doubles(int nlay, bool hswb) {
 
 cudaError_t overlap_aux_launch(int ncols, int nlay, int ld, int iovr, const double* dz, const double* delg,
                                const double* alpha, double* aux, int ldo, cudaStream_t st);
-cudaError_t optics_launch(const SwArgs& a, const SwScratch& s, int p0, int nc, const double* T, cudaStream_t st);
+// T = the coefficient blob, K = the same with the g-point fastest in every k-table (gpoint_fastest)
+cudaError_t optics_launch(const SwArgs& a, const SwScratch& s, int p0, int nc, const double* T, const double* K,
+                          cudaStream_t st);
+void gpoint_fastest(double* blob);
 cudaError_t rt_prepare(int max_smem);
 cudaError_t rt_launch(const SwArgs& a, const SwScratch& s, int p0, int nc, const double* T, const double* ET,
                       cudaStream_t st);
@@ -77,8 +80,8 @@ cudaError_t gas_unpack_launch(const SwScratch& s, int nc, int nlay, const double
 // = columns / daytime points before block b (dayp has nb + 1 entries)
 cudaError_t blocks_prepare(const SwArgs* tab, const int* colpre, const int* dayp, int nb, int total_cols,
                            int2* pts, int* bad, cudaStream_t st);
-cudaError_t optics_blocks_launch(const SwArgs* tab, const int2* pts, const SwScratch& s, int p0, int nc,
-                                 const double* T, cudaStream_t st);
+cudaError_t optics_blocks_launch(const SwArgs* tab, const int2* pts, const SwScratch& s, int p0, int nc, int nlay,
+                                 const double* T, const double* K, cudaStream_t st);
 cudaError_t rt_blocks_launch(const SwArgs* tab, const int2* pts, bool grid, bool want_b, const SwScratch& s, int p0,
                              int nc, int nlay, const double* T, const double* ET, cudaStream_t st);
 
