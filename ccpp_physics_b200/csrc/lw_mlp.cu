@@ -19,7 +19,7 @@
 //                         the Planck fractions as FP16 8-layer blocks of its
 //                         compact hand-off, and the list of the columns that
 //                         have a layer outside the envelope.
-//   gemm_tn_kernel<EPI>   C = A * B^T for the backward pass: dH = dZ W with
+//   gemm_tn_kernel        C = A * B^T for the backward pass: dH = dZ W with
 //                         the activation derivative fused (EPI_DACT), and
 //                         split-K weight gradients dW = dZ^T H with FP32
 //                         atomics (EPI_ATOMIC).  Bias gradients come out as
@@ -958,92 +958,137 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) mlp_h_kernel(FwdArgs a) {
 enum { EPI_ATOMIC = 0, EPI_DACT = 1 };
 
 struct GemmArgs {
-  const bf16* A; long lda;
+  int epi;
+  const bf16* A; long lda;          // rows up to a multiple of 128 are readable
   const bf16* B; long ldb;
-  int M, N, K, kslice;
+  int M, N, K, kslice;              // N <= 144; kslice a multiple of 64
   float* C; long ldc;               // EPI_ATOMIC
   const bf16* Z; long ldz;          // EPI_DACT
   bf16* D; long ldd;                // EPI_DACT row-major out (nullable)
   bf16* Dt; long lddt;              // EPI_DACT transposed out (nullable)
   int* err;
+  __host__ __device__ int mtiles() const { return (M + 127) / 128; }
+  __host__ __device__ int ctas() const { return mtiles() * ((K + kslice - 1) / kslice); }
 };
 
-constexpr int GK = 64;                                   // K per staged chunk
-constexpr uint32_t GSM_A = 0;                            // canon [128][64]
-constexpr uint32_t GSM_B = GSM_A + 128 * GK * 2;         // canon [288][64]
-constexpr uint32_t GSM_BAR = GSM_B + 288 * GK * 2;
-constexpr uint32_t GEMM_SMEM_MIN = GSM_BAR + 32;
-constexpr uint32_t GEMM_SMEM = 120 * 1024;               // > half an SM: one CTA per SM (512 TMEM columns)
-static_assert(GEMM_SMEM >= GEMM_SMEM_MIN, "gemm shared memory");
+// One or two independent products per launch: CTAs [0, n0) work on j[0], the
+// rest on j[1], a 128-row tile and a K slice each.
+//
+// Bound by latency: the largest product is 0.7 GFLOP.  A CTA therefore brings
+// its whole K slice (up to 320) in one go, 16 bytes per cp.async, and issues
+// every MMA behind one barrier (in 64-wide chunks, each with its own round trip
+// and its own wait, a product took 16 to 36 us); the weight gradients leave as
+// 16-byte vector reductions; and two products that do not depend on each other
+// share a launch.  Batch 8,192: five launches 130 us, three launches now 36 us.
+struct BwdArgs {
+  GemmArgs j[2];
+  int n0;
+};
 
-template <int EPI>
-__global__ void __launch_bounds__(128, 1) gemm_tn_kernel(GemmArgs g) {
+constexpr int GEMM_THREADS = 256, GK = 320;              // K per staged chunk
+constexpr uint32_t GSM_A = 0;                            // canon [128][GK]
+constexpr uint32_t GSM_B = GSM_A + 128 * GK * 2;         // canon [144][GK]
+constexpr uint32_t GSM_BAR = GSM_B + 144 * GK * 2;
+constexpr uint32_t GEMM_SMEM = GSM_BAR + 32;             // > half an SM: one CTA per SM
+static_assert(GEMM_SMEM > 116 * 1024 && GEMM_SMEM <= 227 * 1024, "gemm shared memory");
+
+// rows x kc (a multiple of 32) of a K-major matrix into a canonical tile: a
+// warp's copies are 8 rows x 64 bytes, contiguous per 8 lanes in shared memory
+__device__ __forceinline__ void stage_tile(unsigned char* tile, const bf16* src, long ld, int rows, int kc, int tid) {
+  const int quads = kc >> 5, lane = tid & 31;
+  for (int c = tid >> 5; c < (rows >> 3) * quads; c += GEMM_THREADS / 32) {
+    const int r = ((c / quads) << 3) + (lane & 7), k = ((c % quads) << 5) + ((lane >> 3) << 3);
+    umma::cp_async16(tile + umma::canon_off(r, k, GK), src + (size_t)r * ld + k);
+  }
+}
+
+__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tn_kernel(BwdArgs args) {
   extern __shared__ __align__(1024) unsigned char sm[];
+  const int second = (int)blockIdx.x >= args.n0;
+  const GemmArgs& g = args.j[second];
+  const int cta = (int)blockIdx.x - (second ? args.n0 : 0);
   const int tid = threadIdx.x, warp = tid >> 5;
   uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + GSM_BAR);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + GSM_BAR + 8);
+  const int mt = g.mtiles(), m0 = cta % mt * 128;
+  const int kb = cta / mt * g.kslice, ke = min(g.K, kb + g.kslice);
+  const bf16* A = g.A + (size_t)m0 * g.lda;
+  // the first chunk's copies run while tensor memory is allocated
+  int kc = min(GK, ke - kb);
+  stage_tile(sm + GSM_A, A + kb, g.lda, 128, kc, tid);
+  stage_tile(sm + GSM_B, g.B + kb, g.ldb, g.N, kc, tid);
+  umma::cp_async_commit();
   if (warp == 0) {
-    umma::tmem_alloc(tslot, 512);
+    umma::tmem_alloc(tslot, 256);
     umma::tmem_relinquish();
   }
   if (tid == 0) umma::mbar_init(mbar, 1);
+  // this thread's row, and its half of the columns
+  const int m = m0 + (tid & 127), nmid = ((g.N >> 4) + 1) / 2 * 16;
+  const int n_lo = warp < 4 ? 0 : nmid, n_hi = warp < 4 ? nmid : g.N;
+  uint4 z[8];   // Z of the row's columns (EPI_DACT: N = 128)
+  if (g.epi == EPI_DACT && m < g.M) {
+    const uint4* zp = reinterpret_cast<const uint4*>(g.Z + (size_t)m * g.ldz + n_lo);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) z[q] = __ldg(zp + q);
+  }
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
   const uint32_t tb = *tslot;
   const uint32_t sbase = umma::smem_u32(sm);
-  const int m0 = blockIdx.x * 128;
-  const int kb = blockIdx.y * g.kslice, ke = min(g.K, kb + g.kslice);
-  const int nsplit = g.N > 256 ? 2 : 1, nh = g.N / nsplit;
-  const uint32_t idesc = umma::idesc_bf16(128, nh);
+  const uint32_t idesc = umma::idesc_bf16(128, g.N);
   uint32_t phase = 0;
-  bool ok = true, any = false;
+  bool ok = true;
   for (int k0 = kb; k0 < ke; k0 += GK) {
-    const int kc = min(GK, ke - k0);   // multiple of 16
-    // stage A [128 x kc] and B [N x kc] (zero-fill the unused K of a short chunk)
-    for (int c = tid; c < 128 * (GK / 8); c += 128) {
-      const int r = c / (GK / 8), k = (c % (GK / 8)) * 8;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (k < kc && m0 + r < g.M) v = __ldg(reinterpret_cast<const uint4*>(g.A + (size_t)(m0 + r) * g.lda + k0 + k));
-      *reinterpret_cast<uint4*>(sm + GSM_A + umma::canon_off(r, k, GK)) = v;
+    if (k0 > kb) {
+      kc = min(GK, ke - k0);
+      stage_tile(sm + GSM_A, A + k0, g.lda, 128, kc, tid);
+      stage_tile(sm + GSM_B, g.B + k0, g.ldb, g.N, kc, tid);
+      umma::cp_async_commit();
     }
-    for (int c = tid; c < g.N * (GK / 8); c += 128) {
-      const int r = c / (GK / 8), k = (c % (GK / 8)) * 8;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (k < kc) v = __ldg(reinterpret_cast<const uint4*>(g.B + (size_t)r * g.ldb + k0 + k));
-      *reinterpret_cast<uint4*>(sm + GSM_B + umma::canon_off(r, k, GK)) = v;
-    }
+    umma::cp_async_wait_all();
     umma::fence_smem_async();
     umma::fence_before_sync();
     __syncthreads();
     if (tid == 0) {
       umma::fence_after_sync();
       for (int s = 0; s < kc / 16; ++s)
-        for (int h = 0; h < nsplit; ++h)
-          umma::mma(tb + (uint32_t)(h * nh), umma::tile_desc(sbase + GSM_A, GK, s),
-                    umma::tile_desc(sbase + GSM_B + (uint32_t)(h * nh * GK * 2), GK, s), idesc,
-                    (any || s > 0) ? 1u : 0u);
+        umma::mma(tb, umma::tile_desc(sbase + GSM_A, GK, s), umma::tile_desc(sbase + GSM_B, GK, s), idesc,
+                  (k0 > kb || s > 0) ? 1u : 0u);
       umma::commit(mbar);
     }
-    any = true;
     ok = umma::mbar_wait(mbar, phase);
     phase ^= 1u;
     umma::fence_after_sync();
     if (__syncthreads_or(!ok)) { ok = false; break; }
   }
-  if (ok && any) {
-    const int m = m0 + tid;
-    for (int n0 = 0; n0 < g.N; n0 += 16) {
+  if (ok && kb < ke) {
+#pragma unroll 1
+    for (int n0 = n_lo; n0 < n_hi; n0 += 16) {
       float v[16];
-      umma::tmem_ld16(umma::tmem_addr(tb, warp, n0), v);
+      umma::tmem_ld16(umma::tmem_addr(tb, warp & 3, n0), v);
       if (m >= g.M) continue;
-      if (EPI == EPI_ATOMIC) {
+      if (g.epi == EPI_ATOMIC) {
+        float4* c = reinterpret_cast<float4*>(g.C + (size_t)m * g.ldc + n0);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) atomicAdd(g.C + (size_t)m * g.ldc + n0 + j, v[j]);
+        for (int j = 0; j < 4; ++j) atomicAdd(c + j, make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]));
       } else {
+        uint4 zz[2];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (((n0 - n_lo) >> 4) == q) {
+            zz[0] = z[2 * q];
+            zz[1] = z[2 * q + 1];
+          }
+        const __nv_bfloat162* zb = reinterpret_cast<const __nv_bfloat162*>(zz);
         float d[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) d[j] = v[j] * dsilu(__bfloat162float(g.Z[(size_t)m * g.ldz + n0 + j]));
+        for (int j = 0; j < 8; ++j) {
+          const float2 zf = __bfloat1622float2(zb[j]);
+          d[2 * j] = v[2 * j] * dsilu(zf.x);
+          d[2 * j + 1] = v[2 * j + 1] * dsilu(zf.y);
+        }
         if (g.D) {
           __nv_bfloat162 dp[8];
 #pragma unroll
@@ -1059,10 +1104,11 @@ __global__ void __launch_bounds__(128, 1) gemm_tn_kernel(GemmArgs g) {
       }
     }
   }
+  if (!ok) umma::mbar_wait(mbar, phase ^ 1u, 1u << 20);   // one more bounded wait for the MMA in flight
   umma::fence_before_sync();
   __syncthreads();
   if (tid == 0 && !ok && g.err) atomicCAS(g.err, 0, 1);
-  if (warp == 0) umma::tmem_dealloc(tb, 512);
+  if (warp == 0) umma::tmem_dealloc(tb, 256);
 }
 
 // ---------------------------------------------------------------------------
@@ -1083,12 +1129,13 @@ __device__ inline void pack_param(int p, float w, bf16* ops) {
   }
 }
 
-__device__ inline float grad_of(int p, const float* G) {
-  if (p < P_W2) { const int r = p / NIN, c = p % NIN; return G[G_W1 + r * KIN + c]; }
-  if (p < P_B2) { const int q = p - P_W2; return G[G_W2 + (q / HID) * GW2_LD + q % HID]; }
-  if (p < P_W3) { return G[G_W2 + (p - P_B2) * GW2_LD + HID]; }
-  if (p < P_B3) { const int q = p - P_W3; return G[G_W3 + (q / HID) * GW2_LD + q % HID]; }
-  return G[G_W3 + (p - P_B3) * GW2_LD + HID];
+// where parameter p's gradient lies
+__device__ inline int grad_at(int p) {
+  if (p < P_W2) { const int r = p / NIN, c = p % NIN; return G_W1 + r * KIN + c; }
+  if (p < P_B2) { const int q = p - P_W2; return G_W2 + (q / HID) * GW2_LD + q % HID; }
+  if (p < P_W3) { return G_W2 + (p - P_B2) * GW2_LD + HID; }
+  if (p < P_B3) { const int q = p - P_W3; return G_W3 + (q / HID) * GW2_LD + q % HID; }
+  return G_W3 + (p - P_B3) * GW2_LD + HID;
 }
 
 __device__ inline bool frozen_param(int p) {   // padded output rows stay zero
@@ -1097,12 +1144,14 @@ __device__ inline bool frozen_param(int p) {   // padded output rows stay zero
   return false;
 }
 
-__global__ void adam_kernel(float* P, float* M, float* V, const float* G, bf16* ops, float lr, float b1, float b2,
+// also leaves every gradient it used at zero, for the next step's sums
+__global__ void adam_kernel(float* P, float* M, float* V, float* G, bf16* ops, float lr, float b1, float b2,
                             float c1, float c2, float eps) {
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P_N; p += gridDim.x * blockDim.x) {
     float w = P[p];
     if (!frozen_param(p)) {
-      const float gr = grad_of(p, G);
+      const float gr = G[grad_at(p)];
+      G[grad_at(p)] = 0.0f;
       const float m = b1 * M[p] + (1.0f - b1) * gr;
       const float v = b2 * V[p] + (1.0f - b2) * gr * gr;
       M[p] = m;
@@ -1121,7 +1170,7 @@ __global__ void pack_kernel(const float* P, bf16* ops) {
 // export the gradients in parameter order (gradient check)
 __global__ void grads_kernel(const float* G, float* out) {
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P_N; p += gridDim.x * blockDim.x)
-    out[p] = frozen_param(p) ? 0.0f : grad_of(p, G);
+    out[p] = frozen_param(p) ? 0.0f : G[grad_at(p)];
 }
 
 // layer features and coldry of one block (internal layer order, surface first)
@@ -1166,7 +1215,7 @@ struct Net {
   // training activations for batch `cap`
   long cap = 0;
   bf16 *xt = nullptr, *z1 = nullptr, *h1t = nullptr, *z2 = nullptr, *h2t = nullptr, *dy = nullptr, *dyt = nullptr,
-       *dz2 = nullptr, *dz1t = nullptr;
+       *dz2 = nullptr, *dz2t = nullptr, *dz1t = nullptr;
   bool attrs = false;
 };
 Net net;
@@ -1198,18 +1247,14 @@ cudaError_t set_attrs() {
     return e;
   if ((e = cudaFuncSetAttribute(mlp_h_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, H_SMEM))) return e;
   if ((e = cudaFuncSetAttribute(mlp_h_pack_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PK_SMEM))) return e;
-  if ((e = cudaFuncSetAttribute(gemm_tn_kernel<EPI_ATOMIC>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM)))
-    return e;
-  if ((e = cudaFuncSetAttribute(gemm_tn_kernel<EPI_DACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM)))
-    return e;
+  if ((e = cudaFuncSetAttribute(gemm_tn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM))) return e;
   // one CTA per SM is what makes the 512-column TMEM allocations safe
-  int occ[6] = {0, 0, 0, 0, 0, 0};
+  int occ[5] = {0, 0, 0, 0, 0};
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[0], mlp_fwd_kernel<MODE_FEATS>, FWD_THREADS, FWD_SMEM);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[1], mlp_fwd_kernel<MODE_TRAIN>, FWD_THREADS, FWD_SMEM);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[2], mlp_fwd_kernel<MODE_LW>, FWD_THREADS, FWD_SMEM);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[3], gemm_tn_kernel<EPI_ATOMIC>, 128, GEMM_SMEM);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[4], gemm_tn_kernel<EPI_DACT>, 128, GEMM_SMEM);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[5], mlp_h_kernel, FWD_THREADS, H_SMEM);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[3], gemm_tn_kernel, GEMM_THREADS, GEMM_SMEM);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[4], mlp_h_kernel, FWD_THREADS, H_SMEM);
   for (int o : occ)
     if (o != 1) return cudaErrorLaunchOutOfResources;
   net.attrs = true;
@@ -1238,15 +1283,15 @@ cudaError_t ensure_net(int device, int num_sms) {
 
 cudaError_t ensure_batch(long batch) {
   if (net.cap >= batch) return cudaSuccess;
-  bf16** bufs[] = {&net.xt, &net.z1, &net.h1t, &net.z2, &net.h2t, &net.dy, &net.dyt, &net.dz2, &net.dz1t};
+  bf16** bufs[] = {&net.xt, &net.z1, &net.h1t, &net.z2, &net.h2t, &net.dy, &net.dyt, &net.dz2, &net.dz1t, &net.dz2t};
   for (bf16** b : bufs)
     if (*b) { cudaFree(*b); *b = nullptr; }
   net.cap = 0;
-  // rows: Xt 16, Z [B][128], H^T 144 (row 128 = 1), dY [B][288], dY^T 384, dZ2 [B][128], dZ1^T 128
+  // rows: Xt 16, Z [B][128], H^T 144 (row 128 = 1), dY [B][288], dY^T 384, dZ2 [B][128], dZ1^T 128, dZ2^T 128
   const size_t B = (size_t)batch;
-  const size_t n[] = {16 * B, B * HID, 144 * B, B * HID, 144 * B, B * NOP, GW3_ROWS * B, B * HID, HID * B};
+  const size_t n[] = {16 * B, B * HID, 144 * B, B * HID, 144 * B, B * NOP, GW3_ROWS * B, B * HID, HID * B, HID * B};
   cudaError_t e;
-  for (int k = 0; k < 9; ++k) {
+  for (int k = 0; k < 10; ++k) {
     if ((e = cudaMalloc(bufs[k], n[k] * sizeof(bf16)))) return e;
     if ((e = cudaMemset(*bufs[k], 0, n[k] * sizeof(bf16)))) return e;
   }
@@ -1268,11 +1313,21 @@ FwdArgs base_args() {
   return a;
 }
 
-cudaError_t launch_gemm(int epi, const GemmArgs& g, int ksplit, cudaStream_t st) {
-  dim3 grid((g.M + 127) / 128, ksplit);
-  if (epi == EPI_ATOMIC) gemm_tn_kernel<EPI_ATOMIC><<<grid, 128, GEMM_SMEM, st>>>(g);
-  else gemm_tn_kernel<EPI_DACT><<<grid, 128, GEMM_SMEM, st>>>(g);
+// one product, or two independent ones
+cudaError_t launch_gemm(const GemmArgs& g0, const GemmArgs* g1, cudaStream_t st) {
+  BwdArgs a{};
+  a.j[0] = g0;
+  a.n0 = g0.ctas();
+  if (g1) a.j[1] = *g1;
+  gemm_tn_kernel<<<a.n0 + (g1 ? g1->ctas() : 0), GEMM_THREADS, GEMM_SMEM, st>>>(a);
   return cudaGetLastError();
+}
+// K slice of a weight gradient of mtiles row tiles over `batch` samples, so that
+// its CTAs fill the SMs that `other` CTAs of the same launch leave; at least
+// 256 samples each, since every slice adds its whole product to memory
+int grad_slice(int batch, int mtiles, int other) {
+  const int n = std::max(1, std::min(batch / 256, std::max(8, (net.num_sms - other) / mtiles)));
+  return ((batch + n - 1) / n + 63) / 64 * 64;
 }
 
 // forward (train mode) + backward of one batch: gradients accumulate in net.G
@@ -1297,38 +1352,36 @@ cudaError_t train_batch(const float* feats, const float* targets, long nsamp, lo
   cudaError_t e = cudaGetLastError();
   if (e) return e;
   const int B = (int)batch;
-  // dZ2 = (dY W3) * silu'(Z2): row-major for dH1, transposed for dW2
-  GemmArgs g{};
-  g.err = net.err;
-  g.A = net.dy; g.lda = NOP; g.B = net.ops + O_W3T; g.ldb = NOP; g.M = B; g.N = HID; g.K = NOP; g.kslice = NOP;
-  g.Z = net.z2; g.ldz = HID; g.D = net.dz2; g.ldd = HID; g.Dt = nullptr; g.lddt = 0;
-  // dZ2^T (A operand of dW2) goes to the dZ1^T buffer: dW2 consumes it before dH1 overwrites it
-  g.Dt = net.dz1t;
-  g.lddt = ldt;
-  if ((e = launch_gemm(EPI_DACT, g, 1, st))) return e;
+  // dZ2 = (dY W3) * silu'(Z2): row-major for dZ1, transposed for dW2
+  GemmArgs z2{};
+  z2.epi = EPI_DACT;
+  z2.err = net.err;
+  z2.A = net.dy; z2.lda = NOP; z2.B = net.ops + O_W3T; z2.ldb = NOP; z2.M = B; z2.N = HID; z2.K = z2.kslice = NOP;
+  z2.Z = net.z2; z2.ldz = HID; z2.D = net.dz2; z2.ldd = HID; z2.Dt = net.dz2t; z2.lddt = ldt;
   // dW3 += dY^T H2aug : [288 x B] x [144 x B]^T  (A rows 288..383 are zero)
   GemmArgs w3{};
+  w3.epi = EPI_ATOMIC;
   w3.err = net.err;
   w3.A = net.dyt; w3.lda = ldt; w3.B = net.h2t; w3.ldb = ldt; w3.M = NOP; w3.N = 144; w3.K = B;
-  const int ks = std::max(1, std::min(32, B / 256));
-  w3.kslice = ((B / ks + 63) / 64) * 64;
+  w3.kslice = grad_slice(B, w3.mtiles(), z2.ctas());
   w3.C = net.G + G_W3; w3.ldc = GW2_LD;
-  if ((e = launch_gemm(EPI_ATOMIC, w3, (B + w3.kslice - 1) / w3.kslice, st))) return e;
+  if ((e = launch_gemm(z2, &w3, st))) return e;
+  // dZ1^T = ((dZ2 W2) * silu'(Z1))^T
+  GemmArgs z1{};
+  z1.epi = EPI_DACT;
+  z1.err = net.err;
+  z1.A = net.dz2; z1.lda = HID; z1.B = net.ops + O_W2T; z1.ldb = HID; z1.M = B; z1.N = HID; z1.K = z1.kslice = HID;
+  z1.Z = net.z1; z1.ldz = HID; z1.D = nullptr; z1.Dt = net.dz1t; z1.lddt = ldt;
   // dW2 += dZ2^T H1aug
   GemmArgs w2 = w3;
-  w2.A = net.dz1t; w2.M = HID; w2.B = net.h1t; w2.C = net.G + G_W2;
-  if ((e = launch_gemm(EPI_ATOMIC, w2, (B + w2.kslice - 1) / w2.kslice, st))) return e;
-  // dZ1^T = ((dZ2 W2) * silu'(Z1))^T
-  GemmArgs d1{};
-  d1.err = net.err;
-  d1.A = net.dz2; d1.lda = HID; d1.B = net.ops + O_W2T; d1.ldb = HID; d1.M = B; d1.N = HID; d1.K = HID;
-  d1.kslice = HID;
-  d1.Z = net.z1; d1.ldz = HID; d1.D = nullptr; d1.Dt = net.dz1t; d1.lddt = ldt;
-  if ((e = launch_gemm(EPI_DACT, d1, 1, st))) return e;
+  w2.A = net.dz2t; w2.M = HID; w2.B = net.h1t; w2.C = net.G + G_W2;
+  w2.kslice = grad_slice(B, 1, z1.ctas());
+  if ((e = launch_gemm(z1, &w2, st))) return e;
   // dW1 += dZ1^T X : [128 x B] x [16 x B]^T
   GemmArgs w1 = w3;
   w1.A = net.dz1t; w1.M = HID; w1.B = net.xt; w1.N = 16; w1.C = net.G + G_W1; w1.ldc = KIN;
-  return launch_gemm(EPI_ATOMIC, w1, (B + w1.kslice - 1) / w1.kslice, st);
+  w1.kslice = grad_slice(B, 1, 0);
+  return launch_gemm(w1, nullptr, st);
 }
 
 int check_ready(char* errmsg, int32_t errmsg_len) {
@@ -1654,9 +1707,8 @@ extern "C" int rrtmg_lw_gpu_surrogate_train(const float* feats, const float* tar
       const double fr = (double)done / (double)std::max(1L, total - 1);
       const float lr_t = (float)(lr_final + 0.5 * (lr - lr_final) * (1.0 + std::cos(3.14159265358979323846 * fr)));
       const float c1 = 1.0f - std::pow(b1, (float)net.adam_t), c2 = 1.0f - std::pow(b2, (float)net.adam_t);
-      adam_kernel<<<64, 256, 0, st>>>(net.P, net.Madam, net.Vadam, net.G, net.ops, lr_t, b1, b2, c1, c2, eps);
+      adam_kernel<<<(P_N + 255) / 256, 256, 0, st>>>(net.P, net.Madam, net.Vadam, net.G, net.ops, lr_t, b1, b2, c1, c2, eps);
       SG_CK(cudaGetLastError(), "adam kernel launch");
-      SG_CK(cudaMemsetAsync(net.G, 0, sizeof(float) * G_N, st), "cudaMemsetAsync");
     }
     float l = 0.0f;
     int herr = 0;
