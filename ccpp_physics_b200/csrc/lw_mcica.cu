@@ -29,6 +29,8 @@
 namespace lw {
 
 __device__ __constant__ uint32_t c_pow69069[624];
+constexpr uint32_t pow69069(int n) { return n == 0 ? 1u : 69069u * pow69069(n - 1); }
+constexpr uint32_t kPow69069_32 = pow69069(32);
 
 constexpr uint32_t kMata = 0x9908B0DFu, kUmask = 0x80000000u, kLmask = 0x7FFFFFFFu;
 constexpr uint32_t kTmaskB = 0x9D2C5680u, kTmaskC = 0xEFC60000u;
@@ -110,41 +112,6 @@ struct McicaArgs {
   McicaStage st;  // stage entry point inputs (blocks == nullptr)
 };
 
-// One twister stream kept as a sequence ring of two blocks (1248 words;
-// sequence index s at ring[s mod 1248], draw p = tempered x_{624+p}).  The
-// reader tracks its next sequence index s, its ring position, and how far
-// the sequence has been generated.
-constexpr int kTwoSetRing = 1248;
-struct TwoSetStream {
-  int s;      // sequence index of the next draw
-  int pos;    // s mod 1248
-  int gen;    // sequence indices generated so far (a multiple of 624)
-};
-
-// The next 140 draws (one layer of a layer-major stream, RLM:2006-2024);
-// lane gets the tempered words of g-points n = lane + 32 j (j < 5).  Blocks
-// are appended as the reads advance; the block a new one overwrites was read
-// before the barrier.
-__device__ __forceinline__ void layer_draws(uint32_t* ring, TwoSetStream& st, int lane, uint32_t (&d)[5]) {
-  if (st.gen < st.s + NGPT) {
-    __syncwarp();
-    do {
-      twist_ring(ring, kTwoSetRing, (st.gen / 624) & 1 ? 624 : 0, lane);
-      st.gen += 624;
-    } while (st.gen < st.s + NGPT);
-  }
-#pragma unroll
-  for (int j = 0; j < 5; ++j) {
-    const int n = lane + 32 * j;
-    int q = st.pos + n;
-    if (q >= kTwoSetRing) q -= kTwoSetRing;
-    d[j] = (n < NGPT) ? temper(ring[q]) : 0u;
-  }
-  st.s += NGPT;
-  st.pos += NGPT;
-  if (st.pos >= kTwoSetRing) st.pos -= kTwoSetRing;
-}
-
 // The draw conversion h(u) = u / (2^32 - 1) (u32_unit) is strictly
 // increasing (consecutive u differ by 2^-32, far above a double's spacing),
 // so every comparison of a draw with a per-layer value x is a comparison of
@@ -179,87 +146,300 @@ __device__ long long umax_le(double x) {
 //   iovr = 4/5, exponential / exponential-random: bottom-up, layer k keeps the
 //     value of layer k-1 when set2(k) < alpha(k), else its own draw.
 // Set 1 is stream positions [0, 140 nlay), set 2 the next 140 nlay; two
-// twister states walk them in lockstep, layer by layer, surface first.  The
-// top-down rule is evaluated bottom-up: a layer's value is the set-1 draw of
-// the nearest layer at or above it whose link to the layer above is broken
-// (the top layer always is), so each g-point keeps the run of layers still
-// waiting for that draw and resolves it when the break arrives.
-// The walk runs on tempered words against integer thresholds (above):
-// clr_t[k] = umin_ge(1 - cldf(k)) for the cloud test (RLM:2097-2103), and
+// twister states walk them in lockstep, layer by layer, surface first.
+//
+// Each state is the 624 words x_i..x_{i+623} themselves, updated in place:
+// the next W <= 227 words depend only on words already there, so a layer's
+// 140 draws of a set are computed straight into registers (five per lane) and
+// stored over the words they replace, with one barrier between the reads and
+// the stores of both sets.  Jumping to set 2 takes 224 words at a time.
+//
+// iovr 3's top-down rule is evaluated bottom-up: a layer's value is the set-1
+// draw of the nearest layer at or above it whose link to the layer above is
+// broken (the top layer's always is), so each g-point keeps the run of layers
+// still waiting for that draw.  A break resolves a run: (g-point, run, draw)
+// goes into a queue in shared memory, and 32 of them at a time are turned
+// into flags, one per lane; a tenth of the g-points break at a layer, and
+// resolving them on the spot ran the search with a few lanes active.  Runs
+// without a cloudy layer are not queued.
+//
+// The tests are on tempered words against integer thresholds (above):
+// clr_t[k] = umin_ge(1 - cldf(k)) for the cloud flag (RLM:2097-2103), and
 // aux_t[k] = umax_le(fac_lcf(k)) (iovr 3, 0-based, aux_t[0] unused) or
-// ulim_lt(alpha(k)) (iovr 4, 5).
-__device__ void mcica_two_set(uint32_t* mtA, uint32_t* mtB, const long long* clr_t, const long long* aux_t,
-                              const long long* srt, const uint32_t* pm, int nlay, int iovr, uint32_t s0, int nw,
-                              uint32_t* out, int lane) {
-  for (int n = lane; n < 624; n += 32) {
-    const uint32_t v = s0 * c_pow69069[n];
-    mtA[n] = v;
-    mtB[n] = v;
+// ulim_lt(alpha(k)) (iovr 4, 5).  A clear layer's flag (threshold 2^32 - 1)
+// is set by the draw of all ones alone.  So once the walk is above the top
+// cloudy layer and no run with a cloudy layer waits, the remaining set-1 words
+// are only looked through for that draw; if one turns up, the column is done
+// again to its top (walk_all).
+//
+// Bound by integer issue.  5,003 columns of 127 layers, iovr 3: 1.12 ms with
+// 1,248-word rings read back per draw, runs resolved on the spot and 12 warps
+// per SM; 0.30 ms so (12.6 KB a warp, 16 warps per SM).
+constexpr int kTwoSetWarps = 2;      // per CTA, a column each; the grid holds every column, so warps are refilled as they end
+constexpr int kTwoSetQueue = 192;    // 31 events left over and at most 160 of one layer
+constexpr int kNoCloud = 0x7fff;     // "no cloudy layer at or above"
+
+__device__ __forceinline__ uint32_t wrap624(uint32_t q) { return min(q, q - 624u); }   // q < 1248
+
+// The next 32 W words of a state whose oldest word is x[pos] (W <= 7: 224 of
+// the 227 that depend on present words only), lane + 32 j to r[j].
+template <int W>
+__device__ __forceinline__ void mt_next(const uint32_t* x, uint32_t pos, int lane, uint32_t (&r)[W]) {
+#pragma unroll
+  for (int j = 0; j < W; ++j) {
+    const uint32_t q = pos + lane + 32 * j;
+    r[j] = mt_word(x[wrap624(q)], x[wrap624(q + 1)], x[wrap624(q + 397)]);
+  }
+}
+// Stores the first `count` of them over the words they replace.
+template <int W>
+__device__ __forceinline__ void mt_put(uint32_t* x, uint32_t pos, int count, int lane, const uint32_t (&r)[W]) {
+#pragma unroll
+  for (int j = 0; j < W; ++j)
+    if (lane + 32 * j < count) x[wrap624(pos + lane + 32 * j)] = r[j];
+}
+// Advances by `count` words; whether this lane met the word that tempers to 2^32 - 1.
+__device__ bool mt_skip(uint32_t* x, uint32_t& pos, int count, int lane) {
+  bool hit = false;
+  for (int left = count; left > 0; left -= 224) {
+    const int n = min(left, 224);
+    uint32_t r[7];
+    mt_next(x, pos, lane, r);
+#pragma unroll
+    for (int j = 0; j < 7; ++j) hit |= lane + 32 * j < n && r[j] == kRawAllOnes;
+    __syncwarp();
+    mt_put(x, pos, n, lane, r);
+    __syncwarp();
+    pos = wrap624(pos + n);
+  }
+  return hit;
+}
+
+// Per-warp shared memory of the kernel below.
+struct TwoSetSmem {
+  long long* clr;    // [nlay] cloud thresholds
+  long long* aux;    // [nlay] link thresholds
+  long long* srt;    // [32 nw] per 32-layer word, the cloud thresholds in ascending order
+  uint2* ev;         // [kTwoSetQueue] waiting events: draw; g-point | last layer << 8 | first layer << 16
+  uint32_t* xa;      // [624] state of set 1
+  uint32_t* xb;      // [624] state of set 2
+  uint32_t* pm;      // [33 nw] the mask of a word's layers with the c smallest thresholds
+  uint32_t* ow;      // [140 nw] flags
+  int16_t* nxt;      // [32 nw + 2] lowest cloudy layer at or above
+  __host__ __device__ static size_t bytes(int nlay, int nw) {
+    return ((size_t)16 * nlay + 256 * nw + 8 * kTwoSetQueue + 2 * 624 * 4 + 4 * (33 * nw + NGPT * nw) +
+            2 * (32 * nw + 2) + 15) & ~(size_t)15;
+  }
+  __device__ TwoSetSmem(char* p, int nlay, int nw) {
+    clr = reinterpret_cast<long long*>(p);
+    aux = clr + nlay;
+    srt = aux + nlay;
+    ev = reinterpret_cast<uint2*>(srt + 32 * nw);
+    xa = reinterpret_cast<uint32_t*>(ev + kTwoSetQueue);
+    xb = xa + 624;
+    pm = xb + 624;
+    ow = pm + 33 * nw;
+    nxt = reinterpret_cast<int16_t*>(ow + NGPT * nw);
+  }
+};
+
+// The flags of one event: per 32-layer word of its run, the layers whose
+// threshold the draw reaches are a prefix of the word's sorted thresholds.
+__device__ __forceinline__ void two_set_event(const TwoSetSmem& m, uint2 e, int nw) {
+  const long long v = e.x;
+  const int n = e.y & 255, k1 = (e.y >> 8) & 255, k0 = e.y >> 16;
+  for (int w = k0 >> 5; w <= (k1 >> 5); ++w) {
+    const int lo = max(k0 - 32 * w, 0), hi = min(k1 - 32 * w, 31);
+    const uint32_t run = (0xFFFFFFFFu >> (31 - hi)) & (0xFFFFFFFFu << lo);
+    const long long* sw = m.srt + 32 * w;
+    int cnt = 0;
+#pragma unroll
+    for (int st = 16; st >= 1; st >>= 1)
+      if (sw[cnt + st - 1] <= v) cnt += st;
+    cnt += (sw[31] <= v) ? 1 : 0;   // only when all 32 qualify (then cnt was 31)
+    const uint32_t f = run & m.pm[33 * w + cnt];
+    if (f) atomicOr(m.ow + n * nw + w, f);   // two events of a g-point may be in flight
+  }
+}
+
+__global__ void __launch_bounds__(32 * kTwoSetWarps)
+lw_mcica_two_set_kernel(const Block* __restrict__ blocks, int nblocks, const Block b0, int ncols, McicaArgs a,
+                        uint32_t* __restrict__ bits) {
+  extern __shared__ __align__(16) char smem_raw[];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int nlay = a.nlay, nlp1 = nlay + 1, nw = a.nw;
+  const int c = blockIdx.x * kTwoSetWarps + wib;
+  if (c >= ncols) return;   // the warps share nothing
+  const TwoSetSmem m(smem_raw + TwoSetSmem::bytes(nlay, nw) * wib, nlay, nw);
+
+  // cloud and link thresholds (inputs as in lw_mcica_kernel below)
+  const Block* B = (nblocks > 0) ? ((nblocks == 1) ? &b0 : &blocks[find_block(blocks, nblocks, c)]) : nullptr;
+  const int i = B ? c - B->col0 : 0;
+  int32_t seed;
+  bool any = false;
+  if (B) {
+    for (int k = lane; k < nlay; k += 32) {
+      const double cf = B->in[F_CLDCF][i + (size_t)B->ld * (a.top_at_1 ? nlp1 - (k + 1) - 1 : k)];
+      any |= cf > 1.0e-6;
+      m.clr[k] = umin_ge(1.0 - ((cf < 2.2250738585072014e-308) ? 0.0 : cf));
+    }
+    seed = (a.isubclw == 1) ? 140 + (B->seed0 + i + 1) : B->icseed[i];   // RLM:765-773
+  } else {
+    for (int k = lane; k < nlay; k += 32) m.clr[k] = umin_ge(1.0 - a.st.cldf[c + (size_t)a.st.ld * k]);
+    any = true;
+    seed = a.st.seed[c];
+  }
+  if (!__any_sync(0xffffffffu, any)) return;   // clear column: no draws
+  if (a.iovr == 3) {
+    // fac_lcf(k) = exp(-0.5 (dz(k) + dz(k-1)) / de_lgth), dz in the internal order (RLM:819, 2001)
+    const double dl = B ? B->in[F_DELGTH][i] : a.st.delg[c];
+    for (int k = 1 + lane; k < nlay; k += 32) {
+      double dz0, dz1;
+      if (B) {
+        const int r0 = a.top_at_1 ? nlp1 - (k + 1) - 1 : k, r1 = a.top_at_1 ? nlp1 - k - 1 : k - 1;
+        dz0 = B->in[F_DZLYR][i + (size_t)B->ld * r0];
+        dz1 = B->in[F_DZLYR][i + (size_t)B->ld * r1];
+      } else {
+        dz0 = a.st.dz[c + (size_t)a.st.ld * k];
+        dz1 = a.st.dz[c + (size_t)a.st.ld * (k - 1)];
+      }
+      m.aux[k] = umax_le(exp(-0.5 * (dz0 + dz1) / dl));
+    }
+  } else {
+    // alpha is taken in the caller's row order, unflipped (RLM:820, 933)
+    for (int k = lane; k < nlay; k += 32)
+      m.aux[k] = ulim_lt(B ? B->in[F_ALPHA][i + (size_t)B->ld * k] : a.st.alpha[c + (size_t)a.st.ld * k]);
   }
   __syncwarp();
-  // set 2 starts at draw 140 nlay of the same stream: its first layer_draws
-  // call appends blocks up to there
-  const int P0 = NGPT * nlay;
-  TwoSetStream sa{624, 624, 624}, sb{624 + P0, (624 + P0) % kTwoSetRing, 624};
-  uint32_t cdf[5], c1[5], c2[5];
-  uint32_t word[5] = {0u, 0u, 0u, 0u, 0u};
-  int start[5] = {0, 0, 0, 0, 0}, wi[5] = {0, 0, 0, 0, 0};
-  for (int k = 0; k < nlay; ++k) {
-    layer_draws(mtA, sa, lane, c1);
-    layer_draws(mtB, sb, lane, c2);
-    if (iovr == 3) {
-      const bool top = (k == nlay - 1);
-      const long long fk = top ? 0 : aux_t[k + 1];
-#pragma unroll
-      for (int j = 0; j < 5; ++j) {
-        const int n = lane + 32 * j;
-        if (n >= NGPT) continue;
-        if (!top && (long long)c2[j] <= fk) continue;   // linked to the layer above: still waiting
-        // the run start[j]..k takes this layer's set-1 draw: per 32-layer word,
-        // the layers whose threshold it reaches are a prefix of the word's
-        // sorted thresholds (RLM:2097-2103)
-        const long long v = c1[j];
-        for (int w = start[j] >> 5; w <= (k >> 5); ++w) {
-          const int lo = max(start[j], 32 * w) - 32 * w, hi = min(k, 32 * w + 31) - 32 * w;
-          const uint32_t rm = (hi == 31 ? 0xFFFFFFFFu : ((1u << (hi + 1)) - 1u)) & ~((1u << lo) - 1u);
-          const long long* sw = srt + 32 * w;
-          int cnt = 0;
-#pragma unroll
-          for (int st = 16; st >= 1; st >>= 1)
-            if (sw[cnt + st - 1] <= v) cnt += st;
-          cnt += (sw[31] <= v) ? 1 : 0;   // only when all 32 qualify (then cnt was 31)
-          if (w != wi[j]) {
-            out[n * nw + wi[j]] = word[j];
-            word[j] = 0u;
-            wi[j] = w;
-          }
-          word[j] |= rm & pm[33 * w + cnt];
-        }
-        start[j] = k + 1;
+  // the next cloudy layer above each, and iovr 3's sorted thresholds and
+  // prefix masks per 32-layer word (layers past nlay never qualify)
+  int up = kNoCloud, ktop = -1;
+  if (lane == 0) m.nxt[32 * nw] = kNoCloud;
+  for (int w = nw - 1; w >= 0; --w) {
+    const int k = 32 * w + lane;
+    const long long th = (k < nlay) ? m.clr[k] : LLONG_MAX;
+    const uint32_t cloudy = __ballot_sync(0xffffffffu, th < 0xFFFFFFFFLL);
+    const uint32_t here = cloudy & (0xFFFFFFFFu << lane);
+    m.nxt[k] = (int16_t)(here ? 32 * w + __ffs(here) - 1 : up);
+    if (cloudy) {
+      up = 32 * w + __ffs(cloudy) - 1;
+      if (ktop < 0) ktop = 32 * w + 31 - __clz(cloudy);
+    }
+    if (a.iovr == 3) {
+      int rank = 0;
+      for (int o = 0; o < 32; ++o) {
+        const long long t2 = __shfl_sync(0xffffffffu, th, o);
+        rank += (t2 < th || (t2 == th && o < lane)) ? 1 : 0;
       }
-    } else {
-      const long long ak = aux_t[k];
-      const long long ck = clr_t[k];
-#pragma unroll
-      for (int j = 0; j < 5; ++j) {
-        const int n = lane + 32 * j;
-        if (n >= NGPT) continue;
-        cdf[j] = (k > 0 && (long long)c2[j] < ak) ? cdf[j] : c1[j];
-        if ((long long)cdf[j] >= ck) word[j] |= 1u << (k & 31);
-        if ((k & 31) == 31 || k == nlay - 1) {
-          out[n * nw + (k >> 5)] = word[j];
-          word[j] = 0u;
-        }
+      m.srt[32 * w + rank] = th;
+      for (int q = 0; q <= 32; ++q) {
+        const uint32_t b = __ballot_sync(0xffffffffu, rank < q);
+        if (lane == 0) m.pm[33 * w + q] = b;
       }
     }
   }
-  if (iovr == 3) {
+  const uint32_t s0 = (uint32_t)(seed == 0 ? 4357 : seed);   // random_setseed_t (MT:285-299)
+  const uint32_t below = (1u << lane) - 1u;
+
+  for (bool walk_all = false;; walk_all = true) {
+    // mt(i) = 69069^i seed; set 2 starts 140 nlay draws on
+    uint32_t v = s0 * c_pow69069[lane];
+    for (int n = lane; n < 624; n += 32) {
+      m.xa[n] = m.xb[n] = v;
+      v *= kPow69069_32;
+    }
+    for (int n = lane; n < NGPT * nw; n += 32) m.ow[n] = 0u;
+    __syncwarp();
+    uint32_t pa = 0, pb = 0;
+    mt_skip(m.xb, pb, NGPT * nlay, lane);
+
+    int start[5], nc[5];          // iovr 3: the waiting run's first layer and its lowest cloudy one
+    uint32_t cdf[5], word[5];     // iovr 4, 5: the value carried up, the flags of this 32-layer word
+    const int nc0 = m.nxt[0];
 #pragma unroll
     for (int j = 0; j < 5; ++j) {
-      const int n = lane + 32 * j;
-      if (n < NGPT) out[n * nw + wi[j]] = word[j];
+      start[j] = 0;
+      nc[j] = (lane + 32 * j < NGPT) ? nc0 : kNoCloud;
+      cdf[j] = word[j] = 0u;
     }
+    int nev = 0, k = 0;
+    for (; k < nlay; ++k) {
+      if (k > ktop && !walk_all) {   // nothing cloudy from here on
+        bool more = false;
+#pragma unroll
+        for (int j = 0; j < 5; ++j) more |= (a.iovr == 3) ? nc[j] < k : cdf[j] == 0xFFFFFFFFu;
+        if (!__any_sync(0xffffffffu, more)) break;
+      }
+      uint32_t c1[5], c2[5];
+      mt_next(m.xa, pa, lane, c1);
+      mt_next(m.xb, pb, lane, c2);
+      __syncwarp();
+      mt_put(m.xa, pa, NGPT, lane, c1);
+      mt_put(m.xb, pb, NGPT, lane, c2);
+      __syncwarp();
+      pa = wrap624(pa + NGPT);
+      pb = wrap624(pb + NGPT);
+#pragma unroll
+      for (int j = 0; j < 5; ++j) {
+        c1[j] = temper(c1[j]);
+        c2[j] = temper(c2[j]);
+      }
+      if (a.iovr == 3) {
+        const bool top = (k == nlay - 1);
+        const long long fk = top ? -1 : m.aux[k + 1];
+        const int nc1 = m.nxt[k + 1];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+          const int n = lane + 32 * j;
+          const bool brk = n < NGPT && (long long)c2[j] > fk;   // not linked to the layer above
+          const bool put = brk && (k >= nc[j] || c1[j] == 0xFFFFFFFFu);
+          const uint32_t b = __ballot_sync(0xffffffffu, put);
+          if (put) m.ev[nev + __popc(b & below)] = make_uint2(c1[j], n | (k << 8) | (start[j] << 16));
+          nev += __popc(b);
+          if (brk) {
+            start[j] = k + 1;
+            nc[j] = nc1;
+          }
+        }
+        if (nev >= 32) {
+          __syncwarp();
+          do {
+            nev -= 32;
+            two_set_event(m, m.ev[nev + lane], nw);
+          } while (nev >= 32);
+          __syncwarp();
+        }
+      } else {
+        const long long ak = m.aux[k], ck = m.clr[k];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+          const int n = lane + 32 * j;
+          if (n >= NGPT) continue;
+          cdf[j] = (k > 0 && (long long)c2[j] < ak) ? cdf[j] : c1[j];
+          if ((long long)cdf[j] >= ck) word[j] |= 1u << (k & 31);
+          if ((k & 31) == 31) {
+            m.ow[n * nw + (k >> 5)] = word[j];
+            word[j] = 0u;
+          }
+        }
+      }
+    }
+    // what the walk left out may hold the one draw that flags a clear layer
+    const bool again = k < nlay && __any_sync(0xffffffffu, mt_skip(m.xa, pa, NGPT * (nlay - k), lane));
+    if (again) continue;
+    __syncwarp();
+    if (a.iovr == 3) {
+      if (lane < nev) two_set_event(m, m.ev[lane], nw);
+    } else if (k & 31) {   // the last word begun
+#pragma unroll
+      for (int j = 0; j < 5; ++j)
+        if (lane + 32 * j < NGPT) m.ow[(lane + 32 * j) * nw + (k >> 5)] = word[j];
+    }
+    break;
   }
+  __syncwarp();
+  uint32_t* out = bits + (size_t)c * NGPT * nw;
+  for (int n = lane; n < NGPT * nw; n += 32) out[n] = m.ow[n];
 }
 
 // The draws of random (iovr=0) and maximum-random (iovr=1) overlap come from
@@ -282,19 +462,15 @@ __host__ __device__ constexpr uint32_t temper_c(uint32_t y) {
 }
 static_assert(temper_c(kRawAllOnes) == 0xFFFFFFFFu, "kRawAllOnes tempers to 2^32 - 1");
 
-// Per-warp shared memory: clear[nlay] = 1 - cldf (double), ring[cap].  For
-// iovr 3..5 the ring's space holds the two twister states and the per-layer
-// overlap parameter instead.
+// Per-warp shared memory: clear[nlay] = 1 - cldf (double), ring[cap].
 __host__ __device__ inline size_t mcica_warp_bytes(int nlay, int cap) {
   return ((nlay * 8 + 15) & ~15) + (size_t)cap * 4;
 }
 
 constexpr int kMcicaWarps = 6;   // 6 warps x 18.5 KB (127 layers): two CTAs, twelve warps per SM
 
-// NG g-points per column: 140 for the longwave path (every overlap, block or
-// stage inputs), 112 for the shortwave path (stage inputs, iovr 0..2: the
-// shortwave decorrelation-length and exponential overlaps draw in another
-// order, radsw_main.F90:2101-2198, and are not built here).
+// iovr 0..2.  NG g-points per column: 140 for the longwave path (block or
+// stage inputs), 112 for the shortwave path (stage inputs).
 template <int NG>
 __global__ void __launch_bounds__(32 * kMcicaWarps)
 lw_mcica_kernel(const Block* __restrict__ blocks, int nblocks, const Block b0, int ncols, McicaArgs a,
@@ -335,71 +511,6 @@ lw_mcica_kernel(const Block* __restrict__ blocks, int nblocks, const Block b0, i
     const uint32_t s0 = (uint32_t)(seed == 0 ? 4357 : seed);   // random_setseed_t (MT:285-299)
 
     uint32_t* out = bits + (size_t)c * NG * a.nw;
-    if constexpr (NG == NGPT) {
-    if (a.iovr >= 3) {
-      // two sequence rings, the per-layer overlap parameter and the walk's
-      // thresholds in the ring's space
-      uint32_t* mtA = ring;
-      uint32_t* mtB = ring + kTwoSetRing;
-      double* aux = reinterpret_cast<double*>(ring + 2 * kTwoSetRing);
-      const Block* B = (nblocks > 0) ? ((nblocks == 1) ? &b0 : &blocks[find_block(blocks, nblocks, c)]) : nullptr;
-      const int i = B ? c - B->col0 : 0;
-      if (a.iovr == 3) {
-        // fac_lcf(k) = exp(-0.5 (dz(k) + dz(k-1)) / de_lgth), dz in the internal order (RLM:819, 2001)
-        const double dl = B ? B->in[F_DELGTH][i] : a.st.delg[c];
-        for (int k = 1 + lane; k < nlay; k += 32) {
-          double dz0, dz1;
-          if (B) {
-            const int r0 = a.top_at_1 ? nlp1 - (k + 1) - 1 : k, r1 = a.top_at_1 ? nlp1 - k - 1 : k - 1;
-            dz0 = B->in[F_DZLYR][i + (size_t)B->ld * r0];
-            dz1 = B->in[F_DZLYR][i + (size_t)B->ld * r1];
-          } else {
-            dz0 = a.st.dz[c + (size_t)a.st.ld * k];
-            dz1 = a.st.dz[c + (size_t)a.st.ld * (k - 1)];
-          }
-          aux[k] = exp(-0.5 * (dz0 + dz1) / dl);
-        }
-      } else {
-        // alpha is taken in the caller's row order, unflipped (RLM:820, 933)
-        for (int k = lane; k < nlay; k += 32)
-          aux[k] = B ? B->in[F_ALPHA][i + (size_t)B->ld * k] : a.st.alpha[c + (size_t)a.st.ld * k];
-      }
-      // the walk's integer thresholds, after the rings and aux
-      long long* aux_t = reinterpret_cast<long long*>(aux + nlay);
-      long long* clr_t = aux_t + nlay;
-      __syncwarp();
-      for (int k = lane; k < nlay; k += 32) {
-        clr_t[k] = umin_ge(clr[k]);
-        if (a.iovr == 3) aux_t[k] = (k > 0) ? umax_le(aux[k]) : 0;
-        else aux_t[k] = ulim_lt(aux[k]);
-      }
-      __syncwarp();
-      // iovr 3: per 32-layer word, the cloud thresholds in ascending order and,
-      // for each count c, the mask of the word's layers with the c smallest
-      // (layers past nlay never qualify)
-      long long* srt = clr_t + nlay;
-      uint32_t* pm = reinterpret_cast<uint32_t*>(srt + 32 * a.nw);
-      if (a.iovr == 3) {
-        for (int w = 0; w < a.nw; ++w) {
-          const int m = 32 * w + lane;
-          const long long th = (m < nlay) ? clr_t[m] : LLONG_MAX;
-          int rank = 0;
-          for (int o = 0; o < 32; ++o) {
-            const long long t2 = __shfl_sync(0xffffffffu, th, o);
-            rank += (t2 < th || (t2 == th && o < lane)) ? 1 : 0;
-          }
-          srt[32 * w + rank] = th;
-          for (int c = 0; c <= 32; ++c) {
-            const uint32_t b = __ballot_sync(0xffffffffu, rank < c);
-            if (lane == 0) pm[33 * w + c] = b;
-          }
-        }
-        __syncwarp();
-      }
-      mcica_two_set(mtA, mtB, clr_t, aux_t, srt, pm, nlay, a.iovr, s0, a.nw, out, lane);
-      continue;
-    }
-    }
     // seeding x_0..x_623 at ring[0..623]: mt(i) = 69069^i seed
     for (int n = lane; n < 624; n += 32) ring[n] = s0 * c_pow69069[n];
     __syncwarp();
@@ -614,19 +725,17 @@ cudaError_t seed_gather_launch(const uint32_t* raw, const int32_t* imap, const i
   return cudaGetLastError();
 }
 
-// ring words: one round's draws plus a twist block, and at least the two
-// rings, the overlap parameter, the two threshold arrays and the per-word
-// sorted thresholds and masks of iovr 3..5; a multiple of 624
+// ring words: one round's draws plus a twist block (at least two blocks, for
+// iovr 2), a multiple of 624
 int mcica_ring_capacity(int nlay) {
-  const long round = (long)kMcicaRound * nlay + 623;
-  const long nw = (nlay + 31) / 32;
-  const long two_set = 2L * kTwoSetRing + 6L * nlay + 97L * nw;   // + sorted thresholds, prefix masks
-  const long need = round > two_set ? round : two_set;
+  const long need = std::max((long)kMcicaRound * nlay + 623, 1248L);
   return (int)((need + 623) / 624 * 624);
 }
 
 cudaError_t mcica_prepare(int max_smem) {
   cudaError_t e = cudaFuncSetAttribute(lw_mcica_kernel<NGPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(lw_mcica_two_set_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(lw_mcica_kernel<kSwNgpt>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
 }
@@ -648,6 +757,13 @@ cudaError_t mcica_launch(const Block* blocks, int nblocks, const Block& b0, int 
   a.top_at_1 = top_at_1;
   a.cap = mcica_ring_capacity(nlay);
   a.st = stage;
+  if (iovr >= 3) {
+    if (ncols < 1) return cudaSuccess;
+    const size_t smem = TwoSetSmem::bytes(nlay, a.nw) * kTwoSetWarps;
+    lw_mcica_two_set_kernel<<<(ncols + kTwoSetWarps - 1) / kTwoSetWarps, 32 * kTwoSetWarps, smem, st>>>(
+        blocks, nblocks, b0, ncols, a, bits);
+    return cudaGetLastError();
+  }
   const int wpb = kMcicaWarps;
   size_t smem = mcica_warp_bytes(nlay, a.cap) * wpb;
   int per_sm = 0;
@@ -668,97 +784,98 @@ cudaError_t mcica_launch(const Block* blocks, int nblocks, const Block& b0, int 
 // Shortwave sub-columns with decorrelation-length (iovr 3) or exponential /
 // exponential-random (iovr 4, 5) overlap (radsw_main.F90:2101-2198).  Both
 // random sets are g-major, set 1 = draws [0, 112 nlay) and set 2 = draws
-// [112 nlay, 224 nlay) of one stream, cdfunc(k, n) = draw (n-1) nlay + k.
-// Set 2 is read from a second sequence ring that runs 112 nlay draws ahead
-// of the first; each ring holds one round's draws plus the twist history,
-// as in the iovr 0/1 walk.  Each lane walks its g-point: top-down for iovr
-// 3 (cdfunc(k) = cdfunc(k+1) when cdfun2(k) <= fac_lcf(k+1)), bottom-up for
-// 4, 5 (cdfunc(k) = cdfunc(k-1) when cdfun2(k) < alpha(k)), flagging
-// cdfunc(k) >= 1 - cldf(k).  stage.alpha holds fac_lcf (iovr 3, entry k is
-// the factor between layers k-1 and k) or alpha (iovr 4, 5), per layer in
-// internal order.
-constexpr int kSwTwoSetMaxWarps = 8;   // warps per CTA: as many as the shared memory holds, up to 8
+// [112 nlay, 224 nlay) of one stream, cdfunc(k, n) = draw (n-1) nlay + k, so
+// the draws of a g-point lie side by side: lanes are the layers of a 32-layer
+// word.  cdfunc(k) = cdfunc(k+1) when cdfun2(k) <= fac_lcf(k+1) (iovr 3), or
+// cdfunc(k-1) when cdfun2(k) < alpha(k) (iovr 4, 5): a layer's value is the
+// draw of the nearest layer above (below) it that is not linked.  The ballot
+// of the broken links names that lane, a shuffle brings its draw, runs that
+// cross a word take the value carried from the word before, and the ballot of
+// cdfunc(k) >= 1 - cldf(k) is the word of flags.  The comparisons are of
+// tempered words with integer thresholds (umin_ge and its like).
+// stage.alpha holds fac_lcf (iovr 3, entry k is the factor between layers k-1
+// and k) or alpha (iovr 4, 5), per layer in internal order.
+//
+// Each set is read from its own ring of two twister blocks; set 2's runs 112
+// nlay draws ahead.  A g-point needs at most 255 draws, so a block is
+// overwritten only once it has been read.
+//
+// Bound by integer issue.  3,001 columns of 64 layers (1,800 daylit), iovr 3,
+// with the kernel that forms fac_lcf: 0.25 ms with a lane per g-point (28 of
+// 32 lanes, rings of 28 g-points, draws converted to FP64), 0.11 ms so.
+constexpr int kSwTwoSetRing = 1248;
+constexpr int kSwTwoSetWarps = 2;   // per CTA, a column each
 
-__host__ __device__ inline size_t sw_two_set_warp_bytes(int nlay, int cap) {
-  return 2 * (((size_t)nlay * 8 + 15) & ~(size_t)15) + 2 * (size_t)cap * 4;
+__host__ __device__ inline size_t sw_two_set_warp_bytes(int nlay) {
+  return (2 * (size_t)nlay * 8 + 2 * (size_t)kSwTwoSetRing * 4 + 15) & ~(size_t)15;
 }
 
-__global__ void __launch_bounds__(32 * kSwTwoSetMaxWarps)
+__global__ void __launch_bounds__(32 * kSwTwoSetWarps)
 sw_mcica_two_set_kernel(int ncols, McicaArgs a, uint32_t* __restrict__ bits) {
   extern __shared__ __align__(16) char smem_raw[];
+  constexpr uint32_t kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int nlay = a.nlay, cap = a.cap, nw = a.nw;
-  const size_t lb = ((size_t)nlay * 8 + 15) & ~(size_t)15;
-  char* my = smem_raw + sw_two_set_warp_bytes(nlay, cap) * wib;
-  double* clr = reinterpret_cast<double*>(my);         // 1 - cldf(k)
-  double* aux = reinterpret_cast<double*>(my + lb);    // fac_lcf or alpha
-  uint32_t* ra = reinterpret_cast<uint32_t*>(my + 2 * lb);
-  uint32_t* rb = ra + cap;
-  const int wpb = blockDim.x >> 5;
-  const int warps_total = gridDim.x * wpb;
-  const long long P0 = (long long)kSwNgpt * nlay;   // set 2 starts here
-  for (int c = blockIdx.x * wpb + wib; c < ncols; c += warps_total) {
-    __syncwarp();
-    for (int k = lane; k < nlay; k += 32) {
-      clr[k] = 1.0 - a.st.cldf[c + (size_t)a.st.ld * k];
-      aux[k] = a.st.alpha[c + (size_t)a.st.ld * k];
+  const int nlay = a.nlay, nw = a.nw;
+  const int c = blockIdx.x * kSwTwoSetWarps + wib;
+  if (c >= ncols) return;   // the warps share nothing
+  long long* clr = reinterpret_cast<long long*>(smem_raw + sw_two_set_warp_bytes(nlay) * wib);
+  long long* aux = clr + nlay;   // layer k is not linked when its set-2 word is >= aux[k]
+  uint32_t* ra = reinterpret_cast<uint32_t*>(aux + nlay);
+  uint32_t* rb = ra + kSwTwoSetRing;
+  for (int k = lane; k < nlay; k += 32) {
+    clr[k] = umin_ge(1.0 - a.st.cldf[c + (size_t)a.st.ld * k]);
+    if (a.iovr == 3)
+      aux[k] = (k == nlay - 1) ? 0 : umax_le(a.st.alpha[c + (size_t)a.st.ld * (k + 1)]) + 1;
+    else
+      aux[k] = (k == 0) ? 0 : ulim_lt(a.st.alpha[c + (size_t)a.st.ld * k]);
+  }
+  const int32_t seed = a.st.seed[c];
+  uint32_t x = (uint32_t)(seed == 0 ? 4357 : seed) * c_pow69069[lane];   // random_setseed_t (MT:285-299)
+  for (int n = lane; n < 624; n += 32) {
+    ra[n] = rb[n] = x;
+    x *= kPow69069_32;
+  }
+  __syncwarp();
+  // sequence indices: of the g-point's first draw in each set, and generated so far
+  int sa = 624, sb = 624 + kSwNgpt * nlay, ga = 624, gb = 624;
+  uint32_t* out = bits + (size_t)c * kSwNgpt * nw;
+  for (int n = 0; n < kSwNgpt; ++n) {
+    while (ga < sa + nlay) {
+      twist_ring(ra, kSwTwoSetRing, (ga / 624) & 1 ? 624 : 0, lane);
+      ga += 624;
     }
-    const int32_t seed = a.st.seed[c];
-    const uint32_t s0 = (uint32_t)(seed == 0 ? 4357 : seed);   // random_setseed_t (MT:285-299)
-    for (int n = lane; n < 624; n += 32) ra[n] = rb[n] = s0 * c_pow69069[n];
-    __syncwarp();
-    long long ga = 624, gb = 624;    // sequence words generated in each ring
-    int ja = 624 % cap, jb = 624 % cap;
-    uint32_t* out = bits + (size_t)c * kSwNgpt * nw;
-    for (int n0 = 0; n0 < kSwNgpt; n0 += kMcicaRound) {
-      const long long need_a = 624 + (long long)(n0 + kMcicaRound) * nlay;
-      while (ga < need_a) {
-        twist_ring(ra, cap, ja, lane);
-        ga += 624;
-        ja += 624;
-        if (ja == cap) ja = 0;
-      }
-      const long long need_b = need_a + P0;
-      while (gb < need_b) {
-        twist_ring(rb, cap, jb, lane);
-        gb += 624;
-        jb += 624;
-        if (jb == cap) jb = 0;
-      }
-      const int n = n0 + lane;
-      if (lane < kMcicaRound) {
-        const int qa = (int)((624 + (long long)n * nlay) % cap);
-        const int qb = (int)((624 + P0 + (long long)n * nlay) % cap);
-        auto at = [&](const uint32_t* r, int q0, int k) {
-          int q = q0 + k;
-          if (q >= cap) q -= cap;
-          return u32_unit(temper(r[q]));
-        };
-        uint32_t word = 0;
-        if (a.iovr == 3) {
-          double cur = at(ra, qa, nlay - 1);
-          for (int k = nlay - 1; k >= 0; --k) {
-            if (k < nlay - 1 && !(at(rb, qb, k) <= aux[k + 1])) cur = at(ra, qa, k);
-            if (cur >= clr[k]) word |= 1u << (k & 31);
-            if ((k & 31) == 0) {
-              out[n * nw + (k >> 5)] = word;
-              word = 0;
-            }
-          }
-        } else {
-          double cur = 0.0;
-          for (int k = 0; k < nlay; ++k) {
-            if (k == 0 || !(at(rb, qb, k) < aux[k])) cur = at(ra, qa, k);
-            if (cur >= clr[k]) word |= 1u << (k & 31);
-            if ((k & 31) == 31 || k == nlay - 1) {
-              out[n * nw + (k >> 5)] = word;
-              word = 0;
-            }
-          }
-        }
-      }
-      __syncwarp();
+    while (gb < sb + nlay) {
+      twist_ring(rb, kSwTwoSetRing, (gb / 624) & 1 ? 624 : 0, lane);
+      gb += 624;
     }
+    const int qa = sa % kSwTwoSetRing, qb = sb % kSwTwoSetRing;
+    uint32_t carry = 0;   // the value at the edge of the word before
+    for (int i = 0; i < nw; ++i) {
+      const int w = (a.iovr == 3) ? nw - 1 - i : i;
+      const int k = 32 * w + lane;
+      const bool in = k < nlay;
+      uint32_t v = 0, l = 0;
+      long long lk = 0, ck = 0;
+      if (in) {
+        const int ia = qa + k, ib = qb + k;
+        v = temper(ra[ia >= kSwTwoSetRing ? ia - kSwTwoSetRing : ia]);
+        l = temper(rb[ib >= kSwTwoSetRing ? ib - kSwTwoSetRing : ib]);
+        lk = aux[k];
+        ck = clr[k];
+      }
+      const uint32_t brk = __ballot_sync(kAll, in && (long long)l >= lk);
+      // the nearest broken link at or above (iovr 3) or at or below this layer
+      const uint32_t at = brk & ((a.iovr == 3) ? kAll << lane : kAll >> (31 - lane));
+      const int src = (a.iovr == 3) ? __ffs(at) - 1 : 31 - __clz(at);
+      const uint32_t got = __shfl_sync(kAll, v, src & 31);
+      const uint32_t cdf = at ? got : carry;
+      const uint32_t flags = __ballot_sync(kAll, in && (long long)cdf >= ck);
+      if (lane == 0) out[n * nw + w] = flags;
+      carry = __shfl_sync(kAll, cdf, (a.iovr == 3) ? 0 : 31);
+    }
+    sa += nlay;
+    sb += nlay;
+    __syncwarp();   // the reads of a block before it is overwritten
   }
 }
 
@@ -775,25 +892,12 @@ cudaError_t mcica_sw_two_set_launch(int ncols, int nlay, int iovr, const McicaSt
   a.iovr = iovr;
   a.isubclw = 2;
   a.top_at_1 = 0;
-  const long round = (long)kMcicaRound * nlay + 623;
-  a.cap = (int)((round + 623) / 624 * 624);
+  a.cap = kSwTwoSetRing;
   a.st = stage;
-  static const int max_smem = [] {   // initialised once, thread-safe
-    int dev = 0, v = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    return v;
-  }();
-  const size_t per_warp = sw_two_set_warp_bytes(nlay, a.cap);
-  const int wpb = (int)std::min<size_t>(kSwTwoSetMaxWarps, (size_t)max_smem / per_warp);
-  if (wpb < 1) return cudaErrorInvalidValue;
-  const size_t smem = per_warp * wpb;
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sw_mcica_two_set_kernel, 32 * wpb, smem);
-  if (per_sm < 1) per_sm = 1;
-  const int grid = min((ncols + wpb - 1) / wpb, num_sms * per_sm);
-  if (grid < 1) return cudaSuccess;
-  sw_mcica_two_set_kernel<<<grid, 32 * wpb, smem, st>>>(ncols, a, bits);
+  if (ncols < 1) return cudaSuccess;
+  const size_t smem = sw_two_set_warp_bytes(nlay) * kSwTwoSetWarps;
+  sw_mcica_two_set_kernel<<<(ncols + kSwTwoSetWarps - 1) / kSwTwoSetWarps, 32 * kSwTwoSetWarps, smem, st>>>(ncols, a,
+                                                                                                           bits);
   return cudaGetLastError();
 }
 
