@@ -228,6 +228,16 @@ extern "C" int rrtmg_lw_gpu_init(const rrtmg_lw_init_args* a, char* errmsg, int3
   std::vector<double> kt(RRTMG_LW_TABLES_NDOUBLE);
   std::memcpy(kt.data(), rrtmg_lw_tables_blob, nblob);
   std::vector<float> kt32(kt.begin(), kt.end());
+  // band-fastest copies behind the blob (lw_common.cuh, bandtab)
+  kt.resize(bandtab::end, 0.0);
+  const auto band_fastest = [&kt](int dst, int src, int rows) {
+    for (int r = 0; r < rows; ++r)
+      for (int b = 0; b < NBANDS; ++b) kt[dst + NBANDS * r + b] = kt[src + r + rows * b];
+  };
+  band_fastest(bandtab::totplnk, lwtab::totplnk, 181);
+  band_fastest(bandtab::absliq1, lwtab::absliq1, 58);
+  band_fastest(bandtab::absice2, lwtab::absice2, 43);
+  band_fastest(bandtab::absice3, lwtab::absice3, 46);
 
   if (!g.kt64) {
     CK(cudaMalloc(&g.kt64, kt.size() * sizeof(double)), "cudaMalloc(tables)");

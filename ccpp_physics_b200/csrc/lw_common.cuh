@@ -54,6 +54,16 @@ struct Tables {
   const R* trec;     // the rlwinit tables
 };
 
+// Copies of the Planck and cloud tables with the band fastest, behind the blob
+// in the FP64 arrays (offsets into kt): a row is one 128-byte line.
+namespace bandtab {
+constexpr int totplnk = (RRTMG_LW_TABLES_NDOUBLE + 15) & ~15;
+constexpr int absliq1 = totplnk + 181 * NBANDS;
+constexpr int absice2 = absliq1 + 58 * NBANDS;
+constexpr int absice3 = absice2 + 43 * NBANDS;
+constexpr int end = absice3 + 46 * NBANDS;
+}  // namespace bandtab
+
 // exp_tbl(it), tfn_tbl(it), tau_tbl(it) of one record.
 __device__ __forceinline__ void tbl_exp_tfn(const double* trec, int it, double& ex, double& tf) {
   const double2 v = __ldg(reinterpret_cast<const double2*>(trec) + it);

@@ -69,7 +69,7 @@ static __device__ __constant__ double c_a2[16] = {0.00, -12.0, -11.7, 0.00, -0.7
 
 // checked read of the FP64 coefficient tables
 __device__ __forceinline__ double t64(const double* kt, long long o) {
-  if (!LW_OK(o >= 0 && o < RRTMG_LW_TABLES_NDOUBLE, 11, o)) return 0.0;
+  if (!LW_OK(o >= 0 && o < bandtab::end, 11, o)) return 0.0;
   return __ldg(kt + o);
 }
 

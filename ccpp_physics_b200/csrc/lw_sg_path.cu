@@ -64,14 +64,20 @@ static_assert(SR_WARPS * SR_GPW == NGPT, "g-points per column");
 // shared memory of one column group
 struct SrGroup {
   float4 bf[SR_NL][NBANDS];             // {pklay, pklev above - pklay, pklev below - pklay, secdiff * taucld}
-  float part[SR_WARPS][4][SR_NL + 1];   // per-warp level sums: total down, clear down, total up, clear up
   union {
+    struct {                            // prologue: what a layer's bands share
+      double frlay[SR_NL], frlev[SR_NL];           // Planck interpolation fractions, layer and its upper level
+      double fliq[SR_NL], fice[SR_NL], refice[SR_NL], clwp[SR_NL], ciwp[SR_NL], cda1[SR_NL], tauran[SR_NL],
+          tausnw[SR_NL];                           // CloudLayer
+      int indlay[SR_NL], indlev[SR_NL], iliq[SR_NL], iice[SR_NL];   // iliq 0: no cloud
+    } lay;
     struct {
-      float pkv[SR_NL + 1][NBANDS];     // pklev(b, l) (prologue)
-    } p;
-    double fn[2][SR_NL + 1];            // net flux (total, clear sky; output)
+      float part[SR_WARPS][4][SR_NL + 1];   // per-warp level sums: total down, clear down, total up, clear up
+      double fn[2][SR_NL + 1];              // net flux (total, clear sky; output)
+    } o;
   } u;
   double pw[SR_WARPS][2];               // per-warp sums of coldry + colh2o and of colh2o (prologue)
+  double tz0, stemp, plev0;             // surface level and skin temperature, surface level pressure
   float secd[NBANDS];                   // diffusivity angle per band
   float pk0[NBANDS];                    // pklay(b, 0) (surface temperature)
   float semis;
@@ -156,14 +162,15 @@ __device__ __forceinline__ void cloud_terms(float od, int it, float odcld, const
 
 // cldprop band optics of one layer (RLM:1589-1799), FP64: the layer's
 // band-independent terms once (set: indices and interpolation fractions,
-// one division), then each band's table interpolation (band); the
-// arithmetic of band_taucld (lw_gas.cuh) with the per-band work hoisted.
+// one division; kept in the group's shared memory), then each band's table
+// interpolation (band); the arithmetic of band_taucld (lw_gas.cuh) with the
+// per-band work hoisted and the tables band-fastest (bandtab).
 struct CloudLayer {
-  double cf, clwp, ciwp, cda1, tauran, tausnw, fliq, fice, refice;
+  double clwp, ciwp, cda1, tauran, tausnw, fliq, fice, refice;
   int iliq, iice;
-  __device__ __forceinline__ void set(const Flags& f, double cf_, double clwp_, double relw, double ciwp_,
-                                      double reiw, double cda1_, double cda3, double cda4) {
-    cf = cf_; clwp = clwp_; ciwp = ciwp_; cda1 = cda1_;
+  __device__ __forceinline__ void set(const Flags& f, double clwp_, double relw, double ciwp_, double reiw,
+                                      double cda1_, double cda3, double cda4) {
+    clwp = clwp_; ciwp = ciwp_; cda1 = cda1_;
     tauran = kAbsrain * cda1;
     tausnw = (cda3 > 0.0 && cda4 > 10.0) ? kAbssnow0 * 1.05756 * cda3 / cda4 : 0.0;
     const double lfac = relw - 1.5;
@@ -178,31 +185,34 @@ struct CloudLayer {
     fice = ifac - (double)iice;
   }
   __device__ __forceinline__ double band(int b, const Flags& f, const double* kt) const {
-    if (!(cf > 2.2250738585072014e-308)) return 0.0;   // cfrac(k) > cldmin = tiny
     if (f.ilwcliq <= 0) return cda1;                    // diagnostic cloud optical depth
     double tauliq = 0.0, tauice = 0.0;
     if (clwp > 0.0 && f.ilwcliq == 1) {
-      const double a = t64(kt, lwtab::absliq1 + (iliq - 1) + 58 * b);
-      const double c = t64(kt, lwtab::absliq1 + iliq + 58 * b);
+      const double a = t64(kt, bandtab::absliq1 + NBANDS * (iliq - 1) + b);
+      const double c = t64(kt, bandtab::absliq1 + NBANDS * iliq + b);
       tauliq = fmax(0.0, clwp * (a + fliq * (c - a)));
     }
     if (ciwp > 0.0) {
       if (f.ilwcice == 1) {
         const int ia = (int)t64(kt, lwtab::ipat + b);
         tauice = fmax(0.0, ciwp * (t64(kt, lwtab::absice1 + 2 * (ia - 1)) + t64(kt, lwtab::absice1 + 1 + 2 * (ia - 1)) / refice));
-      } else if (f.ilwcice == 2) {
-        const double a = t64(kt, lwtab::absice2 + (iice - 1) + 43 * b);
-        const double c = t64(kt, lwtab::absice2 + iice + 43 * b);
-        tauice = fmax(0.0, ciwp * (a + fice * (c - a)));
-      } else if (f.ilwcice == 3) {
-        const double a = t64(kt, lwtab::absice3 + (iice - 1) + 46 * b);
-        const double c = t64(kt, lwtab::absice3 + iice + 46 * b);
+      } else if (f.ilwcice == 2 || f.ilwcice == 3) {
+        const int o = (f.ilwcice == 2 ? bandtab::absice2 : bandtab::absice3) + NBANDS * (iice - 1) + b;
+        const double a = t64(kt, o), c = t64(kt, o + NBANDS);
         tauice = fmax(0.0, ciwp * (a + fice * (c - a)));
       }
     }
     return tauice + tauliq + tauran + tausnw;
   }
 };
+
+// planck_int (lw_gas.cuh) from the band-fastest table; dw = delwave(b)
+__device__ __forceinline__ float planck_band(const double* kt, int b, double dw, int ind, double frac) {
+  const double p0 = t64(kt, bandtab::totplnk + NBANDS * (ind - 1) + b);
+  const double p1 = t64(kt, bandtab::totplnk + NBANDS * ind + b);
+  return (float)(dw * (p0 + frac * (p1 - p0)));
+}
+__device__ __forceinline__ int planck_index(double t) { return min(180, max(1, (int)(t - 159.0))); }
 
 __device__ __forceinline__ int band_of(int g) {
   return g < 10 ? 0 : g < 22 ? 1 : g < 38 ? 2 : g < 52 ? 3 : g < 68 ? 4 : g < 76 ? 5 : g < 88 ? 6 : g < 96 ? 7
@@ -264,19 +274,19 @@ __global__ void __launch_bounds__(SR_THREADS, 1) lw_sg_rt_kernel(SrArgs a) {
     const size_t ld = (size_t)B.ld;
     auto IN = [&](int fld, int row) -> double { return B.in[fld][i + ld * row]; };
 
-    // ---------------- column terms and band fields (thread <-> layer) ----------------
+    // ---------------- column terms (thread <-> layer) ----------------
+    bool cldk = false;
     {
+      auto& L = S.u.lay;
       const int t = gt;
       const bool live = t < nlay;
       const int r = top ? nlay - 1 - t : t;   // input row of layer t (and of its top level)
       const int rl = top ? nlay - 1 - t : t + 1;
-      float pkl[NBANDS];
-      bool cldk = false;
       double colw = 0.0, colh = 0.0;   // this layer's coldry and water column
-      double cf = 0.0, clwp = 0.0, relw = 0.0, ciwp = 0.0, reiw = 0.0, cda1 = 0.0, cda3 = 0.0, cda4 = 0.0;
       if (live) {
         const double delp = IN(F_DELPIN, r), q = IN(F_QLYR, r), tavel = IN(F_TLYR, r), tz = IN(F_TLVL, rl);
-        cf = IN(F_CLDCF, r);
+        const double cf = IN(F_CLDCF, r);
+        double clwp = 0.0, relw = 0.0, ciwp = 0.0, reiw = 0.0, cda1 = 0.0, cda3 = 0.0, cda4 = 0.0;
         if (f.ilwcliq > 0) {
           clwp = IN(F_LWP, r); relw = IN(F_RELIQ, r); ciwp = IN(F_IWP, r); reiw = IN(F_REICE, r);
           cda1 = IN(F_RWP, r); cda3 = IN(F_SWP, r); cda4 = IN(F_RESNOW, r);
@@ -291,23 +301,24 @@ __global__ void __launch_bounds__(SR_THREADS, 1) lw_sg_rt_kernel(SrArgs a) {
         const double coldry = tem2c * delp / (tem1c * tem0 * (1.0 + h2ovmr));
         colw = coldry;
         colh = fmax(0.0, coldry * h2ovmr);
-        const int indlay = min(180, max(1, (int)(tavel - 159.0)));
-        const double tlyrfr = tavel - (int)tavel;
-        const int indlev = min(180, max(1, (int)(tz - 159.0)));
-        const double tlvlfr = tz - (int)tz;
-#pragma unroll
-        for (int b = 0; b < NBANDS; ++b) {
-          pkl[b] = (float)planck_int(kt64, b, indlay, tlyrfr);
-          S.u.p.pkv[t + 1][b] = (float)planck_int(kt64, b, indlev, tlvlfr);
-        }
+        L.indlay[t] = planck_index(tavel);
+        L.frlay[t] = tavel - (int)tavel;
+        L.indlev[t] = planck_index(tz);
+        L.frlev[t] = tz - (int)tz;
         cldk = cf > kEps;
+        CloudLayer CL;
+        CL.set(f, clwp, relw, ciwp, reiw, cda1, cda3, cda4);
+        L.fliq[t] = CL.fliq; L.fice[t] = CL.fice; L.refice[t] = CL.refice; L.clwp[t] = CL.clwp; L.ciwp[t] = CL.ciwp;
+        L.cda1[t] = CL.cda1; L.tauran[t] = CL.tauran; L.tausnw[t] = CL.tausnw;
+        L.iliq[t] = (cf > 2.2250738585072014e-308) ? CL.iliq : 0;   // cfrac(k) > cldmin = tiny
+        L.iice[t] = CL.iice;
       }
-      if (t < NBANDS) {
-        // surface level and surface temperature (RLM:2251-2262)
-        const double tz0 = top ? IN(F_TLVL, nlay) : IN(F_TLVL, 0);
-        const double stemp = B.in[F_SFGTMP][i];
-        S.u.p.pkv[0][t] = (float)planck_int(kt64, t, min(180, max(1, (int)(tz0 - 159.0))), tz0 - (int)tz0);
-        S.pk0[t] = (float)planck_int(kt64, t, min(180, max(1, (int)(stemp - 159.0))), stemp - (int)stemp);
+      if (t == SR_GT - 1) {   // a thread without a layer
+        S.tz0 = top ? IN(F_TLVL, nlay) : IN(F_TLVL, 0);
+        S.stemp = B.in[F_SFGTMP][i];
+        S.plev0 = top ? IN(F_PLVL, nlay) : IN(F_PLVL, 0);
+        const double sfe = B.in[F_SFEMIS][i];
+        S.semis = (float)((sfe > kEps && sfe <= 1.0) ? sfe : 1.0);
       }
       // the column sums of the precipitable water (RLM:910-919) as a warp
       // tree, then over the group's warps: the reference adds layer by layer,
@@ -324,39 +335,71 @@ __global__ void __launch_bounds__(SR_THREADS, 1) lw_sg_rt_kernel(SrArgs a) {
           S.pw[gw][1] = s2;
         }
       }
-      const int lcf1 = sync.any(live && cldk);   // also: pw[] and pkv[] complete
-      if (t < NBANDS) {
-        // precipitable water (every band's thread forms the same sum) and the
-        // diffusivity angle (RLM:1041-1050)
-        double tem1 = 0.0, tem2 = 0.0;
-#pragma unroll
-        for (int w = 0; w < SR_WARPS; ++w) {
-          tem1 += S.pw[w][0];
-          tem2 += S.pw[w][1];
-        }
-        const double amdw = kConAmd / kConAmw;
-        const double tem0 = 10.0 * tem2 / (amdw * tem1 * kConG);
-        const double pwvcm = tem0 * (top ? IN(F_PLVL, nlay) : IN(F_PLVL, 0));
-        const double secd = (t == 0 || t == 3 || t == 9)
-                                ? 1.66
-                                : fmin(1.80, fmax(1.50, c_a0[t] + c_a1[t] * exp(c_a2[t] * pwvcm)));
-        S.secd[t] = (float)secd;
-        if (t == 0) {
-          const double sfe = B.in[F_SFEMIS][i];
-          S.semis = (float)((sfe > kEps && sfe <= 1.0) ? sfe : 1.0);
-          S.lcf1 = lcf1;
+    }
+    // also: pw[] and the layers' terms complete
+    const int lcf1 = sync.any(cldk);
+
+    // ---------------- band fields (thread <-> band, ten layer ranges) ----------------
+    // With a thread per layer and the bands in a loop, each band's table reads
+    // waited on L2 in turn and its stores (256 bytes apart) met in one bank.
+    // With the bands along a half warp a layer's row of a band-fastest table
+    // is one 128-byte line and its stores are consecutive, and the layers'
+    // shared terms fit where the level sums go later, which leaves the L1 60 KB
+    // instead of 28.  147,456 columns, network and transfer: 23.1 -> 20.4 ms.
+    // The tables in shared memory (21.9 ms: the L1 is what the inputs' sectors
+    // of four columns live in) and reads of clear layers too, for more of them
+    // in flight (21.4 ms), were slower.
+    {
+      auto& L = S.u.lay;
+      const int b = gt & (NBANDS - 1), h = gt >> 4;
+      constexpr int kRanges = SR_GT / NBANDS;
+      const double dw = c_delwave[b];
+      {
+        const int n = (nlay + kRanges - 1) / kRanges, k0 = h * n, k1 = min(k0 + n, nlay);
+        // pklev below the range's first layer (RLM:2251-2262)
+        float below = 0.0f;
+        if (k0 == 0) below = planck_band(kt64, b, dw, planck_index(S.tz0), S.tz0 - (int)S.tz0);
+        else if (k0 < nlay) below = planck_band(kt64, b, dw, L.indlev[k0 - 1], L.frlev[k0 - 1]);
+#pragma unroll 4
+        for (int k = k0; k < k1; ++k) {
+          const float pl = planck_band(kt64, b, dw, L.indlay[k], L.frlay[k]);
+          const float up = planck_band(kt64, b, dw, L.indlev[k], L.frlev[k]);
+          float* p = &S.bf[k][b].x;
+          *reinterpret_cast<float2*>(p) = make_float2(pl, up - pl);
+          p[2] = below - pl;
+          below = up;
         }
       }
-      sync.sync();
-      if (live) {
-        CloudLayer CL;
-        CL.set(f, cf, clwp, relw, ciwp, reiw, cda1, cda3, cda4);
-#pragma unroll 1
-        for (int b = 0; b < NBANDS; ++b) {
-          const double tc = lcf1 ? CL.band(b, f, kt64) : 0.0;
-          if (b == 6) B.out[O_CLDTAU][i + ld * r] = tc;   // band 7 cloud optical depth (RLM:1087-1097)
-          S.bf[t][b] = make_float4(pkl[b], S.u.p.pkv[t + 1][b] - pkl[b], S.u.p.pkv[t][b] - pkl[b], S.secd[b] * (float)tc);
+      // precipitable water (every thread forms the same sum) and the
+      // diffusivity angle (RLM:1041-1050)
+      double tem1 = 0.0, tem2 = 0.0;
+#pragma unroll
+      for (int w = 0; w < SR_WARPS; ++w) {
+        tem1 += S.pw[w][0];
+        tem2 += S.pw[w][1];
+      }
+      const double amdw = kConAmd / kConAmw;
+      const double tem0 = 10.0 * tem2 / (amdw * tem1 * kConG);
+      const double pwvcm = tem0 * S.plev0;
+      const float secd = (float)((b == 0 || b == 3 || b == 9)
+                                     ? 1.66
+                                     : fmin(1.80, fmax(1.50, c_a0[b] + c_a1[b] * exp(c_a2[b] * pwvcm))));
+      if (h == 0) {
+        S.secd[b] = secd;
+        S.pk0[b] = planck_band(kt64, b, dw, planck_index(S.stemp), S.stemp - (int)S.stemp);
+        if (b == 0) S.lcf1 = lcf1;
+      }
+      // cloud optical depths, the ranges interleaved: cloudy layers lie together
+#pragma unroll 2
+      for (int k = h; k < nlay; k += kRanges) {
+        double tc = 0.0;
+        if (lcf1 && L.iliq[k] > 0) {
+          const CloudLayer CL{L.clwp[k], L.ciwp[k], L.cda1[k], L.tauran[k], L.tausnw[k], L.fliq[k], L.fice[k],
+                              L.refice[k], L.iliq[k], L.iice[k]};
+          tc = CL.band(b, f, kt64);
         }
+        if (b == 6) B.out[O_CLDTAU][i + ld * (top ? nlay - 1 - k : k)] = tc;   // band 7 (RLM:1087-1097)
+        S.bf[k][b].w = secd * (float)tc;
       }
       sync.sync();   // band fields complete
     }
@@ -384,7 +427,7 @@ __global__ void __launch_bounds__(SR_THREADS, 1) lw_sg_rt_kernel(SrArgs a) {
       // this g-point's 8-layer blocks: tau at hq[j * 2 * NGPT], fractions at hq[j * 2 * NGPT + NGPT]
       const uint4* hq = reinterpret_cast<const uint4*>(a.hnd + (size_t)cc * nch * SR_HCH) + g;
       const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
-      float* P = &S.part[gw][0][0];
+      float* P = &S.u.o.part[gw][0][0];
       auto chunk_bits = [&](int j) -> uint32_t {
         const int k0 = SR_CH * j;
         const int wd = k0 >> 5;
@@ -565,10 +608,10 @@ __global__ void __launch_bounds__(SR_THREADS, 1) lw_sg_rt_kernel(SrArgs a) {
 #pragma unroll
         for (int q = 0; q < 4; ++q)
 #pragma unroll
-          for (int w = 0; w < SR_WARPS; ++w) s4[q] += (double)S.part[w][q][l];
+          for (int w = 0; w < SR_WARPS; ++w) s4[q] += (double)S.u.o.part[w][q][l];
         const double td = s4[0] * flxfac, cd = s4[1] * flxfac, tu = s4[2] * flxfac, cu = s4[3] * flxfac;
-        S.u.fn[0][l] = tu - td;
-        S.u.fn[1][l] = cu - cd;
+        S.u.o.fn[0][l] = tu - td;
+        S.u.o.fn[1][l] = cu - cd;
         if (l == nlay) {
           B.out[O_TOPFLX][2 * i + 0] = tu;
           B.out[O_TOPFLX][2 * i + 1] = cu;
@@ -590,8 +633,8 @@ __global__ void __launch_bounds__(SR_THREADS, 1) lw_sg_rt_kernel(SrArgs a) {
         const int k = gt;
         const int r = top ? nlay - 1 - k : k;
         const double rfdelp = a.cs.heatfac / IN(F_DELPIN, r);
-        B.out[O_HLWC][i + ld * r] = (S.u.fn[0][k] - S.u.fn[0][k + 1]) * rfdelp;
-        if (f.want_hlw0) B.out[O_HLW0][i + ld * r] = (S.u.fn[1][k] - S.u.fn[1][k + 1]) * rfdelp;
+        B.out[O_HLWC][i + ld * r] = (S.u.o.fn[0][k] - S.u.o.fn[0][k + 1]) * rfdelp;
+        if (f.want_hlw0) B.out[O_HLW0][i + ld * r] = (S.u.o.fn[1][k] - S.u.o.fn[1][k + 1]) * rfdelp;
       }
       sync.sync();   // fn[] is read before the next column's prologue reuses its space
     }
