@@ -31,7 +31,7 @@ namespace {
 
 constexpr int kNtbmx = 10000;
 constexpr double kS0 = 1368.22;                  // RSM:343
-constexpr size_t kScratchBudget = (size_t)12 << 30;   // 16,384 columns of 127 layers in one chunk
+constexpr size_t kScratchBudget = (size_t)12 << 30;   // 7,251 columns of 127 layers in one chunk
 
 struct SwState {
   bool ready = false;
@@ -125,13 +125,16 @@ size_t scratch_per_col(int nlay) {
 }
 
 // Columns of a chunk of a call of n: equal chunks that fit the scratch budget,
-// in whole waves of the upward kernel.
+// in whole rounds of the upward kernel.
 int chunk_columns(int n, int nlay) {
   const int most = (int)std::max<size_t>(1, kScratchBudget / scratch_per_col(nlay));
   if (n <= most) return std::max(n, 1);
-  const int wave = sw::kRtPerSm * g.num_sms, chunks = (n + most - 1) / most, even = (n + chunks - 1) / chunks;
-  const int whole = (even + wave - 1) / wave * wave;
-  return whole <= most ? whole : std::max(most / wave * wave, std::min(most, wave));
+  const long long round = (long long)sw::kUpThreads * g.num_sms;   // (column, g-point) pairs
+  const auto rounds_of = [round](long long cols) { return cols * sw::kSwNg / round; };
+  const auto cols_of = [round](long long rounds) { return (int)(rounds * round / sw::kSwNg); };
+  const int chunks = (n + most - 1) / most, even = (n + chunks - 1) / chunks;
+  const int whole = cols_of(rounds_of(even - 1) + 1);
+  return whole <= most ? std::max(whole, even) : std::max(cols_of(rounds_of(most)), std::min(most, cols_of(1)));
 }
 
 // carve one chunk's scratch out of the workspace (base null: only its size;

@@ -852,12 +852,12 @@ __device__ __forceinline__ void mix_grid(double zc1, const LayOpt& o, LayOpt& w)
 // layer and sweep in place of four.  sw_down_kernel does that and the outputs.
 //
 // Two kernels, because they want different things: the way up is a chain of
-// FP64 operations per layer (128 registers, sixteen warps per SM, 58 % of the
-// issue slots), the way down streams the stored layers (80 registers, 4.9 TB/s).
+// FP64 operations per layer (128 registers, sixteen warps per SM, 57 % of the
+// issue slots), the way down streams the stored layers (80 registers, 6.4 TB/s).
 // As phases of one kernel, with a slot of the store per resident column, the
-// same loops took 13.0 ms at 16,384 x 127; as two they take 9.1 ms (a column
-// per warp, both adding recurrences and four 10-shuffle sums per level took
-// 21.3 ms).  Down at 4, 5, 6 and 7 CTAs per SM: 9.4, 9.1, 9.1 and 9.8 ms.
+// same loops took 13.0 ms at 16,384 x 127; as two, with whole columns per CTA,
+// they took 9.1 ms (a column per warp, both adding recurrences and four
+// 10-shuffle sums per level took 21.3 ms).  Down at 4, 5, 6 and 7 CTAs per SM: 9.4, 9.1, 9.1 and 9.8 ms.
 constexpr int kRtAhead = 2;   // layers whose stored records are in flight on the way down (even)
 constexpr int kRtLay = kRtVals * kSwNg;   // store doubles of a layer
 
@@ -1304,30 +1304,34 @@ struct RtTable<true> {
 template <bool SHT>
 __host__ __device__ constexpr size_t rt_table_doubles() { return SHT ? kNtbmx + 1 : 0; }
 
-// COLS columns at a time per CTA, which walks the chunk
-template <bool GRID, int COLS, bool SHT>
-__global__ void __launch_bounds__(COLS* kSwNg, kRtPerSm / COLS)
+// CTAs of NT threads walk the chunk's (column, g-point) pairs.  Nothing is
+// shared between the g-points of a column on the way up, so the wide form
+// (NT = kUpThreads) fills the four warps that a scheduler holds at 128
+// registers; as whole columns, four of 3.5 warps, a call of 16,384 x 127 took
+// 12.37 ms instead of 11.66 (five columns at 96 registers spilled: 13.50).
+template <bool GRID, int NT, bool SHT>
+__global__ void __launch_bounds__(NT, kUpThreads / NT)
 sw_up_kernel(SwArgs a, SwScratch s, int p0, int nc, const double* __restrict__ T, const double* __restrict__ ET) {
   extern __shared__ double sm[];
   const auto tbl = RtTable<SHT>::get(ET, sm);
-  const int h = threadIdx.x / kSwNg, g = threadIdx.x - h * kSwNg;
-  for (int pl = blockIdx.x * COLS + h; pl < nc; pl += gridDim.x * COLS) {
+  for (int q = blockIdx.x * NT + threadIdx.x; q < nc * kSwNg; q += gridDim.x * NT) {
+    const int pl = q / kSwNg, g = q - pl * kSwNg;
     const int j1 = a.idxday[p0 + pl];
     if (j1 < 1 || j1 > a.npts) continue;   // reported by the optics kernel
     up_body<GRID>(a, s, pl, nc, j1, g, T, tbl);
   }
 }
 
-template <bool GRID, int COLS, bool SHT>
-__global__ void __launch_bounds__(COLS* kSwNg, kRtPerSm / COLS)
+template <bool GRID, int NT, bool SHT>
+__global__ void __launch_bounds__(NT, kUpThreads / NT)
 sw_up_blocks_kernel(const SwArgs* __restrict__ tab, const int2* __restrict__ pts, SwScratch s, int p0, int nc,
                     const double* __restrict__ T, const double* __restrict__ ET) {
   extern __shared__ double sm[];
   const auto tbl = RtTable<SHT>::get(ET, sm);
-  const int h = threadIdx.x / kSwNg, g = threadIdx.x - h * kSwNg;
-  for (int pl = blockIdx.x * COLS + h; pl < nc; pl += gridDim.x * COLS) {
-    const int2 q = pts[p0 + pl];
-    up_body<GRID>(tab[q.x], s, pl, nc, q.y, g, T, tbl);
+  for (int q = blockIdx.x * NT + threadIdx.x; q < nc * kSwNg; q += gridDim.x * NT) {
+    const int pl = q / kSwNg, g = q - pl * kSwNg;
+    const int2 at = pts[p0 + pl];
+    up_body<GRID>(tab[at.x], s, pl, nc, at.y, g, T, tbl);
   }
 }
 
@@ -1466,9 +1470,9 @@ size_t down_smem(int nlay, bool hswb) { return rt_col_doubles(nlay, hswb) * size
 constexpr size_t kUpSmem = rt_table_doubles<true>() * sizeof(double);
 
 cudaError_t rt_prepare(int max_smem) {
-  const void* up[] = {(const void*)sw_up_kernel<false, kRtPerSm, true>, (const void*)sw_up_kernel<true, kRtPerSm, true>,
-                      (const void*)sw_up_blocks_kernel<false, kRtPerSm, true>,
-                      (const void*)sw_up_blocks_kernel<true, kRtPerSm, true>};
+  const void* up[] = {(const void*)sw_up_kernel<false, kUpThreads, true>, (const void*)sw_up_kernel<true, kUpThreads, true>,
+                      (const void*)sw_up_blocks_kernel<false, kUpThreads, true>,
+                      (const void*)sw_up_blocks_kernel<true, kUpThreads, true>};
   const void* down[] = {(const void*)sw_down_kernel<false, false>,        (const void*)sw_down_kernel<true, false>,
                         (const void*)sw_down_kernel<false, true>,         (const void*)sw_down_kernel<true, true>,
                         (const void*)sw_down_blocks_kernel<false, false>, (const void*)sw_down_blocks_kernel<true, false>,
@@ -1500,13 +1504,13 @@ cudaError_t optics_blocks_launch(const SwArgs* tab, const int2* pts, const SwScr
 cudaError_t rt_blocks_launch(const SwArgs* tab, const int2* pts, bool grid, bool want_b, const SwScratch& s, int p0,
                              int nc, int nlay, const double* T, const double* ET, cudaStream_t st) {
   if (nc <= 0) return cudaSuccess;
-  // as many columns per CTA as an SM holds, exp_tbl in shared memory, once every SM gets such a CTA; below that a
-  // column per CTA, which spreads a small call over the SMs
-  if (nc >= s.num_sms * kRtPerSm) {
-    const auto up = grid ? sw_up_blocks_kernel<true, kRtPerSm, true> : sw_up_blocks_kernel<false, kRtPerSm, true>;
-    up<<<s.num_sms, kRtPerSm * kSwNg, kUpSmem, st>>>(tab, pts, s, p0, nc, T, ET);
+  // one CTA per SM, exp_tbl in shared memory, once they have work for nearly all their threads; below that a column per
+  // CTA, which spreads a small call over the SMs
+  if (nc >= s.num_sms * kUpWide) {
+    const auto up = grid ? sw_up_blocks_kernel<true, kUpThreads, true> : sw_up_blocks_kernel<false, kUpThreads, true>;
+    up<<<s.num_sms, kUpThreads, kUpSmem, st>>>(tab, pts, s, p0, nc, T, ET);
   } else {
-    const auto up = grid ? sw_up_blocks_kernel<true, 1, false> : sw_up_blocks_kernel<false, 1, false>;
+    const auto up = grid ? sw_up_blocks_kernel<true, kSwNg, false> : sw_up_blocks_kernel<false, kSwNg, false>;
     up<<<nc, kSwNg, 0, st>>>(tab, pts, s, p0, nc, T, ET);
   }
   const auto down = want_b ? (grid ? sw_down_blocks_kernel<true, true> : sw_down_blocks_kernel<false, true>)
@@ -1519,11 +1523,11 @@ cudaError_t rt_launch(const SwArgs& a, const SwScratch& s, int p0, int nc, const
                       cudaStream_t st) {
   if (nc <= 0) return cudaSuccess;
   const bool want_b = a.hswb != nullptr, grid = a.isubcsw <= 0;
-  if (nc >= s.num_sms * kRtPerSm) {   // as in rt_blocks_launch
-    const auto up = grid ? sw_up_kernel<true, kRtPerSm, true> : sw_up_kernel<false, kRtPerSm, true>;
-    up<<<s.num_sms, kRtPerSm * kSwNg, kUpSmem, st>>>(a, s, p0, nc, T, ET);
+  if (nc >= s.num_sms * kUpWide) {   // as in rt_blocks_launch
+    const auto up = grid ? sw_up_kernel<true, kUpThreads, true> : sw_up_kernel<false, kUpThreads, true>;
+    up<<<s.num_sms, kUpThreads, kUpSmem, st>>>(a, s, p0, nc, T, ET);
   } else {
-    const auto up = grid ? sw_up_kernel<true, 1, false> : sw_up_kernel<false, 1, false>;
+    const auto up = grid ? sw_up_kernel<true, kSwNg, false> : sw_up_kernel<false, kSwNg, false>;
     up<<<nc, kSwNg, 0, st>>>(a, s, p0, nc, T, ET);
   }
   const auto down = want_b ? (grid ? sw_down_kernel<true, true> : sw_down_kernel<false, true>)

@@ -52,9 +52,9 @@ __host__ __device__ inline size_t tg_offset(int nlay, size_t pl, int k, int g) {
   return pl * tg_doubles(nlay) + ((size_t)(k >> 2) * kSwNg + g) * kTgStride + (k & 3);
 }
 
-// transfer kernels: 112 threads per column; kRtPerSm columns per SM on the way
-// up, kDownPerSm on the way down
-constexpr int kRtPerSm = 4, kDownPerSm = 6;
+// transfer kernels, thread = g-point: kUpThreads per SM on the way up (in one
+// CTA from kUpWide columns per SM on), kDownPerSm columns on the way down
+constexpr int kUpThreads = 512, kUpWide = 4, kDownPerSm = 6;
 constexpr int kRtGroups = kSwNg / 16;       // 16-lane groups of a column
 constexpr int kRtVals = 14;                 // stored values per layer and g-point
 constexpr int kRtBandSlots = 14 + kRtGroups - 1;   // (band, group) pairs: slot band + group

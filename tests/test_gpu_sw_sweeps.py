@@ -15,6 +15,7 @@ pytestmark = pytest.mark.gpu
     (1, 1, {}, True), (2, 2, {}, False), (3, 3, dict(iovr=3), True), (5, 4, dict(isubcsw=0), True),
     (7, 5, {}, False), (9, 31, dict(top_at_1=1), False), (11, 33, dict(isubcsw=0, top_at_1=1), False),
     (6, 65, {}, True), (591, 33, {}, False), (592, 32, dict(isubcsw=0), False), (595, 34, dict(iovr=3), True),
+    (681, 5, {}, True),
 ])
 def test_sweeps_match_oracle(npts, nlay, flags, hswb):
     torch = pytest.importorskip("torch")
