@@ -63,8 +63,10 @@ cudaError_t mcica_sw_launch(int ncols, int nlay, int iovr, const McicaStage& sta
 cudaError_t mcica_sw_two_set_prepare(int max_smem);
 cudaError_t mcica_sw_two_set_launch(int ncols, int nlay, int iovr, const McicaStage& stage, uint32_t* bits,
                                     int num_sms, cudaStream_t st);
-// raw state words of one twister stream (lw_mcica.cu): raw[j] is what draw j tempers
-cudaError_t seed_stream_launch(int32_t seed, long long m, uint32_t* raw, cudaStream_t st);
+// raw state words of one twister stream (lw_mcica.cu): raw[j] is what draw j
+// tempers; state: seed_state_words() of workspace
+size_t seed_state_words();
+cudaError_t seed_stream_launch(int32_t seed, long long m, uint32_t* raw, uint32_t* state, cudaStream_t st);
 // icsdsw/icsdlw of n columns from the raw words of a face's stream
 // (lw_mcica.cu); *bad receives the smallest column whose grid index is outside
 // the face

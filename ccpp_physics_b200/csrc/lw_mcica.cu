@@ -635,57 +635,109 @@ lw_mcica_kernel(const Block* __restrict__ blocks, int nblocks, const Block b0, i
 
 // The raw (untempered) words of one twister stream after
 // random_setseed_t(seed) (MT:285-299): out[j] is the state word that draw j
-// of random_number_t (MT:330-372) tempers.  One CTA walks the stream; the
-// 624-word state is double-buffered in shared memory, so a twist is its
-// three dependency phases (words 0..226 from the old state, 227..453 and
-// 454..622 from words 227 back in the new one, word 623 from new words 0 and
-// 396) with one barrier each and no read-before-write hazard.  Only integer
-// work sits on this serial path; tempering and the conversion to a random
-// index run later, in parallel, for the words that are used
-// (seed_index_of).
-constexpr int kSeedThreads = 256;
+// of random_number_t (MT:330-372) tempers.  One CTA walks a stream, a ring of
+// sequence words in shared memory, 227 words per barrier (word i + 624 needs
+// words i, i + 1 and i + 397); tempering and the conversion to a random index
+// run later, in parallel, for the words that are used (seed_index_of).
+//
+// The walk is a serial chain, so a longer stream is cut into segments of
+// kSeedJump words and each segment's state is jumped to: the state N words on
+// is the GF(2) sum of the states i = 0 .. 19936 whose bit is set in
+// x^N mod p(x), and those states' words are the stream's first kSeedJump ones
+// (c_seed_jump, and how it is made: data/make_mt_jump.py).  Rounds of
+// kSeedSegs segments: the first segment by one CTA, the sums by many, the other
+// segments a CTA each.  The seeds of a 384 x 384 face (294,912 words) take 166 us
+// with one walk and 86 us so; at 82,418 words, past the line, 83 and 80 us, and
+// at 61,952 words 72 and 78 us.
+constexpr int kSeedThreads = 256, kSeedPhase = 227, kSeedRing = 2048;
+constexpr int kSeedJump = 33 * 624, kSeedSegs = 16;
+constexpr int kSeedPolyBits = 19937, kSeedChunk = 512;   // polynomial bits per CTA of the sums
+constexpr int kSeedSumThreads = 160;                     // four words of the state each
+constexpr int kSeedWalk = 4 * kSeedJump;                 // words up to which one CTA walks
+static_assert(kSeedJump + 624 >= kSeedPolyBits + 624 && 4 * kSeedSumThreads >= 624, "words of the sums");
 
-__global__ void __launch_bounds__(kSeedThreads) lw_seed_stream_kernel(uint32_t seed, long long m,
-                                                                      uint32_t* __restrict__ out) {
-  __shared__ uint32_t s[2][624];
+__device__ const uint32_t c_seed_jump[kSeedSegs - 1][624] = {
+#include "../data/mt_jump.inc"
+};
+
+// n words from the state in ring[0..623]; every thread of the CTA calls it,
+// after a barrier.  The state behind them is then ring[(n + q) % kSeedRing].
+__device__ void seed_walk(uint32_t* ring, int n, uint32_t* __restrict__ out) {
   const int t = threadIdx.x;
-  if (t == 0) {   // MT:290-296, signed wrap = unsigned multiply
+  for (int b = 0; b < n; b += kSeedPhase) {
+    if (t < kSeedPhase) {
+      const uint32_t i = b + t;
+      const uint32_t v = mt_word(ring[i % kSeedRing], ring[(i + 1) % kSeedRing], ring[(i + 397) % kSeedRing]);
+      ring[(i + 624) % kSeedRing] = v;
+      if (i < (uint32_t)n) out[i] = v;
+    }
+    __syncthreads();
+  }
+}
+
+// The first segment of a round (or the whole stream): from the seed, or from
+// state[kSeedSegs] where the round before ended.  Leaves its first state in
+// state[0] and clears the others for the sums (state null: neither).
+__global__ void __launch_bounds__(kSeedThreads)
+lw_seed_stream_kernel(uint32_t seed, bool first, int n, uint32_t* __restrict__ state, uint32_t* __restrict__ out) {
+  __shared__ uint32_t ring[kSeedRing];
+  const int t = threadIdx.x;
+  if (!first) {
+    for (int q = t; q < 624; q += kSeedThreads) ring[q] = state[kSeedSegs * 624 + q];
+  } else if (t < 32) {   // MT:290-296, signed wrap = unsigned multiply
     uint32_t v = seed;
-    s[0][0] = v;
-    for (int i = 1; i < 624; ++i) { v *= 69069u; s[0][i] = v; }
+    for (int q = 0; q < t; ++q) v *= 69069u;
+    for (int q = t; q < 624; q += 32) {
+      ring[q] = v;
+      v *= kPow69069_32;
+    }
   }
   __syncthreads();
-  int cur = 0;
-  for (long long base = 0; base < m; base += 624) {
-    const uint32_t* o = s[cur];
-    uint32_t* w = s[cur ^ 1];
-    const long long left = m - base;
-    if (t < 227) {   // words 0..226
-      const uint32_t v = mt_word(o[t], o[t + 1], o[t + 397]);
-      w[t] = v;
-      if (t < left) out[base + t] = v;
-    }
-    __syncthreads();
-    if (t < 227) {   // words 227..453
-      const int kk = 227 + t;
-      const uint32_t v = mt_word(o[kk], o[kk + 1], w[kk - 227]);
-      w[kk] = v;
-      if (kk < left) out[base + kk] = v;
-    }
-    __syncthreads();
-    if (t < 169) {   // words 454..622
-      const int kk = 454 + t;
-      const uint32_t v = mt_word(o[kk], o[kk + 1], w[kk - 227]);
-      w[kk] = v;
-      if (kk < left) out[base + kk] = v;
-    } else if (t == 169) {   // word 623
-      const uint32_t v = mt_word(o[623], w[0], w[396]);
-      w[623] = v;
-      if (623 < left) out[base + 623] = v;
-    }
-    __syncthreads();
-    cur ^= 1;
+  if (state) {
+    for (int q = t; q < 624; q += kSeedThreads) state[q] = ring[q];
+    for (int q = 624 + t; q < kSeedSegs * 624; q += kSeedThreads) state[q] = 0u;
   }
+  seed_walk(ring, n, out);
+}
+
+// state[s] ^= the states of this CTA's kSeedChunk polynomial bits, s = blockIdx.y + 1
+__global__ void __launch_bounds__(kSeedSumThreads)
+lw_seed_jump_kernel(uint32_t* __restrict__ state, const uint32_t* __restrict__ out) {
+  __shared__ uint32_t x[kSeedChunk + 4 * kSeedSumThreads];
+  const int t = threadIdx.x, i0 = blockIdx.x * kSeedChunk;
+  for (int q = t; q < kSeedChunk + 624; q += kSeedSumThreads) {   // sequence words i0 + q
+    const int i = i0 + q;
+    x[q] = i < 624 ? state[i] : out[i - 624];
+  }
+  __syncthreads();
+  const uint32_t* g = c_seed_jump[blockIdx.y] + i0 / 32;
+  uint32_t acc[4] = {0u, 0u, 0u, 0u};
+  for (int w = 0; w < kSeedChunk / 32 && i0 / 32 + w < 624; ++w) {
+    uint32_t m = __ldg(g + w);
+    while (m) {
+      const int b = 32 * w + __ffs(m) - 1;
+      m &= m - 1;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[q] ^= x[b + t + kSeedSumThreads * q];
+    }
+  }
+  uint32_t* y = state + (blockIdx.y + 1) * 624;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (t + kSeedSumThreads * q < 624) atomicXor(y + t + kSeedSumThreads * q, acc[q]);
+}
+
+// segments 1 .. of a round of m words; the state behind the last of a full
+// round goes to state[kSeedSegs]
+__global__ void __launch_bounds__(kSeedThreads)
+lw_seed_segment_kernel(int m, uint32_t* __restrict__ state, uint32_t* __restrict__ out) {
+  __shared__ uint32_t ring[kSeedRing];
+  const int t = threadIdx.x, s = blockIdx.x + 1, n = min(kSeedJump, m - s * kSeedJump);
+  for (int q = t; q < 624; q += kSeedThreads) ring[q] = state[s * 624 + q];
+  __syncthreads();
+  seed_walk(ring, n, out + (size_t)s * kSeedJump);
+  if (s == kSeedSegs - 1)
+    for (int q = t; q < 624; q += kSeedThreads) state[kSeedSegs * 624 + q] = ring[(uint32_t)(n + q) % kSeedRing];
 }
 
 // random_index_t (MT:489-503) of one raw word: max(ceiling(h * imax), 1)
@@ -716,10 +768,26 @@ __global__ void lw_seed_gather_kernel(const uint32_t* __restrict__ raw, const in
 
 // host side ------------------------------------------------------------------
 
-cudaError_t seed_stream_launch(int32_t seed, long long m, uint32_t* raw, cudaStream_t st) {
+size_t seed_state_words() { return (size_t)(kSeedSegs + 1) * 624; }
+
+cudaError_t seed_stream_launch(int32_t seed, long long m, uint32_t* raw, uint32_t* state, cudaStream_t st) {
   if (m <= 0) return cudaSuccess;
+  if (m > INT_MAX) return cudaErrorInvalidValue;
   const uint32_t s = (uint32_t)(seed == 0 ? 4357 : seed);   // MT:291
-  lw_seed_stream_kernel<<<1, kSeedThreads, 0, st>>>(s, m, raw);
+  if (m <= kSeedWalk) {
+    lw_seed_stream_kernel<<<1, kSeedThreads, 0, st>>>(s, true, (int)m, nullptr, raw);
+    return cudaGetLastError();
+  }
+  constexpr int round = kSeedSegs * kSeedJump;
+  for (long long done = 0; done < m; done += round) {
+    const int n = (int)std::min<long long>(round, m - done), segs = (n + kSeedJump - 1) / kSeedJump;
+    uint32_t* out = raw + done;
+    lw_seed_stream_kernel<<<1, kSeedThreads, 0, st>>>(s, done == 0, std::min(n, kSeedJump), state, out);
+    if (segs > 1) {
+      lw_seed_jump_kernel<<<dim3((kSeedPolyBits + kSeedChunk - 1) / kSeedChunk, segs - 1), kSeedSumThreads, 0, st>>>(state, out);
+      lw_seed_segment_kernel<<<segs - 1, kSeedThreads, 0, st>>>(n, state, out);
+    }
+  }
   return cudaGetLastError();
 }
 

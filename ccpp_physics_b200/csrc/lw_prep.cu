@@ -509,13 +509,13 @@ extern "C" int rrtmg_lw_gpu_seeds(const rrtmg_lw_seed_args* a, const rrtmg_lw_ex
   S.add(b.icsdlw, n, true);
   char* extra = nullptr;
   const size_t raw_bytes = ((size_t)(2 * face) * sizeof(uint32_t) + 255) / 256 * 256;
-  CK(S.upload(raw_bytes + 256, &extra), "staging");
+  CK(S.upload(raw_bytes + 256 + lw::seed_state_words() * sizeof(uint32_t), &extra), "staging");
   uint32_t* raw = (uint32_t*)extra;
   int* bad = (int*)(extra + raw_bytes);
   const int none = INT_MAX;
   int first_bad = INT_MAX;
   CK(cudaMemcpyAsync(bad, &none, sizeof(int), cudaMemcpyHostToDevice, st), "cudaMemcpyAsync");
-  CK(lw::seed_stream_launch(ipseed, 2 * face, raw, st), "seed stream launch");
+  CK(lw::seed_stream_launch(ipseed, 2 * face, raw, (uint32_t*)(extra + raw_bytes + 256), st), "seed stream launch");
   CK(lw::seed_gather_launch(raw, b.imap, b.jmap, n, a->isc, a->jsc, a->cnx, face, a->ipsdlim, b.icsdsw, b.icsdlw,
                             bad, st), "seed gather launch");
   CK(cudaMemcpyAsync(&first_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
