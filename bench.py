@@ -534,7 +534,7 @@ def sw_leg(args, torch, timed, sh):
         ach_tf = tr["sw_fp64_flop_per_column_rt"] * n / t_rt / 1e12
         ach_gbs = tr["sw_dram_bytes_per_column_rt"] * n / t_rt / 1e9
         hbm = _peaks()[0]
-        roof = {"kernel": "sw_rt_kernel<false>", "fp64_tflops": ach_tf,
+        roof = {"kernel": "sw_up_kernel + sw_down_kernel", "fp64_tflops": ach_tf,
                 "fp64_peak_tflops": p64.value if rc_peak == 0 else None,
                 "fp64_frac": ach_tf / p64.value if rc_peak == 0 and p64.value > 0 else None,
                 "dram_gbs": ach_gbs, "hbm_peak_gbs": hbm, "hbm_frac": ach_gbs / hbm if hbm else None,
@@ -946,7 +946,7 @@ def main():
         "e2e": e2e,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic, "peak_source": peak_kind,
-                     "kernel": "lw_gas_kernel<double,4> + lw_rt_kernel<double,4> (per chunk)"},
+                     "kernel": "lw_gas_kernel<double> + lw_rt64_kernel (per chunk)"},
         "fp_pipe": fp_pipe,
         "cpu_baseline": cpu,
         "paths": paths,

@@ -150,15 +150,8 @@ __device__ __forceinline__ int find_block(const Block* blocks, int nblocks, int 
 template <typename T>
 __device__ __forceinline__ T ldg(const T* p) { return __ldg(p); }
 
-// Barrier of a group of threads: the whole CTA (gas_column in lw_gas_kernel
-// and the fallback kernel of the learned-gas-optics path), or a named
-// barrier over `n` threads of a CTA that holds several groups (that path's
-// network and transfer kernels).
-struct CtaSync {
-  __device__ __forceinline__ void sync() const { __syncthreads(); }
-  __device__ __forceinline__ int count(bool p) const { return __syncthreads_count(p); }
-  __device__ __forceinline__ int any(bool p) const { return __syncthreads_or(p); }
-};
+// Barrier of a group of threads of a CTA that holds several groups (the
+// network and transfer kernels of the learned-gas-optics path).
 struct GroupSync {
   int id, n;   // named barrier id (1..15) and thread count (a multiple of 32)
   __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }

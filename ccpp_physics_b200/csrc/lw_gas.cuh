@@ -9,10 +9,11 @@
 // walked in order, so every table gather of a band happens while the band's
 // coefficients are hot in L1/L2.
 //
-// Output (device scratch, read by kernel B in lw_rt.cuh), per column c of the
-// chunk and layer k (0-based, surface first), NLP = 32*V >= nlay+1:
+// Output (device scratch, read by kernel B in lw_rt.cuh or lw_rt64.cuh), per
+// column c of the chunk and layer k (0-based, surface first), NLP = 32*V >= nlay+1:
 //   tau  [c][g][NLP]      gas + aerosol optical depth  (taumol tautot)
 //   frac [c][g][NLP]      Planck fraction              (taumol fracs)
+//                         (for lw_rt64.cuh [c][k / 4][g][4])
 //   band [c][0][b][NLP]   pklay(b, k+1)
 //        [c][1][b][NLP]   pklev(b, k)      k = 0..nlay
 //        [c][2][b][NLP]   taucld(b, k+1)

@@ -1,4 +1,6 @@
-// lw_rt.cuh -- kernel B of the RRTMG-LW path: McICA radiative transfer.
+// lw_rt.cuh -- kernel B of the RRTMG-LW path: McICA radiative transfer in FP32,
+// and in FP64 where the spectral heating rates (hlwb) are asked for; FP64
+// without them runs lw_rt64.cuh.
 //
 // Replaces rtrnmc (physics/Radiation/RRTMG/radlw_main.F90, RLM:3420-3785)
 // and the output mapping of rrtmg_lw_run (RLM:1228-1304).  One warp owns

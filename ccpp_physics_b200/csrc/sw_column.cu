@@ -1,23 +1,24 @@
 // sw_column.cu -- the RRTMG-SW column kernels for B200 (FP64).
 //
 // rrtmg_sw_run (physics/Radiation/RRTMG/radsw_main.F90:493-1379, RSM below)
-// for the McICA configurations runs as three launches over a chunk of
-// daytime columns:
+// runs as four launches over a chunk of daytime columns (three with grid-mean
+// clouds):
 //   sw_optics_kernel  one warp per 32 layers of a column, a lane per layer: the driver's
 //                     layer prologue (RSM:910-1094), setcoef (RSM:2242-2389),
 //                     taumol16..29 (RSM:4094-5573; every lane runs the same
 //                     band's code, so the band branches never diverge),
 //                     the solar source sfluxzen, the clear/cloudy column test
 //                     (RSM:1101-1125) and cldprop (RSM:1566-1938);
-//   lw_mcica_kernel<112>  the sub-column generator (lw_mcica.cu);
-//   sw_rt_kernel      two columns per CTA, one g-point per thread: spcvrtm
-//                     (RSM:3228-3942) with vrtqdr (RSM:3959-4051) and the
-//                     flux / heating-rate outputs (RSM:1225-1373).
+//   lw_mcica_kernel<112> or sw_mcica_two_set_kernel  the sub-column generator
+//                     (lw_mcica.cu);
+//   sw_up_kernel, sw_down_kernel  one g-point per thread: spcvrtm
+//                     (RSM:3228-3942) or spcvrtc with vrtqdr (RSM:3959-4051)
+//                     and the flux / heating-rate outputs (RSM:1225-1373).
 //
 // Built with -fmad=false: every statement that feeds a table index or a
 // difference of nearly equal numbers keeps the reference's evaluation order
 // and rounding; the recurrences behind them use fma() where that is exact
-// enough (see sw_rt_kernel).
+// enough (see sw_up_kernel).
 #include <cstdint>
 #include <cstdio>
 #include <vector>
