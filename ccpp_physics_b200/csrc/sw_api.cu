@@ -274,24 +274,55 @@ cudaError_t zero_outputs(const sw::SwArgs& d, const Sizes& z, int nlay, cudaStre
   return e;
 }
 
+// Stage times of a call, [McICA, optics, transfer], the order of the longwave
+// timings, summed over its chunks: each chunk's are read, and waited for, before
+// the next one's events are recorded.  Without kernel_ms it does nothing.
+class StageTimes {
+ public:
+  explicit StageTimes(float* kernel_ms) : ms_(kernel_ms) {
+    if (ms_) ms_[0] = ms_[1] = ms_[2] = 0.0f;
+  }
+  ~StageTimes() {
+    for (auto& e : ev_)
+      if (e) cudaEventDestroy(e);
+  }
+  StageTimes(const StageTimes&) = delete;
+  StageTimes& operator=(const StageTimes&) = delete;
+  // i = 0: in front of the optics, 1: behind it, 2: behind McICA, 3: behind the transfer
+  cudaError_t mark(int i, cudaStream_t st) {
+    if (!ms_) return cudaSuccess;
+    cudaError_t e = ev_[i] ? cudaSuccess : cudaEventCreate(&ev_[i]);
+    if (e == cudaSuccess) e = cudaEventRecord(ev_[i], st);
+    if (e != cudaSuccess || i < 3) return e;
+    if ((e = cudaEventSynchronize(ev_[3])) != cudaSuccess) return e;
+    const int from[3] = {1, 0, 2};
+    for (int q = 0; q < 3; ++q) {
+      float t = 0.0f;
+      if ((e = cudaEventElapsedTime(&t, ev_[from[q]], ev_[from[q] + 1])) != cudaSuccess) return e;
+      ms_[q] += t;
+    }
+    return cudaSuccess;
+  }
+
+ private:
+  float* ms_;
+  cudaEvent_t ev_[4] = {};
+};
+
 // all kernels of one call on device arguments
 int run_device(SwWorkspace* w, const sw::SwArgs& d, int nday, cudaStream_t st, float* kernel_ms, char* errmsg,
                int32_t errmsg_len, const Sizes& z) {
   CK(zero_outputs(d, z, d.nlay, st), "zeroing the outputs");
   const int chunk = chunk_columns(nday, d.nlay);
   CK(grow(&w->scratch, &w->scratch_bytes, carve_bytes(chunk, d.nlay)), "scratch allocation");
-  cudaEvent_t ev[4] = {};
-  if (kernel_ms) {
-    for (auto& e : ev) CK(cudaEventCreate(&e), "cudaEventCreate");
-  }
+  StageTimes times(kernel_ms);
   for (int p0 = 0; p0 < nday; p0 += chunk) {
     const int nc = std::min(chunk, nday - p0);
     sw::SwScratch s = carve(w->scratch, nc, d.nlay);
     s.bad = w->bad;
-    const bool first = kernel_ms && p0 == 0;
-    if (first) CK(cudaEventRecord(ev[0], st), "cudaEventRecord");
+    CK(times.mark(0, st), "stage timing");
     CK(sw::optics_launch(d, s, p0, nc, g.tab, g.ktab, st), "optics kernel launch");
-    if (first) CK(cudaEventRecord(ev[1], st), "cudaEventRecord");
+    CK(times.mark(1, st), "stage timing");
     lw::McicaStage ms;
     ms.cldf = s.cldf;
     ms.seed = s.seed;
@@ -304,17 +335,9 @@ int run_device(SwWorkspace* w, const sw::SwArgs& d, int nday, cudaStream_t st, f
     } else {
       CK(lw::mcica_sw_two_set_launch(nc, d.nlay, d.iovr, ms, s.bits, g.num_sms, st), "McICA kernel launch");
     }
-    if (first) CK(cudaEventRecord(ev[2], st), "cudaEventRecord");
+    CK(times.mark(2, st), "stage timing");
     CK(sw::rt_launch(d, s, p0, nc, g.tab, g.etab, st), "transfer kernel launch");
-    if (first) CK(cudaEventRecord(ev[3], st), "cudaEventRecord");
-  }
-  if (kernel_ms) {
-    CK(cudaEventSynchronize(ev[3]), "kernel execution");
-    // [McICA, optics, transfer], the order of the longwave timings
-    cudaEventElapsedTime(&kernel_ms[0], ev[1], ev[2]);
-    cudaEventElapsedTime(&kernel_ms[1], ev[0], ev[1]);
-    cudaEventElapsedTime(&kernel_ms[2], ev[2], ev[3]);
-    for (auto& e : ev) cudaEventDestroy(e);
+    CK(times.mark(3, st), "stage timing");
   }
   return 0;
 }
@@ -720,18 +743,14 @@ extern "C" int rrtmg_sw_gpu_run_blocks(const rrtmg_sw_run_args* blocks, int32_t 
   const sw::SwArgs& f = w->h_tab[0];
   const int chunk = chunk_columns(ndays, nlay);
   CK(grow(&w->scratch, &w->scratch_bytes, carve_bytes(chunk, nlay)), "scratch allocation");
-  cudaEvent_t ev[4] = {};
-  float* kms = x->kernel_ms;
-  if (kms)
-    for (auto& e : ev) CK(cudaEventCreate(&e), "cudaEventCreate");
+  StageTimes times(x->kernel_ms);
   for (int p0 = 0; p0 < ndays; p0 += chunk) {
     const int nc = std::min(chunk, ndays - p0);
     sw::SwScratch sc = carve(w->scratch, nc, nlay);
     sc.bad = w->bad;
-    const bool first_chunk = kms && p0 == 0;
-    if (first_chunk) CK(cudaEventRecord(ev[0], st), "cudaEventRecord");
+    CK(times.mark(0, st), "stage timing");
     CK(sw::optics_blocks_launch(d_tab, d_pts, sc, p0, nc, nlay, g.tab, g.ktab, st), "optics kernel launch");
-    if (first_chunk) CK(cudaEventRecord(ev[1], st), "cudaEventRecord");
+    CK(times.mark(1, st), "stage timing");
     lw::McicaStage ms;
     ms.cldf = sc.cldf;
     ms.seed = sc.seed;
@@ -741,19 +760,12 @@ extern "C" int rrtmg_sw_gpu_run_blocks(const rrtmg_sw_run_args* blocks, int32_t 
       CK(lw::mcica_sw_launch(nc, nlay, f.iovr, ms, sc.bits, g.num_sms, st), "McICA kernel launch");
     else if (f.isubcsw > 0)
       CK(lw::mcica_sw_two_set_launch(nc, nlay, f.iovr, ms, sc.bits, g.num_sms, st), "McICA kernel launch");
-    if (first_chunk) CK(cudaEventRecord(ev[2], st), "cudaEventRecord");
+    CK(times.mark(2, st), "stage timing");
     CK(sw::rt_blocks_launch(d_tab, d_pts, f.isubcsw <= 0, f.hswb != nullptr, sc, p0, nc, nlay, g.tab, g.etab, st),
        "transfer kernel launch");
-    if (first_chunk) CK(cudaEventRecord(ev[3], st), "cudaEventRecord");
+    CK(times.mark(3, st), "stage timing");
   }
-  if (kms) {
-    CK(cudaEventSynchronize(ev[3]), "kernel execution");
-    cudaEventElapsedTime(&kms[0], ev[1], ev[2]);
-    cudaEventElapsedTime(&kms[1], ev[0], ev[1]);
-    cudaEventElapsedTime(&kms[2], ev[2], ev[3]);
-    for (auto& e : ev) cudaEventDestroy(e);
-  }
-  if (x->sync || kms) return check_bad(w, st, errmsg, errmsg_len);
+  if (x->sync || x->kernel_ms) return check_bad(w, st, errmsg, errmsg_len);
   return 0;
 }
 
