@@ -743,9 +743,11 @@ extern "C" int rrtmg_lw_gpu_run_ex(const rrtmg_lw_run_args* a, const rrtmg_lw_ex
   if (v == 2) {
     // the reference zeroes cldtau before the optional-argument check (RLM:736)
     if (a->cldtau) {
-      FieldSizes fs = sizes_of(a);
-      if (x->memory == RRTMG_LW_DEVICE) cudaMemset(a->cldtau, 0, fs.n2 * sizeof(double));
-      else std::memset(a->cldtau, 0, fs.n2 * sizeof(double));
+      const size_t ld = a->ldim > 0 ? (size_t)a->ldim : (size_t)a->npts, np = (size_t)a->npts;
+      if (x->memory == RRTMG_LW_DEVICE)
+        cudaMemset2D(a->cldtau, ld * sizeof(double), 0, np * sizeof(double), a->nlay);
+      else
+        for (int k = 0; k < a->nlay; ++k) std::memset(a->cldtau + ld * k, 0, np * sizeof(double));
     }
     return 1;
   }
@@ -831,12 +833,13 @@ extern "C" int rrtmg_lw_gpu_run_ex(const rrtmg_lw_run_args* a, const rrtmg_lw_ex
   int r = launch(w, st, &B, 1, a->npts, f, kp, default_shape(kp, pick_v(f.nlay)), x->kernel_ms, errmsg,
                  errmsg_len);
   if (r) return r;
+  // outputs: the first npts records of every row of ldim; the columns beyond npts are the caller's
+  const size_t ld = a->ldim > 0 ? (size_t)a->ldim : (size_t)a->npts, np = (size_t)a->npts, L = (size_t)a->nlay;
+  const size_t width[] = {1, 2, 4, 1, 1, 1, 4}, rows[] = {L, 0, 0, L, L, L * NBANDS, L + 1};   // 0: per-column records
   if (staged) {
     CK(cudaMemcpyAsync(w->stage.p + out0, w->dbuf + out0, off - out0, cudaMemcpyDeviceToHost, st),
        "cudaMemcpyAsync(D2H)");
     CK(cudaStreamSynchronize(st), "kernel execution");
-    const size_t ld = a->ldim > 0 ? (size_t)a->ldim : (size_t)a->npts, np = (size_t)a->npts, L = (size_t)a->nlay;
-    const size_t width[] = {1, 2, 4, 1, 1, 1, 4}, rows[] = {L, 0, 0, L, L, L * NBANDS, L + 1};   // 0: per-column records
     for (int k = 0; k < nout; ++k) {
       if (!host_out[k]) continue;
       const char* src = w->stage.p + (reinterpret_cast<char*>(*outs[k]) - w->dbuf);
@@ -847,8 +850,13 @@ extern "C" int rrtmg_lw_gpu_run_ex(const rrtmg_lw_run_args* a, const rrtmg_lw_ex
   }
   for (int k = 0; k < nout; ++k) {
     if (!host_out[k]) continue;
-    CK(cudaMemcpyAsync(host_out[k], *outs[k], out_n[k] * sizeof(double), cudaMemcpyDeviceToHost, st),
-       "cudaMemcpyAsync(D2H)");
+    const size_t rec = width[k] * sizeof(double);
+    if (rows[k] && ld != np)
+      CK(cudaMemcpy2DAsync(host_out[k], ld * rec, *outs[k], ld * rec, np * rec, rows[k], cudaMemcpyDeviceToHost, st),
+         "cudaMemcpy2DAsync(D2H)");
+    else
+      CK(cudaMemcpyAsync(host_out[k], *outs[k], np * rec * std::max<size_t>(rows[k], 1), cudaMemcpyDeviceToHost, st),
+         "cudaMemcpyAsync(D2H)");
   }
   CK(cudaStreamSynchronize(st), "kernel execution");
   return 0;
