@@ -801,21 +801,24 @@ extern "C" int rrtmg_lw_gpu_run_ex(const rrtmg_lw_run_args* a, const rrtmg_lw_ex
   const bool staged = w->stage.ensure(total);
   HostGather up{w->stage.p, w->dbuf, st};
   size_t off = 0;
-  auto put = [&](const void* src, size_t bytes) -> cudaError_t {   // the next field of the device buffer
-    const size_t at = off;
-    off += al(bytes);
+  // the next field of the device buffer: n elements, without the last row's columns beyond npts, which for a
+  // slice of (ldim, ..) arrays lie behind the array
+  const size_t beyond = a->ldim > 0 ? (size_t)a->ldim - (size_t)a->npts : 0;
+  auto put = [&](const void* src, size_t n, size_t elem) -> cudaError_t {
+    const size_t at = off, bytes = (n > fs.n1 ? n - beyond : n) * elem;
+    off += al(n * elem);
     if (staged) return up.put(at, src, bytes, off);
     return cudaMemcpyAsync(w->dbuf + at, src, bytes, cudaMemcpyHostToDevice, st);
   };
   for (int k = 0; k < nin; ++k) {
     if (!*ins[k]) continue;
     const double* dp = reinterpret_cast<const double*>(w->dbuf + off);
-    CK(put(*ins[k], in_n[k] * sizeof(double)), "cudaMemcpyAsync(H2D)");
+    CK(put(*ins[k], in_n[k], sizeof(double)), "cudaMemcpyAsync(H2D)");
     *ins[k] = dp;
   }
   if (d.icseed) {
     const int32_t* dp = reinterpret_cast<const int32_t*>(w->dbuf + off);
-    CK(put(d.icseed, fs.n1 * sizeof(int32_t)), "cudaMemcpyAsync(H2D)");
+    CK(put(d.icseed, fs.n1, sizeof(int32_t)), "cudaMemcpyAsync(H2D)");
     d.icseed = dp;
   }
   if (staged) CK(up.send(off), "cudaMemcpyAsync(H2D)");

@@ -593,22 +593,24 @@ extern "C" int rrtmg_sw_gpu_run_ex(const rrtmg_sw_run_args* a, const rrtmg_sw_ex
   HostGather up{w->pin.p, w->stage, st};
   size_t off = 0;
   auto place = [&](size_t bytes) { char* p = w->stage + off; off += align256(bytes); return p; };
-  auto put = [&](const void* src, size_t bytes, cudaError_t* e) {   // the next field of the device buffer
-    const size_t at = off;
-    char* p = place(bytes);
+  // the next field of the device buffer: n elements, without the last row's columns beyond npts, which for a
+  // slice of (ldim, ..) arrays lie behind the array
+  auto put = [&](const void* src, size_t n, size_t elem, cudaError_t* e) {
+    const size_t at = off, bytes = (n > z.np ? n - (ldz - z.np) : n) * elem;
+    char* p = place(n * elem);
     *e = staged ? up.put(at, src, bytes, off) : cudaMemcpyAsync(p, src, bytes, cudaMemcpyHostToDevice, st);
     return p;
   };
   cudaError_t ce = cudaSuccess;
   if (a->icseed) {
-    da.icseed = (int32_t*)put(a->icseed, z.np * 4, &ce);
+    da.icseed = (int32_t*)put(a->icseed, z.np, 4, &ce);
     CK(ce, "cudaMemcpyAsync");
   }
-  da.idxday = (int32_t*)put(a->idxday, z.nd * 4, &ce);
+  da.idxday = (int32_t*)put(a->idxday, z.nd, 4, &ce);
   CK(ce, "cudaMemcpyAsync");
   for (auto& p : ins) {
     if (!*p.first) continue;
-    *p.first = (double*)put(*p.first, p.second * 8, &ce);
+    *p.first = (double*)put(*p.first, p.second, 8, &ce);
     CK(ce, "cudaMemcpyAsync");
   }
   if (staged) CK(up.send(off), "cudaMemcpyAsync");
