@@ -424,6 +424,7 @@ int run_host_pipelined(SwWorkspace* w, const rrtmg_sw_run_args* a, cudaStream_t 
   // the kernels' scratch for a whole chunk, allocated before any launch
   CK(grow(&w->scratch, &w->scratch_bytes, carve_bytes(chunk_columns(kSwHostChunk, nlay), nlay)), "scratch allocation");
   CK(cudaMemsetAsync(w->bad, 0, sizeof(int), st), "cudaMemsetAsync");
+  if (kernel_ms) kernel_ms[0] = kernel_ms[1] = kernel_ms[2] = 0.0f;   // summed over the chunks
   for (int j = 0; j < nch; ++j) {
     const int b = j & 1, c0 = j * kSwHostChunk, n = std::min(kSwHostChunk, npts - c0);
     char* base = w->pbuf + (size_t)b * per;
@@ -455,8 +456,10 @@ int run_host_pipelined(SwWorkspace* w, const rrtmg_sw_run_args* a, cudaStream_t 
     sw::SwArgs da = device_args(&dc);
     da.seed0 = c0;
     const Sizes z = sizes_of(&dc);
-    int r = run_device(w, da, dc.nday, st, (j == 0) ? kernel_ms : nullptr, errmsg, errmsg_len, z);
+    float ms[3];
+    int r = run_device(w, da, dc.nday, st, kernel_ms ? ms : nullptr, errmsg, errmsg_len, z);
     if (r) return r;
+    for (int q = 0; kernel_ms && q < 3; ++q) kernel_ms[q] += ms[q];
     CK(cudaEventRecord(w->ev_done[b], st), "cudaEventRecord");
     CK(cudaStreamWaitEvent(w->d2h, w->ev_done[b], 0), "cudaStreamWaitEvent");
     for (size_t k = 0; k < fl.size(); ++k) {

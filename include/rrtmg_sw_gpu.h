@@ -107,7 +107,10 @@ typedef struct rrtmg_sw_exec {
   int32_t sync;
   int32_t reserved;
   float *kernel_ms;        /* optional float[3]: device ms of the McICA, gas
-                              optics and transfer kernels (forces a sync) */
+                              optics and transfer kernels, summed over the
+                              chunks of a large call.  Each chunk is waited
+                              for, so a timed call on host arrays does not
+                              overlap its copies with its kernels. */
 } rrtmg_sw_exec;
 
 /* rswinit (radsw_main.F90:1388): validates iovr, sets heatfac, builds the
