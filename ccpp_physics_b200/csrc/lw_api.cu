@@ -1060,11 +1060,14 @@ extern "C" int rrtmg_lw_gpu_autotune(const rrtmg_lw_run_args* blocks, int32_t nb
   cudaStream_t st = stream ? (cudaStream_t)stream : w->stream;
   const int V = pick_v(f.nlay);
   precision = kernel_precision(precision, &f);
-  // candidates: transfer CTA of 1, 2, 4 columns x hand-off chunk (all, 1/2, 1/4 of the columns)
+  // candidates: transfer CTA of 1, 2, 4 columns x hand-off chunk (all, 1/2, 1/4 of the columns);
+  // only lw_rt_kernel has the choice of columns, and for the others the default stands
+  const bool rt_kernel = f.isubclw > 0 && (precision == RRTMG_LW_FP64 ? f.want_hlwb != 0 : !(g.sgpath && sg_path_applies(f)));
   std::vector<Shape> cands;
   for (int wv : {4, 2, 1})
     for (long ch : {0L, (long)(ncols + 1) / 2, (long)(ncols + 3) / 4}) {
       if (ch > 0 && ch < 1024) continue;
+      if (!rt_kernel && wv != Shape().rt_warps) continue;
       Shape s;
       s.rt_warps = wv;
       s.chunk = ch;

@@ -127,8 +127,8 @@ struct Scratch {
 };
 
 // Launch shape of the column kernels (host side; chosen by the autotuner
-// or defaulted).  rt_warps: columns (one warp each) per CTA of the transfer
-// kernel; chunk: columns per gas-optics -> transfer hand-off (0 = as many as
+// or defaulted).  rt_warps: columns (one warp each) per CTA of lw_rt_kernel (FP32,
+// and FP64 with hlwb); chunk: columns per gas-optics -> transfer hand-off (0 = as many as
 // the scratch budget holds); gas_per_sm: resident gas CTAs per SM to launch
 // (0 = the occupancy limit).
 struct Shape {

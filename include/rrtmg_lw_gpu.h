@@ -171,8 +171,11 @@ int rrtmg_lw_gpu_run_noalloc(const rrtmg_lw_run_args *args, int32_t precision,
 /* Launch shape of the column kernels.  Chosen by rrtmg_lw_gpu_autotune or
  * given by the caller; zero fields take the defaults. */
 typedef struct rrtmg_lw_tuning {
-  int32_t rt_warps;        /* columns (one warp each) per CTA of the transfer
-                              kernel: 1, 2 or 4 (default 4) */
+  int32_t rt_warps;        /* columns (one warp each) per CTA of the McICA
+                              transfer kernel in FP32, and in FP64 with hlwb:
+                              1, 2 or 4 (default 4); the other transfer
+                              kernels do not read it and the autotuner leaves
+                              it at the default */
   int32_t gas_per_sm;      /* resident gas-optics CTAs per SM to launch
                               (0 = the occupancy limit) */
   int32_t chunk_cols;      /* columns per gas-optics -> transfer hand-off
