@@ -1694,7 +1694,6 @@ extern "C" int rrtmg_lw_gpu_surrogate_grads(const float* feats, const float* tar
   if (grads) SG_CK(cudaMemcpyAsync(grads, dgr, sizeof(float) * P_N, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
   SG_CK(cudaFreeAsync(dgr, st), "cudaFreeAsync");
   SG_CK(cudaStreamSynchronize(st), "training kernels");
-  SG_CK(cudaMemsetAsync(net.G, 0, sizeof(float) * G_N, st), "cudaMemsetAsync");
   if (herr[0]) { smsg(errmsg, errmsg_len, "rrtmg_lw_gpu_surrogate_grads: tensor-core wait timed out"); return 1; }
   if (loss) { float l; std::memcpy(&l, &herr[1], sizeof(float)); *loss = l / (float)((long)batch * SG_NOUT); }
   return 0;
@@ -1717,6 +1716,9 @@ extern "C" int rrtmg_lw_gpu_surrogate_train(const float* feats, const float* tar
   }
   cudaStream_t st = (cudaStream_t)stream;
   SG_CK(ensure_batch(batch), "cudaMalloc(activations)");
+  // the sums start from zero whatever the call before left (a gradient check, or
+  // a step that failed before its update); within the call Adam leaves them at zero
+  SG_CK(cudaMemsetAsync(net.G, 0, sizeof(float) * G_N, st), "cudaMemsetAsync");
   SG_CK(cudaMemsetAsync(net.err, 0, sizeof(int), st), "cudaMemsetAsync");
   std::mt19937_64 rng(seed);
   const long steps = n / batch;
