@@ -721,12 +721,8 @@ struct TblGlobal {
   __device__ __forceinline__ double operator()(int i) const { return __ldg(p + i); }
 };
 struct TblShared {
-  unsigned base;
-  __device__ __forceinline__ double operator()(int i) const {
-    double v;
-    asm("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(base + 8u * (unsigned)i));
-    return v;
-  }
+  const double* p;   // shared memory
+  __device__ __forceinline__ double operator()(int i) const { return p[i]; }
 };
 
 __device__ __forceinline__ double exp_small(double z) { return 1.0 - z + 0.5 * z * z; }
@@ -1299,7 +1295,7 @@ struct RtTable<true> {
   static __device__ __forceinline__ type get(const double* ET, double* sm) {
     for (int q = threadIdx.x; q <= kNtbmx; q += blockDim.x) sm[q] = ET[q];
     __syncthreads();
-    return {(unsigned)__cvta_generic_to_shared(sm)};
+    return {sm};
   }
 };
 template <bool SHT>
