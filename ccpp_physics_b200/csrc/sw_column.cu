@@ -897,14 +897,15 @@ __device__ __forceinline__ void rt_cloudy(const RtCol& c, const Tbl& ET) {
       const int k = 32 * w + __ffs(m) - 1;
       m &= m - 1;
       const ptrdiff_t xo = c.xstep * k;
-      const double tae = __ldg(c.aod + xo), sae = __ldg(c.ssa + xo), gae = __ldg(c.asy + xo);
+      const double tae = finite_od(__ldg(c.aod + xo)), sae = __ldg(c.ssa + xo), gae = __ldg(c.asy + xo);
       const double tr = c.ray.p[c.ray.stride * k] * c.ray.coef, tg = c.tg[(size_t)(k >> 2) * kSwNg * kTgStride + (k & 3)];
       const double ztau0 = fmax(kFtiny, tr + tg + tae);
       const double zssa0 = tr + tae * sae;
       const double zasy0 = gae * sae * tae;
       const size_t x = (size_t)k * 14;
       LayOpt v;
-      two_stream(ztau0 + c.tcw[x], zssa0 + c.scw[x], zasy0 + c.gcw[x], c.cosz, c.sntz, c.iswmode, ET, v);
+      const double tc = c.tcw[x], down = __double2hiint(tc) < 0x7e700000 ? 1.0 : 0x1p-64;   // finite_od, for all three
+      two_stream(ztau0 + tc * down, zssa0 + c.scw[x] * down, zasy0 + c.gcw[x] * down, c.cosz, c.sntz, c.iswmode, ET, v);
       if (GRID) {
         LayOpt o;
         two_stream(ztau0, zssa0, zasy0, c.cosz, c.sntz, c.iswmode, ET, o);
@@ -963,9 +964,10 @@ __device__ __forceinline__ void rt_up(const RtCol& c, const Tbl& ET, double ub, 
       if (k + 1 < c.nlay) fetch(nx);   // issued ahead of this layer's arithmetic
       const double tg = (kk & 2) ? ((kk & 1) ? c23.y : c23.x) : ((kk & 1) ? c01.y : c01.x);
       const double tr = cur.tr * c.ray.coef;
+      const double tae = finite_od(cur.tae);
       LayOpt o;
-      two_stream(fmax(kFtiny, tr + tg + cur.tae), tr + cur.tae * cur.sae, cur.gae * cur.sae * cur.tae, c.cosz, c.sntz,
-                 c.iswmode, ET, o);
+      two_stream(fmax(kFtiny, tr + tg + tae), tr + tae * cur.sae, cur.gae * cur.sae * tae, c.cosz, c.sntz, c.iswmode,
+                 ET, o);
       double tbd = o.tb - o.e3;
       __stcg(st, o.td);
       __stcg(st + kSwNg, tbd);
