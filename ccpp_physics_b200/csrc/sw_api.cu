@@ -31,7 +31,10 @@ namespace {
 
 constexpr int kNtbmx = 10000;
 constexpr double kS0 = 1368.22;                  // RSM:343
-constexpr size_t kScratchBudget = (size_t)12 << 30;   // 7,251 columns of 127 layers in one chunk
+// Scratch of one call (RRTMG_SW_GPU_SCRATCH_MB overrides it): 7,631 columns of
+// 127 layers, 1.55 MB each, in one chunk.  16,384 columns with 12 / 6 / 4 / 2 GiB:
+// 11.6, 11.9, 12.4 and 13.3 ms; 3,001: 2.40, 2.38, 2.56 and 2.68 ms.
+constexpr size_t kScratchBudget = (size_t)11 << 30;
 
 struct SwState {
   bool ready = false;
@@ -49,6 +52,7 @@ struct SwWorkspace {
   cudaStream_t stream = nullptr;
   char* scratch = nullptr;
   size_t scratch_bytes = 0;
+  size_t refused = SIZE_MAX;   // the least scratch that the device did not have
   char* stage = nullptr;     // device copies of host arguments
   size_t stage_bytes = 0;
   int* bad = nullptr;
@@ -124,17 +128,24 @@ size_t scratch_per_col(int nlay) {
          4 + (size_t)sw::kSwNg * nw * 4 + 64;
 }
 
+size_t scratch_budget() {
+  const char* env = std::getenv("RRTMG_SW_GPU_SCRATCH_MB");
+  return env ? (size_t)std::atol(env) << 20 : kScratchBudget;
+}
+
 // Columns of a chunk of a call of n: equal chunks that fit the scratch budget,
 // in whole rounds of the upward kernel.
 int chunk_columns(int n, int nlay) {
-  const int most = (int)std::max<size_t>(1, kScratchBudget / scratch_per_col(nlay));
+  const int most = (int)std::max<size_t>(1, scratch_budget() / scratch_per_col(nlay));
   if (n <= most) return std::max(n, 1);
   const long long round = (long long)sw::kUpThreads * g.num_sms;   // (column, g-point) pairs
   const auto rounds_of = [round](long long cols) { return cols * sw::kSwNg / round; };
   const auto cols_of = [round](long long rounds) { return (int)(rounds * round / sw::kSwNg); };
-  const int chunks = (n + most - 1) / most, even = (n + chunks - 1) / chunks;
-  const int whole = cols_of(rounds_of(even - 1) + 1);
-  return whole <= most ? std::max(whole, even) : std::max(cols_of(rounds_of(most)), std::min(most, cols_of(1)));
+  if (most < cols_of(1)) return most;
+  for (int chunks = (n + most - 1) / most;; ++chunks) {   // ends at one round a chunk at the latest
+    const int even = (n + chunks - 1) / chunks, whole = std::max(cols_of(rounds_of(even - 1) + 1), even);
+    if (whole <= most) return whole;
+  }
 }
 
 // carve one chunk's scratch out of the workspace (base null: only its size;
@@ -168,6 +179,20 @@ sw::SwScratch carve(char* base, int nc, int nlay, bool transfer = true) {
   sw::SwScratch s;
   carve(base, nc, nlay, transfer, &s);
   return s;
+}
+
+// The scratch of a call of n columns, and the columns of a chunk: as many as the
+// budget holds, or where the device does not have that much memory left, half as
+// many until it does (a workspace does not ask for a refused size again).
+cudaError_t reserve(SwWorkspace* w, int n, int nlay, int* chunk) {
+  for (*chunk = chunk_columns(n, nlay);; *chunk = (*chunk + 1) / 2) {
+    const size_t need = carve_bytes(*chunk, nlay);
+    if (need >= w->refused && *chunk > 1) continue;
+    const cudaError_t e = grow(&w->scratch, &w->scratch_bytes, need);
+    if (e != cudaErrorMemoryAllocation || *chunk == 1) return e;
+    (void)cudaGetLastError();
+    w->refused = need;
+  }
 }
 
 // Sizes (in elements) of the caller's arrays.
@@ -313,8 +338,8 @@ class StageTimes {
 int run_device(SwWorkspace* w, const sw::SwArgs& d, int nday, cudaStream_t st, float* kernel_ms, char* errmsg,
                int32_t errmsg_len, const Sizes& z) {
   CK(zero_outputs(d, z, d.nlay, st), "zeroing the outputs");
-  const int chunk = chunk_columns(nday, d.nlay);
-  CK(grow(&w->scratch, &w->scratch_bytes, carve_bytes(chunk, d.nlay)), "scratch allocation");
+  int chunk = 0;
+  CK(reserve(w, nday, d.nlay, &chunk), "scratch allocation");
   StageTimes times(kernel_ms);
   for (int p0 = 0; p0 < nday; p0 += chunk) {
     const int nc = std::min(chunk, nday - p0);
@@ -422,7 +447,8 @@ int run_host_pipelined(SwWorkspace* w, const rrtmg_sw_run_args* a, cudaStream_t 
   }
   CK(grow(&w->pbuf, &w->pbuf_bytes, 2 * per), "staging allocation");
   // the kernels' scratch for a whole chunk, allocated before any launch
-  CK(grow(&w->scratch, &w->scratch_bytes, carve_bytes(chunk_columns(kSwHostChunk, nlay), nlay)), "scratch allocation");
+  int chunk = 0;
+  CK(reserve(w, kSwHostChunk, nlay, &chunk), "scratch allocation");
   CK(cudaMemsetAsync(w->bad, 0, sizeof(int), st), "cudaMemsetAsync");
   if (kernel_ms) kernel_ms[0] = kernel_ms[1] = kernel_ms[2] = 0.0f;   // summed over the chunks
   for (int j = 0; j < nch; ++j) {
@@ -746,8 +772,8 @@ extern "C" int rrtmg_sw_gpu_run_blocks(const rrtmg_sw_run_args* blocks, int32_t 
   CK(sw::blocks_prepare(d_tab, d_pre, d_pre + nb, nb, total_cols, d_pts, w->bad, st), "block table kernels");
   // the kernels over all daytime points, in scratch-sized chunks
   const sw::SwArgs& f = w->h_tab[0];
-  const int chunk = chunk_columns(ndays, nlay);
-  CK(grow(&w->scratch, &w->scratch_bytes, carve_bytes(chunk, nlay)), "scratch allocation");
+  int chunk = 0;
+  CK(reserve(w, ndays, nlay, &chunk), "scratch allocation");
   StageTimes times(x->kernel_ms);
   for (int p0 = 0; p0 < ndays; p0 += chunk) {
     const int nc = std::min(chunk, ndays - p0);

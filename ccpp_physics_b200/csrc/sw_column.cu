@@ -885,7 +885,8 @@ __device__ __forceinline__ bool cloud_at(const RtCol& c, int k, uint32_t word) {
   return GRID ? (c.cloudy && c.cfr[(size_t)k * c.cfs] > kFtiny) : ((word >> (k & 31)) & 1u);
 }
 
-// all-sky optics of the cloudy layers, into store values 8..13
+// all-sky optics of the cloudy layers, into store values 8..11, and what the way
+// up alone needs (rb, e4) where it then leaves zrupb, zrupd (6, 7)
 template <bool GRID, typename Tbl>
 __device__ __forceinline__ void rt_cloudy(const RtCol& c, const Tbl& ET) {
 #pragma unroll 1
@@ -916,8 +917,8 @@ __device__ __forceinline__ void rt_cloudy(const RtCol& c, const Tbl& ET) {
       __stcg(q + 9 * kSwNg, v.tb - v.e3);
       __stcg(q + 10 * kSwNg, v.e3);
       __stcg(q + 11 * kSwNg, v.rd);
-      __stcg(q + 12 * kSwNg, v.rb);
-      __stcg(q + 13 * kSwNg, v.e4);
+      __stcg(q + 6 * kSwNg, v.rb);
+      __stcg(q + 7 * kSwNg, v.e4);
     }
   }
 }
@@ -980,16 +981,16 @@ __device__ __forceinline__ void rt_up(const RtCol& c, const Tbl& ET, double ub, 
       ub = fma(o.td * fma(tbd, ud, o.e3 * ub), q, o.rb);
       ud = fma(o.td * o.td * ud, q, o.rd);
       if (c.cloudy) {
-        __stcg(st + 6 * kSwNg, ubw);
-        __stcg(st + 7 * kSwNg, udw);
         if (cloud_at<GRID>(c, k, word)) {
+          o.rb = __ldcg(st + 6 * kSwNg);
+          o.e4 = __ldcg(st + 7 * kSwNg);
           o.td = __ldcg(st + 8 * kSwNg);
           tbd = __ldcg(st + 9 * kSwNg);
           o.e3 = __ldcg(st + 10 * kSwNg);
           o.rd = __ldcg(st + 11 * kSwNg);
-          o.rb = __ldcg(st + 12 * kSwNg);
-          o.e4 = __ldcg(st + 13 * kSwNg);
         }
+        __stcg(st + 6 * kSwNg, ubw);
+        __stcg(st + 7 * kSwNg, udw);
         beam0w *= o.e4;
         const double qw = recip_newton(fma(-udw, o.rd, 1.0));
         ubw = fma(o.td * fma(tbd, udw, o.e3 * ubw), qw, o.rb);

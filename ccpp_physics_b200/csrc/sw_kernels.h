@@ -56,7 +56,7 @@ __host__ __device__ inline size_t tg_offset(int nlay, size_t pl, int k, int g) {
 // CTA from kUpWide columns per SM on), kDownPerSm columns on the way down
 constexpr int kUpThreads = 512, kUpWide = 4, kDownPerSm = 6;
 constexpr int kRtGroups = kSwNg / 16;       // 16-lane groups of a column
-constexpr int kRtVals = 14;                 // stored values per layer and g-point
+constexpr int kRtVals = 12;                 // stored values per layer and g-point
 constexpr int kRtBandSlots = 14 + kRtGroups - 1;   // (band, group) pairs: slot band + group
 __host__ __device__ inline size_t rt_col_store(int nlay) { return (size_t)(nlay + 1) * kRtVals * kSwNg; }
 // shared memory of one column: the groups' partial flux sums
