@@ -109,6 +109,7 @@ void set_msg(char* errmsg, int32_t len, const char* fmt, ...) {
 
 int cuda_fail(char* errmsg, int32_t len, const char* what, cudaError_t e) {
   set_msg(errmsg, len, "rrtmg_lw_gpu: %s failed: %s", what, cudaGetErrorString(e));
+  (void)cudaGetLastError();   // reported here: the next launch check must not meet it again
   return 1;
 }
 

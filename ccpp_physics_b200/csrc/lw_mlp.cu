@@ -1236,6 +1236,7 @@ std::mutex net_mu;
 
 void msg(char* e, int32_t n, const char* fmt, const char* what, cudaError_t c) {
   if (e && n > 0) std::snprintf(e, (size_t)n, fmt, what, cudaGetErrorString(c));
+  (void)cudaGetLastError();   // reported here: the next launch check must not meet it again
 }
 #define SG_CK(call, what)                                                                 \
   do {                                                                                    \

@@ -152,6 +152,7 @@ extern "C" int rrtmg_lw_gpu_run_noalloc(const rrtmg_lw_run_args* a, int32_t prec
   void* base = nullptr;
   if ((e = scratch_address(v.device, &base)) != cudaSuccess) {
     msg(errmsg, errmsg_len, "rrtmg_lw_gpu_run_noalloc: cudaGetSymbolAddress: %s", cudaGetErrorString(e));
+    (void)cudaGetLastError();   // reported here: the next launch check must not meet it again
     return 1;
   }
   uint32_t* bits = static_cast<uint32_t*>(base);
@@ -181,6 +182,7 @@ extern "C" int rrtmg_lw_gpu_run_noalloc(const rrtmg_lw_run_args* a, int32_t prec
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
     msg(errmsg, errmsg_len, "rrtmg_lw_gpu_run_noalloc: kernels failed: %s", cudaGetErrorString(e));
+    (void)cudaGetLastError();
     return 1;
   }
   return 0;

@@ -331,6 +331,7 @@ void set_msg(char* errmsg, int32_t len, const char* fmt, ...) {
 
 int fail(char* errmsg, int32_t len, const char* what, cudaError_t e) {
   set_msg(errmsg, len, "%s: %s failed: %s", tl_who, what, cudaGetErrorString(e));
+  (void)cudaGetLastError();   // reported here: the next launch check must not meet it again
   return 1;
 }
 

@@ -81,6 +81,7 @@ void set_msg(char* m, int32_t n, const char* fmt, ...) {
 }
 int cuda_fail(char* m, int32_t n, const char* what, cudaError_t e) {
   set_msg(m, n, "rrtmg_sw_gpu: %s failed: %s", what, cudaGetErrorString(e));
+  (void)cudaGetLastError();   // reported here: the next launch check must not meet it again
   return 1;
 }
 #define CK(call, what)                                                      \
