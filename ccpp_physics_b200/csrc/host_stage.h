@@ -41,13 +41,22 @@ struct HostStage {
   }
 };
 
-// Gathers fields into a stage laid out like the device buffer dev.
+// Gathers fields into a stage laid out like the device buffer dev.  A call that
+// ends early waits for the copies it has sent, so that the next one, on whatever
+// stream, finds the stage at rest.
 struct HostGather {
   static constexpr size_t kPiece = (size_t)256 << 10;
   char *host, *dev;
   cudaStream_t st;
   size_t sent = 0;
+  bool waited = false;   // the call has synchronised st
 
+  HostGather(char* h, char* d, cudaStream_t s) : host(h), dev(d), st(s) {}
+  HostGather(const HostGather&) = delete;
+  HostGather& operator=(const HostGather&) = delete;
+  ~HostGather() {
+    if (sent && !waited) (void)cudaStreamSynchronize(st);
+  }
   cudaError_t put(size_t off, const void* src, size_t n, size_t next) {   // next: where the following field starts
     std::memcpy(host + off, src, n);
     return next - sent >= kPiece ? send(next) : cudaSuccess;

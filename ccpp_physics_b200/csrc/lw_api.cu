@@ -844,6 +844,7 @@ extern "C" int rrtmg_lw_gpu_run_ex(const rrtmg_lw_run_args* a, const rrtmg_lw_ex
     CK(cudaMemcpyAsync(w->stage.p + out0, w->dbuf + out0, off - out0, cudaMemcpyDeviceToHost, st),
        "cudaMemcpyAsync(D2H)");
     CK(cudaStreamSynchronize(st), "kernel execution");
+    up.waited = true;
     for (int k = 0; k < nout; ++k) {
       if (!host_out[k]) continue;
       const char* src = w->stage.p + (reinterpret_cast<char*>(*outs[k]) - w->dbuf);

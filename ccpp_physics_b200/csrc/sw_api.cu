@@ -617,7 +617,7 @@ extern "C" int rrtmg_sw_gpu_run_ex(const rrtmg_sw_run_args* a, const rrtmg_sw_ex
   size_t total = align256(z.np * 4) + align256(z.nd * 4);
   for (auto& p : ins) if (*p.first) total += align256(p.second * 8);
   for (auto& p : outs) if (*p.p) total += align256(p.n * 8);
-  CK(cudaStreamSynchronize(st), "cudaStreamSynchronize");   // an earlier call that failed may still read the staging
+  CK(cudaStreamSynchronize(st), "cudaStreamSynchronize");
   CK(grow(&w->stage, &w->stage_bytes, total), "staging allocation");
   const bool staged = w->pin.ensure(total + 256);   // and the flag of a bad idxday
   HostGather up{w->pin.p, w->stage, st};
@@ -661,6 +661,7 @@ extern "C" int rrtmg_sw_gpu_run_ex(const rrtmg_sw_run_args* a, const rrtmg_sw_ex
     CK(cudaMemcpyAsync(w->pin.p + out0, w->stage + out0, off - out0, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
     CK(cudaMemcpyAsync(bad, w->bad, sizeof(int), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
     CK(cudaStreamSynchronize(st), "kernel execution");
+    up.waited = true;
     for (const Back& b : back) {
       const char* src = w->pin.p + ((char*)b.dev - w->stage);
       if (b.o.w == 0) std::memcpy(b.host, src, b.o.n * 8);
