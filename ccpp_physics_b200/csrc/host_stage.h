@@ -8,13 +8,17 @@
 // layers of rrtmg_lw_run: 361 -> 309 us; 57 x 127 of rrtmg_sw_run: 1,000 -> 933 us.
 // The buffer belongs to a calling thread's workspace, is freed with it and never
 // exceeds kHostStageMax; larger calls keep the copies per field, whose cost
-// their own size hides.
+// their own size hides, while the gathering grows with it.  Staged / per field,
+// us: longwave, 64 layers, 300 columns (9.7 MiB) 978 / 1,008, 400 (12.9) 1,204 /
+// 1,199, 540 (17) 1,628 / 1,535; 127 layers, 200 (12.8) 1,248 / 1,252, 270 (17)
+// 1,644 / 1,517, 400 (26) 2,290 / 2,019; shortwave, 127 layers, 100 (7.2) 1,099 /
+// 1,155, 200 (14) 1,574 / 1,524, 480 (34) 3,108 / 2,644: the line lies at 12 MiB.
 #pragma once
 #include <algorithm>
 #include <cstring>
 #include <cuda_runtime.h>
 
-constexpr size_t kHostStageMax = (size_t)16 << 20;
+constexpr size_t kHostStageMax = (size_t)12 << 20;
 
 struct HostStage {
   char* p = nullptr;

@@ -1,6 +1,6 @@
 """Host arrays with ldim > npts: the columns beyond npts are the caller's and
 stay as they were, whichever way the call's size takes the arrays to the
-device: one pinned buffer (up to 16 MiB of arguments), a copy per array, or
+device: one pinned buffer (up to 12 MiB of arguments), a copy per array, or
 chunks of 4,096 columns (from 8,192 columns on)."""
 import numpy as np
 import pytest
