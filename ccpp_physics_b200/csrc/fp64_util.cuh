@@ -1,6 +1,6 @@
-// fp64_util.cuh -- FP64 helpers of the transfer kernels (lw_rt64.cuh,
+// fp64_util.cuh -- FP64 helpers of the column kernels (lw_gas.cuh, lw_rt64.cuh,
 // sw_column.cu): quotients without the IEEE slow path, table indices that
-// equal the reference's, sums over lanes.
+// equal the reference's, the split of the atmosphere, sums over lanes.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -57,6 +57,12 @@ __device__ __forceinline__ int pade_index(double z) {
 // layer, cost the scheme 0.8 %, a branch around the layer's first quotients 0.7 %).
 __device__ __forceinline__ double finite_od(double z) {
   return __hiloint2double(min(__double2hiint(z), 0x7e700000), __double2loint(z));
+}
+
+// ln p > 4.56 (the lower atmosphere, RLM:2344, RSM:2305): p against e^4.56 =
+// 95.58347984, by the logarithm itself where rounding could decide.
+__device__ __forceinline__ bool lower_atm(double p) {
+  return (p > 95.5834 && p < 95.5836) ? log(p) > 4.56 : p > 95.5835;
 }
 
 // read-once inputs: no L1 line, which stays with exp_tbl

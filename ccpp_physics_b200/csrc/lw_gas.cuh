@@ -20,6 +20,7 @@
 //   col  [c][48]          secdiff(16), pklay(b,0)(16), semiss, lcf1
 #pragma once
 
+#include "fp64_util.cuh"
 #include "lw_bands.cuh"
 #include "lw_common.cuh"
 #include "lw_features.cuh"
@@ -144,12 +145,6 @@ struct GasWork {
   }
 };
 
-// ln p > 4.56 (the lower atmosphere, RLM:2344): p against e^4.56 =
-// 95.58347984, by the logarithm itself where rounding could decide.
-__device__ __forceinline__ bool lower_atm(double p) {
-  return (p > 95.5834 && p < 95.5836) ? log(p) > 4.56 : p > 95.5835;
-}
-
 // dry-air and water-vapour column amounts of a layer (RLM:823-836)
 struct ColAmt {
   double coldry, h2ovmr;
@@ -204,7 +199,7 @@ __device__ __forceinline__ void gas_unit(int cc, int seg, int b_lo, int b_hi, in
       bool lo = false, cl = false;
       if (k < nlay) {
         const int rk = top ? nlay - 1 - k : k;
-        lo = lower_atm(IN(F_PLYR, rk));
+        lo = fp64::lower_atm(IN(F_PLYR, rk));
         cl = IN(F_CLDCF, rk) > kEps;
         if (rec) {
           const ColAmt ca = col_amounts(IN(F_QLYR, rk), IN(F_DELPIN, rk));

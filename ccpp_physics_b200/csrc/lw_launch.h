@@ -62,7 +62,7 @@ cudaError_t mcica_sw_launch(int ncols, int nlay, int iovr, const McicaStage& sta
 // the same for iovr 3..5 (two g-major sets); stage.alpha = fac_lcf (iovr 3) or alpha (4, 5) per layer
 cudaError_t mcica_sw_two_set_prepare(int max_smem);
 cudaError_t mcica_sw_two_set_launch(int ncols, int nlay, int iovr, const McicaStage& stage, uint32_t* bits,
-                                    int num_sms, cudaStream_t st);
+                                    cudaStream_t st);
 // raw state words of one twister stream (lw_mcica.cu): raw[j] is what draw j
 // tempers; state: seed_state_words() of workspace
 size_t seed_state_words();

@@ -109,7 +109,7 @@ __device__ bool twist_ring(uint32_t* ring, int cap, int jp, int lane) {
 
 struct McicaArgs {
   int nlay, nw, iovr, isubclw, top_at_1;
-  int cap;        // ring capacity in words
+  int cap;        // ring capacity in words (iovr 0..2)
   McicaStage st;  // stage entry point inputs (blocks == nullptr)
 };
 
@@ -829,7 +829,7 @@ cudaError_t mcica_launch(const Block* blocks, int nblocks, const Block& b0, int 
   a.iovr = iovr;
   a.isubclw = isubclw;
   a.top_at_1 = top_at_1;
-  a.cap = mcica_ring_capacity(nlay);
+  a.cap = iovr < 3 ? mcica_ring_capacity(nlay) : 0;
   a.st = stage;
   if (iovr >= 3) {
     if (ncols < 1) return cudaSuccess;
@@ -958,7 +958,7 @@ cudaError_t mcica_sw_two_set_prepare(int max_smem) {
 }
 
 cudaError_t mcica_sw_two_set_launch(int ncols, int nlay, int iovr, const McicaStage& stage, uint32_t* bits,
-                                    int num_sms, cudaStream_t st) {
+                                    cudaStream_t st) {
   if (iovr < 3 || iovr > 5) return cudaErrorInvalidValue;
   McicaArgs a;
   a.nlay = nlay;
@@ -966,7 +966,7 @@ cudaError_t mcica_sw_two_set_launch(int ncols, int nlay, int iovr, const McicaSt
   a.iovr = iovr;
   a.isubclw = 2;
   a.top_at_1 = 0;
-  a.cap = kSwTwoSetRing;
+  a.cap = 0;
   a.st = stage;
   if (ncols < 1) return cudaSuccess;
   const size_t smem = sw_two_set_warp_bytes(nlay) * kSwTwoSetWarps;

@@ -121,7 +121,6 @@ SwWorkspace* workspace(char* errmsg, int32_t errmsg_len, int* rc) {
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-
 // per-column scratch bytes of the kernels
 size_t scratch_per_col(int nlay) {
   const int nw = (nlay + 31) / 32;
@@ -359,7 +358,7 @@ int run_device(SwWorkspace* w, const sw::SwArgs& d, int nday, cudaStream_t st, f
     } else if (d.iovr <= 2) {
       CK(lw::mcica_sw_launch(nc, d.nlay, d.iovr, ms, s.bits, g.num_sms, st), "McICA kernel launch");
     } else {
-      CK(lw::mcica_sw_two_set_launch(nc, d.nlay, d.iovr, ms, s.bits, g.num_sms, st), "McICA kernel launch");
+      CK(lw::mcica_sw_two_set_launch(nc, d.nlay, d.iovr, ms, s.bits, st), "McICA kernel launch");
     }
     CK(times.mark(2, st), "stage timing");
     CK(sw::rt_launch(d, s, p0, nc, g.tab, g.etab, st), "transfer kernel launch");
@@ -792,7 +791,7 @@ extern "C" int rrtmg_sw_gpu_run_blocks(const rrtmg_sw_run_args* blocks, int32_t 
     if (f.isubcsw > 0 && f.iovr <= 2)
       CK(lw::mcica_sw_launch(nc, nlay, f.iovr, ms, sc.bits, g.num_sms, st), "McICA kernel launch");
     else if (f.isubcsw > 0)
-      CK(lw::mcica_sw_two_set_launch(nc, nlay, f.iovr, ms, sc.bits, g.num_sms, st), "McICA kernel launch");
+      CK(lw::mcica_sw_two_set_launch(nc, nlay, f.iovr, ms, sc.bits, st), "McICA kernel launch");
     CK(times.mark(2, st), "stage timing");
     CK(sw::rt_blocks_launch(d_tab, d_pts, f.isubcsw <= 0, f.hswb != nullptr, sc, p0, nc, nlay, g.tab, g.etab, st),
        "transfer kernel launch");
@@ -827,7 +826,7 @@ extern "C" int rrtmg_sw_gpu_mcica(int32_t npts, int32_t nlay, int32_t ldim, int3
     double* aux = (double*)w->scratch;
     CK(sw::overlap_aux_launch(npts, nlay, ld, iovr, dz, de_lgth, alpha, aux, ld, st), "overlap kernel launch");
     ms.alpha = aux;
-    CK(lw::mcica_sw_two_set_launch(npts, nlay, iovr, ms, bits, g.num_sms, st), "McICA kernel launch");
+    CK(lw::mcica_sw_two_set_launch(npts, nlay, iovr, ms, bits, st), "McICA kernel launch");
   } else {
     CK(lw::mcica_sw_launch(npts, nlay, iovr, ms, bits, g.num_sms, st), "McICA kernel launch");
   }

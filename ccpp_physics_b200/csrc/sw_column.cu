@@ -60,12 +60,6 @@ struct Lay {
   bool lower_plog;   // plog > 4.56
 };
 
-// ln p > 4.56 (RSM:2305): p against e^4.56 = 95.58347983, by the logarithm
-// itself where rounding could decide.
-__device__ __forceinline__ bool lower_atm(double p) {
-  return (p > 95.5834 && p < 95.5836) ? log(p) > 4.56 : p > 95.5835;
-}
-
 // rrtmg_sw_run's layer prologue (RSM:910-946 / 1001-1040) for internal
 // layer k (0-based, surface first) of caller column i, then setcoef.
 __device__ void layer_record(const SwArgs& a, int i, int k, const double* __restrict__ T, Lay& L) {
@@ -1504,8 +1498,10 @@ cudaError_t optics_blocks_launch(const SwArgs* tab, const int2* pts, const SwScr
 cudaError_t rt_blocks_launch(const SwArgs* tab, const int2* pts, bool grid, bool want_b, const SwScratch& s, int p0,
                              int nc, int nlay, const double* T, const double* ET, cudaStream_t st) {
   if (nc <= 0) return cudaSuccess;
-  // one CTA per SM, exp_tbl in shared memory, once they have work for nearly all their threads; below that a column per
-  // CTA, which spreads a small call over the SMs
+  // one CTA per SM, exp_tbl in shared memory, once they have work for nearly all their threads (four columns' 448 of
+  // 512); below that a column per CTA, which spreads a small call over the SMs.  A call, wide / narrow, us: 64 layers,
+  // 100 columns 397 / 372, 300 420 / 405, 592 (four per SM) 447 / 454, 600 438 / 530, 1,800 922 / 1,022; 127 layers, 100
+  // 544 / 505, 300 583 / 563, 592 632 / 658, 600 704 / 903, 1,800 1,596 / 1,826
   if (nc >= s.num_sms * kUpWide) {
     const auto up = grid ? sw_up_blocks_kernel<true, kUpThreads, true> : sw_up_blocks_kernel<false, kUpThreads, true>;
     up<<<s.num_sms, kUpThreads, kUpSmem, st>>>(tab, pts, s, p0, nc, T, ET);
