@@ -37,7 +37,8 @@ __device__ __forceinline__ double sqrt_markstein(double x) {
 // finite_od first.  The quotient comes from one Newton step (error below
 // 1e-8 in index units) and is rounded by adding 1.5 2^52; only a value within
 // 1e-6 of a tie takes the IEEE division, so the entry is the reference's in every
-// case.
+// case.  NaN and infinity take it too, and the clamp, since the conversion of
+// NaN is INT_MIN: index 0.
 __device__ __forceinline__ int pade_index(double z) {
   constexpr double kBpade = 1.0 / 0.278, kRound = 6755399441055744.0;
   const double d = kBpade + z;
@@ -47,16 +48,18 @@ __device__ __forceinline__ int pade_index(double z) {
   const double q = z * y, t = fma(q, 10000.0, kRound);
   int i = __double2loint(t);
   const double f = fma(q, 10000.0, kRound - t);
-  if (!(fabs(f) < 0.5 - 1.0e-6)) i = (int)(z / d * 10000 + 0.5);
+  if (!(fabs(f) < 0.5 - 1.0e-6)) i = max(0, min(10000, (int)(z / d * 10000 + 0.5)));
   return i;
 }
 
-// An optical depth >= 0, from 2^1000 on a value there, opaque as well: neither it
-// nor its slant path is then out of the helpers' range.  By the high word, one
-// integer minimum (range tests in pade_index, at all four lookups of a shortwave
-// layer, cost the scheme 0.8 %, a branch around the layer's first quotients 0.7 %).
+// A finite optical depth from 2^1000 on held there (opaque as well), so that
+// neither it nor its slant path is out of the helpers' range; infinity and NaN
+// stay.  By the high word.  (Range tests in pade_index, at all four lookups of a
+// shortwave layer, cost the scheme 0.8 %, a branch around the layer's first
+// quotients 0.7 %.)
+__device__ __forceinline__ bool huge_od(double z) { return (unsigned)(__double2hiint(z) - 0x7e700000) < 0x01800000u; }
 __device__ __forceinline__ double finite_od(double z) {
-  return __hiloint2double(min(__double2hiint(z), 0x7e700000), __double2loint(z));
+  return __hiloint2double(huge_od(z) ? 0x7e700000 : __double2hiint(z), __double2loint(z));
 }
 
 // ln p > 4.56 (the lower atmosphere, RLM:2344, RSM:2305): p against e^4.56 =

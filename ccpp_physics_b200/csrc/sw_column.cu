@@ -899,7 +899,7 @@ __device__ __forceinline__ void rt_cloudy(const RtCol& c, const Tbl& ET) {
       const double zasy0 = gae * sae * tae;
       const size_t x = (size_t)k * 14;
       LayOpt v;
-      const double tc = c.tcw[x], down = __double2hiint(tc) < 0x7e700000 ? 1.0 : 0x1p-64;   // finite_od, for all three
+      const double tc = c.tcw[x], down = huge_od(tc) ? 0x1p-64 : 1.0;   // finite_od, for all three
       two_stream(ztau0 + tc * down, zssa0 + c.scw[x] * down, zasy0 + c.gcw[x] * down, c.cosz, c.sntz, c.iswmode, ET, v);
       if (GRID) {
         LayOpt o;
