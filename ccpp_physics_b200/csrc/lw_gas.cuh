@@ -361,6 +361,8 @@ __device__ __forceinline__ void gas_unit(int cc, int seg, int b_lo, int b_hi, in
     R* tcol = write_scratch ? sc.tau + hoff : nullptr;
     R* fcol = write_scratch ? sc.frac + hoff : nullptr;
     R* bcol = write_scratch ? sc.band + (size_t)cc * 3 * NBANDS * NLP : nullptr;
+    // FP64 inputs without a bound of their own, within the range of lw_rt64.cuh's table index
+    const auto hold = [](double od) { return sizeof(R) == 8 ? fp64::finite_od(od) : od; };
 #pragma unroll 1
     for (int b = b_lo; b < b_hi; ++b) {
       if (t < nlay) {
@@ -374,11 +376,11 @@ __device__ __forceinline__ void gas_unit(int cc, int seg, int b_lo, int b_hi, in
         if (bcol && LW_OK(cc < sc.cap && t + 1 < NLP, 14, cc)) {   // evict-first stores: the hand-off must not push the tables out of L2
           __stcs(bcol + (0 * NBANDS + b) * NLP + t, R(planck_int(kt64, b, indlay, tlyrfr)));
           __stcs(bcol + (1 * NBANDS + b) * NLP + t + 1, R(planck_int(kt64, b, indlev, tlvlfr)));
-          __stcs(bcol + (2 * NBANDS + b) * NLP + t, R(tcld));
+          __stcs(bcol + (2 * NBANDS + b) * NLP + t, R(hold(tcld)));
         }
         const size_t ab = i + ld * ((size_t)r + (size_t)nlay * b);
         R tauaer = R(0);
-        if (!sg_skip && LW_OK(r < nlay && i < B.npts, 15, r)) tauaer = R(B.in[F_AERAOD][ab] * (1.0 - B.in[F_AERSSA][ab]));
+        if (!sg_skip && LW_OK(r < nlay && i < B.npts, 15, r)) tauaer = R(hold(B.in[F_AERAOD][ab] * (1.0 - B.in[F_AERSSA][ab])));
         const int ns = ns_of(b);
         const size_t go = ((size_t)c * nlay + t) * NGPT + ns;
         if (!sg_skip) band_gas_optics<R>(b, tab.kt, LR, [&](int g0, auto tau, auto frac) {

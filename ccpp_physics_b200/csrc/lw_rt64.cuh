@@ -126,7 +126,7 @@ lw_rt64_kernel(const Block* __restrict__ blocks, int nblocks, const Block b0, in
       double ex[4], tf[4];
       int i[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) i[j] = od[j] > 0.06 ? fp64::pade_index(fp64::finite_od(od[j])) : 0;
+      for (int j = 0; j < 4; ++j) i[j] = od[j] > 0.06 ? fp64::pade_index(od[j]) : 0;
 #pragma unroll
       for (int j = 0; j < 4; ++j) exp_tfn(i[j], ex[j], tf[j]);
       next();   // behind the gathers: a warp's loads return in order, and these come from further away
@@ -162,7 +162,7 @@ lw_rt64_kernel(const Block* __restrict__ blocks, int nblocks, const Block b0, in
           a = odtot - 0.5 * odtot * odtot;
         } else {
           double ex;
-          exp_tfn(fp64::pade_index(fp64::finite_od(odtot)), ex, totfac);
+          exp_tfn(fp64::pade_index(odtot), ex, totfac);
           a = 1.0 - ex;
         }
         const double fa = v.frac[j] * a;
