@@ -12,8 +12,8 @@
 // layers across the lanes (both sweeps as affine scans: a composition, five
 // shuffle steps and a replay per g-point, lw_rt.cuh), a layer's terms cost two
 // evaluations but no scan, a column spreads over five warps, and a layer count
-// of 64 leaves no lane idle.  16,384 x 127: 5.02 ms as scans, 4.22 here
-// (3.3 down, 1.3 up); 1,024 x 64: 493 -> 150 us; 32 x 64: 569 -> 46 us.
+// of 64 leaves no lane idle.  16,384 x 127: 5.02 ms as scans, 4.26 here;
+// 5,003 x 127: 2.06 -> 1.35 ms; 1,024 x 64: 493 -> 174 us; 32 x 64: 569 -> 47 us.
 // The way down leaves {transmittance, upward source} in place of {tau, frac}
 // (recomputing both on the way up: 6.06 ms); with exp_tbl and tfn_tbl in shared
 // memory, three columns per CTA: 5.83 ms; four CTAs per SM at 96 registers:

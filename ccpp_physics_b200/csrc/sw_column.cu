@@ -843,7 +843,7 @@ __device__ __forceinline__ void mix_grid(double zc1, const LayOpt& o, LayOpt& w)
 // layer and sweep in place of four.  sw_down_kernel does that and the outputs.
 //
 // Two kernels, because they want different things: the way up is a chain of
-// FP64 operations per layer (128 registers, sixteen warps per SM, 57 % of the
+// FP64 operations per layer (128 registers, sixteen warps per SM, 63 % of the
 // issue slots), the way down streams the stored layers (80 registers, 6.4 TB/s).
 // As phases of one kernel, with a slot of the store per resident column, the
 // same loops took 13.0 ms at 16,384 x 127; as two, with whole columns per CTA,
